@@ -40,23 +40,23 @@ def listed():
         # range, one realization): a long chain of short dependency levels
         dict(name="defaults_300x300", kind="plan", nx=300, ny=300, nz=1, vario="sph", range=30.0, ratio=1.0,
              nugget=0.05, ball=0.0, ndata=0, k=26, reals=1, path="linear", precision="fp32", warm=False),
-        # conditional simulation of an ill-conditioned smooth model on a 2D
-        # map, data at cell centres: create, prepare, simulate, destroy
+        # conditional simulation of a smooth model on a 2D map, data at cell
+        # centres (some systems are singular): create, prepare, simulate, destroy
         dict(name="conditional_500x500", kind="plan", nx=500, ny=500, nz=1, vario="gau", range=30.0, ratio=1.0,
-             nugget=0.01, ball=0.0, ndata=1000, k=32, reals=64, path="random", precision="fp32", warm=False),
+             nugget=0.1, ball=0.0, ndata=1000, k=32, reals=64, path="random", precision="fp32", warm=False),
         # the large 3D reservoir grid: anisotropic, 5,000 data, 48 neighbours
         # and 256 realizations
-        dict(name="reservoir_200x200x100", kind="plan", nx=200, ny=200, nz=100, vario="exp", range=50.0, ratio=2.0, rz=5.0,
-             nugget=0.05, ball=1.0, ndata=5000, k=48, reals=256, path="random", precision="fp32", warm=False),
+        dict(name="reservoir_200x200x100", kind="plan", nx=200, ny=200, nz=100, vario="exp", range=50.0, ratio=2.0,
+             rz=5.0, nugget=0.05, ball=1.0, ndata=5000, k=48, reals=256, path="random", precision="fp32", warm=False),
         # the largest grid, unconditional, solved from the learned warm start
-        dict(name="learned_256x256x256", kind="plan", nx=256, ny=256, nz=256, vario="sph", range=40.0, ratio=2.0, rz=8.0,
-             nugget=0.1, ball=1.0, ndata=0, k=32, reals=64, path="random", precision="fp32", warm=True),
+        dict(name="learned_256x256x256", kind="plan", nx=256, ny=256, nz=256, vario="sph", range=40.0, ratio=2.0,
+             rz=8.0, nugget=0.1, ball=1.0, ndata=0, k=32, reals=64, path="random", precision="fp32", warm=True),
         # many uneven 2D / 3D domains with their own models in one batch
         dict(name="batch_24_domains", kind="batch", domains=24, shapes=6, side0=32, side1=256, depth0=8, depth1=64,
              reals=8),
         # further realizations from a prepared plan, values left on the device
-        dict(name="sweep_160x160x48_r100", kind="sweep", nx=160, ny=160, nz=48, vario="exp", range=30.0, ratio=2.0, rz=5.0,
-             nugget=0.05, ball=1.0, ndata=500, k=24, reals=100, path="random", precision="fp32"),
+        dict(name="sweep_160x160x48_r100", kind="sweep", nx=160, ny=160, nz=48, vario="exp", range=30.0, ratio=2.0,
+             rz=5.0, nugget=0.05, ball=1.0, ndata=500, k=24, reals=100, path="random", precision="fp32"),
         # posterior mean and variance: simple kriging from the data alone
         dict(name="posterior_500x500", kind="krige", nx=500, ny=500, nz=1, vario="exp", range=60.0, ratio=1.0,
              nugget=0.02, ndata=1000, k=10),
@@ -204,8 +204,8 @@ def _batch_items(c, seed):
             dims.append(int(shape.integers(c["depth0"], c["depth1"] + 1)))
         cls = VARIOS[("sph", "exp", "gau")[int(shape.integers(3))]]
         gau = cls is VARIOS["gau"]
-        model = cls(range=float(shape.uniform(5.0, 80.0)) / (4.0 if gau else 1.0), sill=1.0,
-                    nugget=float(shape.uniform(0.05 if gau else 0.0, 0.1)))
+        model = cls(range=float(shape.uniform(5.0, 80.0)), sill=1.0,
+                    nugget=float(shape.uniform(0.12, 0.2) if gau else shape.uniform(0.0, 0.1)))
         nd, k = int(shape.integers(0, 501)), int(shape.choice([8, 16, 32, 48]))
         data = None
         if nd:
