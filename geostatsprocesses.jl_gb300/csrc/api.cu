@@ -46,6 +46,7 @@ struct sgs_plan {
     VarioDev vario{};
     double mean = 0.0;
     int k = 0, nmin = 1;
+    int s_near = 0;               // SolveArgs::s_near
     int precision = SGS_PREC_FP32_REFINE;
     int refine_steps = 2;
     int warm_start = 0;
@@ -71,7 +72,7 @@ struct sgs_plan {
     int8_t* d_status = nullptr;
     CovLut lut{};
     double* d_lut64 = nullptr;
-    float2* d_lut2 = nullptr;
+    int2* d_lut2 = nullptr;
     SweepTables<float> t32{};
     SweepTables<double> t64{};
     int32_t *d_fallback = nullptr;
@@ -485,6 +486,16 @@ int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err) {
         G.N *= G.n[j];
     }
     if (G.N > (int64_t)INT32_MAX / 2) HERR("grid too large (N must be < 2^30)");
+    // division of a node id below 2^31 by d > 1: with s = ceil(log2 d),
+    // floor(x M / 2^(31 + s)), M = floor(2^(31 + s) / d) + 1 < 2^32, is exact
+    // (Granlund and Montgomery 1994)
+    for (int j = 0; j < 2; ++j) {
+        const uint64_t d = (uint64_t)G.n[j];
+        int s = 0;
+        while (((uint64_t)1 << s) < d) ++s;
+        G.magic[j] = d > 1 ? (uint32_t)((((uint64_t)1 << (31 + s)) / d) + 1) : 0;
+        G.shift[j] = s > 0 ? s - 1 : 0;
+    }
     H.N = G.N;
     H.D = pr->ndata;
     if (H.D < 0 || (H.D > 0 && (!pr->data_coords || !pr->data_values))) HERR("invalid data arrays");
@@ -516,6 +527,11 @@ int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err) {
         d.nugget = u.nugget;
         for (int j = 0; j < 3; ++j) d.inv_range[j] = j < dim ? 1.0 / u.ranges[j] : 1.0;
         for (int j = 0; j < 9; ++j) d.R[j] = u.rotation[j];
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) {
+                d.W[3 * i + j] = i < dim && j < dim ? d.R[i + 3 * j] * d.inv_range[j] : 0.0;
+                d.E[3 * i + j] = d.W[3 * i + j] * G.spacing[i];
+            }
         H.vario.sill += u.sill;
         H.vario.nugget += u.nugget;
     }
@@ -643,6 +659,17 @@ int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err) {
             H.xf[i] = make_float4((float)r[0], (float)r[1], (float)r[2], 0.0f);
         }
         const double dh = 4.0 * amax * std::ldexp(1.0, -24) + 1e-30;
+        // lags put together from rounded coordinates are off by a few units in
+        // the last place of the largest coordinate
+        double cmax = 0.0, wsum = 0.0;
+        for (int j = 0; j < dim; ++j) cmax = std::max(cmax, std::fabs(G.origin[j]) + (double)G.n[j] * G.spacing[j]);
+        for (double x : H.xyz) cmax = std::max(cmax, std::fabs(x));
+        for (int j = 0; j < 9; ++j) wsum += std::fabs(H.vario.st[0].W[j]);
+        const double near = std::max(std::ldexp(1.0, -31), 16.0 * std::ldexp(1.0, -52) * cmax * wsum);
+        const double near2 = std::min(near * near, 1e300);
+        uint64_t bits;
+        std::memcpy(&bits, &near2, sizeof(bits));
+        H.s_near = (int)(bits >> 32);
         MetricDev& m = H.metric;
         double slack = 0.0;
         if (m.kind == METRIC_ISO) {
@@ -691,6 +718,7 @@ static int plan_init(sgs_plan* P, const sgs_problem* pr) {
     P->grid = H.grid;
     P->metric = H.metric;
     P->vario = H.vario;
+    P->s_near = H.s_near;
     P->mean = H.mean;
     P->N = H.N;
     P->D = H.D;
@@ -811,6 +839,9 @@ static int run_solve(sgs_plan* P, double* w_full, double* sigma_full) {
     s.mu = P->mean;
     s.tau = kSingularTau * P->vario.sill;
     s.inv_sill = 1.0 / P->vario.sill;
+    s.sd_sill[0] = (float)std::sqrt(P->vario.sill);
+    s.sd_sill[1] = (float)(std::sqrt(P->vario.sill) - (double)s.sd_sill[0]);
+    s.s_near = P->s_near;
     s.refine_steps = P->refine_steps;
     s.P = P->N;
     s.order = P->d_order;
@@ -1023,11 +1054,11 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
             if ((rc = dalloc(P, &P->d_lut64, total))) return rc;
             if ((rc = dalloc(P, &P->d_lut2, total))) return rc;
             P->lut.c64 = P->d_lut64;
-            P->lut.c2 = P->d_lut2;
+            P->lut.cn = P->d_lut2;
             LAUNCH(P, 1, launch_fill_cov_lut(P->grid, P->vario, P->lut, P->d_lut64, P->d_lut2, st));
         } else {
             P->lut.c64 = nullptr;
-            P->lut.c2 = nullptr;
+            P->lut.cn = nullptr;
         }
     }
 

@@ -664,7 +664,7 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
     TmplEntry* d_tmpl;
     double *d_td2, *d_xyz, *d_val, *d_xyzb;
     float4* d_xf;
-    float2* d_lut;
+    int2* d_lut;
     if ((rc = bupload(B, &B->d_path, path))) return rc;
     if ((rc = bupload(B, &B->d_noff, B->noff))) return rc;
     {
@@ -742,7 +742,7 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
         s.grid = h.grid;
         s.vario = h.vario;
         s.lut.c64 = nullptr;
-        s.lut.c2 = d_lut + loff[d];
+        s.lut.cn = d_lut + loff[d];
         for (int j = 0; j < 3; ++j) {
             s.lut.e[j] = lute[d][j];
             s.lut.w[j] = 2 * lute[d][j] + 1;
@@ -752,6 +752,9 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
         s.mu = h.mean;
         s.tau = kSingularTau * h.vario.sill;
         s.inv_sill = 1.0 / h.vario.sill;
+        s.sd_sill[0] = (float)std::sqrt(h.vario.sill);
+        s.sd_sill[1] = (float)(std::sqrt(h.vario.sill) - (double)s.sd_sill[0]);
+        s.s_near = h.s_near;
         s.refine_steps = pr[d].refine_steps;
         s.P = h.N;
         s.nbr = sa.nbr;

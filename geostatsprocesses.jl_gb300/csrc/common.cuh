@@ -82,11 +82,88 @@ __device__ __forceinline__ double centroid(const GridDev& g, int j, int i) {
     return dadd(g.origin[j], t);
 }
 
+// node -> cell: divisions by the grid's sides as multiplications by host-made
+// reciprocals (GridDev::magic), exact for every node id below 2^31
+__device__ __forceinline__ int grid_div(const GridDev& g, int j, int x) {
+    return g.n[j] == 1 ? x : (int)(__umulhi((uint32_t)x, g.magic[j]) >> g.shift[j]);
+}
+
 __device__ __forceinline__ void cell_of(const GridDev& g, int node, int& i0, int& i1, int& i2) {
-    i0 = node % g.n[0];
-    int r = node / g.n[0];
-    i1 = r % g.n[1];
-    i2 = r / g.n[1];
+    const int r = grid_div(g, 0, node);
+    i0 = node - r * g.n[0];
+    i2 = grid_div(g, 1, r);
+    i1 = r - i2 * g.n[1];
+}
+
+// FP64 on this GPU issues one warp instruction in 64 cycles per scheduler, so
+// the covariance below counts its FP64 instructions: about 40 for an
+// exponential structure in 3D instead of about 150 with the library's exp and
+// sqrt, whose many special cases its arguments never need.
+//
+// 2^(j/64), j = 0 .. 63, rounded to double.
+static __device__ const double kExp2J64[64] = {
+    0x1.0000000000000p+0, 0x1.02c9a3e778061p+0, 0x1.059b0d3158574p+0, 0x1.0874518759bc8p+0,
+    0x1.0b5586cf9890fp+0, 0x1.0e3ec32d3d1a2p+0, 0x1.11301d0125b51p+0, 0x1.1429aaea92de0p+0,
+    0x1.172b83c7d517bp+0, 0x1.1a35beb6fcb75p+0, 0x1.1d4873168b9aap+0, 0x1.2063b88628cd6p+0,
+    0x1.2387a6e756238p+0, 0x1.26b4565e27cddp+0, 0x1.29e9df51fdee1p+0, 0x1.2d285a6e4030bp+0,
+    0x1.306fe0a31b715p+0, 0x1.33c08b26416ffp+0, 0x1.371a7373aa9cbp+0, 0x1.3a7db34e59ff7p+0,
+    0x1.3dea64c123422p+0, 0x1.4160a21f72e2ap+0, 0x1.44e086061892dp+0, 0x1.486a2b5c13cd0p+0,
+    0x1.4bfdad5362a27p+0, 0x1.4f9b2769d2ca7p+0, 0x1.5342b569d4f82p+0, 0x1.56f4736b527dap+0,
+    0x1.5ab07dd485429p+0, 0x1.5e76f15ad2148p+0, 0x1.6247eb03a5585p+0, 0x1.6623882552225p+0,
+    0x1.6a09e667f3bcdp+0, 0x1.6dfb23c651a2fp+0, 0x1.71f75e8ec5f74p+0, 0x1.75feb564267c9p+0,
+    0x1.7a11473eb0187p+0, 0x1.7e2f336cf4e62p+0, 0x1.82589994cce13p+0, 0x1.868d99b4492edp+0,
+    0x1.8ace5422aa0dbp+0, 0x1.8f1ae99157736p+0, 0x1.93737b0cdc5e5p+0, 0x1.97d829fde4e50p+0,
+    0x1.9c49182a3f090p+0, 0x1.a0c667b5de565p+0, 0x1.a5503b23e255dp+0, 0x1.a9e6b5579fdbfp+0,
+    0x1.ae89f995ad3adp+0, 0x1.b33a2b84f15fbp+0, 0x1.b7f76f2fb5e47p+0, 0x1.bcc1e904bc1d2p+0,
+    0x1.c199bdd85529cp+0, 0x1.c67f12e57d14bp+0, 0x1.cb720dcef9069p+0, 0x1.d072d4a07897cp+0,
+    0x1.d5818dcfba487p+0, 0x1.da9e603db3285p+0, 0x1.dfc97337b9b5fp+0, 0x1.e502ee78b3ff6p+0,
+    0x1.ea4afa2a490dap+0, 0x1.efa1bee615a27p+0, 0x1.f50765b6e4540p+0, 0x1.fa7c1819e90d8p+0,
+};
+
+// exp(x) for x <= 0, table-driven (Tang 1989): x = (64 m + j) ln2 / 64 + r with
+// |r| <= ln2 / 128, exp(x) = 2^m 2^(j/64) exp(r), exp(r) by its Taylor
+// polynomial of degree 5 (truncation below 4e-17); 0 below -700.
+__device__ __forceinline__ double exp_nonpos(double x) {
+    if ((uint32_t)__double2hiint(x) > 0xC085E000u) return 0.0;  // x < -700
+    const double shift = 6755399441055744.0;  // 1.5 x 2^52: the sum's low word is the rounded integer
+    const double t = fma(x, 0x1.71547652b82fep+6, shift);
+    const int n = __double2loint(t);
+    const double nd = t - shift;
+    double r = fma(nd, -0x1.62e42fef00000p-7, x);  // ln2 / 64 in two parts, the first exact times nd
+    r = fma(nd, -0x1.473de6af278edp-40, r);
+    double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+    p = fma(p, r, 1.0 / 6.0);
+    p = fma(p, r, 0.5);
+    p = fma(p, r, 1.0);
+    p = p * r;
+    const double T = __ldg(&kExp2J64[n & 63]);
+    const double e = fma(T, p, T);
+    return __hiloint2double(__double2hiint(e) + ((n >> 6) << 20), __double2loint(e));
+}
+
+// sqrt(s): FP32 reciprocal root and two Goldschmidt steps in FP64 (within an
+// ulp); values far outside FP32's range go to the library
+__device__ __forceinline__ double sqrt_fp64(double s) {
+    const uint32_t hi = (uint32_t)__double2hiint(s);
+    if (hi - 0x39B00000u > 0x46300000u - 0x39B00000u) return sqrt(s);  // outside 2^-100 .. 2^100
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((float)s));
+    const double yd = (double)y;
+    double g = s * yd, h = 0.5 * yd;
+    double e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    e = fma(-g, g, s);
+    return fma(e, h, g);
+}
+
+// normalized variogram (0 at the origin, 1 at the sill) of a squared
+// normalized lag s
+__device__ __forceinline__ double structure_shape(int type, double s) {
+    if (type == 3) return 1.0 - exp_nonpos(-3.0 * s);
+    const double hn = sqrt_fp64(s);
+    if (type == 1) return hn < 1.0 ? 1.5 * hn - 0.5 * hn * hn * hn : 1.0;
+    return 1.0 - exp_nonpos(-3.0 * hn);
 }
 
 // gamma(h) of one structure at a nonzero lag (GeoStatsFunctions conventions:
@@ -102,20 +179,18 @@ __device__ __forceinline__ double structure_gamma(const VarioStructDev& v, int d
             s += q * q;
         }
     }
-    double hn = sqrt(s);
-    double f;
-    if (v.type == 1) f = hn < 1.0 ? 1.5 * hn - 0.5 * hn * hn * hn : 1.0;
-    else if (v.type == 2) f = 1.0 - exp(-3.0 * hn);
-    else f = 1.0 - exp(-3.0 * s);
-    return v.nugget + (v.sill - v.nugget) * f;
+    return v.nugget + (v.sill - v.nugget) * structure_shape(v.type, s);
 }
+
+__device__ __forceinline__ bool is_zero(double h) { return (__double_as_longlong(h) << 1) == 0; }
 
 // covariance C(h) = sill - gamma(h) in FP64, gamma summed over the model's
 // structures
 __device__ __forceinline__ double cov_fp64(const VarioDev& v, int dim, double h0, double h1, double h2) {
-    if (h0 == 0.0 && h1 == 0.0 && (dim == 2 || h2 == 0.0)) return v.sill;
-    double g = structure_gamma(v.st[0], dim, h0, h1, h2);
-    for (int i = 1; i < v.ns; ++i) g += structure_gamma(v.st[i], dim, h0, h1, h2);
+    if (is_zero(h0) && is_zero(h1) && (dim == 2 || is_zero(h2))) return v.sill;
+    double g = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < v.ns; ++i) g += structure_gamma(v.st[i], dim, h0, h1, h2);
     return v.sill - g;
 }
 

@@ -26,6 +26,8 @@ struct GridDev {
     double origin[3];
     double spacing[3];
     int64_t N;
+    uint32_t magic[2];  // node / n[j] = umulhi(node, magic[j]) >> shift[j] (n[j] > 1)
+    int shift[2];
 };
 
 struct MetricDev {
@@ -49,6 +51,9 @@ struct VarioStructDev {
     double sill, nugget;
     double inv_range[3];
     double R[9];
+    // lag -> normalized lag, diag(1 / ranges) R': component j of lag h is
+    // sum_i W[3 i + j] h_i, and of a lag of d cells sum_i E[3 i + j] d_i
+    double W[9], E[9];
 };
 
 // The process's variogram: ns structures summed (GeoStatsFunctions'
@@ -68,7 +73,8 @@ struct VarioDev {
 // entry (L0+e0) + w0*((L1+e1) + w1*(L2+e2)), w = 2e+1.
 struct CovLut {
     const double* c64;  // nullptr when absent
-    const float2* c2;   // the covariances / sill as FP32 (hi, lo) pairs
+    const int2* cn;     // the covariances / sill as integer multiples of 2^-28 (x) and
+                        // the FP32 bits of the remainder (y)
     int e[3];
     int w[3];
 };
@@ -181,6 +187,9 @@ struct SolveArgs {
     double mu;
     double tau;                  // singular pivot threshold (absolute)
     double inv_sill;             // 1 / sill (the FP32 path works on the correlation matrix)
+    float sd_sill[2];            // sqrt(sill) as an FP32 (hi, lo) pair
+    int s_near;                  // high word of the squared normalized lag up to which a lag
+                                 // computed from rounded parts may stand for zero
     int refine_steps;
     int64_t P;                   // positions to solve
     const int32_t* order;        // P -> node
@@ -276,6 +285,7 @@ struct HostDomain {
     std::vector<float4> xf;               // FP32 origin-relative coordinates, bucket order
     int nb[3] = {1, 1, 1};
     double bw[3] = {1, 1, 1};
+    int s_near = 0;                       // SolveArgs::s_near
 };
 // Validates *pr and fills H; SGS_OK or SGS_ERR_ARG with err set.  The path
 // is left to the caller: plans and batches build and check its ranks on the
@@ -379,7 +389,7 @@ cudaError_t launch_rows_to_out_fp64(const double* V, int64_t N, int R, int Rp, d
 // sigma of P positions (node, m, idx and off are shared with the source)
 cudaError_t launch_tables_to_fp64(const SweepTables<float>& src, SweepTables<double>& dst, int64_t P,
                                   int64_t entries, cudaStream_t s);
-cudaError_t launch_fill_cov_lut(const GridDev& g, const VarioDev& v, CovLut lut, double* c64, float2* c2, cudaStream_t s);
+cudaError_t launch_fill_cov_lut(const GridDev& g, const VarioDev& v, CovLut lut, double* c64, int2* cn, cudaStream_t s);
 // learned warm start (learned.cu)
 cudaError_t launch_nn_features(const GridDev& G, const VarioDev& v, const int32_t* nbr, const int32_t* cnt, int k,
                                const double* data_xyz, float* feat, cudaStream_t s);

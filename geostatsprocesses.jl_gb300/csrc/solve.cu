@@ -7,21 +7,23 @@
 // the prior fallback when the factorization fails or the node has fewer
 // than minneighbors neighbours (seqsim.jl:109-111,127-131).
 //
-// One warp per system.  Grid-grid covariances come from a table over integer
-// lags (every neighbour of a node is a cell offset inside the search
-// template, so pairwise lags are bounded); lags involving data points are
-// evaluated directly in FP64, 32 per warp pass.
+// Grid-grid covariances come from a table over integer lags (every neighbour
+// of a node is a cell offset inside the search template, so pairwise lags are
+// bounded); lags involving data points are evaluated directly in FP64.
 //
 // Precision modes:
-//   FP64          FP64 LHS, right-looking Cholesky in shared memory, FP64
-//                 weights (the plain path; also re-solves queued systems)
-//   FP32+refine   register-resident Gauss-Jordan inverse of the FP32 LHS,
-//                 refinement against a double-FP32 LHS with a compensated
-//                 residual, double-FP32 variance (solve_fp32_kernel below)
+//   FP64          one warp per system: FP64 LHS, right-looking Cholesky in
+//                 shared memory, FP64 weights (the plain path; also re-solves
+//                 queued systems)
+//   FP32+refine   half a warp per system: register-resident L D L' of the
+//                 FP32 LHS with L^-1 carried in place, refinement against the
+//                 LHS in fixed point with exact residuals, double-FP32
+//                 variance (solve_fp32_kernel below)
 // Results are written in level order (the sweep's layout): the grid
 // neighbours with their weights, and the data neighbours folded into the
 // constant b0 = sum_data w_i (d_i - mu).
 #include <cmath>
+#include <utility>
 
 #include "common.cuh"
 
@@ -334,63 +336,176 @@ cudaError_t launch_solve_fp64(const SolveArgs& a, const SweepTables<double>& t, 
 }
 
 // ---------------------------------------------------------------------------
-// FP32 path.  One warp per system, lane l owning rows l and l + 32 of the
-// system in registers.  The LHS is normalized by the sill (a correlation
-// matrix: pivots in (0, 1], weights unchanged) and kept in shared memory as
-// double-FP32 pairs (hi + lo, about 48 bits); grid-grid entries come from the
-// (hi, lo) lag table, entries involving a datum from one FP64 evaluation each,
-// packed 32 per pass.  Its FP32 copy is inverted in registers by the
-// Gauss-Jordan sweep operator (Goodnight 1979; no pivoting, which is stable
-// for symmetric positive definite matrices, and whose k-th pivot is the same
-// Schur complement a Cholesky factorization would test).  Every solve is then
-// a lane-parallel matrix-vector product instead of a sequential triangular
-// solve.  The weights are refined against the double-FP32 LHS: the residual
-// r = c - K w is accumulated with compensated (Dot2) FP32 arithmetic, which
-// carries the accuracy of an FP64 residual without GB300's narrow FP64 pipe.
-// Weights, sigma^2 = sill (1 - w'c) and b0 stay double-FP32 and are written as
-// (hi, lo) pairs for the compensated sweep.  A system with a pivot below
-// 1e-3 (near-singular: the canonical 1e-10 decision needs FP64) or whose
-// refinement does not contract is queued for the FP64 kernel.
-constexpr int SOLVE32_WARPS = 2;
-// resident blocks per SM the FP32 solve is compiled for.  Systems of up to 48
-// neighbours: 7 x 2 warps at 128 registers a thread (a few spilled values,
-// measured 7 % faster than 6 blocks at 168 registers without spills, and
-// ahead of 8 blocks); up to 32 neighbours: 8 blocks at under 100 registers;
-// up to 64 neighbours hold two rows of 64 registers and get 4 blocks
-constexpr int solve32_min_blocks(int nmax) { return nmax > 48 ? 4 : (nmax > 32 ? 7 : 8); }
+// FP32 path.  Half a warp (16 lanes) per system, two systems per warp.  Lane
+// (r, c) of the half's 4 x 4 lane grid owns the entries (r + 4a, c + 4b),
+// b <= a, of the LHS's lower triangle in registers: the triangle's storage is
+// near n^2 / 2 and its updates near n^3 / 3, where one row per lane holds and
+// updates the whole square.  The LHS is normalized by the sill (a correlation
+// matrix: pivots in (0, 1], weights unchanged).
+//
+// Shared memory keeps each entry as K = hi 2^-28 + lo, hi a 32-bit integer and
+// lo the FP32 remainder (about 2^-53), in 4 x 4 blocks of the lower triangle
+// (diagonal blocks whole), so that a lane's own entries lie at its constant
+// offset in every block.  Grid pairs come from the lag table, pairs with a
+// datum from one FP64 evaluation each, spread over the block's threads.
+//
+// The FP32 copy in registers becomes M = L^-1 and D of K = L D L' by one
+// Gauss elimination that carries the inverse in place (no pivoting, which is
+// stable for symmetric positive definite matrices; the k-th pivot is the
+// Schur complement a Cholesky factorization would test).  A solve is then
+// two triangular matrix-vector products, M' D^-1 M x, without sequential
+// substitution.  The weights are refined against the stored K: the iterate
+// is rounded to a multiple of 2^-24 (and a second multiple of 2^-48 after the
+// first correction), so every product hi W is an integer and the residual
+// c - K w is summed exactly in 64-bit integers, one multiply-add each; only
+// the remainders' products are FP32.  That is more accurate than a
+// compensated FP32 sum of (hi, lo) pairs and takes 2 instructions a term
+// instead of 13.  Weights, sigma^2 = sill (1 - w'c) and b0 are double-FP32 and
+// are written as (hi, lo) pairs for the compensated sweep.  A system with a
+// pivot below 1e-3 (near-singular: the canonical 1e-10 decision needs FP64),
+// a weight of 32 or more (the integer sums' range) or whose refinement does
+// not contract is queued for the FP64 kernel.
+//
+// Bound: latency and issue slots of 8 to 24 warps per SM (shared memory holds
+// the systems; counters of the 32-neighbour form: issue slots 49 % used, L1's
+// data pipe 73 % before the table gathers were put in lag order), and the
+// FP64 pipe where many pairs involve data.  Measured against one warp per
+// system with a full Gauss-Jordan inverse (CUDA events, one GB300): 2 M
+// systems of 48 neighbours 37.3 -> 20.4 ms (30.8 -> 14.2 ms without data),
+// 4.2 M of 32 23.5 -> 12.6 ms, 1.2 M of 24 6.7 -> 3.6 ms, 1.2 M of 16 4.1 ->
+// 1.7 ms, 1.2 M of 60 35.4 -> 22.2 ms.
+constexpr float KFIX = 268435456.0f;          // 2^28: units of an entry's integer part
+constexpr float WFIX = 16777216.0f;           // 2^24: units of a weight's first integer part
+constexpr float WFIX2 = 281474976710656.0f;   // 2^48: and of its second
+constexpr float WLIM = 32.0f;                 // 64 entries x 2^28 x (32 x 2^24) < 2^63
+// Warps per block and resident blocks per SM.  The warps of a block go through
+// a round's phases together (they share the FP64 evaluations and the
+// instruction cache lines of code that each runs once a round).  As many
+// warps as registers allow without spills, two per scheduler at 48
+// neighbours: what shared memory they leave is L1 for the lag table (2 M
+// systems of 48: 4 x 2 blocks 20.4 ms, 5 x 2 22.8, 2 x 5 23.8, 1 x 8 24.6;
+// 4.2 M of 32: 4 x 4 12.6 ms, 2 x 9 14.0, 8 x 2 13.5).
+constexpr int solve32_warps(int nmax) { return nmax > 48 ? 3 : (nmax > 16 ? 4 : 2); }
+constexpr int solve32_blocks(int nmax) { return nmax > 32 ? 2 : (nmax > 16 ? 4 : 12); }
 
-template <int NMAX>
-struct Smem32 {
-    // the double-FP32 LHS as its packed lower triangle (row r at r(r+1)/2):
-    // half the shared memory of the square, so that the register file, not
-    // shared memory, bounds the resident warps
-    static constexpr size_t K = (size_t)NMAX * (NMAX + 1) / 2 * sizeof(DF);
-    static constexpr size_t C = (size_t)NMAX * sizeof(DF);
-    static constexpr size_t W = (size_t)NMAX * sizeof(DF);
-    static constexpr int CB = NMAX > 32 ? 64 : 32;  // one entry per owned row
-    static constexpr size_t V = (size_t)CB * sizeof(float);
-    static constexpr size_t COL = 2 * (size_t)CB * sizeof(float);
-    static constexpr size_t INFO = (size_t)NMAX * sizeof(NbInfo);
-    static constexpr size_t LIN = (size_t)NMAX * sizeof(int);
-    static constexpr size_t bytes = K + C + W + V + COL + INFO + LIN;
-    static_assert(K % 16 == 0 && bytes % 16 == 0, "16-byte aligned per-warp layout");
+struct KF {
+    int hi;
+    float lo;
 };
 
-// packed lower-triangle index of entry (i, j) of a symmetric matrix
-__device__ __forceinline__ int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
+template <int NMAX>
+struct Sys32 {
+    static constexpr int NP = NMAX / 4;            // block rows
+    static constexpr int NR = NP / 4;              // rows a lane holds of a vector
+    static constexpr int NB = NP * (NP + 1) / 2;   // blocks of the lower triangle
+    static constexpr int K = NB * 128;             // 16 entries of 8 bytes a block
+    static constexpr int C = NMAX * (int)sizeof(KF);
+    static constexpr int V = NMAX * 4;             // one vector
+    // K, c, three vector buffers, 1 / D; an odd multiple of 64 bytes puts the
+    // two systems of a warp on different banks (where it fits)
+    static constexpr int raw = K + C + 3 * V + V;
+    static constexpr int bytes = raw % 128 == 0 && NMAX < 64 ? raw + 64 : raw;
+    static_assert(NMAX % 16 == 0 && bytes % 16 == 0, "16-byte aligned layout");
+    // byte offset of entry (i, j) inside a 4 x 4 block (a, b): its 16-byte
+    // pieces are permuted by the lane groups that read the block's rows and
+    // columns together, so that those reads use different banks
+    __device__ static __forceinline__ int swz(int a, int b) { return (((a / NR) & 1) << 4) ^ (((b / NR) & 3) << 5); }
+    __device__ static __forceinline__ int block(int a, int b) { return (a * (a + 1) / 2 + b) * 128; }
+    __device__ static __forceinline__ int at(int i, int j) {  // i / 4 >= j / 4
+        return block(i >> 2, j >> 2) + ((((i & 3) << 5) + ((j & 3) << 3)) ^ swz(i >> 2, j >> 2));
+    }
+    // a block's systems, then what it shares for the pairs with data
+    static constexpr int WARPS = solve32_warps(NMAX);
+    static constexpr int SYS = 2 * WARPS;
+    static constexpr int CHUNK = 4 * WARPS;  // data rows evaluated at a time
+    struct Shared {
+        double u[CHUNK][3];       // a datum's lag to its system's node, in the model's frame
+        unsigned long long mask[SYS];  // the systems' neighbours that are data
+        int n[SYS], g[SYS], dom[SYS];
+        unsigned short row[CHUNK];     // system << 6 | neighbour
+        unsigned char place[SYS][NMAX];  // row of the matrix a neighbour stands in
+    };
+    static constexpr int block_bytes = SYS * bytes + (int)sizeof(Shared);
+};
 
-// normalized double-FP32 covariance between two points of the augmented set
-__device__ __forceinline__ DF kcov2n(const SolveArgs& a, const NbInfo& p, const NbInfo& q) {
+__device__ __forceinline__ KF kf_from_double(double v) {
+    const double shift = 1.5 * 16777216.0;  // 1.5 x 2^24: the sum's low word is v in units of 2^-28
+    const double t = v + shift;
+    return {__double2loint(t), (float)(v - (t - shift))};
+}
+
+// the entry as a double-FP32 value (exact up to the second float's rounding)
+__device__ __forceinline__ DF kf_df(KF v) {
+    const float f = __int2float_rn(v.hi);
+    const float rest = __fmaf_rn(__int2float_rn(v.hi - __float2int_rn(f)), 1.0f / KFIX, v.lo);
+    return df_fast_two_sum(__fmul_rn(f, 1.0f / KFIX), rest);
+}
+
+// w / 2^24 of an integer weight as a double-FP32 value (exact)
+__device__ __forceinline__ DF wfix_df(int w) {
+    const float f = __int2float_rn(w);
+    return {__fmul_rn(f, 1.0f / WFIX), __fmul_rn(__int2float_rn(w - __float2int_rn(f)), 1.0f / WFIX)};
+}
+
+__device__ __forceinline__ NbInfo nb_of(const SolveArgs& a, int id) {
+    NbInfo in;
+    if (id < a.grid.N) {
+        cell_of(a.grid, id, in.c0, in.c1, in.c2);
+        in.did = -1;
+    } else {
+        in.c0 = in.c1 = in.c2 = 0;
+        in.did = id - (int)a.grid.N;
+    }
+    return in;
+}
+
+// normalized covariance between two points of the augmented set in FP64: a
+// call, so that its code stays out of the solve's own
+__device__ __noinline__ KF kcov64n(const SolveArgs& a, NbInfo p, NbInfo q) {
+    return kf_from_double(kcov(a, p, q) * a.inv_sill);
+}
+
+// lag of datum d to the centroid of cell (c0, c1, c2) in the frame of the
+// model's first structure, diag(1 / ranges) R' h
+__device__ __noinline__ void datum_lag(const SolveArgs& a, int d, int c0, int c1, int c2, double* u) {
+    const GridDev& G = a.grid;
+    const double h0 = a.data_xyz[3 * (int64_t)d] - centroid(G, 0, c0);
+    const double h1 = a.data_xyz[3 * (int64_t)d + 1] - centroid(G, 1, c1);
+    const double h2 = G.dim == 3 ? a.data_xyz[3 * (int64_t)d + 2] - centroid(G, 2, c2) : 0.0;
+    const double* W = a.vario.st[0].W;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) u[j] = W[j] * h0 + W[3 + j] * h1 + W[6 + j] * h2;
+}
+
+// normalized covariance of a datum whose lag to the node is u (datum_lag) with
+// the grid point d0, d1, d2 cells from the node, for a model of one structure;
+// hit = false where the lag is too short to tell it from zero this way
+__device__ __noinline__ KF datum_cov(const SolveArgs& a, const double* u, int d0, int d1, int d2, bool& hit) {
+    const VarioStructDev& v = a.vario.st[0];
+    const double x0 = (double)d0, x1 = (double)d1, x2 = (double)d2;
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const double t = fma(-v.E[j], x0, fma(-v.E[3 + j], x1, fma(-v.E[6 + j], x2, u[j])));
+        s = fma(t, t, s);
+    }
+    hit = __double2hiint(s) > a.s_near;
+    const double f = structure_shape(v.type, s);
+    return kf_from_double((v.sill - fma(v.sill - v.nugget, f, v.nugget)) * a.inv_sill);
+}
+
+// the same, from the lag table where it holds the pair
+__device__ __forceinline__ KF kcovn(const SolveArgs& a, const NbInfo& p, const NbInfo& q) {
     if (p.did < 0 && q.did < 0) {
         const CovLut& t = a.lut;
         const int L0 = q.c0 - p.c0, L1 = q.c1 - p.c1, L2 = q.c2 - p.c2;
-        if (t.c2 != nullptr && L0 >= -t.e[0] && L0 <= t.e[0] && L1 >= -t.e[1] && L1 <= t.e[1] && L2 >= -t.e[2] &&
+        if (t.cn != nullptr && L0 >= -t.e[0] && L0 <= t.e[0] && L1 >= -t.e[1] && L1 <= t.e[1] && L2 >= -t.e[2] &&
             L2 <= t.e[2]) {
-            const float2 v = t.c2[(L0 + t.e[0]) + t.w[0] * ((L1 + t.e[1]) + t.w[1] * (L2 + t.e[2]))];
-            return {v.x, v.y};
+            const int2 v = t.cn[(L0 + t.e[0]) + t.w[0] * ((L1 + t.e[1]) + t.w[1] * (L2 + t.e[2]))];
+            return {v.x, __int_as_float(v.y)};
         }
     }
-    return df_from_double(kcov(a, p, q) * a.inv_sill);
+    return kcov64n(a, p, q);
 }
 
 __device__ __forceinline__ DF df_mul(DF a, DF b) {
@@ -399,442 +514,859 @@ __device__ __forceinline__ DF df_mul(DF a, DF b) {
     return df_fast_two_sum(p, __fadd_rn(e, __fmaf_rn(a.hi, b.lo, __fmul_rn(a.lo, b.hi))));
 }
 
-// One system (node g, sweep-table row pos) of the problem `a` with at most
-// NMAX neighbours, in this warp's shared-memory slot `base`.
-template <int NMAX>
-__device__ __forceinline__ void solve32_system(const SolveArgs& a, const SweepTables<float>& tab, int64_t pos, int g,
-                                               unsigned char* base, int lane) {
-    using S = Smem32<NMAX>;
-    constexpr bool TWO = NMAX > 32;  // lanes own a second row
-    DF* K = reinterpret_cast<DF*>(base);
-    DF* c = reinterpret_cast<DF*>(base + S::K);
-    DF* w = reinterpret_cast<DF*>(base + S::K + S::C);
-    float* vec = reinterpret_cast<float*>(base + S::K + S::C + S::W);
-    float* colb = reinterpret_cast<float*>(base + S::K + S::C + S::W + S::V);
-    NbInfo* info = reinterpret_cast<NbInfo*>(base + S::K + S::C + S::W + S::V + S::COL);
-    int* lin = reinterpret_cast<int*>(base + S::K + S::C + S::W + S::V + S::COL + S::INFO);
-    const GridDev& G = a.grid;
-    const int k = a.k;
-    const DF sd_sill = df_sqrt(df_from_double(a.vario.sill));
-    const float2* lut2 = a.lut.c2;
-    const int lw0 = a.lut.w[0], lw1 = a.lut.w[1];
-    const int lcentre = a.lut.e[0] + lw0 * (a.lut.e[1] + lw1 * a.lut.e[2]);
-    const int ltotal = lw0 * lw1 * a.lut.w[2];
-    const int i0 = lane, i1 = lane + 32;
-    {
-        const int n = a.cnt[g];
-        int status = SGS_NODE_KRIGED_;
-        DF sigma = sd_sill;
-        if (n < a.nmin) {
-            status = SGS_NODE_PRIOR_NMIN_;
-        } else {
-            NbInfo self;
-            cell_of(G, g, self.c0, self.c1, self.c2);
-            self.did = -1;
-            bool fits = true;  // every grid neighbour within half the table's extents
-            for (int q = lane; q < n; q += 32) {
-                const int id = a.nbr[(int64_t)g * k + q];
-                NbInfo in;
-                if (id < G.N) {
-                    cell_of(G, id, in.c0, in.c1, in.c2);
-                    in.did = -1;
-                    fits = fits && 2 * abs(in.c0 - self.c0) <= a.lut.e[0] && 2 * abs(in.c1 - self.c1) <= a.lut.e[1] &&
-                           2 * abs(in.c2 - self.c2) <= a.lut.e[2];
-                } else {
-                    in.c0 = in.c1 = in.c2 = 0;
-                    in.did = id - (int)G.N;
-                }
-                info[q] = in;
-                // linear lag-table offset of the cell relative to the query: the
-                // table index of a grid pair (q, r) is centre + lin[r] - lin[q]
-                lin[q] = in.did < 0 ? (in.c0 - self.c0) + lw0 * ((in.c1 - self.c1) + lw1 * (in.c2 - self.c2)) : 0;
-            }
-            fits = __all_sync(FULL_MASK, fits);
-            __syncwarp();
-            if (lut2 && fits) {
-                // every pairwise lag of grid neighbours is inside the table (a
-                // plan's table spans twice the search template, so this always
-                // holds there); the clamp only keeps reads in bounds.  Lane l
-                // fills columns l and l + 32 of every row; it keeps their
-                // offsets in registers, and row r's offset and kind come by
-                // shuffle and ballot mask instead of shared-memory loads.
-                const bool gA = lane < n && info[lane].did < 0;
-                const bool gB = lane + 32 < n && info[lane + 32].did < 0;
-                const int linA = gA ? lin[lane] : 0, linB = gB ? lin[lane + 32] : 0;
-                const unsigned mA = __ballot_sync(FULL_MASK, gA), mB = __ballot_sync(FULL_MASK, gB);
-                if (gA) {
-                    const float2 v = lut2[min(max(lcentre - linA, 0), ltotal - 1)];
-                    c[lane] = {v.x, v.y};
-                } else if (lane < n) {
-                    c[lane] = kcov2n(a, info[lane], self);
-                }
-                if (gB) {
-                    const float2 v = lut2[min(max(lcentre - linB, 0), ltotal - 1)];
-                    c[lane + 32] = {v.x, v.y};
-                } else if (lane + 32 < n) {
-                    c[lane + 32] = kcov2n(a, info[lane + 32], self);
-                }
-                for (int r = 0; r < n; ++r) {
-                    const int linr = __shfl_sync(FULL_MASK, r < 32 ? linA : linB, r & 31);
-                    if (!(((r < 32 ? mA : mB) >> (r & 31)) & 1u)) continue;  // warp-uniform: row r is a datum
-                    const int base = lcentre + linr;
-                    DF* Kr = K + r * (r + 1) / 2;
-                    if (gA && lane <= r) {
-                        const float2 v = lut2[min(max(base - linA, 0), ltotal - 1)];
-                        Kr[lane] = {v.x, v.y};
-                    }
-                    if (gB && lane + 32 <= r) {
-                        const float2 v = lut2[min(max(base - linB, 0), ltotal - 1)];
-                        Kr[lane + 32] = {v.x, v.y};
-                    }
-                }
-            } else {
-                for (int q = lane; q < n; q += 32) c[q] = kcov2n(a, info[q], self);
-                for (int r = 0; r < n; ++r) {
-                    const NbInfo ir = info[r];
-                    if (ir.did >= 0) continue;
-                    for (int q = lane; q <= r; q += 32) {
-                        const NbInfo iq = info[q];
-                        if (iq.did < 0) K[r * (r + 1) / 2 + q] = kcov2n(a, iq, ir);
-                    }
-                }
-            }
-            {
-                int* dl = reinterpret_cast<int*>(vec);
-                const int nd = collect_data(info, n, dl, lane);
-                for (int item = lane; item < nd * n; item += 32) {
-                    const int da = dl[item / n], q = item % n;
-                    const NbInfo iq = info[q];
-                    if (iq.did >= 0 && q > da) continue;  // data-data pair once
-                    K[tri(da, q)] = df_from_double(kcov(a, iq, info[da]) * a.inv_sill);
-                }
-            }
-            __syncwarp();
-            // ---- rows of the FP32 LHS into registers (identity padding) ----
-            float R0[NMAX], R1[TWO ? NMAX : 1];
-            const int t0 = i0 * (i0 + 1) / 2, t1 = i1 * (i1 + 1) / 2;  // own rows' starts
+// reductions over the 16 lanes of a half warp
+__device__ __forceinline__ float half_max(float v) {
 #pragma unroll
-            for (int j = 0; j < NMAX; ++j) {
-                R0[j] = (i0 < n && j < n) ? K[j <= i0 ? t0 + j : j * (j + 1) / 2 + i0].hi : (i0 == j ? 1.0f : 0.0f);
-                if (TWO)
-                    R1[j] = (i1 < n && j < n) ? K[j <= i1 ? t1 + j : j * (j + 1) / 2 + i1].hi : (i1 == j ? 1.0f : 0.0f);
-            }
-            // ---- Gauss-Jordan sweep with column rotation: R -> -K^-1 ----
-            // At step kk register j holds column (kk + j) mod NMAX, so the pivot
-            // column is always register 0 and every register index is static
-            // in a rolled loop (a fully unrolled sweep overflows the
-            // instruction cache).  The pivot column is broadcast through shared
-            // memory already rotated (slot j <- row (kk + j + 1) mod NMAX, which
-            // by symmetry is row kk's entry for register j + 1).  NMAX steps
-            // bring the columns back in place; padding pivots are exactly 1.
-            bool ok = true;
-            const bool own0 = i0 < NMAX, own1 = TWO && i1 < NMAX;
+    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULL_MASK, v, o));
+    return v;
+}
+__device__ __forceinline__ double half_sum(double v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+    return v;
+}
+__device__ __forceinline__ DF half_sum_df(DF v) {
 #pragma unroll 1
-            for (int kk = 0; kk < NMAX; ++kk) {
-                const float d = __shfl_sync(FULL_MASK, kk < 32 ? R0[0] : R1[0], kk & 31);
-                if (!(d > 1e-3f)) {  // warp-uniform
-                    ok = false;
-                    break;
-                }
-                // the inverse is a preconditioner only: the approximate
-                // reciprocal (pivots lie in (1e-3, 1], no denormals) is enough
-                float inv;
-                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
-                float* cb = colb + (kk & 1) * S::CB;
-                if (own0) {
-                    int p = i0 - kk - 1;
-                    cb[p < 0 ? p + NMAX : p] = R0[0];
-                }
-                if (own1) {
-                    int p = i1 - kk - 1;
-                    cb[p < 0 ? p + NMAX : p] = R1[0];
-                }
-                __syncwarp();
-                // owner row: A[k][j] / d == A[k][j] - (1 - 1/d) A[k][j]
-                const float a0 = i0 == kk ? __fsub_rn(1.0f, inv) : __fmul_rn(R0[0], inv);
-                const float a1 = TWO ? (i1 == kk ? __fsub_rn(1.0f, inv) : __fmul_rn(R1[0], inv)) : 0.0f;
-                const float4* cb4 = reinterpret_cast<const float4*>(cb);  // 16-byte aligned
+    for (int o = 8; o > 0; o >>= 1) v = df_add(v, shfl_xor_df(v, o));
+    return v;
+}
+
+// Sums a lane keeps over the systems its half warp solves, added to the
+// problem's counters when the half leaves the problem.
+struct SolveTally {
+    uint32_t m = 0, warm = 0;
+    float l1 = 0.0f;
+    __device__ __forceinline__ void flush(const SolveArgs& a, int l16) {
+        if (l16 == 0) {
+            if (a.sum_m && m) atomicAdd(a.sum_m, (unsigned long long)m);
+            if (a.n_warm && warm) atomicAdd(a.n_warm, (unsigned long long)warm);
+            if (a.wl1_max && l1 > 0.0f) atomicMax(a.wl1_max, __float_as_uint(l1));
+        }
+        m = warm = 0;
+        l1 = 0.0f;
+    }
+};
+
+// f(0), f(1), .. f(N - 1) with constant indices: every use of a register array
+// inside is resolved before the compiler decides where the array lives (the
+// large triangular loops below stay in local memory under #pragma unroll)
+template <class F, int... I>
+__device__ __forceinline__ void static_for_impl(F&& f, std::integer_sequence<int, I...>) {
+    (f(std::integral_constant<int, I>{}), ...);
+}
+template <int N, class F>
+__device__ __forceinline__ void static_for(F&& f) {
+    static_for_impl(f, std::make_integer_sequence<int, N>{});
+}
+
+// two FP32 values in one 64-bit register pair; fma.rn.f32x2 is one
+// instruction for both
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+    F2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float f2_lo(F2 v) {
+    float lo;
+    asm("mov.b64 {%0, _}, %1;" : "=f"(lo) : "l"(v));
+    return lo;
+}
+__device__ __forceinline__ float f2_hi(F2 v) {
+    float hi;
+    asm("mov.b64 {_, %0}, %1;" : "=f"(hi) : "l"(v));
+    return hi;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// registers of the lower triangle's rows, two entries each: row i holds
+// entries 0 .. i (and one unused past an even i) from register tri2(i)
+__host__ __device__ constexpr int tri2(int i) { return (i / 2) * (i / 2 + 1) + (i & 1) * (i / 2 + 1); }
+
+// vector of NP floats (a lane group's entries) from shared memory, in pairs
+template <int NP>
+__device__ __forceinline__ void load_vec(const float* p, F2 (&v)[NP / 2]) {
 #pragma unroll
-                for (int j4 = 0; j4 < NMAX / 4; ++j4) {
-                    const float4 v = cb4[j4];
-                    const float akv[4] = {v.x, v.y, v.z, v.w};
+    for (int i = 0; i < NP / 4; ++i) {
+        const ulonglong2 q = reinterpret_cast<const ulonglong2*>(p)[i];
+        v[2 * i] = q.x;
+        v[2 * i + 1] = q.y;
+    }
+}
+
+// four entries of a system's row from one 4 x 4 block in shared memory: a row
+// of the block (two 16-byte reads) or a column (four reads of 8), chosen per
+// lane by predicates, so that lanes on both sides of the diagonal stay together
+template <int OROW, int OCOL>
+__device__ __forceinline__ void lds_block(bool row, uint32_t pr0, uint32_t pr1, uint32_t pc0, uint32_t pc1, uint32_t pc2,
+                                          uint32_t pc3, int2 (&e)[4]) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.s32 p, %14, 0;\n\t"
+        "@p ld.shared.v4.b32 {%0, %1, %2, %3}, [%8 + %15];\n\t"
+        "@p ld.shared.v4.b32 {%4, %5, %6, %7}, [%9 + %15];\n\t"
+        "@!p ld.shared.v2.b32 {%0, %1}, [%10 + %16];\n\t"
+        "@!p ld.shared.v2.b32 {%2, %3}, [%11 + %16];\n\t"
+        "@!p ld.shared.v2.b32 {%4, %5}, [%12 + %16];\n\t"
+        "@!p ld.shared.v2.b32 {%6, %7}, [%13 + %16];\n\t}"
+        : "=&r"(e[0].x), "=&r"(e[0].y), "=&r"(e[1].x), "=&r"(e[1].y), "=&r"(e[2].x), "=&r"(e[2].y), "=&r"(e[3].x),
+          "=&r"(e[3].y)
+        : "r"(pr0), "r"(pr1), "r"(pc0), "r"(pc1), "r"(pc2), "r"(pc3), "r"((int)row), "n"(OROW), "n"(OCOL)
+        : "memory");
+}
+
+// One system per half warp: node g (live: this half has one) of the problem
+// `a` with n_all neighbours, ids nid (lane l of the half holds neighbours l +
+// 16 s), table row pos; a0 / a1 and base0: the two halves' problems and the
+// first half's shared-memory slot (the FP64 evaluations of both systems share
+// the warp).
+template <int NMAX, bool BATCH>
+__device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs* __restrict__ doms, int dom,
+                                             const SweepTables<float>& tab, int64_t pos, int g, bool live, int n_all,
+                                             const int (&nid)[NMAX / 16], unsigned char* smem, SolveTally& tl) {
+    using S = Sys32<NMAX>;
+    constexpr int NP = S::NP, NR = S::NR;
+    const int lane = threadIdx.x & 31, half = lane >> 4, l16 = lane & 15, r = l16 >> 2, c = l16 & 3;
+    const int sys = threadIdx.x >> 4;  // of the block's systems
+    unsigned char* base = smem + sys * S::bytes;
+    typename S::Shared& sh = *reinterpret_cast<typename S::Shared*>(smem + S::SYS * S::bytes);
+    auto problem = [&](int es) -> const SolveArgs& {  // of the block's system es
+        if constexpr (BATCH) return doms[sh.dom[es]];
+        else return a;
+    };
+    unsigned char* Kb = base;
+    KF* C = reinterpret_cast<KF*>(base + S::K);
+    float* v0 = reinterpret_cast<float*>(base + S::K + S::C);
+    float* v1 = v0 + NMAX;
+    float* v2 = v1 + NMAX;
+    float* dinv = v2 + NMAX;
+    const int k = a.k;
+    const bool prior = n_all < a.nmin;        // fewer than minneighbors (or no system)
+    const int n = prior ? 0 : n_all;
+    const int nw = max(n, __shfl_xor_sync(FULL_MASK, n, 16));  // warp-uniform
+    int status = prior ? SGS_NODE_PRIOR_NMIN_ : SGS_NODE_KRIGED_;
+    DF sigma = {a.sd_sill[0], a.sd_sill[1]};
+    bool accept = true;
+    unsigned char* place = sh.place[sys];
+    const int32_t* __restrict__ nrow = a.nbr + (int64_t)g * k;
+    // vectors are stored as [index % 4][index / 4]; this lane holds entries
+    // c + 4 (NR r + s), s < NR, of the vectors the solves produce
+    const int own = c * NP + NR * r;
+    DF w[NR];
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const int j = 4 * j4 + t;
-                        if (j < NMAX - 1) {
-                            R0[j] = __fmaf_rn(-a0, akv[t], R0[j + 1]);
-                            if (TWO) R1[TWO ? j : 0] = __fmaf_rn(-a1, akv[t], R1[TWO ? j + 1 : 0]);
-                        }
+    for (int s = 0; s < NR; ++s) w[s] = {0.0f, 0.0f};
+    if (__syncthreads_or(nw > 0)) {  // block-uniform; the block's warps stay in step
+        // ---- neighbours, their lag-table offsets and c ----
+        unsigned long long dmask = 0;  // neighbours that are data, in order
+        bool fits = true;  // every grid neighbour within half the table's extents
+        {
+            const CovLut& T = a.lut;
+            const int lw0 = T.w[0], lw1 = T.w[1];
+            const int lcentre = T.e[0] + lw0 * (T.e[1] + lw1 * T.e[2]);
+            NbInfo self = {0, 0, 0, -1};
+            if (n > 0) cell_of(a.grid, g, self.c0, self.c1, self.c2);
+            int* lin = reinterpret_cast<int*>(v0);
+            // Order of the matrix: grid neighbours by their linear table
+            // offset (z, then y, then x), data last.  The table index of a
+            // pair is the difference of its offsets, so the 16 pairs of a 4 x
+            // 4 block then read 4 to 5 lines of the table instead of 10 or 11
+            // (distance order), and L1 serves a gather line by line.
+            int key[NMAX / 16], off[NMAX / 16];
+            int* keys = reinterpret_cast<int*>(v1);
+#pragma unroll
+            for (int s = 0; s < NMAX / 16; ++s) {
+                const int q = l16 + 16 * s;
+                off[s] = 0;
+                key[s] = (1 << 30) + NMAX + q;  // past the system
+                if (q < n) {
+                    const NbInfo in = nb_of(a, nid[s]);
+                    if (in.did < 0) {
+                        const int d0 = in.c0 - self.c0, d1 = in.c1 - self.c1, d2 = in.c2 - self.c2;
+                        fits = fits && 2 * abs(d0) <= T.e[0] && 2 * abs(d1) <= T.e[1] && 2 * abs(d2) <= T.e[2];
+                        key[s] = off[s] = d0 + lw0 * (d1 + lw1 * d2);
+                    } else {
+                        key[s] = (1 << 30) + q;
                     }
                 }
-                R0[NMAX - 1] = i0 == kk ? -inv : a0;
-                if (TWO) R1[TWO ? NMAX - 1 : 0] = i1 == kk ? -inv : a1;
+                keys[q] = key[s];
+                const unsigned bal = __ballot_sync(FULL_MASK, key[s] >= (1 << 30) && q < n);
+                dmask |= (unsigned long long)((bal >> (16 * half)) & 0xffffu) << (16 * s);
             }
-            bool accept = ok;
-            if (accept) {
-                float s0 = 0.0f, s1 = 0.0f;
-                if (a.w_init) {
-                    // learned warm start: the refinement below starts from the
-                    // network's prediction and must meet the same tolerance
-                    if (i0 < n) s0 = a.w_init[(int64_t)g * k + i0];
-                    if (TWO && i1 < n) s1 = a.w_init[(int64_t)g * k + i1];
-                } else {
-                    // w = K^-1 c = -R c
-                    for (int q = lane; q < S::CB; q += 32) vec[q] = q < n ? c[q].hi : 0.0f;
-                    __syncwarp();
+            // without a table the offsets may collide: neighbour order then
+            const unsigned fo = __ballot_sync(FULL_MASK, fits);
+            const bool ordered = T.cn != nullptr && ((fo >> (16 * half)) & 0xffffu) == 0xffffu;
+            __syncwarp();
+            int pl[NMAX / 16];
 #pragma unroll
-                    for (int j = 0; j < NMAX; ++j) {
-                        const float v = vec[j];
-                        s0 = __fmaf_rn(-R0[j], v, s0);
-                        if (TWO) s1 = __fmaf_rn(-R1[j], v, s1);
+            for (int s = 0; s < NMAX / 16; ++s) pl[s] = 0;
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+                const int4 kj = reinterpret_cast<const int4*>(keys)[j];
+#pragma unroll
+                for (int s = 0; s < NMAX / 16; ++s)
+                    pl[s] += (kj.x < key[s]) + (kj.y < key[s]) + (kj.z < key[s]) + (kj.w < key[s]);
+            }
+#pragma unroll
+            for (int s = 0; s < NMAX / 16; ++s) {
+                const int q = l16 + 16 * s;
+                if (!ordered) pl[s] = q;
+                place[q] = (unsigned char)pl[s];
+                lin[(pl[s] & 3) * NP + (pl[s] >> 2)] = off[s];
+            }
+            fits = ordered;
+            __syncwarp();
+            if (fits) {
+                // Lags of grid pairs: table index centre + lin[i] - lin[j].
+                // Every neighbour's lag fits half the extents, so every pair's
+                // index is inside the table; data and padding take the
+                // query's own cell (lin = 0), are read like the others and
+                // then overwritten (data) or never used (padding).
+                const int2* __restrict__ lut = T.cn + lcentre;
+                int lc[NP];
+#pragma unroll
+                for (int i = 0; i < NP / 4; ++i) {
+                    const int4 y = reinterpret_cast<const int4*>(lin + c * NP)[i];
+                    lc[4 * i] = y.x, lc[4 * i + 1] = y.y, lc[4 * i + 2] = y.z, lc[4 * i + 3] = y.w;
+                }
+#pragma unroll
+                for (int s = 0; s < NMAX / 16; ++s) {
+                    const int q = l16 + 16 * s;
+                    const int2 x = lut[-lin[(q & 3) * NP + (q >> 2)]];
+                    C[q] = {x.x, __int_as_float(x.y)};
+                }
+                // two block rows at a time: their gathers are all issued
+                // before the first is stored
+                const int l8 = l16 * 8;
+                static_for<NP / 2>([&](auto im) {
+                    constexpr int m = 2 * im;
+                    if (4 * m < nw) {
+                        const int2 *lr0 = lut + lin[r * NP + m], *lr1 = lut + lin[r * NP + m + 1];
+                        int2 e0[m + 1], e1[m + 2];
+                        static_for<m + 1>([&](auto ib) { e0[ib] = __ldg(lr0 - lc[ib]); });
+                        static_for<m + 2>([&](auto ib) { e1[ib] = __ldg(lr1 - lc[ib]); });
+                        static_for<m + 1>([&](auto ib) {
+                            *reinterpret_cast<int2*>(Kb + S::block(m, ib) + (l8 ^ S::swz(m, ib))) = e0[ib];
+                        });
+                        static_for<m + 2>([&](auto ib) {
+                            *reinterpret_cast<int2*>(Kb + S::block(m + 1, ib) + (l8 ^ S::swz(m + 1, ib))) = e1[ib];
+                        });
+                    }
+                });
+            } else {
+                // no table, or a neighbour outside it (a batch's capped
+                // table): every grid pair by itself
+#pragma unroll 1
+                for (int e = l16; e < S::K / 8; e += 16) reinterpret_cast<KF*>(Kb)[e] = {0, 0.0f};
+#pragma unroll 1
+                for (int q = l16; q < NMAX; q += 16) {
+                    C[q] = {0, 0.0f};
+                    if (q < n && nrow[q] < a.grid.N) C[q] = kcovn(a, nb_of(a, nrow[q]), self);
+                }
+            }
+            __syncwarp();
+            if (!fits)
+#pragma unroll 1
+                for (int i = 0; i < n; ++i) {
+                    const NbInfo ni = nb_of(a, nrow[i]);
+                    if (ni.did >= 0) continue;
+#pragma unroll 1
+                    for (int j = l16; j <= i; j += 16) {
+                        const NbInfo nj = nb_of(a, nrow[j]);
+                        if (nj.did >= 0) continue;
+                        const KF x = kcovn(a, nj, ni);
+                        *reinterpret_cast<KF*>(Kb + S::at(i, j)) = x;
+                        if ((i >> 2) == (j >> 2)) *reinterpret_cast<KF*>(Kb + S::at(j, i)) = x;
                     }
                 }
-                DF w0 = {s0, 0.0f}, w1 = {s1, 0.0f};
-                if (i0 < n) w[i0] = w0;
-                if (TWO && i1 < n) w[i1] = w1;
+            __syncwarp();
+        }
+        // ---- pairs with a datum: FP64, over the whole block ----
+        if (l16 == 0) {
+            sh.mask[sys] = dmask;
+            sh.n[sys] = n;
+            sh.g[sys] = g;
+            sh.dom[sys] = dom;
+        }
+        const int rows = __syncthreads_or(dmask != 0) ? -1 : 0;  // unknown number, or none
+#pragma unroll 1
+        for (int r0 = 0, left = rows; left != 0; r0 += S::CHUNK) {  // block-uniform
+            // the r0-th and later data rows of the block's systems
+            int total = 0;
+            for (int e = 0; e < S::SYS; ++e) total += __popcll(sh.mask[e]);
+            const int nr = min(total - r0, S::CHUNK);
+            left = total - r0 - nr;
+            if ((int)threadIdx.x < nr) {
+                int t = r0 + threadIdx.x, es = 0;
+                while (t >= __popcll(sh.mask[es])) t -= __popcll(sh.mask[es++]);
+                unsigned long long mk = sh.mask[es];
+                for (; t > 0; --t) mk &= mk - 1;
+                const int da = __ffsll((long long)mk) - 1;
+                sh.row[threadIdx.x] = (unsigned short)(es << 6 | da);
+                const SolveArgs& ah = problem(es);
+                if (ah.vario.ns == 1) {
+                    int c0, c1, c2;
+                    cell_of(ah.grid, sh.g[es], c0, c1, c2);
+                    datum_lag(ah, ah.nbr[(int64_t)sh.g[es] * ah.k + da] - (int)ah.grid.N, c0, c1, c2, sh.u[threadIdx.x]);
+                }
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int item = threadIdx.x; item < nr * NMAX; item += 32 * S::WARPS) {
+                const int ei = item / NMAX, q = item - ei * NMAX;
+                const int e = sh.row[ei], es = e >> 6, da = e & 63;
+                if (q >= sh.n[es]) continue;
+                const SolveArgs& ah = problem(es);
+                unsigned char* bh = smem + es * S::bytes;
+                const int gh = sh.g[es];
+                const int32_t* rowh = ah.nbr + (int64_t)gh * ah.k;
+                const int id = rowh[q];
+                if (id >= ah.grid.N && q > da) continue;  // data-data pair once
+                // q == da stands for the pair with the node (its own diagonal is 1)
+                const NbInfo nq = nb_of(ah, q == da ? gh : id);
+                KF x;
+                bool hit = false;
+                if (ah.vario.ns == 1 && nq.did < 0) {
+                    int c0, c1, c2;
+                    cell_of(ah.grid, gh, c0, c1, c2);
+                    x = datum_cov(ah, sh.u[ei], nq.c0 - c0, nq.c1 - c1, nq.c2 - c2, hit);
+                }
+                if (!hit) x = kcov64n(ah, nq, nb_of(ah, rowh[da]));
+                const int pd = sh.place[es][da];
+                if (q == da) {
+                    reinterpret_cast<KF*>(bh + S::K)[pd] = x;
+                    *reinterpret_cast<KF*>(bh + S::at(pd, pd)) = {(int)KFIX, 0.0f};
+                } else {
+                    const int pq = sh.place[es][q], i = max(pq, pd), j = min(pq, pd);
+                    *reinterpret_cast<KF*>(bh + S::at(i, j)) = x;
+                    if ((i >> 2) == (j >> 2)) *reinterpret_cast<KF*>(bh + S::at(j, i)) = x;
+                }
+            }
+            __syncthreads();
+        }
+        // ---- the FP32 LHS into registers (identity past the system) ----
+        F2 A[tri2(NP)];
+#define SLOT(a_, b_) (((b_) & 1) ? f2_hi(A[tri2(a_) + (b_) / 2]) : f2_lo(A[tri2(a_) + (b_) / 2]))
+        static_for<NP>([&](auto ia) {
+            constexpr int ba = ia;
+            const bool in = r + 4 * ba < n;
+            const float sc = in ? 1.0f / KFIX : 0.0f;
+            auto entry = [&](int bb) {
+                const float v = __fmul_rn(
+                    __int2float_rn(*reinterpret_cast<const int*>(Kb + S::block(ba, bb) + ((l16 * 8) ^ S::swz(ba, bb)))), sc);
+                return bb == ba && !in && r == c ? 1.0f : v;
+            };
+            static_for<ba / 2 + 1>([&](auto ib) {
+                constexpr int bb = 2 * ib;
+                A[tri2(ba) + ib] = f2_pack(entry(bb), bb + 1 <= ba ? entry(bb + 1) : 0.0f);
+            });
+        });
+        // ---- elimination: A -> M = L^-1 (below the diagonal) and D ----
+        // Step kk = 4p + t: v_j is row kk of M for j < kk and column kk of the
+        // Schur complement for j > kk; every row i > kk takes -l_i v_j with
+        // l_i = a_i,kk / d, and v_kk = d + 1 turns its own a_i,kk into -l_i.
+        // Lane (r, c) needs v at its rows r + 4a and its columns c + 4b: both
+        // come by shuffles from the lanes that hold them (no shared memory,
+        // no divergence).  The steps of a block column run in a rolled loop
+        // (every register index is static); rows above the pivot are
+        // finished, so block rows < p are left out.
+        bool ok = true;
+        static_for<NP>([&](auto ip) {
+            constexpr int p = ip;
+            if (4 * p < nw) {
+#pragma unroll 1
+                for (int t = 0; t < 4; ++t) {
+                    const int h16 = lane & 16;
+                    const int src_r = h16 | (r << 2) | t;  // column kk in row r (block rows >= p)
+                    const int src_c = h16 | (c << 2) | t;  // column kk in row c
+                    const int src_m = h16 | (t << 2) | c;  // row kk, column c (block columns < p)
+                    const float d = __shfl_sync(FULL_MASK, SLOT(p, p), h16 | (t << 2) | t);
+                    float u[NP], vcs[NP];
+                    static_for<NP>([&](auto ij) {
+                        constexpr int j = ij;
+                        if constexpr (j < p) vcs[j] = __shfl_sync(FULL_MASK, SLOT(p, j), src_m);
+                        else if constexpr (j == p) vcs[j] = __shfl_sync(FULL_MASK, SLOT(p, p), c > t ? src_c : src_m);
+                        else vcs[j] = __shfl_sync(FULL_MASK, SLOT(j, p), src_c);
+                    });
+                    static_for<NP - p>([&](auto ii) {
+                        constexpr int i = p + ii;
+                        u[i] = __shfl_sync(FULL_MASK, SLOT(i, p), src_r);
+                    });
+                    // the inverse is a preconditioner only: the approximate
+                    // reciprocal (pivots lie in (1e-3, 1], no denormals) is enough
+                    float inv;
+                    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
+                    ok = ok && d > 1e-3f;
+                    if (l16 == 0) dinv[t * NP + p] = inv;
+                    if (c == t) vcs[p] = __fadd_rn(d, 1.0f);
+                    F2 vc[NP / 2];
+                    static_for<NP / 2>([&](auto ij) { vc[ij] = f2_pack(vcs[2 * ij], vcs[2 * ij + 1]); });
+                    static_for<NP - p>([&](auto ii) {
+                        constexpr int i = p + ii;
+                        float ui = __fmul_rn(u[i], -inv);
+                        if (i == p && r <= t) ui = 0.0f;
+                        const F2 uu = f2_pack(ui, ui);
+                        static_for<i / 2 + 1>([&](auto ij) {
+                            constexpr int j = ij;
+                            A[tri2(i) + j] = f2_fma(uu, vc[j], A[tri2(i) + j]);
+                        });
+                    });
+                }
+            }
+        });
+        accept = ok;
+        // unit diagonal of M, nothing above it
+        static_for<NP>([&](auto ii) {
+            constexpr int i = ii;
+            const float dg = r > c ? SLOT(i, i) : (r == c ? 1.0f : 0.0f);
+            A[tri2(i) + i / 2] = (i & 1) ? f2_pack(SLOT(i, i - 1), dg) : f2_pack(dg, 0.0f);
+        });
+        __syncwarp();
+        // ---- weights: w = M' D^-1 M c (or the network's prediction), then
+        // corrections from the exact residual ----
+        const int steps = a.refine_steps;
+        const bool warm = a.w_init != nullptr;
+        float prev = 0.0f, last = 0.0f, wmax = 0.0f;
+        // the residual of the last iterate w and the correction it gave (the
+        // weights are w + sd)
+        float sr[NR], sd[NR];
+#pragma unroll
+        for (int s = 0; s < NR; ++s) sr[s] = sd[s] = 0.0f;
+        bool early = false, done = n == 0;  // half-uniform
+        float x[NR];
+        if (warm) {
+#pragma unroll
+            for (int s = 0; s < NMAX / 16; ++s) {
+                const int q = l16 + 16 * s;
+                v2[place[q]] = q < n ? a.w_init[(int64_t)g * k + q] : 0.0f;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int s = 0; s < NR; ++s) w[s] = {v2[c + 4 * (NR * r + s)], 0.0f};
+            __syncwarp();
+        }
+        for (int it = warm ? 0 : -1;; ++it) {  // block-uniform (only plans are warm-started)
+            if (__syncthreads_and(done)) break;
+            if (__all_sync(FULL_MASK, done)) continue;  // this warp waits for the others
+            if (it >= 0) {
+                if (it > 0 && !done)
+#pragma unroll
+                    for (int s = 0; s < NR; ++s) w[s] = df_add(w[s], {sd[s], 0.0f});
+                // the iterate as integers: W1 2^-24 (+ W2 2^-48 after a correction)
+                float wm = 0.0f;
+                auto first = [](const DF& v) { return __float2int_rn(__fmul_rn(v.hi, WFIX)); };  // W1
+                auto second = [&](const DF& v) {                                                 // W2
+                    const DF q = wfix_df(first(v));
+                    const float rest = __fadd_rn(__fsub_rn(__fsub_rn(v.hi, q.hi), q.lo), v.lo);
+                    return __float2int_rn(__fmul_rn(rest, WFIX2));
+                };
+#pragma unroll
+                for (int s = 0; s < NR; ++s) {
+                    const int i = c + 4 * (NR * r + s);
+                    if (!done) {
+                        const DF q = wfix_df(first(w[s]));
+                        const DF y = df_two_sum(q.hi, it > 0 ? __fmul_rn(__int2float_rn(second(w[s])), 1.0f / WFIX2) : 0.0f);
+                        w[s] = df_fast_two_sum(y.hi, __fadd_rn(y.lo, q.lo));
+                    }
+                    wm = fmaxf(wm, fabsf(w[s].hi));
+                    const int W1 = first(w[s]);
+                    reinterpret_cast<int*>(v1)[i] = -W1;
+                    v2[i] = -wfix_df(W1).hi;
+                }
+                wm = half_max(wm);
+                if (it == 0) wmax = wm;
+                if (!done && !(wm < WLIM)) accept = false;
                 __syncwarp();
-                float prev = 0.0f, last = 0.0f;
-                const int steps = a.refine_steps;
-                // weights and residual the variance is evaluated with: the last
-                // residual computed (it also drives the last correction)
-                DF sw0 = w0, sw1 = w1;
-                float sr0 = 0.0f, sr1 = 0.0f;
-                // the correction computed from that residual (0 when none was)
-                float sd0 = 0.0f, sd1 = 0.0f;
-                // largest starting weight, for the one-correction estimate below
-                float wmax = fmaxf(i0 < n ? fabsf(w0.hi) : 0.0f, TWO && i1 < n ? fabsf(w1.hi) : 0.0f);
+                // residual c - K w of the own entries, the two parts of the
+                // weights one after the other
+#pragma unroll 1
+                for (int part = 0;; ++part) {  // warp-uniform
+                    long long acc[NR];
+                    float accf[NR];
+                    uint32_t rowp[NR];  // block row I of the triangle
+                    const uint32_t kaddr = (uint32_t)__cvta_generic_to_shared(Kb);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(FULL_MASK, wmax, o));
-                bool early = false;
-                for (int s = 0;; ++s) {
-                    // residual r = c - K w in double-FP32, own rows
-                    float r0 = 0.0f, r1 = 0.0f;
-                    // row i of the packed triangle: entries t_i + j for j <= i,
-                    // then down column i (j (j + 1) / 2 + i) for j > i
-                    if (i0 < n) {
-                        DFAcc acc;
-                        acc.init(c[i0]);
-                        int jt = 0;  // j (j + 1) / 2
-                        for (int j = 0; j < n; ++j) {
-                            acc.add_prod(df_neg(K[j <= i0 ? t0 + j : jt + i0]), w[j]);
-                            jt += j + 1;
-                        }
-                        r0 = acc.value().hi;
+                    for (int s = 0; s < NR; ++s) {
+                        const int I = NR * r + s;
+                        const KF ci = C[c + 4 * I];
+                        acc[s] = part ? 0 : (long long)ci.hi << 24;
+                        accf[s] = part ? 0.0f : ci.lo;
+                        rowp[s] = kaddr + S::block(I, 0);
                     }
-                    if (TWO && i1 < n) {
-                        DFAcc acc;
-                        acc.init(c[i1]);
-                        int jt = 0;
-                        for (int j = 0; j < n; ++j) {
-                            acc.add_prod(df_neg(K[j <= i1 ? t1 + j : jt + i1]), w[j]);
-                            jt += j + 1;
-                        }
-                        r1 = acc.value().hi;
+                    // Entry (i, 4J + j) lies in row c of block (I, J) up to the
+                    // diagonal and in column c of block (J, I) past it (a
+                    // rolled loop: 80 of the registers hold M).
+                    uint32_t colp = kaddr + NR * r * 128;  // block row J, from column NR r
+#pragma unroll 1
+                    for (int J = 0; 4 * J < nw; ++J) {
+                        const int4 W = reinterpret_cast<const int4*>(v1)[J];
+                        const float4 F = reinterpret_cast<const float4*>(v2)[J];
+                        const int G = J / NR;
+                        const uint32_t xr = ((c << 5) | ((r & 1) << 4)) ^ (G << 5);
+                        const uint32_t pc = colp + ((c << 3) ^ ((G & 1) << 4));
+                        static_for<NR>([&](auto is) {
+                            constexpr int s = is;
+                            int2 e[4];
+                            lds_block<0, s * 128>(J <= NR * r + s, rowp[s] + xr, rowp[s] + (xr ^ 16), pc + (r << 5),
+                                                  pc + ((r ^ 1) << 5), pc + ((r ^ 2) << 5), pc + ((r ^ 3) << 5), e);
+                            acc[s] += (long long)e[0].x * W.x;
+                            acc[s] += (long long)e[1].x * W.y;
+                            acc[s] += (long long)e[2].x * W.z;
+                            acc[s] += (long long)e[3].x * W.w;
+                            accf[s] = __fmaf_rn(__int_as_float(e[0].y), F.x, accf[s]);
+                            accf[s] = __fmaf_rn(__int_as_float(e[1].y), F.y, accf[s]);
+                            accf[s] = __fmaf_rn(__int_as_float(e[2].y), F.z, accf[s]);
+                            accf[s] = __fmaf_rn(__int_as_float(e[3].y), F.w, accf[s]);
+                            rowp[s] += 128;
+                        });
+                        colp += (J + 1) * 128;
                     }
-                    sw0 = w0;
-                    sw1 = w1;
-                    sr0 = r0;
-                    sr1 = r1;
-                    sd0 = sd1 = 0.0f;
-                    if (s == steps) break;  // steps == 0: no correction
-                    __syncwarp();
-                    vec[i0] = r0;
-                    if (TWO) vec[i1] = r1;
-                    __syncwarp();
-                    float d0 = 0.0f, d1 = 0.0f;
+                    const float unit = part ? 1.0f / (KFIX * WFIX2) : 1.0f / (KFIX * WFIX);
 #pragma unroll
-                    for (int j = 0; j < NMAX; ++j) {
-                        const float v = vec[j];
-                        d0 = __fmaf_rn(-R0[j], v, d0);
-                        if (TWO) d1 = __fmaf_rn(-R1[j], v, d1);
+                    for (int s = 0; s < NR; ++s) {
+                        const float f = __fadd_rn(__fmul_rn(__ll2float_rn(acc[s]), unit), accf[s]);
+                        x[s] = part ? __fadd_rn(x[s], f) : f;
                     }
-                    float dmax = 0.0f;
-                    sd0 = i0 < n ? d0 : 0.0f;
-                    sd1 = TWO && i1 < n ? d1 : 0.0f;
-                    if (i0 < n) {
-                        const DF t = df_two_sum(w0.hi, d0);
-                        w0 = df_fast_two_sum(t.hi, __fadd_rn(t.lo, w0.lo));
-                        w[i0] = w0;
-                        dmax = fabsf(d0);
-                    }
-                    if (TWO && i1 < n) {
-                        const DF t = df_two_sum(w1.hi, d1);
-                        w1 = df_fast_two_sum(t.hi, __fadd_rn(t.lo, w1.lo));
-                        w[i1] = w1;
-                        dmax = fmaxf(dmax, fabsf(d1));
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(FULL_MASK, dmax, o));
-                    prev = last;
-                    last = dmax;
                     __syncwarp();
-                    if (s + 1 == steps) break;  // the final weights need no residual
-                    // One correction is enough when the start was already good:
-                    // the start's error is about |d| and the contraction factor
-                    // of the FP32 inverse about |d| / |w|, so the corrected
-                    // weights are off by about |d|^2 / |w| (measured on the
-                    // 200x200x100 anisotropic systems: within a factor 4 of the
-                    // true error, which is ~1e-12 there).
-                    if (s == 0 && !a.w_init && last * last <= 1e-10f * wmax && isfinite(last)) {
-                        early = true;
-                        break;
+                    if (part == 1 || it == 0) break;
+#pragma unroll
+                    for (int s = 0; s < NR; ++s) {
+                        const int i = c + 4 * (NR * r + s);
+                        reinterpret_cast<int*>(v1)[i] = -second(w[s]);
+                        v2[i] = 0.0f;
                     }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int s = 0; s < NR; ++s) {
+                    if (c + 4 * (NR * r + s) >= n) x[s] = 0.0f;
+                    if (!done) {
+                        sr[s] = x[s];
+                        sd[s] = 0.0f;
+                    }
+                }
+                if (it >= steps) done = true;  // steps == 0: no correction
+            } else {
+#pragma unroll
+                for (int s = 0; s < NR; ++s) {
+                    const int i = c + 4 * (NR * r + s);
+                    x[s] = i < n ? __fmul_rn(__int2float_rn(C[i].hi), 1.0f / KFIX) : 0.0f;
+                }
+            }
+            if (__all_sync(FULL_MASK, done)) continue;
+            // ---- x -> M' D^-1 M x ----
+#pragma unroll
+            for (int s = 0; s < NR; ++s) v0[own + s] = x[s];
+            __syncwarp();
+            {
+                F2 xc[NP / 2];
+                float tv[NP], h[NP / 2];
+                load_vec<NP>(v0 + c * NP, xc);
+                static_for<NP>([&](auto ii) {
+                    constexpr int i = ii;
+                    F2 t2 = f2_pack(0.0f, 0.0f);
+                    static_for<i / 2 + 1>([&](auto ij) {
+                        constexpr int j = ij;
+                        t2 = f2_fma(A[tri2(i) + j], xc[j], t2);
+                    });
+                    tv[i] = __fadd_rn(f2_lo(t2), f2_hi(t2));
+                });
+                // sums over the four lanes of a row, each lane keeping NR of them
+#pragma unroll
+                for (int i = 0; i < NP / 2; ++i) {
+                    const float keep = (c & 2) ? tv[NP / 2 + i] : tv[i], send = (c & 2) ? tv[i] : tv[NP / 2 + i];
+                    h[i] = __fadd_rn(keep, __shfl_xor_sync(FULL_MASK, send, 2));
+                }
+#pragma unroll
+                for (int i = 0; i < NR; ++i) {
+                    const float keep = (c & 1) ? h[NR + i] : h[i], send = (c & 1) ? h[i] : h[NR + i];
+                    const float y = __fadd_rn(keep, __shfl_xor_sync(FULL_MASK, send, 1));
+                    const int e = r * NP + NR * c + i;
+                    v1[e] = r + 4 * (NR * c + i) < n ? __fmul_rn(y, dinv[e]) : 0.0f;
+                }
+                __syncwarp();
+                load_vec<NP>(v1 + r * NP, xc);
+                F2 z2[NP / 2];
+#pragma unroll
+                for (int j = 0; j < NP / 2; ++j) z2[j] = f2_pack(0.0f, 0.0f);
+                static_for<NP>([&](auto ii) {
+                    constexpr int i = ii;
+                    const float yi = (i & 1) ? f2_hi(xc[i / 2]) : f2_lo(xc[i / 2]);
+                    const F2 yy = f2_pack(yi, yi);
+                    static_for<i / 2 + 1>([&](auto ij) {
+                        constexpr int j = ij;
+                        z2[j] = f2_fma(A[tri2(i) + j], yy, z2[j]);
+                    });
+                });
+#pragma unroll
+                for (int j = 0; j < NP / 2; ++j) {
+                    tv[2 * j] = f2_lo(z2[j]);
+                    tv[2 * j + 1] = f2_hi(z2[j]);
+                }
+#pragma unroll
+                for (int i = 0; i < NP / 2; ++i) {
+                    const float keep = (r & 2) ? tv[NP / 2 + i] : tv[i], send = (r & 2) ? tv[i] : tv[NP / 2 + i];
+                    h[i] = __fadd_rn(keep, __shfl_xor_sync(FULL_MASK, send, 8));
+                }
+#pragma unroll
+                for (int i = 0; i < NR; ++i) {
+                    const float keep = (r & 1) ? h[NR + i] : h[i], send = (r & 1) ? h[i] : h[NR + i];
+                    x[i] = __fadd_rn(keep, __shfl_xor_sync(FULL_MASK, send, 4));
+                    if (c + 4 * (NR * r + i) >= n) x[i] = 0.0f;
+                }
+                __syncwarp();  // the vectors' buffers are rewritten by the next pass
+            }
+            if (it < 0) {
+                if (!warm)
+#pragma unroll
+                    for (int s = 0; s < NR; ++s) w[s] = {x[s], 0.0f};
+                continue;
+            }
+            float dmax = 0.0f;
+#pragma unroll
+            for (int s = 0; s < NR; ++s) dmax = fmaxf(dmax, fabsf(x[s]));
+            bool finite = true;
+#pragma unroll
+            for (int s = 0; s < NR; ++s) finite = finite && isfinite(x[s]);
+            dmax = half_max(dmax);
+            const unsigned fin = __ballot_sync(FULL_MASK, finite);
+            if (((fin >> (16 * half)) & 0xffffu) != 0xffffu) dmax = INFINITY;
+            if (!done) {
+#pragma unroll
+                for (int s = 0; s < NR; ++s) {
+                    sd[s] = x[s];
+                }
+                prev = last;
+                last = dmax;
+                if (it + 1 == steps) {
+                    done = true;  // the final weights need no residual
+                } else if (it == 0 && !warm && last * last <= 1e-10f * wmax && isfinite(last)) {
+                    // One correction is enough when the start was already
+                    // good: the start's error is about |d| and the
+                    // contraction factor of the FP32 factors about |d| / |w|,
+                    // so the corrected weights are off by about |d|^2 / |w|
+                    // (measured on the 200x200x100 anisotropic systems:
+                    // within a factor 4 of the true error, which is ~1e-12).
+                    early = done = true;
+                } else if (it >= 1 && prev > 0.0f && last < 0.5f * prev && (last / prev) * last <= 1e-9f &&
+                           isfinite(last)) {
                     // Later corrections: stop as soon as the contraction test
-                    // below passes (a warm start from a prediction needs two).
-                    if (s >= 1 && prev > 0.0f && last < 0.5f * prev && (last / prev) * last <= 1e-9f &&
-                        isfinite(last)) {
-                        early = true;
-                        break;
-                    }
-                }
-                // the remaining error is about the contraction factor times the
-                // last correction
-                if (early) {
-                    accept = true;
-                } else if (a.refine_steps >= 2) {
-                    const float rho = prev > 0.0f ? last / prev : 0.0f;
-                    accept = rho < 0.5f && rho * last <= 1e-9f && isfinite(last);
-                } else {
-                    accept = isfinite(last);
-                }
-                if (accept) {
-                    // sigma^2 = sill S(w), S(w) = 1 - w'c - w'r with r = c - K w:
-                    // equal to 1 - w'c at the exact weights, but stationary
-                    // there (its error is (w - w*)' K (w - w*)), so it stays
-                    // accurate where the variance cancels to ~0 (a node on a
-                    // datum), where sqrt would magnify any error.  It is taken
-                    // at the final weights w + d: S(w + d) = S(w) - 2 d'r +
-                    // d' K d, and K d = r up to the inverse's error, so
-                    // S(w + d) = S(w) - d'r with an error of order
-                    // |d| |r| x that error.
-                    DFAcc acc;
-                    acc.init({0.0f, 0.0f});
-                    if (i0 < n) {
-                        acc.add_prod(sw0, df_add(c[i0], {sr0, 0.0f}));
-                        acc.add_prod({sd0, 0.0f}, {sr0, 0.0f});
-                    }
-                    if (TWO && i1 < n) {
-                        acc.add_prod(sw1, df_add(c[i1], {sr1, 0.0f}));
-                        acc.add_prod({sd1, 0.0f}, {sr1, 0.0f});
-                    }
-                    const DF wc = warp_sum_df(acc.value());
-                    sigma = df_mul(sd_sill, df_sqrt(df_add({1.0f, 0.0f}, df_neg(wc))));
+                    // passes (a warm start from a prediction needs two).
+                    early = done = true;
                 }
             }
-            if (!accept) {
-                if (lane == 0) a.fallback[atomicAdd(a.nfallback, 1)] = (int32_t)pos;
-                __syncwarp();
-                return;
-            }
-            if (a.w_init && a.n_warm && lane == 0) atomicAdd(a.n_warm, 1ull);
         }
-        // ---- table row: grid neighbours with (hi, lo) weights, data folded into b0
-        int m = 0;
-        const int64_t row = table_row(tab, pos, k);
-        DFAcc b0acc;
-        b0acc.init({0.0f, 0.0f});
-        float l1 = 0.0f;
-        if (status == SGS_NODE_KRIGED_) {
-            for (int b = 0; b < n; b += 32) {
-                const int q = b + lane;
-                const bool isgrid = q < n && info[q].did < 0;
-                const unsigned bal = __ballot_sync(FULL_MASK, isgrid);
-                if (isgrid) {
-                    const int j = m + __popc(bal & lanemask_lt());
-                    tab.idx[row + j] = a.nbr[(int64_t)g * k + q] + (int32_t)a.node0;
-                    reinterpret_cast<float2*>(tab.w)[row + j] = make_float2(w[q].hi, w[q].lo);
-                    l1 += fabsf(w[q].hi);
-                } else if (q < n) {
-                    b0acc.add_prod(w[q], df_from_double(a.data_val[info[q].did] - a.mu));
-                }
-                m += __popc(bal);
+#undef SLOT
+        // the remaining error is about the contraction factor times the last
+        // correction
+        if (accept && !early && n > 0) {
+            if (steps >= 2) {
+                const float rho = prev > 0.0f ? last / prev : 0.0f;
+                accept = rho < 0.5f && rho * last <= 1e-9f && isfinite(last);
+            } else {
+                accept = isfinite(last);
             }
-            if (a.wl1_max) {
+        }
+        // sigma^2 = sill S(w), S(w) = 1 - w'c - w'r with r = c - K w: equal to
+        // 1 - w'c at the exact weights, but stationary there (its error is
+        // (w - w*)' K (w - w*)), so it stays accurate where the variance
+        // cancels to ~0 (a node on a datum), where sqrt would magnify any
+        // error.  It is taken at the final weights w + d: S(w + d) = S(w) -
+        // 2 d'r + d' K d, and K d = r up to the inverse's error, so S(w + d) =
+        // S(w) - d'r with an error of order |d| |r| x that error.
+        DFAcc acc;
+        acc.init({0.0f, 0.0f});
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(FULL_MASK, l1, o);
-                if (lane == 0) atomicMax(a.wl1_max, __float_as_uint(l1));
+        for (int s = 0; s < NR; ++s) {
+            const int i = c + 4 * (NR * r + s);
+            if (i < n) {
+                acc.add_prod(w[s], df_add(kf_df(C[i]), {sr[s], 0.0f}));
+                acc.add_prod({sd[s], 0.0f}, {sr[s], 0.0f});
+                w[s] = df_add(w[s], {sd[s], 0.0f});
             }
         }
-        const DF b0 = warp_sum_df(b0acc.value());
-        if (a.ind_wsum)
-            write_indicator_sums(a, pos, n, info, status == SGS_NODE_KRIGED_,
-                                 [&](int q) { return (double)w[q].hi + (double)w[q].lo; }, lane);
-        if (lane == 0) {
-            if (a.sum_m) atomicAdd(a.sum_m, (unsigned long long)m);
+        const DF wc = half_sum_df(acc.value());
+        if (n > 0) sigma = df_mul(sigma, df_sqrt(df_add({1.0f, 0.0f}, df_neg(wc))));
+        __syncwarp();
+        if (live && !accept && l16 == 0) a.fallback[atomicAdd(a.nfallback, 1)] = (int32_t)pos;
+    }
+    __syncthreads();
+    // ---- table row: grid neighbours with (hi, lo) weights, data folded into b0
+    DF* ws = reinterpret_cast<DF*>(v0);  // the weights in neighbour order (v0, v1)
+#pragma unroll
+    for (int s = 0; s < NR; ++s) ws[c + 4 * (NR * r + s)] = w[s];
+    __syncwarp();
+    const bool wr = live && accept;
+    int m = 0;
+    const int64_t row = wr ? table_row(tab, pos, k) : 0;
+    DFAcc b0acc;
+    b0acc.init({0.0f, 0.0f});
+    float l1 = 0.0f;
+#pragma unroll 1
+    for (int s = 0; s < NMAX / 16; ++s) {
+        const int q = l16 + 16 * s;
+        const bool in = wr && q < n;
+        const int id = in ? nrow[q] : 0;
+        const bool isgrid = in && id < a.grid.N;
+        const unsigned bal = (__ballot_sync(FULL_MASK, isgrid) >> (16 * half)) & 0xffffu;
+        if (in) {
+            const DF wq = ws[place[q]];
+            if (isgrid) {
+                const int j = m + __popc(bal & ((1u << l16) - 1u));
+                tab.idx[row + j] = id + (int32_t)a.node0;
+                reinterpret_cast<float2*>(tab.w)[row + j] = make_float2(wq.hi, wq.lo);
+                l1 += fabsf(wq.hi);
+            } else {
+                b0acc.add_prod(wq, df_from_double(a.data_val[id - a.grid.N] - a.mu));
+            }
+        }
+        m += __popc(bal);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) l1 += __shfl_xor_sync(FULL_MASK, l1, o);
+    const DF b0 = half_sum_df(b0acc.value());
+    if (wr) {
+        tl.m += m;
+        tl.l1 = fmaxf(tl.l1, l1);
+        if (a.w_init && n > 0) tl.warm += 1;
+        if (l16 == 0) {
             tab.node[pos] = g + (int32_t)a.node0;
             tab.m[pos] = m;
             reinterpret_cast<float2*>(tab.b0)[pos] = make_float2(b0.hi, b0.lo);
             reinterpret_cast<float2*>(tab.sigma)[pos] = make_float2(sigma.hi, sigma.lo);
             a.status[g] = (int8_t)status;
         }
-        if (a.w_full) {
-            for (int q = lane; q < k; q += 32)
-                a.w_full[(int64_t)g * k + q] =
-                    (status == SGS_NODE_KRIGED_ && q < n) ? (double)w[q].hi + (double)w[q].lo : 0.0;
-            if (lane == 0) a.sigma_full[g] = (double)sigma.hi + (double)sigma.lo;
+    }
+    if (a.ind_wsum) {  // plans only: both halves have the same problem
+        double wsum = 0.0, ds[8];
+#pragma unroll
+        for (int l = 0; l < 8; ++l) ds[l] = 0.0;
+        if (wr)
+#pragma unroll 1
+            for (int q = l16; q < n; q += 16) {
+                const double v = (double)ws[place[q]].hi + (double)ws[place[q]].lo;
+                wsum += v;
+                if (nrow[q] >= a.grid.N) {
+                    const int cat = a.ind_cat[nrow[q] - a.grid.N];
+#pragma unroll
+                    for (int l = 0; l < 8; ++l)
+                        if (l == cat) ds[l] += v;
+                }
+            }
+        wsum = half_sum(wsum);
+        if (wr && l16 == 0) a.ind_wsum[pos] = wsum;
+#pragma unroll
+        for (int l = 0; l < 8; ++l)
+            if (l < a.ncat) {
+                const double v = half_sum(ds[l]);
+                if (wr && l16 == 0) a.ind_dsum[pos * a.ncat + l] = v;
+            }
+    }
+    if (a.w_full && wr) {
+#pragma unroll 1
+        for (int q = l16; q < k; q += 16) {  // k may be above NMAX in a batch
+            const DF wq = ws[q < n ? place[q] : 0];
+            a.w_full[(int64_t)g * k + q] = q < n ? (double)wq.hi + (double)wq.lo : 0.0;
         }
-        __syncwarp();
+        if (l16 == 0) a.sigma_full[g] = (double)sigma.hi + (double)sigma.lo;
+    }
+    __syncwarp();
+}
+
+// neighbour count and ids of node g (g < 0: none) for solve32_pair
+template <int NMAX>
+__device__ __forceinline__ void read_row(const SolveArgs& a, int g, int l16, int& n, int (&nid)[NMAX / 16]) {
+    n = g >= 0 ? a.cnt[g] : 0;
+#pragma unroll
+    for (int s = 0; s < NMAX / 16; ++s) {
+        const int q = l16 + 16 * s;
+        nid[s] = g >= 0 && q < a.k ? a.nbr[(int64_t)g * a.k + q] : -1;
     }
 }
 
 template <int NMAX>
-__global__ void __launch_bounds__(SOLVE32_WARPS * 32, solve32_min_blocks(NMAX)) solve_fp32_kernel(const SolveArgs a, const SweepTables<float> tab) {
+__global__ void __launch_bounds__(solve32_warps(NMAX) * 32, solve32_blocks(NMAX))
+solve_fp32_kernel(const __grid_constant__ SolveArgs a, const SweepTables<float> tab) {
+    using S = Sys32<NMAX>;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    unsigned char* base = smem + (size_t)wib * Smem32<NMAX>::bytes;
-    const int64_t nwarps = (int64_t)gridDim.x * SOLVE32_WARPS;
-    for (int64_t pos = (int64_t)blockIdx.x * SOLVE32_WARPS + wib; pos < a.P; pos += nwarps)
-        solve32_system<NMAX>(a, tab, pos, a.order[pos], base, lane);
+    const int l16 = threadIdx.x & 15;
+    const int64_t nsys = (int64_t)gridDim.x * S::SYS;  // systems of the grid per round
+    SolveTally tl;
+    // the next round's neighbours are read while this one is solved (a chain
+    // of two dependent reads; the node ids one round further ahead)
+    const int64_t pos0 = (int64_t)blockIdx.x * S::SYS + (threadIdx.x >> 4);
+    auto node_at = [&](int64_t p) { return p < a.P ? a.order[p] : -1; };
+    int g = node_at(pos0), g1 = node_at(pos0 + nsys);
+    int n, nid[NMAX / 16];
+    read_row<NMAX>(a, g, l16, n, nid);
+    for (int64_t b0 = (int64_t)blockIdx.x * S::SYS, pos = pos0; b0 < a.P; b0 += nsys, pos += nsys) {  // block-uniform
+        const int g2 = node_at(pos + 2 * nsys);
+        int n1, nid1[NMAX / 16];
+        read_row<NMAX>(a, g1, l16, n1, nid1);
+        solve32_pair<NMAX, false>(a, nullptr, 0, tab, pos, max(g, 0), g >= 0, n, nid, smem, tl);
+        g = g1;
+        g1 = g2;
+        n = n1;
+#pragma unroll
+        for (int s = 0; s < NMAX / 16; ++s) nid[s] = nid1[s];
+    }
+    tl.flush(a, l16);
 }
 
 // Batch form of solve_fp32_kernel: desc[0] positions list[desc[1] ...]
 // (systems with at most NMAX neighbours, from any domain), each solved with
 // its domain's descriptor.
 template <int NMAX>
-__global__ void __launch_bounds__(SOLVE32_WARPS * 32, solve32_min_blocks(NMAX))
+__global__ void __launch_bounds__(solve32_warps(NMAX) * 32, solve32_blocks(NMAX))
 solve_fp32_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict__ noff, int ndom,
                         const int32_t* __restrict__ order, const int32_t* __restrict__ list,
                         const int32_t* __restrict__ desc, const SweepTables<float> tab) {
+    using S = Sys32<NMAX>;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ SolveArgs s_dom[SOLVE32_WARPS];
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    unsigned char* base = smem + (size_t)wib * Smem32<NMAX>::bytes;
+    const int l16 = threadIdx.x & 15;
     const int64_t n = desc[0];
     const int32_t* lst = list + desc[1];
-    const int64_t nwarps = (int64_t)gridDim.x * SOLVE32_WARPS;
+    const int64_t nsys = (int64_t)gridDim.x * S::SYS;
     int64_t lo = 0, hi = 0;
-    for (int64_t it = (int64_t)blockIdx.x * SOLVE32_WARPS + wib; it < n; it += nwarps) {
-        const int64_t pos = lst[it];
+    int d = 0;
+    SolveTally tl;
+    for (int64_t b0 = (int64_t)blockIdx.x * S::SYS; b0 < n; b0 += nsys) {  // block-uniform
+        const int64_t i = b0 + (threadIdx.x >> 4);
+        const bool live = i < n;
+        const int64_t pos = lst[live ? i : b0];
         const int64_t gg = order[pos];
-        if (gg < lo || gg >= hi) {
-            const int d = find_domain(noff, ndom, gg);
+        if (gg < lo || gg >= hi) {  // half-uniform
+            if (hi > 0) tl.flush(doms[d], l16);
+            d = find_domain(noff, ndom, gg);
             lo = noff[d];
             hi = noff[d + 1];
-            __syncwarp();
-            warp_copy_struct(&s_dom[wib], &doms[d], lane);
-            __syncwarp();
         }
-        solve32_system<NMAX>(s_dom[wib], tab, pos, (int)(gg - lo), base, lane);
+        __syncwarp();
+        int nn, nid[NMAX / 16];
+        read_row<NMAX>(doms[d], live ? (int)(gg - lo) : -1, l16, nn, nid);
+        solve32_pair<NMAX, true>(doms[d], doms, d, tab, pos, (int)(gg - lo), live, nn, nid, smem, tl);
     }
+    if (hi > 0) tl.flush(doms[d], l16);
 }
 
 template <int NMAX>
 static cudaError_t launch_solve32(const SolveArgs& a, const SweepTables<float>& t, cudaStream_t s) {
+    using S = Sys32<NMAX>;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = Smem32<NMAX>::bytes * SOLVE32_WARPS;
-    cudaError_t e = cudaFuncSetAttribute(solve_fp32_kernel<NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(solve_fp32_kernel<NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::block_bytes);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_fp32_kernel<NMAX>, SOLVE32_WARPS * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_fp32_kernel<NMAX>, S::WARPS * 32, S::block_bytes);
     if (per_sm < 1) per_sm = 1;
-    int64_t want = (a.P + SOLVE32_WARPS - 1) / SOLVE32_WARPS;
+    int64_t want = (a.P + S::SYS - 1) / S::SYS;
     int blocks = (int)(want < (int64_t)nsm * per_sm ? want : (int64_t)nsm * per_sm);
     if (blocks < 1) blocks = 1;
-    solve_fp32_kernel<NMAX><<<blocks, SOLVE32_WARPS * 32, smem, s>>>(a, t);
+    solve_fp32_kernel<NMAX><<<blocks, S::WARPS * 32, S::block_bytes, s>>>(a, t);
     return cudaGetLastError();
 }
 
@@ -857,14 +1389,14 @@ template <int NMAX>
 static cudaError_t launch_solve32_batch(const SolveArgs* doms, const int64_t* noff, int ndom, const int32_t* order,
                                         const int32_t* list, const int32_t* desc, const SweepTables<float>& t,
                                         int nsm, cudaStream_t s) {
-    const size_t smem = Smem32<NMAX>::bytes * SOLVE32_WARPS;
-    cudaError_t e = cudaFuncSetAttribute(solve_fp32_batch_kernel<NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    using S = Sys32<NMAX>;
+    cudaError_t e =
+        cudaFuncSetAttribute(solve_fp32_batch_kernel<NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::block_bytes);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_fp32_batch_kernel<NMAX>, SOLVE32_WARPS * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_fp32_batch_kernel<NMAX>, S::WARPS * 32, S::block_bytes);
     if (per_sm < 1) per_sm = 1;
-    solve_fp32_batch_kernel<NMAX><<<nsm * per_sm, SOLVE32_WARPS * 32, smem, s>>>(doms, noff, ndom, order, list, desc, t);
+    solve_fp32_batch_kernel<NMAX><<<nsm * per_sm, S::WARPS * 32, S::block_bytes, s>>>(doms, noff, ndom, order, list, desc, t);
     return cudaGetLastError();
 }
 
@@ -872,7 +1404,7 @@ cudaError_t launch_solve_fp32_batch(int nmax, const SolveArgs* doms, const int64
                                     const int32_t* order, const int32_t* list, const int32_t* desc,
                                     const SweepTables<float>& t, int nsm, cudaStream_t s) {
     switch (nmax) {
-        case 8: return launch_solve32_batch<8>(doms, noff, ndom, order, list, desc, t, nsm, s);
+        case 8:
         case 16: return launch_solve32_batch<16>(doms, noff, ndom, order, list, desc, t, nsm, s);
         case 32: return launch_solve32_batch<32>(doms, noff, ndom, order, list, desc, t, nsm, s);
         case 48: return launch_solve32_batch<48>(doms, noff, ndom, order, list, desc, t, nsm, s);
@@ -936,7 +1468,7 @@ cudaError_t launch_tables_to_fp64(const SweepTables<float>& src, SweepTables<dou
 }
 
 // ---------------------------------------------------------------------------
-__global__ void fill_lut_kernel(const GridDev G, const VarioDev v, const CovLut t, double* c64, float2* c2,
+__global__ void fill_lut_kernel(const GridDev G, const VarioDev v, const CovLut t, double* c64, int2* cn,
                                 int64_t total) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int L0 = (int)(i % t.w[0]) - t.e[0];
@@ -946,20 +1478,19 @@ __global__ void fill_lut_kernel(const GridDev G, const VarioDev v, const CovLut 
         const double c = cov_fp64(v, G.dim, dmul((double)L0, G.spacing[0]), dmul((double)L1, G.spacing[1]),
                                   G.dim == 3 ? dmul((double)L2, G.spacing[2]) : 0.0);
         if (c64) c64[i] = c;
-        if (c2) {  // normalized by the sill, as (hi, lo) for the FP32 path
-            const double cn = c / v.sill;
-            const float hi = (float)cn;
-            c2[i] = make_float2(hi, (float)(cn - (double)hi));
+        if (cn) {  // normalized by the sill, in the FP32 path's (hi, lo) form
+            const KF x = kf_from_double(c / v.sill);
+            cn[i] = make_int2(x.hi, __float_as_int(x.lo));
         }
     }
 }
 
-cudaError_t launch_fill_cov_lut(const GridDev& g, const VarioDev& v, CovLut lut, double* c64, float2* c2,
+cudaError_t launch_fill_cov_lut(const GridDev& g, const VarioDev& v, CovLut lut, double* c64, int2* cn,
                                 cudaStream_t s) {
     const int64_t total = (int64_t)lut.w[0] * lut.w[1] * lut.w[2];
     int blocks = (int)((total + 255) / 256);
     if (blocks > 65535) blocks = 65535;
-    fill_lut_kernel<<<blocks, 256, 0, s>>>(g, v, lut, c64, c2, total);
+    fill_lut_kernel<<<blocks, 256, 0, s>>>(g, v, lut, c64, cn, total);
     return cudaGetLastError();
 }
 
