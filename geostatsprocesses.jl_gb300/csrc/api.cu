@@ -47,6 +47,7 @@ struct sgs_plan {
     double mean = 0.0;
     int k = 0, nmin = 1;
     int s_near = 0;               // SolveArgs::s_near
+    int path_linear = 0;          // the path visits the nodes in id order
     int precision = SGS_PREC_FP32_REFINE;
     int refine_steps = 2;
     int warm_start = 0;
@@ -761,6 +762,7 @@ static int plan_init(sgs_plan* P, const sgs_problem* pr) {
     // the device: rank[path[t]] = t, and the path a permutation of the nodes
     int32_t* d_perr = nullptr;
     if ((rc = dalloc(P, &P->d_rank, P->N)) || (rc = dalloc(P, &d_perr, 1))) return rc;
+    P->path_linear = pr->path == nullptr;
     if (pr->path) {
         if ((rc = upload(P, &P->d_path, pr->path, P->N))) return rc;
     } else if ((rc = dalloc(P, &P->d_path, P->N))) {
@@ -1010,6 +1012,7 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
     la.path = P->d_path;
     la.nbr = P->d_nbr;
     la.cnt = P->d_cnt;
+    la.path_linear = P->path_linear;
     la.level = P->d_level;
     la.ticket = P->d_scratch + 1;
     la.maxlevel = P->d_scratch + 2;

@@ -11,6 +11,7 @@
 //                 inside iff d2 <= 1
 #pragma once
 
+#include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -314,32 +315,109 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
-// Level of node c once it is known (>= 0).  Bounded: the wait gives up after
-// wait_ns of wall-clock time (or, should the timer stall, after a count of
-// polls, each at least the 64 ns back-off, reached no earlier), and soon after
-// another warp has raised *err.  The flag and the timer are read every 32nd
-// poll only: the flag shares its cache line with the kernel's ticket counter,
-// which every warp updates.  A warp that gives up raises *err; the returned
-// level is then 0 and the caller's result is void.
-__device__ __forceinline__ int wait_level(const volatile int32_t* vlevel, int64_t c, int32_t* err,
-                                          uint64_t wait_ns) {
-    int l = vlevel[c];
-    if (l >= 0) return l;
+// Dependency levels of 32 consecutive tickets, one node per lane: the lane's
+// node g (active: it has one) has neighbours row[0, n), of which those below
+// N are grid nodes; lev[c] is node c's level, -1 while unknown.  On a linear
+// path first is the rank, and so the id, of lane 0's node (else negative): a
+// neighbour in [first, first + 32) is another lane's node, whose level is read
+// from s_lev (this warp's 32 words) instead of global memory.
+//
+// Every lane reads all its neighbours' levels once, remembers the unknown
+// ones in a mask, and then polls eight of them per turn (the farthest first:
+// along a path the last neighbour to be done is usually the nearest) until
+// none is left.  Lanes finish in any order.  Waits end because tickets are
+// taken in path order by running warps; they are bounded all the same by
+// wait_ns of wall-clock time without progress of the warp (and, should the
+// timer stall, by a count of polls reached no earlier), and stop soon after
+// another warp has raised *err.  A warp that gives up raises *err and returns
+// with its remaining levels unwritten.  Returns the lane's level (0 if none).
+__device__ __forceinline__ int warp_levels(bool active, int g, const int32_t* __restrict__ row, int n, int64_t N,
+                                           volatile int32_t* lev, int64_t first, volatile int32_t* s_lev, int32_t* err,
+                                           uint64_t wait_ns, int lane) {
+    int lv = 0;
+    unsigned long long mask = 0, near = 0;  // unknown levels: elsewhere, in this warp
+    s_lev[lane] = -1;
+    if (!active) n = 0;
+    int nmax = n;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nmax = max(nmax, __shfl_xor_sync(FULL_MASK, nmax, o));
+    for (int q = 0; q < nmax; q += 8) {  // eight levels in flight per lane
+        int c[8], l[8];
+#pragma unroll
+        for (int h = 0; h < 8; ++h) c[h] = q + h < n ? row[q + h] : INT_MAX;
+#pragma unroll
+        for (int h = 0; h < 8; ++h) l[h] = c[h] < N ? lev[c[h]] : -2;
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+            if (l[h] != -1) lv = max(lv, l[h] + 1);
+            else if (first >= 0 && (uint64_t)(c[h] - first) < 32) near |= 1ull << (q + h);
+            else mask |= 1ull << (q + h);
+        }
+    }
+    bool pending = active;
     const volatile int32_t* verr = err;
     const uint64_t max_polls = wait_ns / 32 + 1024;
-    uint64_t t0 = 0;
-    for (uint64_t polls = 1;; ++polls) {
-        __nanosleep(64);
-        l = vlevel[c];
-        if (l >= 0) return l;
-        if ((polls & 31) == 0) {
-            if (*verr) return 0;
-            const uint64_t now = global_ns();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > wait_ns || polls > max_polls) {
-                atomicExch(err, 1);
-                return 0;
+    uint64_t t0 = 0, idle = 0;
+    __syncwarp();
+    for (;;) {
+        // hand levels over within the warp for as long as that moves a lane
+        for (bool any = true; any;) {
+            bool moved = false;
+            if (pending && near) {
+                const int q = 63 - __clzll((long long)near);
+                const int l = s_lev[row[q] - first];
+                if (l >= 0) {
+                    lv = max(lv, l + 1);
+                    near &= ~(1ull << q);
+                    moved = true;
+                }
             }
+            if (pending && !(near | mask)) {
+                lev[g] = lv;
+                s_lev[lane] = lv;
+                pending = false;
+                moved = true;
+            }
+            __syncwarp();
+            any = __any_sync(FULL_MASK, moved);
+        }
+        if (!__any_sync(FULL_MASK, pending)) return lv;
+        // one turn over global memory
+        bool moved = false;
+        if (pending && mask) {
+            unsigned long long left = mask;
+            int c[8], q[8], l[8];
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+                q[h] = left ? 63 - __clzll((long long)left) : -1;
+                left = left ? left & ~(1ull << q[h]) : 0;
+                c[h] = q[h] >= 0 ? row[q[h]] : 0;
+            }
+#pragma unroll
+            for (int h = 0; h < 8; ++h) l[h] = q[h] >= 0 ? lev[c[h]] : -1;
+#pragma unroll
+            for (int h = 0; h < 8; ++h)
+                if (l[h] >= 0) {
+                    lv = max(lv, l[h] + 1);
+                    mask &= ~(1ull << q[h]);
+                    moved = true;
+                }
+        }
+        if (__any_sync(FULL_MASK, moved)) {
+            idle = 0;
+            t0 = 0;
+            continue;
+        }
+        __nanosleep(64);
+        if ((++idle & 31) == 0) {
+            bool stop = *verr != 0;
+            if (!stop) {
+                const uint64_t now = global_ns();
+                if (t0 == 0) t0 = now;
+                stop = now - t0 > wait_ns || idle > max_polls;
+                if (stop) atomicExch(err, 1);
+            }
+            if (__any_sync(FULL_MASK, stop)) return 0;
         }
     }
 }

@@ -121,12 +121,19 @@ struct SearchArgs {
 // so a wait of 2 s only happens on a table that breaks the path order.
 constexpr uint64_t LEVEL_WAIT_NS = 2000000000ull;
 
+// Blocks of 8 warps per SM of the dependency-level kernels.  Warps beyond what
+// throughput needs only wait, and their polls slow the chain of the early
+// ranks: 250 k nodes take 0.39 ms with one block per SM and 0.53 with two,
+// 4 M 1.75 and 1.58 ms, 16.8 M 5.3 and 4.0 ms (four and eight are no faster).
+inline int level_blocks_per_sm(int64_t nodes) { return nodes >= ((int64_t)1 << 21) ? 2 : 1; }
+
 struct LevelArgs {
     int64_t N;
     int k;
     const int32_t* path;
     const int32_t* nbr;
     const int32_t* cnt;
+    int path_linear;             // 1: the path visits the nodes in id order
     int32_t* level;              // N, -1 = not yet known
     int32_t* ticket;             // 1 counter
     int32_t* maxlevel;           // 1 counter
