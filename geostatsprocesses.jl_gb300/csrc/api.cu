@@ -85,11 +85,9 @@ struct sgs_plan {
     unsigned long long* d_stats = nullptr;  // [3] search candidates (grid, data), prior nodes
     float* d_nn = nullptr;        // warm-start network parameters
     float* d_winit = nullptr;     // warm-start predictions [N][k]
-    int32_t* d_done = nullptr;    // dataflow sweep: per-node epoch flags
-    unsigned long long* d_flow = nullptr;  // dataflow sweep: ticket, error flag
-    int32_t flow_epoch = 0;
+    unsigned long long* d_flow = nullptr;  // dataflow sweep: error flag, tickets
     sgs_sweep_config sweep{SGS_SWEEP_FLOW, 1, 0, 1, 0, 0, 0, 0, 0, 0.f};
-    int64_t done_cap = 0;         // flags allocated in d_done (pieces x N)
+    bool sweep_auto = true;  // not set or tuned by the user: the launch chooses `tight`
     int last_sweep_mode = SGS_SWEEP_FLOW;  // mode of the last sweep launched
     int data_only = 0;            // neighbours from the data alone (sgs_krige)
     // indicator simulation (sgs_plan_set_indicator)
@@ -352,7 +350,7 @@ void sgs::set_thread_error(const char* msg) { g_create_err = msg; }
 extern "C" const char* sgs_version(void) { return "geosgs 0.1.0 (sm_103a)"; }
 
 // Diagnostic (exported, not part of the C ABI in include/geosgs.h): runs the
-// dataflow sweep's bounded wait on a flag that nothing sets, with a limit of
+// dataflow sweep's bounded wait on a value that nothing stores, with a limit of
 // wait_ns.  *timed_out = 1 when the wait gave up and said so; *elapsed_ns =
 // the launch's duration.  Returns 0, or a negative SGS_ERR_* code when the
 // launch itself failed.
@@ -360,25 +358,24 @@ extern "C" int sgs_selftest_bounded_wait(int64_t wait_ns, int32_t* timed_out, in
     if (!timed_out || !elapsed_ns || wait_ns <= 0) return SGS_ERR_ARG;
     *timed_out = 0;
     *elapsed_ns = 0;
-    int32_t* d = nullptr;  // [0] the flag, [1] the error word, [2] the neighbour index (0)
-    if (cudaMalloc(&d, 3 * sizeof(int32_t)) != cudaSuccess) {
+    int32_t* d = nullptr;  // [0, 4) a row that nothing stores, [4] the error word
+    if (cudaMalloc(&d, 5 * sizeof(int32_t)) != cudaSuccess) {
         cudaGetLastError();
         return SGS_ERR_CUDA;
     }
     int rc = SGS_OK;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     FlowArgs f{};
-    f.done = d;
-    f.err = d + 1;
-    f.epoch = 1;
+    f.err = d + 4;
     f.wait_ns = (uint64_t)wait_ns;
     int32_t herr = 0;
     float ms = 0.f;
-    if (cudaMemset(d, 0, 3 * sizeof(int32_t)) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
-        cudaEventCreate(&e1) != cudaSuccess || cudaEventRecord(e0) != cudaSuccess ||
-        launch_flow_wait_selftest(d + 2, f, 0) != cudaSuccess || cudaEventRecord(e1) != cudaSuccess ||
-        cudaEventSynchronize(e1) != cudaSuccess ||
-        cudaMemcpy(&herr, d + 1, sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess ||
+    if (cudaMemset(d, 0xff, 4 * sizeof(int32_t)) != cudaSuccess || cudaMemset(d + 4, 0, sizeof(int32_t)) != cudaSuccess ||
+        cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess ||
+        cudaEventRecord(e0) != cudaSuccess ||
+        launch_flow_wait_selftest(reinterpret_cast<const float*>(d), f, 0) != cudaSuccess ||
+        cudaEventRecord(e1) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+        cudaMemcpy(&herr, d + 4, sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess ||
         cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
         cudaGetLastError();
         rc = SGS_ERR_CUDA;
@@ -1086,7 +1083,7 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
             if ((rc = dalloc(P, &P->d_fallback, N))) return rc;
         }
     }
-    if (!P->d_flow && (rc = dalloc(P, &P->d_flow, 2))) return rc;
+    if (!P->d_flow && (rc = dalloc(P, &P->d_flow, FLOW_WORDS))) return rc;
     if (P->ind_ncat && !P->d_ind_wsum) {
         if ((rc = dalloc(P, &P->d_ind_wsum, N))) return rc;
         if ((rc = dalloc(P, &P->d_ind_dsum, (size_t)N * P->ind_ncat))) return rc;
@@ -1166,7 +1163,7 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
 static int check_flow_error(sgs_plan* P) {
     if (!P->d_flow || P->last_sweep_mode != SGS_SWEEP_FLOW) return SGS_OK;
     int32_t err = 0;
-    CK(P, cudaMemcpy(&err, P->d_flow + 1, sizeof(err), cudaMemcpyDeviceToHost));
+    CK(P, cudaMemcpy(&err, P->d_flow, sizeof(err), cudaMemcpyDeviceToHost));
     if (err) return set_err(P, SGS_ERR_TIMEOUT, "dataflow sweep: a dependency wait exceeded its bound");
     return SGS_OK;
 }
@@ -1193,43 +1190,26 @@ static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, v
         // leading levels by per-level launches, the rest in one dataflow launch
         int W = c.lanes_w, G = c.lanes_g;
         const int H = flow_layout(Rp, W, G);
-        const int64_t nflags = P->N * H;
-        if (nflags > P->done_cap) {
-            CK(P, cudaStreamSynchronize(st));
-            dfree(P, P->d_done);
-            P->d_done = nullptr;
-            P->done_cap = 0;
-            int rc;
-            if ((rc = dalloc(P, &P->d_done, nflags))) return rc;
-            P->done_cap = nflags;
-            CK(P, cudaMemsetAsync(P->d_done, 0, nflags * sizeof(int32_t), st));
-            P->flow_epoch = 0;
-        }
-        if (P->flow_epoch >= 0x7ffffff0) {
-            CK(P, cudaMemsetAsync(P->d_done, 0, P->done_cap * sizeof(int32_t), st));
-            P->flow_epoch = 0;
-        }
         // levels [lo, hi) by per-level launches, the rest by dataflow launches
         const int lo = std::max(0, std::min(c.level_lo, P->nlevels));
         const int hi = std::max(lo, std::min(c.level_hi, P->nlevels));
         const int64_t plo = P->h_loff[lo], phi = P->h_loff[hi];
-        const int32_t epoch = ++P->flow_epoch;
-        CK(P, cudaMemsetAsync(P->d_flow, 0, 2 * sizeof(unsigned long long), st));
-        auto flow = [&](int64_t p0, int64_t p1) -> int {
+        CK(P, cudaMemsetAsync(P->d_flow, 0, FLOW_WORDS * sizeof(unsigned long long), st));
+        auto flow = [&](int l0, int l1) -> int {
+            const int64_t p0 = P->h_loff[l0], p1 = P->h_loff[l1];
             FlowArgs f{};
             f.item0 = p0 * H;
             f.item1 = p1 * H;
-            f.N = P->N;
             f.H = H;
-            f.done = P->d_done;
-            f.epoch = epoch;
-            f.ticket = P->d_flow;
-            f.err = reinterpret_cast<int32_t*>(P->d_flow + 1);
+            f.ticket = P->d_flow + FLOW_TICKET_STRIDE + (l0 == 0 ? 0 : FLOW_TICKETS);
+            f.err = reinterpret_cast<int32_t*>(P->d_flow);
             f.chunk = std::max(1, c.chunk);
             f.blocks_per_sm = c.blocks_per_sm;
-            f.tight = c.tight;
+            f.tight = P->sweep_auto ? flow_tight((p1 - p0) * H, l1 - l0, P->nsm) : c.tight;
             f.wait_ns = 10000000000ull;  // 10 s: far beyond any dependency chain
-            cudaError_t e;
+            cudaError_t e = launch_flow_clear(values_fp64(P) ? sweep64(P).node : P->t32.node, p0, p1, P->N,
+                                              (size_t)Rp * (values_fp64(P) ? sizeof(double) : sizeof(float)), V, st);
+            if (e != cudaSuccess) return cuda_err(P, e, "sweep clear");
             if (values_fp64(P))
                 e = launch_sweep_flow_fp64(sweep64(P), P->k, Rp, W, G, (const double*)z, seed, (double*)V, f, P->nsm, st);
             else
@@ -1239,7 +1219,7 @@ static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, v
             return SGS_OK;
         };
         int rc;
-        if (plo > 0 && (rc = flow(0, plo))) return rc;
+        if (plo > 0 && (rc = flow(0, lo))) return rc;
         for (int l = lo; l < hi; ++l) {
             const int64_t p0 = P->h_loff[l], p1 = P->h_loff[l + 1];
             cudaError_t e;
@@ -1251,12 +1231,7 @@ static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, v
             if (e != cudaSuccess) return cuda_err(P, e, "sweep launch");
             if (p1 > p0) P->info.launches++;
         }
-        if (phi < P->N) {
-            const int32_t* node = values_fp64(P) ? sweep64(P).node : P->t32.node;
-            if (phi > plo) LAUNCH(P, 1, launch_flow_mark(node, plo, phi, H, P->N, P->d_done, epoch, st));
-            if (plo > 0) CK(P, cudaMemsetAsync(P->d_flow, 0, sizeof(unsigned long long), st));  // ticket only
-            if ((rc = flow(phi, P->N))) return rc;
-        }
+        if (phi < P->N && (rc = flow(hi, P->nlevels))) return rc;
         return SGS_OK;
     }
     for (int l = 0; l < P->nlevels; ++l) {
@@ -1516,6 +1491,7 @@ extern "C" int sgs_plan_set_sweep(sgs_plan* P, const sgs_sweep_config* c) {
     if (c->mode == SGS_SWEEP_LEVELS && (c->lanes_g < 0 || c->lanes_g > 4 || c->lanes_g == 3 || c->split_nodes < 0))
         return set_err(P, SGS_ERR_ARG, "invalid per-level sweep parameters (lanes_g 0, 1, 2 or 4, split_nodes >= 0)");
     P->sweep = *c;
+    P->sweep_auto = false;
     if (P->sweep.chunk < 1) P->sweep.chunk = 1;
     return SGS_OK;
 }
@@ -1523,6 +1499,7 @@ extern "C" int sgs_plan_set_sweep(sgs_plan* P, const sgs_sweep_config* c) {
 // time one sweep configuration (after a warm-up run); < 0 on failure
 static int time_sweep(sgs_plan* P, const sgs_sweep_config& c, int R, int Rp, void* V, float* ms) {
     P->sweep = c;
+    P->sweep_auto = false;
     cudaStream_t st = P->stream;
     int rc;
     if ((rc = run_sweep(P, R, Rp, nullptr, 7, V, st))) return rc;
@@ -1549,6 +1526,7 @@ extern "C" int sgs_plan_tune_sweep(sgs_plan* P, int32_t R, sgs_sweep_config* cho
     int rc;
     if ((rc = dalloc(P, (unsigned char**)&V, (size_t)P->N * Rp * es))) return rc;
     const sgs_sweep_config saved = P->sweep;
+    const bool saved_auto = P->sweep_auto;
     std::vector<sgs_sweep_config> done;
     int best = -1;
     auto run = [&](sgs_sweep_config c) -> int {
@@ -1643,6 +1621,7 @@ extern "C" int sgs_plan_tune_sweep(sgs_plan* P, int32_t R, sgs_sweep_config* cho
     dfree(P, V);
     if (rc || best < 0) {
         P->sweep = saved;
+        P->sweep_auto = saved_auto;
         return rc ? rc : set_err(P, SGS_ERR_CUDA, "no sweep configuration could be timed");
     }
     P->sweep = done[best];

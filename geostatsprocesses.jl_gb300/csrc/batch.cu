@@ -367,11 +367,9 @@ struct sgs_batch {
     int32_t* d_scratch = nullptr;  // [0] maxlevel [1] level-wait error
     int32_t* d_ticket = nullptr;             // levels tickets, one counter per domain
     unsigned long long* d_sums = nullptr;    // [0] sum of grid neighbours (tables) [1] sum_m [2] priors
-    unsigned long long* d_flow = nullptr;    // sweep ticket, error flag, second launch's ticket
+    unsigned long long* d_flow = nullptr;    // sweep: error flag, tickets
     uint64_t* d_seed = nullptr;
     uint64_t* h_seed = nullptr;    // pinned
-    int32_t* d_done = nullptr;
-    int64_t done_cap = 0;
     int64_t table_entries = 0;
     SweepTables<float> t32{};
     SweepTables<double> t64{};
@@ -387,6 +385,7 @@ struct sgs_batch {
     void* sweep_V = nullptr;
     cudaStream_t sweep_stream = nullptr;
     sgs_sweep_config sweep{SGS_SWEEP_FLOW, 1, 0, 1, 0, 0, 0, 0, 0, 0.f};
+    bool sweep_auto = true;  // not set or tuned by the user: the launch chooses `tight`
     bool sweep_graph_valid = false;
     bool sweep_pending = false;    // a device-resident sweep not yet checked
     unsigned int* d_wl1 = nullptr; // per domain: largest sum of |grid weights| (FP32 bits)
@@ -714,7 +713,7 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
     if ((rc = balloc(B, &B->d_scratch, 4))) return rc;
     if ((rc = balloc(B, &B->d_ticket, nd))) return rc;
     if ((rc = balloc(B, &B->d_sums, 4))) return rc;
-    if ((rc = balloc(B, &B->d_flow, 3))) return rc;
+    if ((rc = balloc(B, &B->d_flow, FLOW_WORDS))) return rc;
     if ((rc = balloc(B, &B->d_seed, 1))) return rc;
     if ((rc = balloc(B, &B->d_wl1, nd))) return rc;
 
@@ -1011,28 +1010,23 @@ extern "C" int sgs_batch_prepare(sgs_batch* B) {
     return SGS_OK;
 }
 
-// The sweep: flags cleared, then one persistent dataflow launch over every
+// The sweep: rows cleared, then one persistent dataflow launch over every
 // position of the batch's level order.
 static int enqueue_sweep(sgs_batch* B, int Rp, const void* z, void* V, cudaStream_t st, int64_t& launched) {
     const sgs_sweep_config& c = B->sweep;
     int W = c.lanes_w, G = c.lanes_g;
     const int H = flow_layout(Rp, W, G);
-    const int64_t nflags = B->Ntot * H;
-    if (nflags > B->done_cap) return berr(B, SGS_ERR_STATE, "sweep flags not allocated");
-    BCK(B, cudaMemsetAsync(B->d_done, 0, nflags * sizeof(int32_t), st));
-    BCK(B, cudaMemsetAsync(B->d_flow, 0, 3 * sizeof(unsigned long long), st));
+    BCK(B, cudaMemsetAsync(V, 0xff, (size_t)B->Ntot * Rp * (values_fp64(B) ? sizeof(double) : sizeof(float)), st));
+    BCK(B, cudaMemsetAsync(B->d_flow, 0, FLOW_WORDS * sizeof(unsigned long long), st));
     FlowArgs f{};
     f.item0 = 0;
     f.item1 = B->Ntot * H;
-    f.N = B->Ntot;
     f.H = H;
-    f.done = B->d_done;
-    f.epoch = 1;
-    f.ticket = B->d_flow;
-    f.err = reinterpret_cast<int32_t*>(B->d_flow + 1);
+    f.ticket = B->d_flow + FLOW_TICKET_STRIDE;
+    f.err = reinterpret_cast<int32_t*>(B->d_flow);
     f.chunk = std::max(1, c.chunk);
     f.blocks_per_sm = c.blocks_per_sm;
-    f.tight = c.tight;
+    f.tight = B->sweep_auto ? flow_tight(f.item1, B->info.nlevels, B->nsm) : c.tight;
     f.wait_ns = 10000000000ull;  // 10 s: far beyond any dependency chain
     f.seed_dev = B->d_seed;
     f.pairs = B->promote ? 1 : 0;
@@ -1046,7 +1040,7 @@ static int enqueue_sweep(sgs_batch* B, int Rp, const void* z, void* V, cudaStrea
         f32.cls = 0;
         BLAUNCH(B, launch_sweep_flow_fp32(B->t32, B->kmax, Rp, W, G, (const float*)z, 0, (float*)V, f32, B->nsm, st));
         FlowArgs f64 = f;
-        f64.ticket = B->d_flow + 2;
+        f64.ticket = f.ticket + FLOW_TICKETS;
         f64.node_class = B->d_cls;
         f64.cls = 1;
         BLAUNCH(B, launch_sweep_flow_fp64(sweep64(B), B->kmax, Rp, W, G, (const double*)z, 0, (double*)V, f64, B->nsm,
@@ -1059,27 +1053,9 @@ static int enqueue_sweep(sgs_batch* B, int Rp, const void* z, void* V, cudaStrea
     return SGS_OK;
 }
 
-static int ensure_flags(sgs_batch* B, int Rp) {
-    int W = B->sweep.lanes_w, G = B->sweep.lanes_g;
-    const int64_t need = B->Ntot * flow_layout(Rp, W, G);
-    if (need <= B->done_cap) return SGS_OK;
-    BCK(B, cudaStreamSynchronize(B->stream));
-    if (B->sweep_exec) {
-        cudaGraphExecDestroy(B->sweep_exec);
-        B->sweep_exec = nullptr;
-    }
-    bfree(B, B->d_done);
-    B->d_done = nullptr;
-    B->done_cap = 0;
-    int rc;
-    if ((rc = balloc(B, &B->d_done, need))) return rc;
-    B->done_cap = need;
-    return SGS_OK;
-}
-
 static int check_sweep_error(sgs_batch* B) {
     int32_t e = 0;
-    BCK(B, cudaMemcpy(&e, B->d_flow + 1, sizeof(e), cudaMemcpyDeviceToHost));
+    BCK(B, cudaMemcpy(&e, B->d_flow, sizeof(e), cudaMemcpyDeviceToHost));
     if (e) return berr(B, SGS_ERR_TIMEOUT, "dataflow sweep: a dependency wait exceeded its bound");
     return SGS_OK;
 }
@@ -1087,7 +1063,6 @@ static int check_sweep_error(sgs_batch* B) {
 // Seeded sweep into V ([Ntot][Rp]) through the cached graph.
 static int run_sweep_graph(sgs_batch* B, int Rp, uint64_t seed, void* V, cudaStream_t st) {
     int rc;
-    if ((rc = ensure_flags(B, Rp))) return rc;
     if (!B->sweep_exec || B->sweep_Rp != Rp || B->sweep_V != V || B->sweep_stream != st || !B->sweep_graph_valid ||
         B->sweep_promote != B->promote || B->sweep_mixed != B->mixed) {
         if (B->sweep_exec) {
@@ -1177,10 +1152,6 @@ extern "C" int sgs_batch_simulate(sgs_batch* B, int32_t R, const double* z, uint
             if (domain_fp64(B, d)) BLAUNCH(B, launch_z_to_rows_fp64(zin, n, R, Rp, (double*)zr + n0 * Rp, st));
             else if (f64) BLAUNCH(B, launch_z_to_rows_fp32(zin, n, R, 2 * Rp, (float*)((double*)zr + n0 * Rp), st));
             else BLAUNCH(B, launch_z_to_rows_fp32(zin, n, R, Rp, (float*)zr + n0 * Rp, st));
-        }
-        if ((rc = ensure_flags(B, Rp))) {
-            cleanup();
-            return rc;
         }
         BCK(B, cudaEventRecord(B->ev[4], st));
         if ((rc = enqueue_sweep(B, Rp, zr, V, st, launched))) {
@@ -1325,6 +1296,7 @@ extern "C" int sgs_batch_set_sweep(sgs_batch* B, const sgs_sweep_config* c) {
         c->tight > 1)
         return berr(B, SGS_ERR_ARG, "invalid dataflow sweep parameters");
     B->sweep = *c;
+    B->sweep_auto = false;
     B->sweep.level_lo = B->sweep.level_hi = B->sweep.split_nodes = 0;
     if (B->sweep.chunk < 1) B->sweep.chunk = 1;
     B->sweep_graph_valid = false;
@@ -1343,13 +1315,14 @@ extern "C" int sgs_batch_tune_sweep(sgs_batch* B, int32_t R, sgs_sweep_config* c
     unsigned char* V = nullptr;
     if ((rc = balloc(B, &V, (size_t)B->Ntot * Rp * es))) return rc;
     const sgs_sweep_config saved = B->sweep;
+    const bool saved_auto = B->sweep_auto;
     std::vector<sgs_sweep_config> done;
     int best = -1;
     cudaStream_t st = B->stream;
     auto time_one = [&](sgs_sweep_config c) -> int {
         B->sweep = c;
+        B->sweep_auto = false;
         int r;
-        if ((r = ensure_flags(B, Rp))) return r;
         int64_t launched = 0;
         *B->h_seed = 7;
         BCK(B, cudaMemcpyAsync(B->d_seed, B->h_seed, sizeof(uint64_t), cudaMemcpyHostToDevice, st));
@@ -1378,6 +1351,7 @@ extern "C" int sgs_batch_tune_sweep(sgs_batch* B, int32_t R, sgs_sweep_config* c
     bfree(B, V);
     if (rc || best < 0) {
         B->sweep = saved;
+        B->sweep_auto = saved_auto;
         B->sweep_graph_valid = false;
         return rc ? rc : berr(B, SGS_ERR_CUDA, "no sweep configuration could be timed");
     }

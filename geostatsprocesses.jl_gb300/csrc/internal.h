@@ -158,23 +158,35 @@ struct SweepTables {
                                  // (P + 1), used by batches of domains
 };
 
+// Item counters of a dataflow launch: one per warp of a block (class), each in
+// its own 256 bytes; class c takes the items c, c + 8, c + 16, ... (in chunks).
+// One counter for all hands out an item every 2.3 ns, which bounded wide
+// launches (5.45 million rows of 8 values: 12.3 ms).
+constexpr int FLOW_CLASSES = 8;
+constexpr int FLOW_TICKET_STRIDE = 32;  // words
+constexpr int FLOW_TICKETS = FLOW_CLASSES * FLOW_TICKET_STRIDE;
+constexpr int FLOW_WORDS = FLOW_TICKET_STRIDE + 2 * FLOW_TICKETS;  // error flag, the counters of two launches
+
+// More warps than a level has items only poll: the kernels compiled for
+// higher residency run from levels of 16 items per SM (the other form's
+// warps) on.  A mean of 4,096 items in a level: 4.29 ms with it, 4.60
+// without; of 905: 1.56 and 0.98.
+inline int flow_tight(int64_t items, int levels, int nsm) { return items >= (int64_t)levels * 16 * nsm; }
+
 // Dataflow sweep state: warps take items (position in level order x piece of
-// the row) from `ticket` and wait, per neighbour, until the neighbour's flag
-// of the same piece equals epoch (set once that piece of this sweep is
-// stored).
+// the row) from `ticket` and wait, per value, until a neighbour's row holds
+// something else than the pattern it was cleared to (launch_flow_clear).
 struct FlowArgs {
     int64_t item0;               // first item of this launch (earlier ones are done)
     int64_t item1;               // one past the last item of this launch
-    int64_t N;                   // nodes (flag stride between pieces)
     int H;                       // pieces per row
-    int32_t* done;               // H x N flags, piece-major
-    int32_t epoch;               // > 0, new for every sweep over the same flags
-    unsigned long long* ticket;  // 1 counter, zero at launch
+    uint64_t rec;                // its reciprocal (set by the launch)
+    unsigned long long* ticket;  // FLOW_TICKETS words, zero at launch
     int32_t* err;                // 1 flag, zero at launch
     int chunk;                   // consecutive items taken per ticket
     int blocks_per_sm;           // resident blocks per SM to launch (<= occupancy)
     int tight;                   // 1: kernel compiled for higher residency (register cap)
-    uint64_t wait_ns;            // longest wait for one flag before giving up
+    uint64_t wait_ns;            // longest wait for one value before giving up
     const uint64_t* seed_dev;    // nullptr, or the draw seed in device memory (read at
                                  // launch; lets a captured graph take a new seed)
     int pairs;                   // FP64 values, packed tables: every 8-byte weight, b0
@@ -378,14 +390,14 @@ cudaError_t launch_sweep_all_fp64(const SweepTables<double>& t, int k, const int
 // per slice of the neighbour list and G chunks of 4 realizations per lane,
 // as returned by flow_layout, which also gives the pieces per row
 int flow_layout(int Rp, int& W, int& G);
-cudaError_t launch_flow_wait_selftest(const int32_t* idx, const FlowArgs& f, cudaStream_t s);
+cudaError_t launch_flow_wait_selftest(const float* row, const FlowArgs& f, cudaStream_t s);
 cudaError_t launch_sweep_flow_fp32(const SweepTables<float>& t, int k, int Rp, int W, int G, const float* z,
                                    uint64_t seed, float* V, const FlowArgs& f, int nsm, cudaStream_t s);
 cudaError_t launch_sweep_flow_fp64(const SweepTables<double>& t, int k, int Rp, int W, int G, const double* z,
                                    uint64_t seed, double* V, const FlowArgs& f, int nsm, cudaStream_t s);
-cudaError_t launch_flow_mark(const int32_t* node, int64_t p0, int64_t p1, int H, int64_t N, int32_t* done,
-                             int32_t epoch, cudaStream_t s);
-int sweep_flow_max_blocks_per_sm(bool fp64, int G, bool tight);
+// the rows of positions [p0, p1) (all N: every row) cleared for a dataflow launch
+cudaError_t launch_flow_clear(const int32_t* node, int64_t p0, int64_t p1, int64_t N, size_t row_bytes, void* V,
+                              cudaStream_t s);
 // host z (R x N, realization-major double) on device -> node-major [N][Rp] of T
 cudaError_t launch_z_to_rows_fp32(const double* zin, int64_t N, int R, int Rp, float* z, cudaStream_t s);
 cudaError_t launch_z_to_rows_fp64(const double* zin, int64_t N, int R, int Rp, double* z, cudaStream_t s);

@@ -38,9 +38,25 @@ __device__ __forceinline__ D4 load_d4(const double* p) {
     const double2 b = reinterpret_cast<const double2*>(p)[1];
     return {a.x, a.y, b.x, b.y};
 }
+// All ones in a value's words stands for "not yet stored" in a dataflow launch
+// (below); no other NaN does, and a stored value never has it.
+__device__ __forceinline__ bool missing(float v) { return __float_as_uint(v) == 0xffffffffu; }
+__device__ __forceinline__ bool missing(double v) { return __double2hiint(v) == -1 && __double2loint(v) == -1; }
+template <typename T>
+__device__ __forceinline__ T unstored();
+template <>
+__device__ __forceinline__ float unstored<float>() { return __uint_as_float(0xffffffffu); }
+template <>
+__device__ __forceinline__ double unstored<double>() { return __hiloint2double(-1, -1); }
+template <typename V>
+__device__ __forceinline__ bool missing4(const V& v) {
+    return missing(v.x) || missing(v.y) || missing(v.z) || missing(v.w);
+}
+__device__ __forceinline__ float settle(float v) { return missing(v) ? __uint_as_float(0x7fffffffu) : v; }
+__device__ __forceinline__ double settle(double v) { return missing(v) ? __hiloint2double(0x7fffffff, -1) : v; }
 __device__ __forceinline__ void store_d4(double* p, D4 v) {
-    reinterpret_cast<double2*>(p)[0] = make_double2(v.x, v.y);
-    reinterpret_cast<double2*>(p)[1] = make_double2(v.z, v.w);
+    reinterpret_cast<double2*>(p)[0] = make_double2(settle(v.x), settle(v.y));
+    reinterpret_cast<double2*>(p)[1] = make_double2(settle(v.z), settle(v.w));
 }
 
 // Compensated dot product in FP32 (Dot2: Ogita, Rump & Oishi 2005, "Accurate
@@ -479,261 +495,332 @@ cudaError_t launch_sweep_all_fp64(const SweepTables<double>& t, int k, const int
 // Dataflow sweep: the dependency levels in one persistent launch, with no
 // barrier between levels.  Realizations are independent, so a node's row is
 // cut into H pieces of P4 chunks of 4 realizations, and every (node, piece)
-// is a work item with its own flag: piece q of a node waits only for piece q
-// of its grid neighbours.  Items are numbered position-major (item = pos * H
-// + q, positions in level order) and warps take `chunk` consecutive items per
-// ticket.  A dependency always has a smaller item number (strictly lower
-// level, same piece), and item numbers are taken in increasing order by
-// warps that are running, so every wait ends: the smallest unfinished item
-// can always proceed.  Waits are bounded anyway (wait_ns of wall-clock time);
-// a warp that gives up sets err, skips the update but still raises its flag,
-// and no warp takes new tickets once err is set.
+// is a work item.  Items are numbered position-major (item = pos * H + q,
+// positions in level order) and warps take `chunk` consecutive items per
+// ticket, the next ticket while the current one is worked on.  A dependency
+// always has a smaller item number (strictly lower level, same piece), and
+// item numbers are taken in increasing order by warps that are running, so
+// every wait ends: the smallest unfinished item can always proceed.
 //
-// Memory ordering: the item's lanes store the piece, each fences (gpu
-// scope), the warp synchronizes, lane 0 stores the flag; a reader's lanes
-// load flags with acquire semantics, synchronize, then read rows with L2-only
-// loads (ld.global.cg), so no stale L1 line of a row written by another SM is
-// used.
+// The values are their own flags.  Before the launch every word of the rows it
+// writes holds a bit pattern no stored value has (all ones, a NaN that
+// arithmetic does not produce; settle() replaces it should one come in with
+// the draws).  A reader loads a neighbour's chunk past L1 and, word by word,
+// either has the value or loads again; nothing is ordered by it but the value
+// itself, so there are no fences and no flag reads.  With a flag per (node,
+// piece), a release fence and acquire polls, one dependent step took 2.6 us
+// (a chain of 2,125 levels: 5.6 ms) instead of 0.94.  Waits are bounded
+// (wait_ns of wall-clock time, or a count of polls reached no earlier); a
+// warp that gives up sets err and stores NaN, and no warp takes new tickets
+// once err is set.
+//
+// What bounds it: the neighbours' rows, gathered from anywhere in the values
+// (no reuse once they exceed L2), or on narrow levels the step above.  4M
+// nodes x 26 neighbours x 256 FP32 values: 40.8 ms, 65 with flags (37.6 by
+// per-level launches, whose half-empty warps of the narrow levels cost the
+// same on other shapes: 16.8M nodes x 64 values 33.7 ms, per level 36.3,
+// with flags 59; 1.2M x 100: 4.3, 5.9 and 6.8).
 //
 // Lane layout inside a warp: W lanes per slice of the neighbour list (a
 // power of two), S = 32 / W slices, each lane G chunks of the piece
 // (P4 = W * G); the S partial sums are combined across lanes at the end.
-__device__ __forceinline__ int ld_flag_acquire(const int32_t* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ float4 ld_value4(const float* p) {
+    float4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p)
+                 : "memory");
     return v;
 }
-__device__ __forceinline__ void st_flag(int32_t* p, int v) {
-    asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ D4 ld_value4(const double* p) {
+    D4 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "l"(p + 2) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_value4(float* p, float4 v) {
+    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(settle(v.x)), "f"(settle(v.y)),
+                 "f"(settle(v.z)), "f"(settle(v.w))
+                 : "memory");
+}
+__device__ __forceinline__ void st_value4(double* p, D4 v) {
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(settle(v.x)), "d"(settle(v.y)) : "memory");
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + 2), "d"(settle(v.z)), "d"(settle(v.w))
+                 : "memory");
 }
 
-// Wait until piece q of every grid neighbour is stored in this sweep (flags
-// of piece q: done_q); false when a wait gave up.  A legitimate wait can last
-// as long as the longest dependency chain, so the bound is wall-clock time.
-// The flag that ends a wait is read with acquire semantics, and the warp
-// barrier orders it before every lane's reads of the neighbours' rows.
-__device__ __forceinline__ bool flow_wait(const int32_t* __restrict__ idx, int m, const int32_t* done_q,
-                                          const FlowArgs& f, int lane) {
-    bool ok = true;
-    // bounded by elapsed time and, should the timer stall, by a count of
-    // polls (each takes at least the 64 ns back-off, so the count bound is
-    // reached no earlier than the time bound)
-    const uint64_t max_polls = f.wait_ns / 32 + 1024;
-    for (int j = lane; j < m; j += 32) {
-        const int32_t* flag = done_q + idx[j];
-        uint64_t t0 = 0, polls = 0;
-        while (ld_flag_acquire(flag) != f.epoch) {
-            const uint64_t now = global_ns();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > f.wait_ns || ++polls > max_polls) {
-                ok = false;
-                break;
-            }
-            __nanosleep(64);
-        }
+// A wait's bound: wait_ns of wall-clock time or, should the timer stall, a
+// count of polls (each a load from L2, far above 16 ns, so the count is
+// reached no earlier).  False once it has run out or another wait has.
+struct FlowBound {
+    uint64_t t0 = 0, polls = 0;
+    __device__ __forceinline__ bool more(int32_t* err, uint64_t wait_ns) {
+        if (++polls > 16) __nanosleep(32);
+        if (polls & 63) return true;
+        const uint64_t now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (!*(volatile int32_t*)err && now - t0 <= wait_ns && polls <= wait_ns / 16 + 1024) return true;
+        atomicExch(err, 1);
+        return false;
     }
-    ok = __all_sync(FULL_MASK, ok);
-    __syncwarp();
-    return ok;
-}
+};
 
-// One piece (chunks [c0, c0 + W*G) of the row, clipped to the row) of one
-// node, FP32 values with compensated sums.
-template <int G, bool CSR>
-__device__ __forceinline__ void flow_piece_fp32(const SweepTables<float>& t, int k, int64_t pos, int g, int m, int Rp,
-                                                int64_t Rs, int c0, int W, int lane, const float* __restrict__ z,
-                                                uint64_t seed, float* __restrict__ V) {
-    const int cpn = Rp >> 2;
-    const int S = 32 / W, s = lane / W, cl = lane % W;
-    const int64_t row = CSR ? t.off[pos] : pos * (int64_t)k;
-    const int32_t* idx = t.idx + row;
-    const float2* w = reinterpret_cast<const float2*>(t.w) + row;
-    Dot2 a[G][4];
+// The sums of one chunk (4 realizations): FP32 values with (hi, lo) weights
+// and compensated sums, FP64 values with plain FMA sums.
+template <typename T>
+struct FlowSum;
+template <>
+struct FlowSum<float> {
+    using Weight = float2;
+    using Value = float4;
+    Dot2 a[4];
+    __device__ __forceinline__ void init() {
 #pragma unroll
-    for (int gi = 0; gi < G; ++gi)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) a[gi][q].init(0.f, 0.f);
-#pragma unroll 4
-    for (int j = s; j < m; j += S) {
-        const float4* row = reinterpret_cast<const float4*>(V + (int64_t)idx[j] * Rs);
-        const float2 wj = w[j];
-#pragma unroll
-        for (int gi = 0; gi < G; ++gi) {
-            const int ch = c0 + cl + gi * W;
-            if (ch < cpn) {
-                const float4 v = __ldcg(row + ch);
-                a[gi][0].add(wj.x, wj.y, v.x);
-                a[gi][1].add(wj.x, wj.y, v.y);
-                a[gi][2].add(wj.x, wj.y, v.z);
-                a[gi][3].add(wj.x, wj.y, v.w);
-            }
-        }
+        for (int q = 0; q < 4; ++q) a[q].init(0.f, 0.f);
     }
-    for (int o = W; o < 32; o <<= 1)
-#pragma unroll
-        for (int gi = 0; gi < G; ++gi)
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                dot2_merge(a[gi][q], __shfl_xor_sync(FULL_MASK, a[gi][q].s, o),
-                           __shfl_xor_sync(FULL_MASK, a[gi][q].c, o));
-    if (s == 0) {
-        const float2 b0 = reinterpret_cast<const float2*>(t.b0)[pos];
-        const float2 sg = reinterpret_cast<const float2*>(t.sigma)[pos];
-#pragma unroll
-        for (int gi = 0; gi < G; ++gi) {
-            const int ch = c0 + cl + gi * W;
-            if (ch < cpn) {
-                const float4 zz =
-                    z ? *reinterpret_cast<const float4*>(z + (int64_t)g * Rs + 4 * ch) : normals4(seed, g, ch);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) dot2_merge(a[gi][q], b0.x, b0.y);
-                a[gi][0].add(sg.x, sg.y, zz.x);
-                a[gi][1].add(sg.x, sg.y, zz.y);
-                a[gi][2].add(sg.x, sg.y, zz.z);
-                a[gi][3].add(sg.x, sg.y, zz.w);
-                Vec4<float>::store(V + (int64_t)g * Rs + 4 * ch, make_float4(a[gi][0].value(), a[gi][1].value(),
-                                                                             a[gi][2].value(), a[gi][3].value()));
-            }
-        }
+    __device__ static Weight entry(const float* p, int64_t i, int) { return reinterpret_cast<const float2*>(p)[i]; }
+    __device__ static Weight shfl(Weight w, int l) {
+        return make_float2(__shfl_sync(FULL_MASK, w.x, l), __shfl_sync(FULL_MASK, w.y, l));
     }
-}
-
-// The same for FP64 values (plain FMA sums).
-template <int G, bool CSR>
-__device__ __forceinline__ void flow_piece_fp64(const SweepTables<double>& t, int k, int64_t pos, int g, int m, int Rp,
-                                                int64_t Rs, int c0, int W, int lane, const double* __restrict__ z,
-                                                uint64_t seed, double* __restrict__ V, int pairs) {
-    const int cpn = Rp >> 2;
-    const int S = 32 / W, s = lane / W, cl = lane % W;
-    const int64_t row = CSR ? t.off[pos] : pos * (int64_t)k;
-    const int32_t* idx = t.idx + row;
-    const double* w = t.w + row;
+    __device__ static Value draws(const float* z, uint64_t seed, int g, int64_t row, int ch) {
+        return z ? *reinterpret_cast<const float4*>(z + row + 4 * ch) : normals4(seed, g, ch);
+    }
+    __device__ __forceinline__ void add(Weight w, const Value& v) {
+        a[0].add(w.x, w.y, v.x);
+        a[1].add(w.x, w.y, v.y);
+        a[2].add(w.x, w.y, v.z);
+        a[3].add(w.x, w.y, v.w);
+    }
+    __device__ __forceinline__ void across(int o) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            dot2_merge(a[q], __shfl_xor_sync(FULL_MASK, a[q].s, o), __shfl_xor_sync(FULL_MASK, a[q].c, o));
+    }
+    __device__ __forceinline__ Value finish(Weight b0, Weight sg, const Value& z) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dot2_merge(a[q], b0.x, b0.y);
+        add(sg, z);
+        return make_float4(a[0].value(), a[1].value(), a[2].value(), a[3].value());
+    }
+};
+template <>
+struct FlowSum<double> {
+    using Weight = double;
+    using Value = D4;
+    D4 a;
+    __device__ __forceinline__ void init() { a = {0.0, 0.0, 0.0, 0.0}; }
     // pairs: each 8-byte table entry holds an FP32 (hi, lo) pair
-    auto entry = [pairs](const double* p, int64_t i) {
+    __device__ static Weight entry(const double* p, int64_t i, int pairs) {
         if (pairs) {
             const float2 v = reinterpret_cast<const float2*>(p)[i];
             return (double)v.x + (double)v.y;
         }
         return p[i];
-    };
-    D4 a[G];
-#pragma unroll
-    for (int gi = 0; gi < G; ++gi) a[gi] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
-    for (int j = s; j < m; j += S) {
-        const double2* row = reinterpret_cast<const double2*>(V + (int64_t)idx[j] * Rs);
-        const double wj = entry(w, j);
-#pragma unroll
-        for (int gi = 0; gi < G; ++gi) {
-            const int ch = c0 + cl + gi * W;
-            if (ch < cpn) {
-                const double2 v0 = __ldcg(row + 2 * ch);
-                const double2 v1 = __ldcg(row + 2 * ch + 1);
-                a[gi].x = fma(wj, v0.x, a[gi].x);
-                a[gi].y = fma(wj, v0.y, a[gi].y);
-                a[gi].z = fma(wj, v1.x, a[gi].z);
-                a[gi].w = fma(wj, v1.y, a[gi].w);
-            }
-        }
     }
-    for (int o = W; o < 32; o <<= 1)
-#pragma unroll
-        for (int gi = 0; gi < G; ++gi) {
-            a[gi].x += __shfl_xor_sync(FULL_MASK, a[gi].x, o);
-            a[gi].y += __shfl_xor_sync(FULL_MASK, a[gi].y, o);
-            a[gi].z += __shfl_xor_sync(FULL_MASK, a[gi].z, o);
-            a[gi].w += __shfl_xor_sync(FULL_MASK, a[gi].w, o);
-        }
-    if (s == 0) {
-        const double b0 = entry(t.b0, pos), sg = entry(t.sigma, pos);
-#pragma unroll
-        for (int gi = 0; gi < G; ++gi) {
-            const int ch = c0 + cl + gi * W;
-            if (ch < cpn) {
-                D4 zz;
-                if (z) {
-                    zz = load_d4(z + (int64_t)g * Rs + 4 * ch);
-                } else {
-                    const float4 f = normals4(seed, g, ch);
-                    zz = {(double)f.x, (double)f.y, (double)f.z, (double)f.w};
-                }
-                D4 r;
-                r.x = fma(sg, zz.x, a[gi].x + b0);
-                r.y = fma(sg, zz.y, a[gi].y + b0);
-                r.z = fma(sg, zz.z, a[gi].z + b0);
-                r.w = fma(sg, zz.w, a[gi].w + b0);
-                store_d4(V + (int64_t)g * Rs + 4 * ch, r);
-            }
-        }
+    __device__ static Weight shfl(Weight w, int l) { return __shfl_sync(FULL_MASK, w, l); }
+    __device__ static Value draws(const double* z, uint64_t seed, int g, int64_t row, int ch) {
+        if (z) return load_d4(z + row + 4 * ch);
+        const float4 n4 = normals4(seed, g, ch);
+        return {(double)n4.x, (double)n4.y, (double)n4.z, (double)n4.w};
     }
-}
+    __device__ __forceinline__ void add(Weight w, const Value& v) {
+        a.x = fma(w, v.x, a.x);
+        a.y = fma(w, v.y, a.y);
+        a.z = fma(w, v.z, a.z);
+        a.w = fma(w, v.w, a.w);
+    }
+    __device__ __forceinline__ void across(int o) {
+        a.x += __shfl_xor_sync(FULL_MASK, a.x, o);
+        a.y += __shfl_xor_sync(FULL_MASK, a.y, o);
+        a.z += __shfl_xor_sync(FULL_MASK, a.z, o);
+        a.w += __shfl_xor_sync(FULL_MASK, a.w, o);
+    }
+    __device__ __forceinline__ Value finish(Weight b0, Weight sg, const Value& z) {
+        return {fma(sg, z.x, a.x + b0), fma(sg, z.y, a.y + b0), fma(sg, z.z, a.z + b0), fma(sg, z.w, a.w + b0)};
+    }
+};
 
 // CSR: packed tables (t.off rows) and the seed read from f.seed_dev, the form
 // used by batches of domains.
-template <typename T, int G, int MINB, bool CSR>
+//
+// A warp has three items under way: the ticket of the one after next, the
+// table rows of the next one (a neighbour per lane, handed round by shuffles),
+// and AHEAD neighbours' values of the current one, loaded before the first
+// of them is looked at.
+template <typename T, int G, int AHEAD, int MINB, bool CSR>
 __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables<T> t, int k, int Rp, int W,
-                                                               const T* __restrict__ z, uint64_t seed,
-                                                               T* __restrict__ V, const FlowArgs f) {
+                                                               const T* __restrict__ z, uint64_t seed, T* V,
+                                                               const __grid_constant__ FlowArgs f) {
+    using Sum = FlowSum<T>;
+    using Weight = typename Sum::Weight;
+    using Value = typename Sum::Value;
     const int lane = threadIdx.x & 31;
     const int64_t items = f.item1;
-    const int P4 = W * G;
+    const int S = 32 / W, s = lane / W, cl = lane % W, cpn = Rp >> 2;
     const int64_t Rs = f.row_stride ? f.row_stride : Rp;
+    const int pairs = CSR && sizeof(T) == 8 ? f.pairs : 0;
     if (CSR && f.seed_dev) seed = *f.seed_dev;
-    for (;;) {
+    // a ticket of the warp's class, or the end once an error is raised (the
+    // two reads overlap)
+    const int cls = threadIdx.x >> 5;
+    auto take = [&]() {
         unsigned long long base = 0;
-        if (lane == 0)
-            base = (*(volatile int32_t*)f.err) ? (unsigned long long)items
-                                                 : f.item0 + atomicAdd(f.ticket, (unsigned long long)f.chunk);
-        base = __shfl_sync(FULL_MASK, base, 0);
-        if ((int64_t)base >= items) break;
-        const int64_t end = min((int64_t)base + f.chunk, items);
-        for (int64_t it = (int64_t)base; it < end; ++it) {
-            const int64_t pos = it / f.H;
-            const int q = (int)(it - pos * f.H);
-            const int g = t.node[pos];
-            if (f.node_class && f.node_class[g] != f.cls) continue;  // the other launch's node
-            const int m = t.m[pos];
-            int32_t* done_q = f.done + (int64_t)q * f.N;
-            const bool ok = flow_wait(t.idx + (CSR ? t.off[pos] : pos * (int64_t)k), m, done_q, f, lane);
-            if (ok) {
-                if constexpr (sizeof(T) == 4)
-                    flow_piece_fp32<G, CSR>(t, k, pos, g, m, Rp, Rs, q * P4, W, lane, z, seed, V);
-                else
-                    flow_piece_fp64<G, CSR>(t, k, pos, g, m, Rp, Rs, q * P4, W, lane, z, seed, V, CSR ? f.pairs : 0);
-            } else if (lane == 0) {
-                atomicExch(f.err, 1);
+        if (lane == 0) {
+            base = f.item0 + (atomicAdd(f.ticket + cls * FLOW_TICKET_STRIDE, 1ull) * FLOW_CLASSES + cls) * f.chunk;
+            if (*(volatile int32_t*)f.err) base = (unsigned long long)items;
+        }
+        return base;
+    };
+    unsigned long long ticket = take();
+    int64_t it = 0, end = 0;  // the next item, and the end of its ticket
+    auto step = [&]() {
+        if (++it < end) return;
+        it = (int64_t)__shfl_sync(FULL_MASK, ticket, 0);
+        end = min(it + f.chunk, items);
+        if (it < items) ticket = take();
+    };
+    // it / H by a reciprocal: exact while it * H < 2^64
+    auto position = [&](int64_t i) { return f.H == 1 ? i : (int64_t)__umul64hi((uint64_t)i, f.rec); };
+    // the next item's tables
+    int64_t nrow = 0;
+    int ng = 0, nm = 0, nidx = 0;
+    Weight nw{};
+    auto tables = [&]() {
+        if (it >= items) return;
+        const int64_t pos = position(it);
+        ng = t.node[pos];
+        nm = t.m[pos];
+        nrow = CSR ? t.off[pos] : pos * (int64_t)k;
+        if (lane < (CSR ? nm : k)) {
+            nidx = t.idx[nrow + lane];
+            nw = Sum::entry(t.w, nrow + lane, pairs);
+        }
+    };
+    step();
+    tables();
+    while (it < items) {
+        const int64_t pos = position(it);
+        const int c0 = (int)(it - pos * f.H) * (W * G);
+        const int64_t row = nrow;
+        const int g = ng, m = nm;
+        int idx = nidx;
+        Weight w = nw;
+        step();
+        tables();
+        if (CSR && f.node_class && f.node_class[g] != f.cls) continue;  // the other launch's node
+        // the draws and the node's own terms: nothing of them waits
+        Value zz[G];
+        Weight b0{}, sg{};
+        if (s == 0) {
+            b0 = Sum::entry(t.b0, pos, pairs);
+            sg = Sum::entry(t.sigma, pos, pairs);
+#pragma unroll
+            for (int gi = 0; gi < G; ++gi) {
+                const int ch = c0 + cl + gi * W;
+                if (ch < cpn) zz[gi] = Sum::draws(z, seed, g, (int64_t)g * Rs, ch);
             }
-            __threadfence();
-            __syncwarp();
-            if (lane == 0) st_flag(done_q + g, f.epoch);
+        }
+        bool stuck = false;
+        Sum a[G];
+#pragma unroll
+        for (int gi = 0; gi < G; ++gi) a[gi].init();
+        for (int jb = 0; jb < m; jb += 32) {
+            if (jb && jb + lane < m) {
+                idx = t.idx[row + jb + lane];
+                w = Sum::entry(t.w, row + jb + lane, pairs);
+            }
+            const int mm = min(32, m - jb);
+            for (int j0 = 0; j0 < mm; j0 += AHEAD * S) {
+                Value v[AHEAD][G];
+                auto wanted = [&](int h, int gi) { return j0 + h * S + s < mm && c0 + cl + gi * W < cpn; };
+                auto chunk = [&](int h) {
+                    return V + (int64_t)__shfl_sync(FULL_MASK, idx, (j0 + h * S + s) & 31) * Rs + 4 * (c0 + cl);
+                };
+#pragma unroll
+                for (int h = 0; h < AHEAD; ++h) {
+                    const T* p = chunk(h);
+#pragma unroll
+                    for (int gi = 0; gi < G; ++gi)
+                        if (wanted(h, gi)) v[h][gi] = ld_value4(p + 4 * gi * W);
+                }
+                // whatever is not stored yet is loaded again
+                FlowBound bound;
+                for (;;) {
+                    bool miss = false;
+#pragma unroll
+                    for (int h = 0; h < AHEAD; ++h)
+#pragma unroll
+                        for (int gi = 0; gi < G; ++gi) miss |= wanted(h, gi) && missing4(v[h][gi]);
+                    if (!__any_sync(FULL_MASK, miss) || stuck) break;
+                    stuck = !bound.more(f.err, f.wait_ns);
+                    stuck = __any_sync(FULL_MASK, stuck);
+#pragma unroll
+                    for (int h = 0; h < AHEAD; ++h) {
+                        const T* p = chunk(h);
+#pragma unroll
+                        for (int gi = 0; gi < G; ++gi)
+                            if (wanted(h, gi) && missing4(v[h][gi])) v[h][gi] = ld_value4(p + 4 * gi * W);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < AHEAD; ++h) {
+                    const Weight wj = Sum::shfl(w, (j0 + h * S + s) & 31);
+#pragma unroll
+                    for (int gi = 0; gi < G; ++gi)
+                        if (wanted(h, gi)) a[gi].add(wj, v[h][gi]);
+                }
+            }
+        }
+        for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+            for (int gi = 0; gi < G; ++gi) a[gi].across(o);
+        if (s == 0) {
+#pragma unroll
+            for (int gi = 0; gi < G; ++gi) {
+                const int ch = c0 + cl + gi * W;
+                if (ch < cpn) {
+                    Value r = a[gi].finish(b0, sg, zz[gi]);
+                    if (stuck) r.x = r.y = r.z = r.w = settle(unstored<T>());
+                    st_value4(V + (int64_t)g * Rs + 4 * ch, r);
+                }
+            }
         }
     }
 }
 
 // Self-test of the dataflow wait: one warp waits, with the sweep's own
-// flow_wait, on a flag that nothing sets; the wait must give up after
+// bound, on a row that nothing stores; the wait must give up after
 // f.wait_ns and report it in *f.err, leaving the context usable.
-__global__ void flow_wait_selftest_kernel(const int32_t* __restrict__ idx, const FlowArgs f) {
-    const int lane = threadIdx.x & 31;
-    const bool ok = flow_wait(idx, 1, f.done, f, lane);
-    if (!ok && lane == 0) atomicExch(f.err, 1);
+__global__ void flow_wait_selftest_kernel(const float* row, const __grid_constant__ FlowArgs f) {
+    FlowBound bound;
+    while (missing4(ld_value4(row)))
+        if (!bound.more(f.err, f.wait_ns)) return;
 }
 
-cudaError_t launch_flow_wait_selftest(const int32_t* idx, const FlowArgs& f, cudaStream_t s) {
-    flow_wait_selftest_kernel<<<1, 32, 0, s>>>(idx, f);
+cudaError_t launch_flow_wait_selftest(const float* row, const FlowArgs& f, cudaStream_t s) {
+    flow_wait_selftest_kernel<<<1, 32, 0, s>>>(row, f);
     return cudaGetLastError();
 }
 
-// Flags of the positions [p0, p1) swept by per-level launches before a
-// dataflow launch takes over (every piece).
-__global__ void flow_mark_kernel(const int32_t* __restrict__ node, int64_t p0, int64_t p1, int H, int64_t N,
-                                 int32_t* __restrict__ done, int32_t epoch) {
-    const int64_t n = (p1 - p0) * H;
+// Rows of the positions [p0, p1) set to the pattern that stands for "not yet
+// stored" (row_bytes a multiple of 16).
+__global__ void flow_clear_kernel(const int32_t* __restrict__ node, int64_t p0, int64_t p1, int row16,
+                                  uint4* __restrict__ V) {
+    const int64_t n = (p1 - p0) * row16;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pos = p0 + i / H;
-        const int q = (int)(i % H);
-        done[(int64_t)q * N + node[pos]] = epoch;
+        const int64_t p = i / row16;
+        V[(int64_t)node[p0 + p] * row16 + (i - p * row16)] = make_uint4(~0u, ~0u, ~0u, ~0u);
     }
+}
+
+cudaError_t launch_flow_clear(const int32_t* node, int64_t p0, int64_t p1, int64_t N, size_t row_bytes, void* V,
+                              cudaStream_t s) {
+    if (p1 <= p0) return cudaSuccess;
+    if (p0 == 0 && p1 == N) return cudaMemsetAsync(V, 0xff, (size_t)N * row_bytes, s);
+    const int64_t n = (p1 - p0) * (int64_t)(row_bytes / 16);
+    const int blocks = (int)std::min<int64_t>((n + 255) / 256, 1 << 14);
+    flow_clear_kernel<<<blocks, 256, 0, s>>>(node, p0, p1, (int)(row_bytes / 16), reinterpret_cast<uint4*>(V));
+    return cudaGetLastError();
 }
 
 // Lane layout for a row of cpn chunks: W lanes per slice (0 = automatic),
@@ -748,35 +835,43 @@ int flow_layout(int Rp, int& W, int& G) {
     return (cpn + W * G - 1) / (W * G);
 }
 
-template <typename T, int G, int MINB, bool CSR>
-static cudaError_t flow_launch(const SweepTables<T>& t, int k, int Rp, int W, const T* z, uint64_t seed, T* V,
+template <typename T, bool CSR>
+using FlowKernel = void (*)(const SweepTables<T>, int, int, int, const T*, uint64_t, T*, const FlowArgs);
+
+// The kernel for G chunks per lane and W lanes per slice.  A lane has 4 loads
+// in flight; 2 where 16 or 32 slices cover a neighbour list with that many
+// (W <= 2: with 4, the empty ones cost 8 % on batches of 8 realizations).
+template <typename T, bool CSR>
+static FlowKernel<T, CSR> flow_kernel(int G, int W, bool tight) {
+    constexpr bool F = sizeof(T) == 4;
+    if (G == 2) return tight ? sweep_flow_kernel<T, 2, 2, F ? 3 : 2, CSR> : sweep_flow_kernel<T, 2, 2, F ? 2 : 1, CSR>;
+    if (W <= 2) return tight ? sweep_flow_kernel<T, 1, 2, F ? 4 : 3, CSR> : sweep_flow_kernel<T, 1, 2, 2, CSR>;
+    return tight ? sweep_flow_kernel<T, 1, 4, F ? 4 : 3, CSR> : sweep_flow_kernel<T, 1, 4, 2, CSR>;
+}
+
+template <typename T, bool CSR>
+static cudaError_t flow_launch(const SweepTables<T>& t, int k, int Rp, int W, int G, const T* z, uint64_t seed, T* V,
                                const FlowArgs& f, int nsm, cudaStream_t s) {
+    const FlowKernel<T, CSR> kernel = flow_kernel<T, CSR>(G, W, f.tight);
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_flow_kernel<T, G, MINB, CSR>, 256, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * FLOW_CLASSES, 0);
     if (e != cudaSuccess) return e;
     if (f.blocks_per_sm > 0 && f.blocks_per_sm < per_sm) per_sm = f.blocks_per_sm;
     if (per_sm < 1) per_sm = 1;
     const int64_t items = (f.item1 - f.item0 + f.chunk - 1) / f.chunk;
-    int64_t blocks = std::min<int64_t>((int64_t)nsm * per_sm, (items + 7) / 8);
+    int64_t blocks = std::min<int64_t>((int64_t)nsm * per_sm, (items + FLOW_CLASSES - 1) / FLOW_CLASSES);
     if (blocks < 1) blocks = 1;
-    sweep_flow_kernel<T, G, MINB, CSR><<<(int)blocks, 256, 0, s>>>(t, k, Rp, W, z, seed, V, f);
+    kernel<<<(int)blocks, 32 * FLOW_CLASSES, 0, s>>>(t, k, Rp, W, z, seed, V, f);
     return cudaGetLastError();
 }
 
 template <typename T>
 static cudaError_t sweep_flow(const SweepTables<T>& t, int k, int Rp, int W, int G, const T* z, uint64_t seed, T* V,
-                              const FlowArgs& f, int nsm, cudaStream_t s) {
+                              FlowArgs f, int nsm, cudaStream_t s) {
     if (f.item1 <= f.item0) return cudaSuccess;
-    if (t.off) {
-        if (G == 2) return f.tight ? flow_launch<T, 2, 4, true>(t, k, Rp, W, z, seed, V, f, nsm, s)
-                                   : flow_launch<T, 2, 1, true>(t, k, Rp, W, z, seed, V, f, nsm, s);
-        return f.tight ? flow_launch<T, 1, 6, true>(t, k, Rp, W, z, seed, V, f, nsm, s)
-                       : flow_launch<T, 1, 1, true>(t, k, Rp, W, z, seed, V, f, nsm, s);
-    }
-    if (G == 2) return f.tight ? flow_launch<T, 2, 4, false>(t, k, Rp, W, z, seed, V, f, nsm, s)
-                               : flow_launch<T, 2, 1, false>(t, k, Rp, W, z, seed, V, f, nsm, s);
-    return f.tight ? flow_launch<T, 1, 6, false>(t, k, Rp, W, z, seed, V, f, nsm, s)
-                   : flow_launch<T, 1, 1, false>(t, k, Rp, W, z, seed, V, f, nsm, s);
+    f.rec = f.H > 1 ? ~0ull / (uint64_t)f.H + 1 : 0;
+    return t.off ? flow_launch<T, true>(t, k, Rp, W, G, z, seed, V, f, nsm, s)
+                 : flow_launch<T, false>(t, k, Rp, W, G, z, seed, V, f, nsm, s);
 }
 
 cudaError_t launch_sweep_flow_fp32(const SweepTables<float>& t, int k, int Rp, int W, int G, const float* z,
@@ -787,31 +882,6 @@ cudaError_t launch_sweep_flow_fp32(const SweepTables<float>& t, int k, int Rp, i
 cudaError_t launch_sweep_flow_fp64(const SweepTables<double>& t, int k, int Rp, int W, int G, const double* z,
                                    uint64_t seed, double* V, const FlowArgs& f, int nsm, cudaStream_t s) {
     return sweep_flow<double>(t, k, Rp, W, G, z, seed, V, f, nsm, s);
-}
-
-cudaError_t launch_flow_mark(const int32_t* node, int64_t p0, int64_t p1, int H, int64_t N, int32_t* done,
-                             int32_t epoch, cudaStream_t s) {
-    if (p1 <= p0) return cudaSuccess;
-    const int64_t n = (p1 - p0) * H;
-    const int blocks = (int)std::min<int64_t>((n + 255) / 256, 1 << 16);
-    flow_mark_kernel<<<blocks, 256, 0, s>>>(node, p0, p1, H, N, done, epoch);
-    return cudaGetLastError();
-}
-
-int sweep_flow_max_blocks_per_sm(bool fp64, int G, bool tight) {
-    int per_sm = 0;
-    if (fp64) {
-        if (G == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, tight ? sweep_flow_kernel<double, 2, 4, false> : sweep_flow_kernel<double, 2, 1, false>, 256, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, tight ? sweep_flow_kernel<double, 1, 6, false> : sweep_flow_kernel<double, 1, 1, false>, 256, 0);
-    } else {
-        if (G == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, tight ? sweep_flow_kernel<float, 2, 4, false> : sweep_flow_kernel<float, 2, 1, false>, 256, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, tight ? sweep_flow_kernel<float, 1, 6, false> : sweep_flow_kernel<float, 1, 1, false>, 256, 0);
-    }
-    return per_sm;
 }
 
 // ---------------------------------------------------------------------------
