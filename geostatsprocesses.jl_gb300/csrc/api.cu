@@ -459,11 +459,96 @@ extern "C" void sgs_plan_destroy(sgs_plan* p) {
     delete p;
 }
 
+// The search template: every cell offset of the box [-e, e] inside the
+// neighbourhood, by (d2, linear offset).  d2(h) = d2(-h) to the bit, so only
+// the half of the box that follows the centre in (z, y, x) order, whose linear
+// offsets are the positive ones, is enumerated and sorted; a run of equal d2
+// is then the half's mirror image followed by the half.  The sort is by 32
+// bits of d2 scaled to its range (3 radix passes), and exact within the runs
+// that these leave equal.  A comparison sort of all of it bounded large
+// neighbourhoods: 1.19M offsets 88 ms, this 15.
+static void host_template(HostDomain& H, const int64_t e[3]) {
+    const GridDev& G = H.grid;
+    std::vector<double> d2;
+    std::vector<TmplEntry> cell;
+    const size_t cap = (size_t)(((2 * e[0] + 1) * (2 * e[1] + 1) * (2 * e[2] + 1)) / 2);
+    d2.reserve(cap);
+    cell.reserve(cap);
+    double dmax = 0.0;
+    for (int64_t c = 0; c <= e[2]; ++c)
+        for (int64_t b = c == 0 ? 0 : -e[1]; b <= e[1]; ++b) {
+            int64_t a0 = e[0] + 1, a1 = -e[0] - 1;  // the row's span inside
+            for (int64_t a = c == 0 && b == 0 ? 1 : -e[0]; a <= e[0]; ++a) {
+                const double h[3] = {(double)a * G.spacing[0], (double)b * G.spacing[1],
+                                     G.dim == 3 ? (double)c * G.spacing[2] : 0.0};
+                const double d = host_d2(H.metric, G.dim, h);
+                if (!host_inside(H.metric, d)) continue;
+                d2.push_back(d);
+                cell.push_back(TmplEntry{(int)a, (int)b, (int)c, (int)(a + (int64_t)G.n[0] * (b + (int64_t)G.n[1] * c))});
+                dmax = std::max(dmax, d);
+                a0 = std::min(a0, a);
+                a1 = std::max(a1, a);
+            }
+            if (a0 > a1) continue;
+            H.tmpl_ext[0] = std::max(H.tmpl_ext[0], (int)std::max(std::abs(a0), std::abs(a1)));
+            H.tmpl_ext[1] = std::max(H.tmpl_ext[1], (int)std::abs(b));
+            H.tmpl_ext[2] = std::max(H.tmpl_ext[2], (int)c);
+        }
+    const size_t n = d2.size();
+    double scale = 4294967295.0 / dmax;
+    if (!std::isfinite(scale) || !std::isfinite(dmax)) scale = 0.0;  // one run
+    std::vector<uint64_t> key(n), tmp(n);  // (scaled d2, index)
+    uint32_t hist[3][2048] = {};
+    for (size_t i = 0; i < n; ++i) {
+        const uint64_t q = scale > 0.0 ? std::min<uint64_t>((uint64_t)(d2[i] * scale), 0xffffffffu) : 0;
+        key[i] = q << 32 | i;
+        for (int r = 0; r < 3; ++r) hist[r][(q >> (11 * r)) & 2047]++;
+    }
+    for (int r = 0; r < 3; ++r) {
+        uint32_t sum = 0;
+        bool one = false;
+        for (uint32_t& x : hist[r]) {
+            one |= x == n;
+            const uint32_t c = x;
+            x = sum;
+            sum += c;
+        }
+        if (one) continue;
+        for (size_t i = 0; i < n; ++i) tmp[hist[r][(key[i] >> (32 + 11 * r)) & 2047]++] = key[i];
+        key.swap(tmp);
+    }
+    auto before = [&](uint64_t x, uint64_t y) {
+        const uint32_t i = (uint32_t)x, j = (uint32_t)y;
+        return d2[i] < d2[j] || (d2[i] == d2[j] && cell[i].dlin < cell[j].dlin);
+    };
+    H.tmpl.resize(2 * n);
+    H.tmpl_d2.resize(2 * n);
+    for (size_t i = 0; i < n;) {
+        size_t j = i + 1;
+        while (j < n && key[j] >> 32 == key[i] >> 32) ++j;
+        // (z, y, x) order, which the radix passes keep, mostly is the linear one
+        if (j - i > 1 && !std::is_sorted(key.begin() + i, key.begin() + j, before))
+            std::sort(key.begin() + i, key.begin() + j, before);
+        while (i < j) {  // runs of equal d2
+            const double d = d2[(uint32_t)key[i]];
+            size_t m = 1;
+            while (i + m < j && d2[(uint32_t)key[i + m]] == d) ++m;
+            for (size_t s = 0; s < m; ++s) {
+                const TmplEntry t = cell[(uint32_t)key[i + s]];
+                H.tmpl[2 * i + m + s] = t;
+                H.tmpl[2 * i + m - 1 - s] = TmplEntry{-t.dx, -t.dy, -t.dz, -t.dlin};
+                H.tmpl_d2[2 * i + s] = H.tmpl_d2[2 * i + m + s] = d;
+            }
+            i += m;
+        }
+    }
+}
+
 // Host-side set-up of one problem: validation (argument errors as the
 // reference's ArgumentError / @assert), the neighbourhood metric, the path
 // and its ranks, the sorted offset template and the data buckets.  Shared by
 // plans and batches of domains.
-int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err) {
+int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err, bool grid_neighbors) {
 #define HERR(msg)              \
     do {                       \
         err = (msg);           \
@@ -580,30 +665,7 @@ int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err) {
         cells *= 2 * e[j] + 1;
     }
     if (cells > (int64_t)1 << 28) HERR("search neighbourhood spans too many cells");
-    struct Ent { double d2; int64_t lin; TmplEntry e; };
-    std::vector<Ent> ents;
-    for (int64_t c = -e[2]; c <= e[2]; ++c)
-        for (int64_t b = -e[1]; b <= e[1]; ++b)
-            for (int64_t a = -e[0]; a <= e[0]; ++a) {
-                if (a == 0 && b == 0 && c == 0) continue;
-                double h[3] = {(double)a * G.spacing[0], (double)b * G.spacing[1], dim == 3 ? (double)c * G.spacing[2] : 0.0};
-                double d = host_d2(H.metric, dim, h);
-                if (!host_inside(H.metric, d)) continue;
-                int64_t lin = a + (int64_t)G.n[0] * (b + (int64_t)G.n[1] * c);
-                ents.push_back({d, lin, TmplEntry{(int)a, (int)b, (int)c, (int)lin}});
-            }
-    std::sort(ents.begin(), ents.end(), [](const Ent& x, const Ent& y) {
-        return x.d2 < y.d2 || (x.d2 == y.d2 && x.lin < y.lin);
-    });
-    H.tmpl.resize(ents.size());
-    H.tmpl_d2.resize(ents.size());
-    for (size_t i = 0; i < ents.size(); ++i) {
-        H.tmpl[i] = ents[i].e;
-        H.tmpl_d2[i] = ents[i].d2;
-        H.tmpl_ext[0] = std::max(H.tmpl_ext[0], std::abs(ents[i].e.dx));
-        H.tmpl_ext[1] = std::max(H.tmpl_ext[1], std::abs(ents[i].e.dy));
-        H.tmpl_ext[2] = std::max(H.tmpl_ext[2], std::abs(ents[i].e.dz));
-    }
+    if (grid_neighbors) host_template(H, e);
 
     // data: id order (solve) and bucket order (search)
     H.xyz.assign((size_t)H.D * 3, 0.0);
@@ -706,11 +768,11 @@ void sgs::search_args_of(const HostDomain& H, SearchArgs& sa) {
     }
 }
 
-static int plan_init(sgs_plan* P, const sgs_problem* pr) {
+static int plan_init(sgs_plan* P, const sgs_problem* pr, bool grid_neighbors = true) {
     HostDomain H;
     {
         std::string err;
-        const int rc = host_domain(pr, H, err);  // path ranks on the device, below
+        const int rc = host_domain(pr, H, err, grid_neighbors);  // path ranks on the device, below
         if (rc != SGS_OK) return set_err(P, rc, err);
     }
     P->grid = H.grid;
@@ -1663,7 +1725,7 @@ extern "C" int sgs_krige(const sgs_problem* problem, double* mean, double* var) 
         sgs_plan_destroy(P);
         return code;
     };
-    int rc = plan_init(P, problem);
+    int rc = plan_init(P, problem, false);
     if (rc != SGS_OK) return fail(rc);
     const int64_t N = P->N;
     if (P->D == 0) {  // no data: the prior (priormean, src/expectation/field/gaussian.jl:5-19)
@@ -1677,34 +1739,16 @@ extern "C" int sgs_krige(const sgs_problem* problem, double* mean, double* var) 
     P->warm_start = 0;
     P->data_only = 1;
     if ((rc = sgs_plan_prepare(P)) != SGS_OK) return fail(rc);
-    std::vector<int32_t> node(N);
-    std::vector<int8_t> st(N);
-    std::vector<double> b0(N), sd(N);
-    if (cudaMemcpy(st.data(), P->d_status, N, cudaMemcpyDeviceToHost) != cudaSuccess)
-        return fail(cuda_err(P, cudaGetLastError(), "status read-back"));
-    if (P->precision == SGS_PREC_FP64) {
-        if (cudaMemcpy(node.data(), P->t64.node, N * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(b0.data(), P->t64.b0, N * 8, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(sd.data(), P->t64.sigma, N * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
-            return fail(cuda_err(P, cudaGetLastError(), "table read-back"));
-    } else {
-        std::vector<float> b2(2 * N), s2(2 * N);
-        if (cudaMemcpy(node.data(), P->t32.node, N * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(b2.data(), P->t32.b0, N * 8, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(s2.data(), P->t32.sigma, N * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
-            return fail(cuda_err(P, cudaGetLastError(), "table read-back"));
-        for (int64_t p = 0; p < N; ++p) {
-            b0[p] = (double)b2[2 * p] + (double)b2[2 * p + 1];
-            sd[p] = (double)s2[2 * p] + (double)s2[2 * p + 1];
-        }
-    }
-    const double nan = std::nan("");
-    for (int64_t p = 0; p < N; ++p) {
-        const int32_t g = node[p];
-        const bool ok = st[g] == SGS_NODE_KRIGED;
-        mean[g] = ok ? P->mean + b0[p] : nan;
-        if (var) var[g] = ok ? sd[p] * sd[p] : nan;
-    }
+    double* d_mv = nullptr;  // mean, variance
+    if ((rc = dalloc(P, &d_mv, 2 * N))) return fail(rc);
+    cudaError_t e = P->precision == SGS_PREC_FP64
+                        ? launch_krige_moments(P->t64, P->d_status, P->mean, N, d_mv, d_mv + N, P->stream)
+                        : launch_krige_moments(P->t32, P->d_status, P->mean, N, d_mv, d_mv + N, P->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(mean, d_mv, N * sizeof(double), cudaMemcpyDeviceToHost, P->stream);
+    if (e == cudaSuccess && var)
+        e = cudaMemcpyAsync(var, d_mv + N, N * sizeof(double), cudaMemcpyDeviceToHost, P->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
+    if (e != cudaSuccess) return fail(cuda_err(P, e, "moments"));
     sgs_plan_destroy(P);
     return SGS_OK;
 }

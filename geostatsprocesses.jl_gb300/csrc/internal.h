@@ -309,7 +309,9 @@ struct HostDomain {
 // Validates *pr and fills H; SGS_OK or SGS_ERR_ARG with err set.  The path
 // is left to the caller: plans and batches build and check its ranks on the
 // device (launch_path_ranks, launch_batch_path_ranks).
-int host_domain(const sgs_problem* pr, HostDomain& H, std::string& err);
+// grid_neighbors: false for kriging from the data alone, whose search has no
+// template (none is built; neighbourhoods too large for one stay refused)
+int host_domain(const sgs_problem* pr, HostDomain& H, std::string& err, bool grid_neighbors = true);
 // rank[path[t]] = t for a path of N nodes on the device (path NULL: the
 // linear path, written into path_out), checking that the path is a
 // permutation of [0, N): *err (zeroed by the caller) is set otherwise.
@@ -395,6 +397,10 @@ cudaError_t launch_sweep_flow_fp32(const SweepTables<float>& t, int k, int Rp, i
                                    uint64_t seed, float* V, const FlowArgs& f, int nsm, cudaStream_t s);
 cudaError_t launch_sweep_flow_fp64(const SweepTables<double>& t, int k, int Rp, int W, int G, const double* z,
                                    uint64_t seed, double* V, const FlowArgs& f, int nsm, cudaStream_t s);
+// mean + b0 and sigma^2 of the kriged nodes, NaN elsewhere, by node
+template <typename T>
+cudaError_t launch_krige_moments(const SweepTables<T>& t, const int8_t* status, double mean, int64_t N, double* m,
+                                 double* v, cudaStream_t s);
 // the rows of positions [p0, p1) (all N: every row) cleared for a dataflow launch
 cudaError_t launch_flow_clear(const int32_t* node, int64_t p0, int64_t p1, int64_t N, size_t row_bytes, void* V,
                               cudaStream_t s);

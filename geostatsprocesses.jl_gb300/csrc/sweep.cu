@@ -516,7 +516,7 @@ cudaError_t launch_sweep_all_fp64(const SweepTables<double>& t, int k, const int
 //
 // What bounds it: the neighbours' rows, gathered from anywhere in the values
 // (no reuse once they exceed L2), or on narrow levels the step above.  4M
-// nodes x 26 neighbours x 256 FP32 values: 40.8 ms, 65 with flags (37.6 by
+// nodes x 48 neighbours x 256 FP32 values: 40.8 ms, 65 with flags (37.6 by
 // per-level launches, whose half-empty warps of the narrow levels cost the
 // same on other shapes: 16.8M nodes x 64 values 33.7 ms, per level 36.3,
 // with flags 59; 1.2M x 100: 4.3, 5.9 and 6.8).
@@ -822,6 +822,38 @@ cudaError_t launch_flow_clear(const int32_t* node, int64_t p0, int64_t p1, int64
     flow_clear_kernel<<<blocks, 256, 0, s>>>(node, p0, p1, (int)(row_bytes / 16), reinterpret_cast<uint4*>(V));
     return cudaGetLastError();
 }
+
+// Posterior mean and variance from the tables of a plan whose neighbours are
+// data only: its data terms and conditional deviations, node by node.
+template <typename T>
+__global__ void krige_moments_kernel(const SweepTables<T> t, const int8_t* __restrict__ status, double mean, int64_t N,
+                                     double* __restrict__ m, double* __restrict__ v) {
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
+        double b0, sd;
+        if constexpr (sizeof(T) == 8) {
+            b0 = t.b0[p];
+            sd = t.sigma[p];
+        } else {
+            b0 = (double)t.b0[2 * p] + (double)t.b0[2 * p + 1];
+            sd = (double)t.sigma[2 * p] + (double)t.sigma[2 * p + 1];
+        }
+        const int32_t g = t.node[p];
+        const bool ok = status[g] == SGS_NODE_KRIGED_;
+        m[g] = ok ? mean + b0 : nan("");
+        v[g] = ok ? sd * sd : nan("");
+    }
+}
+
+template <typename T>
+cudaError_t launch_krige_moments(const SweepTables<T>& t, const int8_t* status, double mean, int64_t N, double* m,
+                                 double* v, cudaStream_t s) {
+    krige_moments_kernel<T><<<(int)std::min<int64_t>((N + 255) / 256, 1 << 14), 256, 0, s>>>(t, status, mean, N, m, v);
+    return cudaGetLastError();
+}
+template cudaError_t launch_krige_moments<float>(const SweepTables<float>&, const int8_t*, double, int64_t, double*,
+                                                 double*, cudaStream_t);
+template cudaError_t launch_krige_moments<double>(const SweepTables<double>&, const int8_t*, double, int64_t, double*,
+                                                  double*, cudaStream_t);
 
 // Lane layout for a row of cpn chunks: W lanes per slice (0 = automatic),
 // G chunks per lane; returns the pieces per row.
