@@ -759,6 +759,7 @@ void sgs::search_args_of(const HostDomain& H, SearchArgs& sa) {
     sa.k = H.k;
     sa.T = (int)H.tmpl.size();
     sa.D = H.D;
+    sa.ring0 = search_ring0(H.k, H.D, H.grid.dim, H.nb);
     for (int j = 0; j < 3; ++j) {
         sa.nb[j] = H.nb[j];
         sa.bw[j] = H.bw[j];
@@ -1029,6 +1030,7 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
     sa.path = P->d_path;
     sa.rank = P->d_rank;
     sa.D = P->D;
+    sa.ring0 = search_ring0(k, P->D, P->grid.dim, P->nb);
     sa.dxyz = P->d_dxyz_b;
     sa.dxyz_f = P->d_dxyz_f;
     sa.did = P->d_did;

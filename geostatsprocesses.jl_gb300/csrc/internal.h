@@ -3,6 +3,8 @@
 // Not part of the public ABI (include/geosgs.h is).
 #pragma once
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -99,6 +101,8 @@ struct SearchArgs {
     const int32_t* did;          // data id of each bucket-ordered entry
     const int32_t* bstart;       // bucket start offsets (nb+1)
     int nb[3];
+    int ring0;                   // buckets on each side of a node's own to start with
+                                 // when its k nearest data are looked for (search_ring0)
     double bw[3];                // bucket widths (physical)
     float inv_bw_f[3];           // FP32 1 / bucket width, for the bucket range
     float ext_f[3];              // FP32 bounding-box half extents
@@ -113,6 +117,12 @@ struct SearchArgs {
     // screened), summed once per warp
     unsigned long long* scanned;
 };
+
+// The ring whose box of buckets holds 1.5 k of D evenly spread data.
+inline int search_ring0(int k, int64_t D, int dim, const int* nb) {
+    const double side = std::pow(1.5 * k * nb[0] * nb[1] * nb[2] / (double)std::max<int64_t>(D, 1), 1.0 / dim);
+    return (int)std::min(std::max(0.0, std::floor(0.5 * (side - 1.0))), 1e6);
+}
 
 // Longest wait of the dependency-level kernels for one neighbour's level.
 // Their waits end by construction (a neighbour's path rank is smaller, and
