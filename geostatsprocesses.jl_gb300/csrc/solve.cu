@@ -22,6 +22,7 @@
 // Results are written in level order (the sweep's layout): the grid
 // neighbours with their weights, and the data neighbours folded into the
 // constant b0 = sum_data w_i (d_i - mu).
+#include <algorithm>
 #include <cmath>
 #include <utility>
 
@@ -313,8 +314,241 @@ solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict
     }
 }
 
+// The plain FP64 path for at most 16 neighbours: GS lanes per system (8 or 16,
+// one per neighbour), 32 / GS systems per warp.  A warp FP64 instruction
+// holds its scheduler for 64 cycles whatever its lanes do, so what counts is
+// the number of instructions and the systems that share them.  Pairs with a
+// datum, the only ones evaluated, are queued and taken 32 at a time; lane i
+// then holds row i of the LHS in registers, and L D L' is eliminated with the
+// right-hand side (the k-th pivot is the one Cholesky's square root would be
+// taken of) by one reciprocal a column and rows broadcast by shuffles, in
+// chunks of 4 entries up to the longest system of the warp.  One warp per
+// system with a Cholesky factorization in shared memory and a division per
+// row in each substitution took 250k systems of 10 data 8.9 ms, this 2.6.
+// 1 / d of a pivot (positive, normal): an FP32 reciprocal r of its mantissa,
+// off by e = 1 - d r of some 2^-22, and one step of third order, r (1 + e +
+// e^2).  The exponents are handled as integers, off the FP64 pipe.
+__device__ __forceinline__ double reciprocal(double d) {
+    const unsigned hi = __double2hiint(d), lo = __double2loint(d);
+    float rf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(__uint_as_float(0x3f800000u | (hi & 0xfffffu) << 3 | lo >> 29)));
+    const unsigned u = __float_as_uint(rf);
+    const double r = __hiloint2double((int)((u >> 3) + (896u << 20) + (1023u << 20) - (hi & 0x7ff00000u)), (int)(u << 29));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+template <int GS>
+struct Sys64 {
+    static constexpr int SYS = 32 / GS;
+    static constexpr int LD = GS + 1;
+    double K[SYS][(GS + 1) * LD];  // row GS: the right-hand side
+    NbInfo info[SYS][GS + 1];      // [n]: the node itself
+    unsigned short queue[64];      // pairs with a datum: is the node's, system, row, column
+};
+
+__device__ __noinline__ double kcov_pair(const SolveArgs& a, const NbInfo& p, const NbInfo& q) { return kcov(a, p, q); }
+
+template <int GS, typename O>
+__global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __grid_constant__ SolveArgs a,
+                                                                      const SweepTables<O> tab) {
+    using S = Sys64<GS>;
+    constexpr int LD = S::LD;
+    extern __shared__ __align__(16) unsigned char smem[];
+    S& sh = reinterpret_cast<S*>(smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, grp = lane / GS, q = lane % GS;
+    const int k = a.k;
+    const GridDev& G = a.grid;
+    const double sill = a.vario.sill;
+    const int64_t count = a.list ? (int64_t)*a.nfallback : a.P;
+    const int64_t rounds = (count + S::SYS - 1) / S::SYS;
+    const int64_t nwarps = (int64_t)gridDim.x * SOLVE_WARPS;
+    unsigned long long msum = 0;
+    float l1max = 0.0f;
+    for (int64_t it = (int64_t)blockIdx.x * SOLVE_WARPS + (threadIdx.x >> 5); it < rounds; it += nwarps) {
+        const int64_t item = it * S::SYS + grp;
+        const bool have = item < count;
+        const int64_t pos = have ? (a.list ? (int64_t)a.list[item] : item) : 0;
+        const int g = have ? a.order[pos] : 0;
+        const int cnt = have ? a.cnt[g] : 0;
+        const int n = have && cnt >= a.nmin ? cnt : 0;  // systems to solve (0: none, or the prior)
+        NbInfo in{0, 0, 0, -1};
+        int id = 0;
+        if (q < n) {
+            id = a.nbr[(int64_t)g * k + q];
+            if (id < G.N) cell_of(G, id, in.c0, in.c1, in.c2);
+            else in.did = id - (int)G.N;
+            sh.info[grp][q] = in;
+        }
+        if (q == 0) {
+            NbInfo self{0, 0, 0, -1};
+            cell_of(G, g, self.c0, self.c1, self.c2);
+            sh.info[grp][n] = self;
+        }
+        __syncwarp();
+        const int nmax = (int)__reduce_max_sync(FULL_MASK, (unsigned)n);
+
+        // ---- covariances of the pairs among the neighbours and the node ----
+        int nq = 0;
+        auto evaluate = [&](int c) {
+            if (lane < c) {
+                const unsigned e = sh.queue[lane];
+                const int sg = (e >> 12) & 3, i = (e >> 6) & 63, j = e & 63;
+                const double v = kcov_pair(a, sh.info[sg][j], sh.info[sg][i]);
+                const int row = e >> 14 ? GS : i;  // the node's own
+                sh.K[sg][row * LD + j] = v;
+                if (row < GS) sh.K[sg][j * LD + i] = v;
+            }
+        };
+        const int pairs = n * (n + 1) / 2, pmax = nmax * (nmax + 1) / 2;
+        for (int p0 = 0; p0 < pmax; p0 += GS) {
+            const int p = p0 + q;
+            // p = i (i - 1) / 2 + j, j < i, i in 1 .. n (n: the node)
+            int i = (int)((1.0f + sqrtf(8.0f * (float)p + 1.0f)) * 0.5f);
+            if (i * (i - 1) / 2 > p) --i;
+            if (i * (i + 1) / 2 <= p) ++i;
+            const int j = p - i * (i - 1) / 2;
+            bool queued = false;
+            // the node's own row is kept as row GS
+            const int row = i == n ? GS : i;
+            if (p < pairs) {
+                const NbInfo pj = sh.info[grp][j], pi = sh.info[grp][i];
+                queued = pj.did >= 0 || pi.did >= 0;
+                if (!queued) {
+                    const double v = lut_or_cov(a, pi.c0 - pj.c0, pi.c1 - pj.c1, pi.c2 - pj.c2);
+                    sh.K[grp][row * LD + j] = v;
+                    if (i < n) sh.K[grp][j * LD + i] = v;
+                }
+            }
+            const unsigned b = __ballot_sync(FULL_MASK, queued);
+            if (queued) sh.queue[nq + __popc(b & lanemask_lt())] = (unsigned short)((i == n) << 14 | grp << 12 | i << 6 | j);
+            nq += __popc(b);
+            __syncwarp();
+            if (nq >= 32) {
+                evaluate(32);
+                __syncwarp();
+                const unsigned short rest = lane + 32 < nq ? sh.queue[lane + 32] : 0;
+                __syncwarp();
+                sh.queue[lane] = rest;
+                __syncwarp();
+                nq -= 32;
+            }
+        }
+        evaluate(nq);
+        __syncwarp();
+
+        // ---- L D L' of the rows in registers, with the right-hand side ----
+        double A[GS];
+#pragma unroll
+        for (int l = 0; l < GS; ++l)
+            A[l] = q < n && l < n && l != q ? sh.K[grp][q * LD + l] : (l == q ? (q < n ? sill : 1.0) : 0.0);
+        const double c = q < n ? sh.K[grp][GS * LD + q] : 0.0;
+        double y = c, dinv = 1.0;
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < GS; ++j) {
+            if (j < nmax) {
+                const double d = __shfl_sync(FULL_MASK, A[j], j, GS);
+                ok = ok && (j >= n || d > a.tau);
+                const double inv = reciprocal(d);
+                if (q == j) dinv = inv;
+                const double f = q > j ? -A[j] * inv : 0.0;
+                y = fma(f, __shfl_sync(FULL_MASK, y, j, GS), y);
+#pragma unroll
+                for (int l0 = 0; l0 < GS; l0 += 4)
+                    if (l0 + 3 > j && l0 < nmax) {
+#pragma unroll
+                        for (int l = l0; l < l0 + 4; ++l)
+                            if (l > j) A[l] = fma(f, __shfl_sync(FULL_MASK, A[l], j, GS), A[l]);
+                    }
+            }
+        }
+        double w = 0.0;
+#pragma unroll
+        for (int j = GS - 1; j >= 0; --j) {
+            if (j < nmax) {
+                const double t = y * dinv;
+                if (q == j) w = t;
+                const double wj = __shfl_sync(FULL_MASK, t, j, GS);
+                if (q < j) y = fma(-A[j], wj, y);
+            }
+        }
+        if (q >= n) w = 0.0;
+
+        // ---- the sweep-table row ----
+        const bool kriged = n > 0 && ok;
+        const bool isgrid = kriged && q < n && in.did < 0;
+        double wc = w * c;
+        double b0 = kriged && q < n && in.did >= 0 ? w * (a.data_val[in.did] - a.mu) : 0.0;
+        float l1 = isgrid ? (float)fabs(w) : 0.0f;
+#pragma unroll
+        for (int o = GS / 2; o > 0; o >>= 1) {
+            wc += __shfl_xor_sync(FULL_MASK, wc, o);
+            b0 += __shfl_xor_sync(FULL_MASK, b0, o);
+            l1 += __shfl_xor_sync(FULL_MASK, l1, o);
+        }
+        const double var = kriged ? sill - wc : sill;
+        const double sigma = sqrt(var > 0.0 ? var : 0.0);
+        const unsigned gb = (__ballot_sync(FULL_MASK, isgrid) >> (grp * GS)) & (0xffffffffu >> (32 - GS));
+        const int m = __popc(gb);
+        if (have) {
+            const int64_t row = table_row(tab, pos, k);
+            if (isgrid) {
+                const int j = __popc(gb & ((1u << q) - 1));
+                tab.idx[row + j] = id + (int32_t)a.node0;
+                put(tab.w, row + j, w);
+            }
+            if (q == 0) {
+                msum += m;
+                l1max = fmaxf(l1max, l1);
+                tab.node[pos] = g + (int32_t)a.node0;
+                tab.m[pos] = m;
+                put(tab.b0, pos, b0);
+                put(tab.sigma, pos, sigma);
+                a.status[g] = (int8_t)(n == 0 ? SGS_NODE_PRIOR_NMIN_ : (ok ? SGS_NODE_KRIGED_ : SGS_NODE_PRIOR_SINGULAR_));
+            }
+            if (a.w_full) {
+                for (int l = q; l < k; l += GS) a.w_full[(int64_t)g * k + l] = l == q && kriged && q < n ? w : 0.0;
+                if (q == 0) a.sigma_full[g] = sigma;
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        msum += __shfl_xor_sync(FULL_MASK, msum, o);
+        l1max = fmaxf(l1max, __shfl_xor_sync(FULL_MASK, l1max, o));
+    }
+    if (lane == 0) {
+        if (a.sum_m && msum) atomicAdd(a.sum_m, msum);
+        if (a.wl1_max && l1max > 0.0f) atomicMax(a.wl1_max, __float_as_uint(l1max));
+    }
+}
+
+template <int GS, typename O>
+static cudaError_t launch_solve64(const SolveArgs& a, const SweepTables<O>& t, cudaStream_t s) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const size_t smem = sizeof(Sys64<GS>) * SOLVE_WARPS;
+    cudaError_t e = cudaFuncSetAttribute(solve64_kernel<GS, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve64_kernel<GS, O>, SOLVE_WARPS * 32, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t full = (int64_t)nsm * std::max(per_sm, 1);
+    const int64_t per_block = SOLVE_WARPS * Sys64<GS>::SYS;
+    const int64_t want = a.list ? full : (a.P + per_block - 1) / per_block;
+    const int blocks = (int)std::max<int64_t>(1, std::min(want, full));
+    solve64_kernel<GS, O><<<blocks, SOLVE_WARPS * 32, smem, s>>>(a, t);
+    return cudaGetLastError();
+}
+
 template <typename T, typename O>
 static cudaError_t launch_solve(const SolveArgs& a, const SweepTables<O>& t, cudaStream_t s) {
+    // several systems share a warp (a lone one of 32 gains nothing: 27.8k took
+    // 1.56 ms in that form, 1.30 in this) and no category sums are wanted
+    if (a.k <= 16 && !a.ind_wsum) return a.k <= 8 ? launch_solve64<8, O>(a, t, s) : launch_solve64<16, O>(a, t, s);
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -362,8 +596,9 @@ cudaError_t launch_solve_fp64(const SolveArgs& a, const SweepTables<double>& t, 
 // compensated FP32 sum of (hi, lo) pairs and takes 2 instructions a term
 // instead of 13.  Weights, sigma^2 = sill (1 - w'c) and b0 are double-FP32 and
 // are written as (hi, lo) pairs for the compensated sweep.  A system with a
-// pivot below 1e-3 (near-singular: the canonical 1e-10 decision needs FP64),
-// a weight of 32 or more (the integer sums' range) or whose refinement does
+// pivot below 1e-3 (near-singular: the canonical 1e-10 decision needs FP64;
+// a datum on another neighbour's point is singular without one: 27.8k such of
+// 250k systems of 32 went through FP64 in 1.3 ms), a weight of 32 or more (the integer sums' range) or whose refinement does
 // not contract is queued for the FP64 kernel.
 //
 // Bound: latency and issue slots of 8 to 24 warps per SM (shared memory holds
@@ -424,6 +659,7 @@ struct Sys32 {
         int n[SYS], g[SYS], dom[SYS];
         unsigned short row[CHUNK];     // system << 6 | neighbour
         unsigned char place[SYS][NMAX];  // row of the matrix a neighbour stands in
+        unsigned char same[SYS];  // 1: a datum and another neighbour are one point
     };
     static constexpr int block_bytes = SYS * bytes + (int)sizeof(Shared);
 };
@@ -645,7 +881,7 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
     float* dinv = v2 + NMAX;
     const int k = a.k;
     const bool prior = n_all < a.nmin;        // fewer than minneighbors (or no system)
-    const int n = prior ? 0 : n_all;
+    int n = prior ? 0 : n_all;
     const int nw = max(n, __shfl_xor_sync(FULL_MASK, n, 16));  // warp-uniform
     int status = prior ? SGS_NODE_PRIOR_NMIN_ : SGS_NODE_KRIGED_;
     DF sigma = {a.sd_sill[0], a.sd_sill[1]};
@@ -786,6 +1022,7 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
         // ---- pairs with a datum: FP64, over the whole block ----
         if (l16 == 0) {
             sh.mask[sys] = dmask;
+            sh.same[sys] = 0;
             sh.n[sys] = n;
             sh.g[sys] = g;
             sh.dom[sys] = dom;
@@ -839,6 +1076,9 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
                     reinterpret_cast<KF*>(bh + S::K)[pd] = x;
                     *reinterpret_cast<KF*>(bh + S::at(pd, pd)) = {(int)KFIX, 0.0f};
                 } else {
+                    // Correlation 1: the variance of their difference, 2 (1 - K), bounds the
+                    // later one's pivot, which is then far below the singular rule's 1e-10.
+                    if (x.hi == (int)KFIX && fabsf(x.lo) <= 1e-12f) sh.same[es] = 1;
                     const int pq = sh.place[es][q], i = max(pq, pd), j = min(pq, pd);
                     *reinterpret_cast<KF*>(bh + S::at(i, j)) = x;
                     if ((i >> 2) == (j >> 2)) *reinterpret_cast<KF*>(bh + S::at(j, i)) = x;
@@ -846,6 +1086,7 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
             }
             __syncthreads();
         }
+        const bool singular = sh.same[sys];
         // ---- the FP32 LHS into registers (identity past the system) ----
         F2 A[tri2(NP)];
 #define SLOT(a_, b_) (((b_) & 1) ? f2_hi(A[tri2(a_) + (b_) / 2]) : f2_lo(A[tri2(a_) + (b_) / 2]))
@@ -934,7 +1175,7 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
         float sr[NR], sd[NR];
 #pragma unroll
         for (int s = 0; s < NR; ++s) sr[s] = sd[s] = 0.0f;
-        bool early = false, done = n == 0;  // half-uniform
+        bool early = false, done = n == 0 || singular;  // half-uniform
         float x[NR];
         if (warm) {
 #pragma unroll
@@ -1188,6 +1429,11 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
             }
         }
         const DF wc = half_sum_df(acc.value());
+        if (singular) {
+            accept = true;
+            status = SGS_NODE_PRIOR_SINGULAR_;
+            n = 0;
+        }
         if (n > 0) sigma = df_mul(sigma, df_sqrt(df_add({1.0f, 0.0f}, df_neg(wc))));
         __syncwarp();
         if (live && !accept && l16 == 0) a.fallback[atomicAdd(a.nfallback, 1)] = (int32_t)pos;
