@@ -12,13 +12,20 @@
 // values, row stride >= R, float or double, centred), and `offset` (the
 // process mean) is added to every value.
 //
-// One warp per node; sums in FP64; the quantile kernel sorts each row in
-// shared memory (bitonic, R <= 1024).  Nothing is allocated: the threshold
-// and probability lists (at most 32 per launch) travel in the kernel
-// parameters, and the host wrapper launches once per 32 of them.
+// FP64 values: one warp per node, sums in FP64, quantiles by a sort in shared
+// memory (bitonic, R <= 1024).  Rows of float, which the FP32 sweep writes,
+// have forms of their own below that keep off the FP64 pipe (a warp FP64
+// instruction holds its scheduler for 64 cycles): exact sums in integers,
+// sorting networks in registers, thresholds moved to the floats between which
+// they fall.  1M nodes x 100 float values, one GB300: mean and variance 4.57
+// -> 0.22 ms, 3 quantiles 4.36 -> 0.30, 3 thresholds 1.79 -> 0.11 (0.06 each
+// to read).  Nothing is allocated: the threshold and probability lists (at
+// most 32 per launch) travel in the kernel parameters, and the host wrapper
+// launches once per 32 of them.
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 
 #include "common.cuh"
 
@@ -38,7 +45,10 @@ struct EnsArgs {
     int nlist;         // entries of `list` used
     int list_stride;   // output row length (all entries of the full list)
     int list0;         // first output column of this launch
-    double list[ENS_LIST];
+    double list[ENS_LIST];   // thresholds or probabilities; float rows' quantiles: the
+                             // weight of the upper order statistic, whose lower one is lo
+    float tf[ENS_LIST];      // float rows: thresholds as floats
+    int lo[ENS_LIST];
 };
 
 __device__ __forceinline__ double ens_val(const EnsArgs& a, int64_t g, int r) {
@@ -138,6 +148,265 @@ __global__ void __launch_bounds__(ENS_WARPS * 32) ens_quantile_kernel(const EnsA
     }
 }
 
+// ---- rows of float ----
+// LPN lanes per node (8, or 32 for long rows), 32 / LPN nodes per warp; lane q
+// holds the values q, q + LPN, ... of the row, V of them at most.
+template <int LPN, int V>
+__device__ __forceinline__ void ens_load(const float* __restrict__ row, int R, int q, bool in, float pad, float (&x)[V]) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) x[i] = in && i * LPN + q < R ? row[i * LPN + q] : pad;
+}
+
+template <int LPN>
+__device__ __forceinline__ long long ens_group_sum(long long v) {
+#pragma unroll
+    for (int o = LPN / 2; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+    return v;
+}
+
+template <int LPN>
+__device__ __forceinline__ double ens_group_sum(double v) {
+#pragma unroll
+    for (int o = LPN / 2; o > 0; o >>= 1) v += __shfl_xor_sync(FULL_MASK, v, o);
+    return v;
+}
+
+// What a node's sums are, until 32 nodes are finished together.
+struct EnsSums {
+    long long s, c, hh, hl, ll;
+    int e;  // ENS_DONE: s and hh hold the mean and the sum of squares (FP64)
+};
+constexpr int ENS_DONE = INT_MIN;
+constexpr int ENS_FIXED_MAX = 512;  // values of a row in the integer form
+
+// Mean and variance in integers.  With |x| < 2^e over a row, X = x 2^(51 - e)
+// is an integer (values below 2^-27 of the largest are rounded to it), sums of
+// at most 512 of them are exact, and so are the three partial sums of the
+// squares of X - M, M an integer near the mean, taken as 26-bit halves:
+// sum (X - M)^2 = hh 2^52 + 2 hl 2^26 + ll.  The variance is the sum less
+// (sum (X - M))^2 / R.  FP64 is left to the last dozen operations, for 32
+// nodes at a time.  Rows with infinities, NaN or magnitudes beyond 2^60 or
+// below 2^-60 are summed in FP64.
+template <int LPN, int V>
+__global__ void __launch_bounds__(ENS_WARPS * 32) ens_stats_fixed_kernel(const EnsArgs a, int rounds, double* mean,
+                                                                         double* var) {
+    __shared__ EnsSums s_sum[ENS_WARPS][32];
+    EnsSums* sum = s_sum[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, grp = lane / LPN, q = lane % LPN;
+    constexpr int NPW = 32 / LPN;
+    const float* vals = reinterpret_cast<const float*>(a.vals);
+    const int span = rounds * NPW;  // nodes a warp finishes together
+    const int64_t step = (int64_t)gridDim.x * ENS_WARPS * span;
+    const float rinv = 1.0f / (float)a.R;
+    for (int64_t g0 = ((int64_t)blockIdx.x * ENS_WARPS + (threadIdx.x >> 5)) * span; g0 < a.N; g0 += step) {
+        for (int it = 0; it < rounds; ++it) {
+            const int64_t g = g0 + it * NPW + grp;
+            const float* row = vals + g * a.stride;
+            float x[V];
+            ens_load<LPN, V>(row, a.R, q, g < a.N, 0.0f, x);
+            unsigned mx = 0;
+#pragma unroll
+            for (int i = 0; i < V; ++i) mx = max(mx, __float_as_uint(x[i]) & 0x7fffffffu);
+#pragma unroll
+            for (int o = LPN / 2; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+            const int e = mx ? (int)(mx >> 23) - 126 : 0;
+            const bool fixed = e >= -60 && e <= 60;
+            const float sc = __uint_as_float((unsigned)(127 + 25 - (fixed ? e : 0)) << 23);
+            long long X[V], s = 0;
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                const float y = __fmul_rn(x[i], sc);
+                const int h = __float2int_rn(y);
+                const int l = __float2int_rn(__fmul_rn(__fadd_rn(y, -__int2float_rn(h)), 67108864.0f));
+                X[i] = (long long)h * (1 << 26) + l;
+                s += X[i];
+            }
+            s = ens_group_sum<LPN>(s);
+            const long long M = __float2ll_rn(__fmul_rn((float)s, rinv));
+            long long hh = 0, hl = 0, ll = 0;
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                const long long d = i * LPN + q < a.R ? X[i] - M : 0;
+                const int dh = (int)(d >> 26), dl = (int)d & ((1 << 26) - 1);
+                hh += (long long)dh * dh;
+                hl += (long long)dh * dl;
+                ll += (long long)dl * dl;
+            }
+            hh = ens_group_sum<LPN>(hh);
+            hl = ens_group_sum<LPN>(hl);
+            ll = ens_group_sum<LPN>(ll);
+            if (q == 0) sum[it * NPW + grp] = {s, s - a.R * M, hh, hl, ll, e};
+            if (__any_sync(FULL_MASK, !fixed)) {
+                double t = 0.0;
+#pragma unroll 1
+                for (int r = q; r < a.R && g < a.N; r += LPN) t += ens_val(a, g, r);
+                const double m = ens_group_sum<LPN>(t) / a.R;
+                t = 0.0;
+#pragma unroll 1
+                for (int r = q; r < a.R && g < a.N; r += LPN) {
+                    const double d = ens_val(a, g, r) - m;
+                    t += d * d;
+                }
+                t = ens_group_sum<LPN>(t);
+                if (!fixed && q == 0)
+                    sum[it * NPW + grp] = {__double_as_longlong(m), 0, __double_as_longlong(t), 0, 0, ENS_DONE};
+            }
+        }
+        __syncwarp();
+        const int64_t g = g0 + lane;
+        if (lane < span && g < a.N) {
+            const EnsSums v = sum[lane];
+            double m, t;
+            if (v.e == ENS_DONE) {
+                m = __longlong_as_double(v.s);
+                t = __longlong_as_double(v.hh);
+            } else {
+                const double u = __hiloint2double((1023 + v.e - 51) << 20, 0);
+                m = (double)v.s / a.R * u + a.offset;
+                t = fma((double)v.hh, 4503599627370496.0, fma((double)v.hl, 134217728.0, (double)v.ll));
+                const double c = (double)v.c;
+                t = fmax(t - c * c / a.R, 0.0) * (u * u);
+            }
+            if (mean) mean[g] = m;
+            if (var) var[g] = a.R > 1 ? t / (a.R - 1) : nan("");
+        }
+        __syncwarp();
+    }
+}
+
+// count(x <= t) or, complement, count(x > t) of the floats t in tf: the
+// largest for which t + offset <= threshold still holds.
+template <int LPN, int LIST>
+__global__ void __launch_bounds__(ENS_WARPS * 32) ens_cdf_float_kernel(const __grid_constant__ EnsArgs a, int complement,
+                                                                       double* out) {
+    extern __shared__ double s_frac[];  // c / R
+    for (int c = threadIdx.x; c <= a.R; c += ENS_WARPS * 32) s_frac[c] = (double)c / a.R;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, grp = lane / LPN, q = lane % LPN;
+    constexpr int NPW = 32 / LPN;
+    const float* vals = reinterpret_cast<const float*>(a.vals);
+    float tf[LIST];
+#pragma unroll
+    for (int i = 0; i < LIST; ++i) tf[i] = a.tf[i];
+    const int64_t step = (int64_t)gridDim.x * ENS_WARPS * NPW;
+    for (int64_t g0 = ((int64_t)blockIdx.x * ENS_WARPS + (threadIdx.x >> 5)) * NPW; g0 < a.N; g0 += step) {
+        const int64_t g = g0 + grp;
+        const float* row = vals + g * a.stride;
+        int cnt[LIST];
+#pragma unroll
+        for (int i = 0; i < LIST; ++i) cnt[i] = 0;
+        if (g < a.N)
+#pragma unroll 4
+            for (int r = q; r < a.R; r += LPN) {
+                const float x = row[r];
+#pragma unroll
+                for (int i = 0; i < LIST; ++i) cnt[i] += complement ? x > tf[i] : x <= tf[i];
+            }
+#pragma unroll
+        for (int o = LPN / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < LIST; ++i) cnt[i] += __shfl_xor_sync(FULL_MASK, cnt[i], o);
+        if (g < a.N)
+            for (int i = q; i < a.nlist; i += LPN) {
+                int c = 0;
+#pragma unroll
+                for (int j = 0; j < LIST; ++j)
+                    if (j == i) c = cnt[j];
+                out[g * a.list_stride + a.list0 + i] = s_frac[c];
+            }
+    }
+}
+
+// order-preserving integer of a float (NaN with a clear sign last) and back
+__device__ __forceinline__ int ens_key(float x) {
+    const int b = __float_as_int(x);
+    return b ^ ((b >> 31) & 0x7fffffff);
+}
+
+// Quantiles: each row sorted in registers, V keys a lane, by merges that
+// compare i with its mirror image in the merged run first (so that every
+// comparison keeps the smaller key at the smaller index) and then at halved
+// distances; only the last log2(LPN) distances of a merge cross lanes.
+template <int LPN, int V>
+__global__ void __launch_bounds__(ENS_WARPS * 32) ens_quantile_float_kernel(const __grid_constant__ EnsArgs a,
+                                                                            double* out) {
+    extern __shared__ int s_keys[];
+    const int lane = threadIdx.x & 31, grp = lane / LPN, q = lane % LPN;
+    constexpr int NPW = 32 / LPN, P = LPN * V;
+    int* sorted = s_keys + (size_t)(threadIdx.x >> 5) * (NPW * (P + 4));
+    const float* vals = reinterpret_cast<const float*>(a.vals);
+    const int64_t step = (int64_t)gridDim.x * ENS_WARPS * NPW;
+    for (int64_t g0 = ((int64_t)blockIdx.x * ENS_WARPS + (threadIdx.x >> 5)) * NPW; g0 < a.N; g0 += step) {
+        const int64_t g = g0 + grp;
+        float x[V];
+        ens_load<LPN, V>(vals + g * a.stride, a.R, q, g < a.N, 0.0f, x);
+        int key[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) key[i] = i * LPN + q < a.R ? ens_key(x[i]) : INT_MAX;
+        auto order = [&](int i, int j) {
+            const int lo = min(key[i], key[j]), hi = max(key[i], key[j]);
+            key[i] = lo;
+            key[j] = hi;
+        };
+        // runs within a lane
+#pragma unroll
+        for (int size = 2; size <= V; size <<= 1) {
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+                if ((i & (size / 2)) == 0) order(i, i ^ (size - 1));
+#pragma unroll
+            for (int d = size / 4; d > 0; d >>= 1)
+#pragma unroll
+                for (int i = 0; i < V; ++i)
+                    if ((i & d) == 0) order(i, i ^ d);
+        }
+        // runs across lanes
+#pragma unroll
+        for (int size = 2; size <= LPN; size <<= 1) {  // lanes merged
+            {
+                const bool low = (q & (size / 2)) == 0;
+                int y[V];
+#pragma unroll
+                for (int i = 0; i < V; ++i) y[i] = __shfl_xor_sync(FULL_MASK, key[V - 1 - i], size - 1);
+#pragma unroll
+                for (int i = 0; i < V; ++i) key[i] = (y[i] < key[i]) == low ? y[i] : key[i];
+            }
+#pragma unroll
+            for (int d = size / 4; d > 0; d >>= 1) {
+                const bool low = (q & d) == 0;
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    const int y = __shfl_xor_sync(FULL_MASK, key[i], d);
+                    key[i] = (y < key[i]) == low ? y : key[i];
+                }
+            }
+#pragma unroll
+            for (int d = V / 2; d > 0; d >>= 1)
+#pragma unroll
+                for (int i = 0; i < V; ++i)
+                    if ((i & d) == 0) order(i, i ^ d);
+        }
+#pragma unroll
+        for (int i = 0; i < V; i += 4)
+            *reinterpret_cast<int4*>(sorted + grp * (P + 4) + q * V + i) = make_int4(key[i], key[i + 1], key[i + 2], key[i + 3]);
+        __syncwarp();
+        for (int t = lane; t < NPW * a.nlist; t += 32) {
+            const int gi = t / a.nlist, i = t - gi * a.nlist;
+            if (g0 + gi < a.N) {
+                const int* srt = sorted + gi * (P + 4);
+                const int lo = a.lo[i], hi = min(lo + 1, a.R - 1);
+                auto value = [&](int p) {
+                    const int b = srt[p];
+                    return (double)__int_as_float(b ^ ((b >> 31) & 0x7fffffff)) + a.offset;
+                };
+                const double vl = value(lo);
+                out[(g0 + gi) * a.list_stride + a.list0 + i] = vl + a.list[i] * (value(hi) - vl);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 }  // namespace sgs
 
 using namespace sgs;
@@ -171,6 +440,35 @@ int ens_grid(int64_t N) {
     return (int)std::max<int64_t>(1, std::min(want, cap));
 }
 
+// nodes one warp finishes together (in rounds of npw), fewer where that would
+// leave warps without work
+int ens_rounds(int64_t N, int lpn) {
+    const int npw = 32 / lpn;
+    const int64_t warps = (int64_t)ens_grid(INT64_MAX / 2) * ENS_WARPS;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(lpn, N / (npw * warps)));
+}
+
+// The largest float t with (double)t + offset <= x: (double)t + offset does
+// not decrease with t, so x <= threshold can be decided on floats.  NaN where
+// nothing compares (x is NaN).
+float ens_threshold(double x, double offset) {
+    if (std::isnan(x)) return NAN;
+    auto value = [](int64_t k) {  // k-th float from -inf = 0 upward
+        int32_t b = (int32_t)(k - 0x7f800000);
+        b = b < 0 ? (int32_t)(0x80000000u | (uint32_t)-(int64_t)b) : b;
+        float f;
+        std::memcpy(&f, &b, sizeof(f));
+        return f;
+    };
+    int64_t lo = 0, hi = 2 * (int64_t)0x7f800000;  // -inf + offset <= x always holds
+    while (lo < hi) {
+        const int64_t mid = (lo + hi + 1) / 2;
+        if ((double)value(mid) + offset <= x) lo = mid;
+        else hi = mid - 1;
+    }
+    return value(lo);
+}
+
 int ens_done(cudaError_t e, const char* where) {
     if (e != cudaSuccess) {
         sgs::set_thread_error(std::string(where) + ": " + cudaGetErrorString(e));
@@ -188,7 +486,17 @@ extern "C" int sgs_ensemble_stats(const void* vals, int32_t precision, int64_t n
     if (rc) return rc;
     if (!mean && !var) return ens_fail(SGS_ERR_ARG, "no output");
     if (nnodes == 0) return SGS_OK;
-    ens_stats_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, 0, (cudaStream_t)stream>>>(a, mean, var);
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (!a.fp64 && nreals <= ENS_FIXED_MAX && std::isfinite(offset)) {
+        const int lpn = nreals <= 128 ? 8 : 32;
+        const int rounds = ens_rounds(nnodes, lpn);
+        const int grid = ens_grid((nnodes + rounds * (32 / lpn) - 1) / (rounds * (32 / lpn)));
+        if (nreals <= 32) ens_stats_fixed_kernel<8, 4><<<grid, ENS_WARPS * 32, 0, st>>>(a, rounds, mean, var);
+        else if (nreals <= 128) ens_stats_fixed_kernel<8, 16><<<grid, ENS_WARPS * 32, 0, st>>>(a, rounds, mean, var);
+        else ens_stats_fixed_kernel<32, 16><<<grid, ENS_WARPS * 32, 0, st>>>(a, rounds, mean, var);
+    } else {
+        ens_stats_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, 0, st>>>(a, mean, var);
+    }
     return ens_done(cudaGetLastError(), "sgs_ensemble_stats");
 }
 
@@ -205,7 +513,19 @@ extern "C" int sgs_ensemble_cdf(const void* vals, int32_t precision, int64_t nno
         a.list0 = i0;
         a.nlist = std::min(ENS_LIST, nx - i0);
         for (int i = 0; i < a.nlist; ++i) a.list[i] = x[i0 + i];
-        ens_cdf_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, 0, (cudaStream_t)stream>>>(a, complement ? 1 : 0, out);
+        const cudaStream_t st = (cudaStream_t)stream;
+        if (!a.fp64 && nreals <= ENS_RMAX && std::isfinite(offset)) {
+            for (int i = 0; i < ENS_LIST; ++i) a.tf[i] = i < a.nlist ? ens_threshold(a.list[i], offset) : 0.0f;
+            const size_t smem = (size_t)(nreals + 1) * sizeof(double);
+            const int lpn = nreals <= 128 ? 8 : 32;
+            const int grid = ens_grid((nnodes + 32 / lpn - 1) / (32 / lpn)), c = complement ? 1 : 0;
+            if (lpn == 8 && a.nlist <= 4) ens_cdf_float_kernel<8, 4><<<grid, ENS_WARPS * 32, smem, st>>>(a, c, out);
+            else if (lpn == 8) ens_cdf_float_kernel<8, ENS_LIST><<<grid, ENS_WARPS * 32, smem, st>>>(a, c, out);
+            else if (a.nlist <= 4) ens_cdf_float_kernel<32, 4><<<grid, ENS_WARPS * 32, smem, st>>>(a, c, out);
+            else ens_cdf_float_kernel<32, ENS_LIST><<<grid, ENS_WARPS * 32, smem, st>>>(a, c, out);
+        } else {
+            ens_cdf_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, 0, st>>>(a, complement ? 1 : 0, out);
+        }
         if ((rc = ens_done(cudaGetLastError(), "sgs_ensemble_cdf"))) return rc;
     }
     return SGS_OK;
@@ -222,18 +542,38 @@ extern "C" int sgs_ensemble_quantile(const void* vals, int32_t precision, int64_
     for (int i = 0; i < np; ++i)
         if (!(p[i] >= 0.0 && p[i] <= 1.0)) return ens_fail(SGS_ERR_ARG, "probabilities must be in [0, 1]");
     if (nnodes == 0) return SGS_OK;
+    a.list_stride = np;
+    const cudaStream_t st = (cudaStream_t)stream;
     int P = 1;
     while (P < nreals) P <<= 1;
-    const size_t smem = (size_t)ENS_WARPS * P * sizeof(double);
-    if ((rc = ens_done(cudaFuncSetAttribute(ens_quantile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem), "sgs_ensemble_quantile")))
-        return rc;
-    a.list_stride = np;
     for (int i0 = 0; i0 < np; i0 += ENS_LIST) {
         a.list0 = i0;
         a.nlist = std::min(ENS_LIST, np - i0);
         for (int i = 0; i < a.nlist; ++i) a.list[i] = p[i0 + i];
-        ens_quantile_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, smem, (cudaStream_t)stream>>>(a, out);
+        if (a.fp64) {
+            const size_t smem = (size_t)ENS_WARPS * P * sizeof(double);
+            if ((rc = ens_done(cudaFuncSetAttribute(ens_quantile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)smem), "sgs_ensemble_quantile")))
+                return rc;
+            ens_quantile_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, smem, st>>>(a, out);
+        } else {
+            for (int i = 0; i < a.nlist; ++i) {
+                const double h = (a.R - 1) * a.list[i], fl = std::floor(h);
+                a.lo[i] = std::min(std::max((int)fl, 0), a.R - 1);
+                a.list[i] = h - fl;
+            }
+            auto launch = [&](auto kernel, int lpn, int v) {
+                const int npw = 32 / lpn;
+                const size_t smem = (size_t)ENS_WARPS * npw * (lpn * v + 4) * sizeof(int);
+                kernel<<<ens_grid((nnodes + npw - 1) / npw), ENS_WARPS * 32, smem, st>>>(a, out);
+            };
+            if (nreals <= 32) launch(ens_quantile_float_kernel<8, 4>, 8, 4);
+            else if (nreals <= 64) launch(ens_quantile_float_kernel<8, 8>, 8, 8);
+            else if (nreals <= 128) launch(ens_quantile_float_kernel<8, 16>, 8, 16);
+            else if (nreals <= 256) launch(ens_quantile_float_kernel<32, 8>, 32, 8);
+            else if (nreals <= 512) launch(ens_quantile_float_kernel<32, 16>, 32, 16);
+            else launch(ens_quantile_float_kernel<32, 32>, 32, 32);
+        }
         if ((rc = ens_done(cudaGetLastError(), "sgs_ensemble_quantile"))) return rc;
     }
     return SGS_OK;
