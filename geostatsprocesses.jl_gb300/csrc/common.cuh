@@ -230,6 +230,30 @@ __device__ __forceinline__ float4 normals4(uint64_t seed, int64_t g, int q) {
     return make_float4(r0 * c0, r0 * s0, r1 * c1, r1 * s1);
 }
 
+// two FP32 values in one 64-bit register pair; fma.rn.f32x2 is one
+// instruction for both
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+    F2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float f2_lo(F2 v) {
+    float lo;
+    asm("mov.b64 {%0, _}, %1;" : "=f"(lo) : "l"(v));
+    return lo;
+}
+__device__ __forceinline__ float f2_hi(F2 v) {
+    float hi;
+    asm("mov.b64 {_, %0}, %1;" : "=f"(hi) : "l"(v));
+    return hi;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 // ---- double-FP32 ("float-float") arithmetic: a value is an unevaluated sum
 // hi + lo of two floats, |lo| <= ulp(hi)/2, about 48 significant bits.  Error-
 // free transformations after Knuth (TwoSum), Dekker (Fast2Sum) and the FMA

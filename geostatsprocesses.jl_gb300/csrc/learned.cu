@@ -14,6 +14,8 @@
 // the mean squared error of y against the weights the method's own solver
 // produced.  One warp per system throughout; parameters live in shared
 // memory.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sgs {
@@ -179,132 +181,327 @@ __global__ void __launch_bounds__(NN_WARPS * 32) nn_forward_kernel(const float* 
 }
 
 // Loss and gradients of a batch: every system adds its mean squared error
-// to *loss and its gradient to grad (accumulated per block in shared memory,
-// then once per block into global memory).
-__global__ void __launch_bounds__(NN_WARPS * 32) nn_backward_kernel(const float* __restrict__ params,
-                                                                    const float* __restrict__ feat,
-                                                                    const int32_t* __restrict__ count,
-                                                                    const float* __restrict__ target, int64_t nsys,
-                                                                    int k, float* grad, float* loss) {
+// to *loss and its gradient to grad.
+//
+// One warp per system, its neighbours in chunks of 32 rows.  All products are
+// 32 x 32 (or x 8) tiles of the warp, 4 x 8 of them per lane, one step of the
+// inner dimension taking 3 shared-memory loads for 32 FP32 multiply-adds (16
+// instructions): H = F W1', Z = H W2a', dW2a = dZ' H, dH = dZ W2a, dW1 = dZ1'
+// F.  The matrices a step reads along both dimensions are kept in both orders.
+// The gradients of the weights stay in registers over all systems of a warp,
+// are added up per block in shared memory and once per block in global
+// memory.  Bound: FP32 issue and shared-memory loads of 12 warps per SM (what
+// shared memory holds).  Shared-memory sums with one neighbour per lane, 32
+// lanes adding to one bank, took 16,384 systems of 32 neighbours 0.66 ms; this
+// 0.13.
+constexpr int NN_LDT = 36;               // tile row: 16-byte aligned, 8 rows of 4 on different banks
+constexpr int NN_TILE = 32 * NN_LDT;
+
+template <int NC>  // chunks of 32 neighbours
+struct NNTiles {
+    static constexpr int WARPS = 12 / NC;
+    struct alignas(16) Warp {
+        float H[NC][NN_TILE];    // h, [neighbour][unit]
+        float T[NC][NN_TILE];    // h, then dz2, [unit][neighbour]
+        float Z[NC][NN_TILE];    // dz2, then dz1, [neighbour][unit]
+        float F[NC][32 * NNF];   // features, [neighbour][feature]
+        float FT[NNF * NN_LDT];  // of one chunk, [feature][neighbour]
+        float g[32], u[32], sz[32], dg[32];
+    };
+    float W1T[NNF * NN_LDT], W2A[NN_TILE], W2AT[NN_TILE], W2B[NN_TILE], W2BT[NN_TILE];
+    float b1[32], b2[32], w3[32], b3[4], warp_loss[16];
+    Warp warp[WARPS];
+    static_assert(sizeof(Warp) % 16 == 0 && NN_TILE % 4 == 0 && WARPS <= 16, "16-byte loads");
+};
+
+// acc[r][p] += A[r] B[2p, 2p + 1], r < 4, p < 4
+__device__ __forceinline__ void nn_step(F2 (&acc)[4][4], const float* A, const float* B) {
+    const float4 a = *reinterpret_cast<const float4*>(A);
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(B), y = *reinterpret_cast<const ulonglong2*>(B + 4);
+    const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const F2 s = f2_pack(av[r], av[r]);
+        acc[r][0] = f2_fma(s, x.x, acc[r][0]);
+        acc[r][1] = f2_fma(s, x.y, acc[r][1]);
+        acc[r][2] = f2_fma(s, y.x, acc[r][2]);
+        acc[r][3] = f2_fma(s, y.y, acc[r][3]);
+    }
+}
+
+__device__ __forceinline__ void nn_load8(const float* p, F2 (&v)[4]) {
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(p), y = *reinterpret_cast<const ulonglong2*>(p + 4);
+    v[0] = x.x, v[1] = x.y, v[2] = y.x, v[3] = y.y;
+}
+
+__device__ __forceinline__ void nn_store8(float* p, const F2 (&v)[4]) {
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]);
+    *reinterpret_cast<ulonglong2*>(p + 4) = make_ulonglong2(v[2], v[3]);
+}
+
+// the lane's tile by columns: X[unit][neighbours]
+__device__ __forceinline__ void nn_store_t(float* X, const F2 (&t)[4][4]) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        *reinterpret_cast<float4*>(X + (2 * p) * NN_LDT) = make_float4(f2_lo(t[0][p]), f2_lo(t[1][p]), f2_lo(t[2][p]), f2_lo(t[3][p]));
+        *reinterpret_cast<float4*>(X + (2 * p + 1) * NN_LDT) =
+            make_float4(f2_hi(t[0][p]), f2_hi(t[1][p]), f2_hi(t[2][p]), f2_hi(t[3][p]));
+    }
+}
+
+// sums over the 8 lanes that hold the same units
+__device__ __forceinline__ void nn_sum_rows(F2 (&v)[4]) {
+    const F2 one = f2_pack(1.0f, 1.0f);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) v[p] = f2_fma(one, __shfl_xor_sync(FULL_MASK, v[p], o), v[p]);
+}
+
+template <int NC>
+__global__ void __launch_bounds__(NNTiles<NC>::WARPS * 32, 1)
+nn_backward_kernel(const float* __restrict__ params, const float* __restrict__ feat, const int32_t* __restrict__ count,
+                   const float* __restrict__ target, int64_t nsys, int k, float* grad, float* loss) {
     extern __shared__ __align__(16) unsigned char raw[];
-    NNSmem& S = *reinterpret_cast<NNSmem*>(raw);
-    float* G = reinterpret_cast<float*>(raw + sizeof(NNSmem));  // block gradient [NN_PARAMS]
-    for (int i = threadIdx.x; i < NN_PARAMS; i += blockDim.x) {
-        S.P[i] = params[i];
-        G[i] = 0.0f;
+    using S = NNTiles<NC>;
+    S& sh = *reinterpret_cast<S*>(raw);
+    const int lane = threadIdx.x & 31, ri = lane >> 2, ui = lane & 3;
+    typename S::Warp& w = sh.warp[threadIdx.x >> 5];
+    for (int i = threadIdx.x; i < NNH * NNH; i += S::WARPS * 32) {
+        const int a = i / NNH, b = i % NNH;
+        sh.W2A[a * NN_LDT + b] = sh.W2AT[b * NN_LDT + a] = params[NN_W2A + i];
+        sh.W2B[a * NN_LDT + b] = sh.W2BT[b * NN_LDT + a] = params[NN_W2B + i];
+        if (i < NNH * NNF) sh.W1T[(i % NNF) * NN_LDT + i / NNF] = params[NN_W1 + i];
+        if (i < NNH) {
+            sh.b1[i] = params[NN_B1 + i];
+            sh.b2[i] = params[NN_B2 + i];
+            sh.w3[i] = params[NN_W3 + i];
+        }
+        if (i == 0) sh.b3[0] = params[NN_B3];
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    float* Hs = S.Hs[wib];
-    float* Qs = S.Qs[wib];
-    float* gs = S.gs[wib];
-    float* us = S.us[wib];
-    const int64_t nw = (int64_t)gridDim.x * NN_WARPS;
-    float block_loss = 0.0f;
-    for (int64_t s = (int64_t)blockIdx.x * NN_WARPS + wib; s < nsys; s += nw) {
+    const bool vec = (reinterpret_cast<uintptr_t>(feat) & 15) == 0;
+    const F2 one = f2_pack(1.0f, 1.0f);
+    F2 dw2a[4][4], dw2b[4][4], dw1[4], dw3[4], db1[4], db2[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) dw2a[r][p] = dw2b[r][p] = 0;
+        dw1[r] = dw3[r] = db1[r] = db2[r] = 0;
+    }
+    float db3 = 0.0f, total = 0.0f;
+    const int64_t nw = (int64_t)gridDim.x * S::WARPS;
+    for (int64_t s = (int64_t)blockIdx.x * S::WARPS + (threadIdx.x >> 5); s < nsys; s += nw) {
         const int n = min(count[s], k);
         if (n <= 0) continue;
-        const float* f = feat + s * k * NNF;
-        float y[2];
-        nn_forward_warp(S.P, f, n, Hs, Qs, gs, us, lane, y);
-        // dL/dy_i = 2 (y_i - t_i) / n, kept per lane; squared error to the loss
-        float dy[2] = {0.f, 0.f}, l2 = 0.0f;
-        for (int t = 0; t < 2; ++t) {
-            const int i = lane + 32 * t;
-            if (i < n) {
-                const float e = y[t] - target[s * k + i];
-                dy[t] = 2.0f * e / (float)n;
-                l2 += e * e;
-            }
-        }
+        const float inv_n = 1.0f / (float)n;
+        // ---- h = relu(W1 f + b1), its mean ----
+        F2 sum[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(FULL_MASK, l2, o);
-        block_loss += l2 / (float)n;
-        // output layer: dw3, db3; dz2_i = dy_i w3 (q_i > 0), stored over Qs
-        // after its use (each lane owns its rows)
-        float dyw[2] = {dy[0], dy[1]};
-        __shared__ float dys[NN_WARPS][64];
-        for (int t = 0; t < 2; ++t) {
-            const int i = lane + 32 * t;
-            if (i < 64) dys[wib][i] = i < n ? dyw[t] : 0.0f;
-        }
-        __syncwarp();
-        {
-            // lane a: dw3[a] = sum_i dy_i q_ia
-            float acc = 0.0f;
-            for (int i = 0; i < n; ++i) acc = fmaf(dys[wib][i], Qs[i * NN_LD + lane], acc);
-            atomicAdd(&G[NN_W3 + lane], acc);
-            if (lane == 0) {
-                float sdy = 0.0f;
-                for (int i = 0; i < n; ++i) sdy += dys[wib][i];
-                atomicAdd(&G[NN_B3], sdy);
-            }
-        }
-        __syncwarp();
-        for (int t = 0; t < 2; ++t) {
-            const int i = lane + 32 * t;
+        for (int c = 0; c < NC; ++c) {
+            if (32 * c >= n) break;
+            const int i = 32 * c + lane;
+            float f[NNF];
+#pragma unroll
+            for (int j = 0; j < NNF; ++j) f[j] = 0.0f;
             if (i < n) {
-                for (int a = 0; a < NNH; ++a) {
-                    const float q = Qs[i * NN_LD + a];
-                    Qs[i * NN_LD + a] = q > 0.0f ? dyw[t] * S.P[NN_W3 + a] : 0.0f;  // dz2
+                const float* fp = feat + (s * k + i) * NNF;
+                if (vec) {
+                    const float4 x = reinterpret_cast<const float4*>(fp)[0], y = reinterpret_cast<const float4*>(fp)[1];
+                    f[0] = x.x, f[1] = x.y, f[2] = x.z, f[3] = x.w, f[4] = y.x, f[5] = y.y, f[6] = y.z, f[7] = y.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < NNF; ++j) f[j] = fp[j];
                 }
             }
-        }
-        __syncwarp();
-        // lane a owns row a of W2a / W2b: dW2a[a][b] = sum_i dz2_ia h_ib
-        float sz = 0.0f;
-        for (int i = 0; i < n; ++i) sz += Qs[i * NN_LD + lane];
-        for (int b = 0; b < NNH; ++b) {
-            float acc = 0.0f;
-            for (int i = 0; i < n; ++i) acc = fmaf(Qs[i * NN_LD + lane], Hs[i * NN_LD + b], acc);
-            atomicAdd(&G[NN_W2A + lane * NNH + b], acc);
-            atomicAdd(&G[NN_W2B + lane * NNH + b], sz * gs[b]);
-        }
-        atomicAdd(&G[NN_B2 + lane], sz);
-        // dg[b] = sum_a W2b[a][b] sz_a  (lane b); reuse us for dg / n
-        us[lane] = sz;
-        __syncwarp();
-        float dg = 0.0f;
-        for (int a = 0; a < NNH; ++a) dg = fmaf(S.P[NN_W2B + a * NNH + lane], us[a], dg);
-        __syncwarp();
-        gs[lane] = dg / (float)n;
-        __syncwarp();
-        // dh_i[b] = sum_a W2a[a][b] dz2_ia + dg_b / n; dz1 = dh (h > 0), over Hs
-        for (int t = 0; t < 2; ++t) {
-            const int i = lane + 32 * t;
-            if (i < n) {
-                float dh[NNH];
+            *reinterpret_cast<float4*>(&w.F[c][lane * NNF]) = make_float4(f[0], f[1], f[2], f[3]);
+            *reinterpret_cast<float4*>(&w.F[c][lane * NNF + 4]) = make_float4(f[4], f[5], f[6], f[7]);
 #pragma unroll
-                for (int b = 0; b < NNH; ++b) dh[b] = gs[b];
-                for (int a = 0; a < NNH; ++a) {
-                    const float z = Qs[i * NN_LD + a];
+            for (int j = 0; j < NNF; ++j) w.FT[j * NN_LDT + lane] = f[j];
+            __syncwarp();
+            F2 h[4][4];
+            nn_load8(sh.b1 + 8 * ui, h[0]);
 #pragma unroll
-                    for (int b = 0; b < NNH; ++b) dh[b] = fmaf(S.P[NN_W2A + a * NNH + b], z, dh[b]);
+            for (int p = 0; p < 4; ++p) h[1][p] = h[2][p] = h[3][p] = h[0][p];
+#pragma unroll
+            for (int j = 0; j < NNF; ++j) nn_step(h, w.FT + j * NN_LDT + 4 * ri, sh.W1T + j * NN_LDT + 8 * ui);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const bool in = 32 * c + 4 * ri + r < n;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    h[r][p] = in ? f2_pack(fmaxf(f2_lo(h[r][p]), 0.0f), fmaxf(f2_hi(h[r][p]), 0.0f)) : 0;
+                    sum[p] = f2_fma(one, h[r][p], sum[p]);
                 }
-#pragma unroll
-                for (int b = 0; b < NNH; ++b) Hs[i * NN_LD + b] = Hs[i * NN_LD + b] > 0.0f ? dh[b] : 0.0f;
+                nn_store8(&w.H[c][(4 * ri + r) * NN_LDT + 8 * ui], h[r]);
             }
+            nn_store_t(&w.T[c][8 * ui * NN_LDT + 4 * ri], h);
+            __syncwarp();
         }
+        nn_sum_rows(sum);
+        if (ri == 0) nn_store8(w.g + 8 * ui, sum);
         __syncwarp();
-        // lane a owns row a of W1: dW1[a][j] = sum_i dz1_ia f_ij
+        w.g[lane] /= (float)n;
+        __syncwarp();
         {
-            float acc[NNF] = {0, 0, 0, 0, 0, 0, 0, 0};
-            float sb = 0.0f;
-            for (int i = 0; i < n; ++i) {
-                const float d = Hs[i * NN_LD + lane];
-                sb += d;
+            float z = sh.b2[lane];
 #pragma unroll
-                for (int j = 0; j < NNF; ++j) acc[j] = fmaf(d, f[i * NNF + j], acc[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < NNF; ++j) atomicAdd(&G[NN_W1 + lane * NNF + j], acc[j]);
-            atomicAdd(&G[NN_B1 + lane], sb);
+            for (int b = 0; b < NNH; ++b) z = fmaf(sh.W2BT[b * NN_LDT + lane], w.g[b], z);
+            w.u[lane] = z;
         }
         __syncwarp();
+        // ---- q = relu(W2a h + u), y = w3 q + b3; dz2 = dL/dy w3 (q > 0) ----
+#pragma unroll
+        for (int p = 0; p < 4; ++p) sum[p] = 0;
+        float l2 = 0.0f;
+        F2 w3[4];
+        nn_load8(sh.w3 + 8 * ui, w3);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (32 * c >= n) break;
+            float t[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int i = 32 * c + 4 * ri + r;
+                t[r] = i < n ? target[s * k + i] : 0.0f;
+            }
+            F2 z[4][4];
+            nn_load8(w.u + 8 * ui, z[0]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) z[1][p] = z[2][p] = z[3][p] = z[0][p];
+#pragma unroll 8
+            for (int b = 0; b < NNH; ++b) nn_step(z, w.T[c] + b * NN_LDT + 4 * ri, sh.W2AT + b * NN_LDT + 8 * ui);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                F2 y2 = 0;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    z[r][p] = f2_pack(fmaxf(f2_lo(z[r][p]), 0.0f), fmaxf(f2_hi(z[r][p]), 0.0f));
+                    y2 = f2_fma(w3[p], z[r][p], y2);
+                }
+                float y = f2_lo(y2) + f2_hi(y2);
+                y += __shfl_xor_sync(FULL_MASK, y, 1);
+                y += __shfl_xor_sync(FULL_MASK, y, 2);
+                const bool in = 32 * c + 4 * ri + r < n;
+                const float e = in ? y + sh.b3[0] - t[r] : 0.0f;
+                const float dy = 2.0f * e / (float)n;
+                if (ui == 0) {
+                    l2 += e * e;
+                    db3 += dy;
+                }
+                const F2 d2 = f2_pack(dy, dy);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    dw3[p] = f2_fma(d2, z[r][p], dw3[p]);
+                    const float wl = f2_lo(w3[p]) * dy, wh = f2_hi(w3[p]) * dy;
+                    z[r][p] = f2_pack(f2_lo(z[r][p]) > 0.0f ? wl : 0.0f, f2_hi(z[r][p]) > 0.0f ? wh : 0.0f);
+                    sum[p] = f2_fma(one, z[r][p], sum[p]);
+                }
+                nn_store8(&w.Z[c][(4 * ri + r) * NN_LDT + 8 * ui], z[r]);
+            }
+            __syncwarp();  // T has been read
+            nn_store_t(&w.T[c][8 * ui * NN_LDT + 4 * ri], z);
+        }
+        total += l2 * inv_n;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) db2[p] = f2_fma(one, sum[p], db2[p]);
+        nn_sum_rows(sum);
+        if (ri == 0) nn_store8(w.sz + 8 * ui, sum);
+        __syncwarp();
+        // ---- dW2a = dz2' h, dW2b = (sum dz2)' g, dg = W2b' sum dz2 / n ----
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int rows = min(32, n - 32 * c);
+#pragma unroll 4
+            for (int i = 0; i < rows; ++i) nn_step(dw2a, w.Z[c] + i * NN_LDT + 4 * ri, w.H[c] + i * NN_LDT + 8 * ui);
+        }
+        nn_step(dw2b, w.sz + 4 * ri, w.g + 8 * ui);
+        {
+            float d = 0.0f;
+#pragma unroll
+            for (int a = 0; a < NNH; ++a) d = fmaf(sh.W2B[a * NN_LDT + lane], w.sz[a], d);
+            w.dg[lane] = d * inv_n;
+        }
+        __syncwarp();
+        // ---- dz1 = (W2a' dz2 + dg) (h > 0), dW1 = dz1' f ----
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (32 * c >= n) break;
+            F2 d[4][4];
+            nn_load8(w.dg + 8 * ui, d[0]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) d[1][p] = d[2][p] = d[3][p] = d[0][p];
+#pragma unroll 8
+            for (int a = 0; a < NNH; ++a) nn_step(d, w.T[c] + a * NN_LDT + 4 * ri, sh.W2A + a * NN_LDT + 8 * ui);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                F2 h[4];
+                nn_load8(&w.H[c][(4 * ri + r) * NN_LDT + 8 * ui], h);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    d[r][p] = f2_pack(f2_lo(h[p]) > 0.0f ? f2_lo(d[r][p]) : 0.0f, f2_hi(h[p]) > 0.0f ? f2_hi(d[r][p]) : 0.0f);
+                    db1[p] = f2_fma(one, d[r][p], db1[p]);
+                }
+                nn_store8(&w.Z[c][(4 * ri + r) * NN_LDT + 8 * ui], d[r]);
+            }
+            __syncwarp();
+            const int rows = min(32, n - 32 * c);
+#pragma unroll 4
+            for (int i = 0; i < rows; ++i) {  // units 4 ri .., features 2 ui ..
+                const float4 x = *reinterpret_cast<const float4*>(&w.Z[c][i * NN_LDT + 4 * ri]);
+                const F2 f = *reinterpret_cast<const F2*>(&w.F[c][i * NNF + 2 * ui]);
+                dw1[0] = f2_fma(f2_pack(x.x, x.x), f, dw1[0]);
+                dw1[1] = f2_fma(f2_pack(x.y, x.y), f, dw1[1]);
+                dw1[2] = f2_fma(f2_pack(x.z, x.z), f, dw1[2]);
+                dw1[3] = f2_fma(f2_pack(x.w, x.w), f, dw1[3]);
+            }
+            __syncwarp();
+        }
     }
-    if (lane == 0) atomicAdd(loss, block_loss);
+    // ---- the block's gradient, over the tiles' memory ----
     __syncthreads();
-    for (int i = threadIdx.x; i < NN_PARAMS; i += blockDim.x) atomicAdd(&grad[i], G[i]);
+    float* G = reinterpret_cast<float*>(&sh.warp[0]);
+    static_assert(sizeof(sh.warp) >= NN_PARAMS * sizeof(float), "room for the gradient");
+    for (int i = threadIdx.x; i < NN_PARAMS; i += S::WARPS * 32) G[i] = 0.0f;
+    __syncthreads();
+    auto add = [&](int i, F2 v) {
+        atomicAdd(&G[i], f2_lo(v));
+        atomicAdd(&G[i + 1], f2_hi(v));
+    };
+    nn_sum_rows(dw3);
+    nn_sum_rows(db1);
+    nn_sum_rows(db2);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int at = (4 * ri + r) * NNH + 8 * ui + 2 * p;
+            add(NN_W2A + at, dw2a[r][p]);
+            add(NN_W2B + at, dw2b[r][p]);
+        }
+        add(NN_W1 + (4 * ri + p) * NNF + 2 * ui, dw1[p]);
+        if (ri == 0) {
+            add(NN_W3 + 8 * ui + 2 * p, dw3[p]);
+            add(NN_B1 + 8 * ui + 2 * p, db1[p]);
+            add(NN_B2 + 8 * ui + 2 * p, db2[p]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        db3 += __shfl_xor_sync(FULL_MASK, db3, o);
+        total += __shfl_xor_sync(FULL_MASK, total, o);
+    }
+    if (lane == 0) {
+        atomicAdd(&G[NN_B3], db3);
+        sh.warp_loss[threadIdx.x >> 5] = total;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {  // once per block: fewer roundings of the whole sum
+        double t = 0.0;
+        for (int i = 0; i < S::WARPS; ++i) t += (double)sh.warp_loss[i];
+        atomicAdd(loss, (float)t);
+    }
+    for (int i = threadIdx.x; i < NN_PARAMS; i += S::WARPS * 32) atomicAdd(&grad[i], G[i]);
 }
 
 // Warm-start predictions for every node of a plan: features computed in
@@ -393,13 +590,25 @@ cudaError_t launch_nn_forward(const float* params, const float* feat, const int3
     return cudaGetLastError();
 }
 
+template <int NC>
+static cudaError_t nn_backward(const float* params, const float* feat, const int32_t* count, const float* target,
+                               int64_t nsys, int k, float* grad, float* loss, cudaStream_t s) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const size_t smem = sizeof(NNTiles<NC>);
+    cudaError_t e = cudaFuncSetAttribute(nn_backward_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    constexpr int W = NNTiles<NC>::WARPS;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(nsm, (nsys + W - 1) / W));
+    nn_backward_kernel<NC><<<blocks, W * 32, smem, s>>>(params, feat, count, target, nsys, k, grad, loss);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_nn_backward(const float* params, const float* feat, const int32_t* count, const float* target,
                                int64_t nsys, int k, float* grad, float* loss, cudaStream_t s) {
-    const size_t smem = sizeof(NNSmem) + NN_PARAMS * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(nn_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    nn_backward_kernel<<<nn_blocks(nsys), NN_WARPS * 32, smem, s>>>(params, feat, count, target, nsys, k, grad, loss);
-    return cudaGetLastError();
+    return k <= 32 ? nn_backward<1>(params, feat, count, target, nsys, k, grad, loss, s)
+                   : nn_backward<2>(params, feat, count, target, nsys, k, grad, loss, s);
 }
 
 cudaError_t launch_nn_adam(float* p, const float* g, float* m, float* v, int step, float lr, float scale,

@@ -795,29 +795,6 @@ __device__ __forceinline__ void static_for(F&& f) {
     static_for_impl(f, std::make_integer_sequence<int, N>{});
 }
 
-// two FP32 values in one 64-bit register pair; fma.rn.f32x2 is one
-// instruction for both
-using F2 = unsigned long long;
-__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
-    F2 v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ float f2_lo(F2 v) {
-    float lo;
-    asm("mov.b64 {%0, _}, %1;" : "=f"(lo) : "l"(v));
-    return lo;
-}
-__device__ __forceinline__ float f2_hi(F2 v) {
-    float hi;
-    asm("mov.b64 {_, %0}, %1;" : "=f"(hi) : "l"(v));
-    return hi;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-    F2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 // registers of the lower triangle's rows, two entries each: row i holds
 // entries 0 .. i (and one unused past an even i) from register tri2(i)
 __host__ __device__ constexpr int tri2(int i) { return (i / 2) * (i / 2 + 1) + (i & 1) * (i / 2 + 1); }
