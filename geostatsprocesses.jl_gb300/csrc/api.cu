@@ -1223,13 +1223,27 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
     return SGS_OK;
 }
 
-// error flag of the last dataflow sweep (the caller has synchronized)
-static int check_flow_error(sgs_plan* P) {
-    if (!P->d_flow || P->last_sweep_mode != SGS_SWEEP_FLOW) return SGS_OK;
+static int check_flow(sgs_plan* P) {
     int32_t err = 0;
     CK(P, cudaMemcpy(&err, P->d_flow, sizeof(err), cudaMemcpyDeviceToHost));
     if (err) return set_err(P, SGS_ERR_TIMEOUT, "dataflow sweep: a dependency wait exceeded its bound");
     return SGS_OK;
+}
+
+// error flag, counters and bound of a dataflow launch (FLOW_WORDS cleared first)
+static FlowArgs plan_flow(const sgs_plan* P) {
+    FlowArgs f{};
+    f.ticket = P->d_flow + FLOW_TICKET_STRIDE;
+    f.err = reinterpret_cast<int32_t*>(P->d_flow);
+    f.chunk = 1;
+    f.wait_ns = 10000000000ull;  // 10 s: far beyond any dependency chain
+    return f;
+}
+
+// error flag of the last dataflow sweep (the caller has synchronized)
+static int check_flow_error(sgs_plan* P) {
+    if (!P->d_flow || P->last_sweep_mode != SGS_SWEEP_FLOW) return SGS_OK;
+    return check_flow(P);
 }
 
 static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, void* V, cudaStream_t st) {
@@ -1261,16 +1275,14 @@ static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, v
         CK(P, cudaMemsetAsync(P->d_flow, 0, FLOW_WORDS * sizeof(unsigned long long), st));
         auto flow = [&](int l0, int l1) -> int {
             const int64_t p0 = P->h_loff[l0], p1 = P->h_loff[l1];
-            FlowArgs f{};
+            FlowArgs f = plan_flow(P);
             f.item0 = p0 * H;
             f.item1 = p1 * H;
             f.H = H;
-            f.ticket = P->d_flow + FLOW_TICKET_STRIDE + (l0 == 0 ? 0 : FLOW_TICKETS);
-            f.err = reinterpret_cast<int32_t*>(P->d_flow);
+            if (l0 > 0) f.ticket += FLOW_TICKETS;
             f.chunk = std::max(1, c.chunk);
             f.blocks_per_sm = c.blocks_per_sm;
             f.tight = P->sweep_auto ? flow_tight((p1 - p0) * H, l1 - l0, P->nsm) : c.tight;
-            f.wait_ns = 10000000000ull;  // 10 s: far beyond any dependency chain
             cudaError_t e = launch_flow_clear(values_fp64(P) ? sweep64(P).node : P->t32.node, p0, p1, P->N,
                                               (size_t)Rp * (values_fp64(P) ? sizeof(double) : sizeof(float)), V, st);
             if (e != cudaSuccess) return cuda_err(P, e, "sweep clear");
@@ -1860,17 +1872,18 @@ extern "C" int sgs_plan_simulate_indicator(sgs_plan* P, int32_t R, const double*
     ia.wsum = P->d_ind_wsum;
     ia.dsum = P->d_ind_dsum;
     CK(P, cudaEventRecord(P->ev[5], st));
-    for (int l = 0; l < P->nlevels; ++l) {
-        const int64_t p0 = P->h_loff[l], p1 = P->h_loff[l + 1];
-        cudaError_t e = P->cok ? launch_cok_level(cok_args(P), P->d_order, P->k, p0, p1, Rp, ur, seed, C, st)
-                        : P->precision == SGS_PREC_FP64
-                            ? launch_sis_level_fp64(P->t64, P->k, p0, p1, Rp, ia, ur, seed, C, st)
-                            : launch_sis_level_fp32(P->t32, P->k, p0, p1, Rp, ia, ur, seed, C, st);
+    {
+        const FlowArgs f = plan_flow(P);
+        cudaError_t e = cudaMemsetAsync(P->d_flow, 0, FLOW_WORDS * sizeof(unsigned long long), st);
+        if (e == cudaSuccess)
+            e = P->cok ? launch_cok_flow(cok_args(P), P->d_order, P->k, N, Rp, ur, seed, C, f, st)
+                : P->precision == SGS_PREC_FP64 ? launch_sis_flow_fp64(P->t64, P->k, N, Rp, ia, ur, seed, C, f, st)
+                                                : launch_sis_flow_fp32(P->t32, P->k, N, Rp, ia, ur, seed, C, f, st);
         if (e != cudaSuccess) {
             cleanup();
             return cuda_err(P, e, "indicator sweep launch");
         }
-        if (p1 > p0) P->info.launches++;
+        P->info.launches++;
     }
     CK(P, cudaEventRecord(P->ev[6], st));
     if ((rc = dalloc(P, &od, (size_t)N * R))) {
@@ -1882,8 +1895,9 @@ extern "C" int sgs_plan_simulate_indicator(sgs_plan* P, int32_t R, const double*
     P->info.d2h_bytes += (int64_t)N * R * sizeof(int32_t);
     CK(P, cudaStreamSynchronize(st));
     P->info.ms_sweep = elapsed(P->ev[5], P->ev[6]);
+    rc = check_flow(P);
     cleanup();
-    return SGS_OK;
+    return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -1977,14 +1991,14 @@ extern "C" int sgs_plan_simulate_multivariate(sgs_plan* P, int32_t R, const doub
     }
     const CokArgs c = cok_args(P);
     CK(P, cudaEventRecord(P->ev[5], st));
-    for (int l = 0; l < P->nlevels; ++l) {
-        const int64_t p0 = P->h_loff[l], p1 = P->h_loff[l + 1];
-        cudaError_t e = launch_mv_level(c, P->d_order, P->k, N, p0, p1, Rp, zr, seed, V, st);
+    {
+        cudaError_t e = cudaMemsetAsync(P->d_flow, 0, FLOW_WORDS * sizeof(unsigned long long), st);
+        if (e == cudaSuccess) e = launch_mv_flow(c, P->d_order, P->k, N, Rp, zr, seed, V, plan_flow(P), st);
         if (e != cudaSuccess) {
             cleanup();
             return cuda_err(P, e, "multivariate sweep launch");
         }
-        if (p1 > p0) P->info.launches++;
+        P->info.launches++;
     }
     CK(P, cudaEventRecord(P->ev[6], st));
     if ((rc = dalloc(P, &od, (size_t)NL * R))) {
@@ -1996,6 +2010,7 @@ extern "C" int sgs_plan_simulate_multivariate(sgs_plan* P, int32_t R, const doub
     P->info.d2h_bytes += NL * R * (int64_t)sizeof(double);
     CK(P, cudaStreamSynchronize(st));
     P->info.ms_sweep = elapsed(P->ev[5], P->ev[6]);
+    rc = check_flow(P);
     cleanup();
-    return SGS_OK;
+    return rc;
 }

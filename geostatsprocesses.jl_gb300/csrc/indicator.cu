@@ -18,14 +18,14 @@
 // The draw is the inverse cdf at a uniform u: the first category whose
 // cumulative probability exceeds u.
 //
-// Categories are bytes, node-major [N][Rp] (4 realizations per 32-bit
-// word); levels run in order, one thread per (node, 4 realizations).
+// Categories are bytes, node-major [N][Rp].
 // Per-category sums are compensated FP32 sums of (hi, lo) weights (about
 // 1e-12), so the category decision equals an FP64 evaluation except at
 // exact ties.
 #include <algorithm>
 
 #include "common.cuh"
+#include "flow.cuh"
 
 namespace sgs {
 
@@ -64,95 +64,211 @@ __device__ __forceinline__ int draw_category(const IndArgs& ia, const double* p,
     return ia.ncat - 1;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) sis_level_kernel(const SweepTables<T> t, int k, int64_t p0, int64_t p1, int Rp,
-                                                        const IndArgs ia, const double* __restrict__ u, uint64_t seed,
-                                                        uint8_t* __restrict__ C) {
-    const int cpn = Rp >> 2;
-    const int64_t total = (p1 - p0) * cpn;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pos = p0 + i / cpn;
-        const int ch = (int)(i % cpn);
-        const int g = t.node[pos];
-        const int m = t.m[pos];
-        const int32_t* idx = t.idx + pos * k;
-        // per realization and category: the weights of grid neighbours of
-        // that category (compensated FP32 sums, or FP64 for FP64 tables)
-        float s[4][IND_MAX_CAT], c[4][IND_MAX_CAT];
-        double d[4][IND_MAX_CAT];
+// The sweeps below are dataflow launches (sweep.cu): an item is a node and up
+// to 32 of its realizations, W lanes one realization each and 32 / W slices of
+// the neighbour list.  A lane loads its realization's value of 8
+// neighbours and adds them once they are stored.  One launch per level, with
+// the categories of 4 realizations and up to 28 FP64 divisions to a thread,
+// took 48 us for a level (174 levels of 256 x 256 nodes x 32: 8.3 ms); this
+// takes 2.4 (0.42 ms).  8, 16 or 24 neighbours at a time are slower, and so is
+// a branch on the category instead of adding zero to the others (0.70 ms).
+constexpr int IND_AHEAD = 4;
+
+// The category drawn at u for probabilities proportional to base + sum,
+// clamped: in FP32 where that decides it.  The FP32 sums differ from exact ones
+// by less than 2^-19 (1 + A), A the sum of the terms' magnitudes; where u falls
+// within twice that of a boundary, or nothing is left after clamping, the FP64
+// evaluation decides.
+template <int LM, class Sum, class Exact>
+__device__ __forceinline__ int draw_category32(const IndArgs& ia, const float (&base)[LM], Sum sum, Exact exact,
+                                               double u) {
+    float q[LM], s = 0.0f, A = 1.0f;
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int l = 0; l < IND_MAX_CAT; ++l) {
-                s[r][l] = 0.f;
-                c[r][l] = 0.f;
-                d[r][l] = 0.0;
-            }
-        for (int j = 0; j < m; ++j) {
-            const uint32_t cats = *reinterpret_cast<const uint32_t*>(C + (int64_t)idx[j] * Rp + 4 * ch);
-            if constexpr (sizeof(T) == 4) {
-                const float2 wj = reinterpret_cast<const float2*>(t.w)[pos * k + j];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int cr = (int)((cats >> (8 * r)) & 0xffu);
-#pragma unroll
-                    for (int l = 0; l < IND_MAX_CAT; ++l)
-                        if (l == cr) {
-                            const DF ts = df_two_sum(s[r][l], wj.x);
-                            s[r][l] = ts.hi;
-                            c[r][l] = __fadd_rn(c[r][l], __fadd_rn(ts.lo, wj.y));
-                        }
-                }
-            } else {
-                const double wj = t.w[pos * k + j];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int cr = (int)((cats >> (8 * r)) & 0xffu);
-#pragma unroll
-                    for (int l = 0; l < IND_MAX_CAT; ++l)
-                        if (l == cr) d[r][l] += wj;
-                }
-            }
+    for (int l = 0; l < LM; ++l) {
+        q[l] = 0.0f;
+        if (l < ia.ncat) {
+            const float b = base[l], g = sum(l);
+            A += fabsf(b) + fabsf(g);
+            q[l] = fminf(fmaxf(b + g, 0.0f), 1.0f);
+            s += q[l];
         }
-        const double W = ia.wsum[pos];
-        const double* D = ia.dsum + pos * ia.ncat;
-        const float4 uf = u ? make_float4(0.f, 0.f, 0.f, 0.f) : uniforms4(seed, g, ch);
-        const float ufa[4] = {uf.x, uf.y, uf.z, uf.w};
-        uint32_t out = 0;
+    }
+    const float margin = A * 3.8e-6f, us = (float)u * s;
+    bool near = !(s > margin);
+    float cum = 0.0f;
+    int cat = ia.ncat - 1;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            double p[IND_MAX_CAT];
-#pragma unroll
-            for (int l = 0; l < IND_MAX_CAT; ++l) {
-                const double gsum = sizeof(T) == 4 ? (double)s[r][l] + (double)c[r][l] : d[r][l];
-                p[l] = l < ia.ncat ? ia.prob[l] * (1.0 - W) + gsum + D[l] : 0.0;
-            }
-            const double ur = u ? u[(int64_t)g * Rp + 4 * ch + r] : (double)ufa[r];
-            out |= (uint32_t)draw_category(ia, p, ur) << (8 * r);
+    for (int l = 0; l < LM - 1; ++l)
+        if (l < ia.ncat - 1) {
+            cum += q[l];
+            near = near || !(fabsf(us - cum) > margin);
+            if (us < cum && cat == ia.ncat - 1) cat = l;
         }
-        *reinterpret_cast<uint32_t*>(C + (int64_t)g * Rp + 4 * ch) = out;
+    if (near) {
+        double p[IND_MAX_CAT];
+#pragma unroll
+        for (int l = 0; l < IND_MAX_CAT; ++l) p[l] = 0.0;
+#pragma unroll
+        for (int l = 0; l < LM; ++l)
+            if (l < ia.ncat) p[l] = exact(l);
+        cat = draw_category(ia, p, u);
+    }
+    return cat;
+}
+
+// uniform (given or seeded) of a node's realization
+__device__ __forceinline__ double uniform_of(const double* __restrict__ u, uint64_t seed, int64_t g, int Rp, int r) {
+    if (u) return u[g * Rp + r];
+    const float4 f = uniforms4(seed, g, r >> 2);
+    return (double)((r & 2) ? ((r & 1) ? f.w : f.z) : ((r & 1) ? f.y : f.x));
+}
+
+// Categories of neighbours j + h S, h < IND_AHEAD, of one realization (C: its
+// column) once they are stored, IND_NONE where there is none; false where the
+// wait was given up.
+constexpr uint32_t IND_NONE = 0xfe;
+__device__ __forceinline__ bool flow_categories(const int32_t* idx, int m, int j, int S, bool on, const uint8_t* C, int Rp,
+                                                const FlowArgs& f, uint32_t (&cat)[IND_AHEAD]) {
+    int g[IND_AHEAD];
+#pragma unroll
+    for (int h = 0; h < IND_AHEAD; ++h) g[h] = on && j + h * S < m ? idx[j + h * S] : -1;
+#pragma unroll
+    for (int h = 0; h < IND_AHEAD; ++h) cat[h] = g[h] >= 0 ? ld_category(C + (int64_t)g[h] * Rp) : IND_NONE;
+    FlowBound bound;
+    for (;;) {
+        bool miss = false;
+#pragma unroll
+        for (int h = 0; h < IND_AHEAD; ++h) miss |= cat[h] == 0xff;
+        if (!miss) return true;
+        if (!bound.more(f.err, f.wait_ns)) return false;
+#pragma unroll
+        for (int h = 0; h < IND_AHEAD; ++h)
+            if (cat[h] == 0xff) cat[h] = ld_category(C + (int64_t)g[h] * Rp);
     }
 }
 
-template <typename T>
-static cudaError_t sis_level(const SweepTables<T>& t, int k, int64_t p0, int64_t p1, int Rp, const IndArgs& ia,
-                             const double* u, uint64_t seed, uint8_t* C, cudaStream_t s) {
-    if (p1 <= p0) return cudaSuccess;
-    int64_t blocks = ((p1 - p0) * (Rp / 4) + 255) / 256;
-    if (blocks > (1 << 20)) blocks = 1 << 20;
-    sis_level_kernel<T><<<(int)blocks, 256, 0, s>>>(t, k, p0, p1, Rp, ia, u, seed, C);
+template <typename T, int LM>
+__global__ void __launch_bounds__(256) sis_flow_kernel(const SweepTables<T> t, int k, int Rp, const IndArgs ia,
+                                                       const double* __restrict__ u, uint64_t seed, uint8_t* C,
+                                                       const __grid_constant__ FlowArgs f, int W) {
+    const int lane = threadIdx.x & 31, S = 32 / W, s = lane / W;
+    bool ok = true;
+    for (FlowItems next(f); next.live(); next.step()) {
+        const int64_t pos = next.position();
+        const int r = (int)(next.it - pos * f.H) * W + lane % W;
+        const bool on = r < Rp;
+        const int g = t.node[pos];
+        const int m = t.m[pos];
+        const int32_t* idx = t.idx + pos * k;
+        // weights: (hi, lo) pairs, or the two words of a double
+        const float2* tw = reinterpret_cast<const float2*>(t.w) + pos * k;
+        float2 w0 = make_float2(0.f, 0.f), w1 = w0;
+        if (lane < m) w0 = tw[lane];
+        if (lane + 32 < m) w1 = tw[lane + 32];
+        const double W1 = 1.0 - ia.wsum[pos];
+        const double* D = ia.dsum + pos * ia.ncat;
+        float b0[LM];
+#pragma unroll
+        for (int l = 0; l < LM; ++l) b0[l] = l < ia.ncat ? (float)(ia.prob[l] * W1 + D[l]) : 0.f;
+        const double ur = on ? uniform_of(u, seed, g, Rp, r) : 0.0;
+        // per category: the weights of grid neighbours of that category
+        // (compensated FP32 sums, or FP64 for FP64 tables)
+        float sh[LM], sc[LM];
+        double sd[LM];
+#pragma unroll
+        for (int l = 0; l < LM; ++l) {
+            sh[l] = sc[l] = 0.f;
+            sd[l] = 0.0;
+        }
+        for (int j0 = 0; j0 < m; j0 += IND_AHEAD * S) {
+            uint32_t cat[IND_AHEAD];
+            ok = flow_categories(idx, ok ? m : 0, j0 + s, S, on, C + r, Rp, f, cat) && ok;
+#pragma unroll
+            for (int h = 0; h < IND_AHEAD; ++h) {
+                const int j = j0 + h * S + s;
+                const float hi0 = __shfl_sync(FULL_MASK, w0.x, j & 31), lo0 = __shfl_sync(FULL_MASK, w0.y, j & 31);
+                float2 wj = make_float2(hi0, lo0);
+                if (m > 32) {
+                    const float hi1 = __shfl_sync(FULL_MASK, w1.x, j & 31), lo1 = __shfl_sync(FULL_MASK, w1.y, j & 31);
+                    if (j >= 32) wj = make_float2(hi1, lo1);
+                }
+                if constexpr (sizeof(T) == 4) {
+#pragma unroll
+                    for (int l = 0; l < LM; ++l) {  // zeros for the other categories
+                        const bool own = l == (int)cat[h];
+                        const DF ts = df_two_sum(sh[l], own ? wj.x : 0.f);
+                        sh[l] = ts.hi;
+                        sc[l] = __fadd_rn(sc[l], __fadd_rn(ts.lo, own ? wj.y : 0.f));
+                    }
+                } else {
+                    const double wd = __hiloint2double(__float_as_int(wj.y), __float_as_int(wj.x));
+#pragma unroll
+                    for (int l = 0; l < LM; ++l) sd[l] += l == (int)cat[h] ? wd : 0.0;
+                }
+            }
+        }
+        for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+            for (int l = 0; l < LM; ++l) {
+                if constexpr (sizeof(T) == 4) {
+                    const DF ts = df_two_sum(sh[l], __shfl_xor_sync(FULL_MASK, sh[l], o));
+                    sc[l] = __fadd_rn(sc[l], __shfl_xor_sync(FULL_MASK, sc[l], o));
+                    sh[l] = ts.hi;
+                    sc[l] = __fadd_rn(sc[l], ts.lo);
+                } else {
+                    sd[l] += __shfl_xor_sync(FULL_MASK, sd[l], o);
+                }
+            }
+        if (s == 0 && on) {
+            const int cat = draw_category32<LM>(
+                ia, b0, [&](int l) { return sizeof(T) == 4 ? sh[l] + sc[l] : (float)sd[l]; },
+                [&](int l) {
+                    return ia.prob[l] * W1 + (sizeof(T) == 4 ? (double)sh[l] + (double)sc[l] : sd[l]) + D[l];
+                },
+                ur);
+            st_category(C + (int64_t)g * Rp + r, ok ? cat : 0);
+        }
+    }
+}
+
+// the items and pieces of a dataflow launch over all N positions, values
+// cleared to the unstored pattern
+template <class K, class... A>
+static cudaError_t ind_flow(K kernel, FlowArgs f, int64_t N, int Rp, void* V, size_t bytes, cudaStream_t s, A... args) {
+    int W = 1;
+    while (W < Rp && W < 32) W <<= 1;
+    f.H = (Rp + W - 1) / W;
+    f.rec = f.H > 1 ? ~0ull / (uint64_t)f.H + 1 : 0;
+    f.item0 = 0;
+    f.item1 = N * f.H;
+    f.chunk = 1;
+    cudaError_t e = cudaMemsetAsync(V, 0xff, bytes, s);
+    if (e != cudaSuccess) return e;
+    int dev = 0, nsm = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * FLOW_CLASSES, 0);
+    if (e != cudaSuccess) return e;
+    const int64_t full = (int64_t)nsm * std::max(per_sm, 1);
+    const int blocks = (int)std::max<int64_t>(1, std::min(full, (f.item1 + FLOW_CLASSES - 1) / FLOW_CLASSES));
+    kernel<<<blocks, 32 * FLOW_CLASSES, 0, s>>>(args..., f, W);
     return cudaGetLastError();
 }
 
-cudaError_t launch_sis_level_fp32(const SweepTables<float>& t, int k, int64_t p0, int64_t p1, int Rp,
-                                  const IndArgs& ia, const double* u, uint64_t seed, uint8_t* C, cudaStream_t s) {
-    return sis_level<float>(t, k, p0, p1, Rp, ia, u, seed, C, s);
+cudaError_t launch_sis_flow_fp32(const SweepTables<float>& t, int k, int64_t N, int Rp, const IndArgs& ia,
+                                 const double* u, uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s) {
+    const size_t bytes = (size_t)N * Rp;
+    if (ia.ncat <= 2) return ind_flow(sis_flow_kernel<float, 2>, f, N, Rp, C, bytes, s, t, k, Rp, ia, u, seed, C);
+    if (ia.ncat <= 4) return ind_flow(sis_flow_kernel<float, 4>, f, N, Rp, C, bytes, s, t, k, Rp, ia, u, seed, C);
+    return ind_flow(sis_flow_kernel<float, 8>, f, N, Rp, C, bytes, s, t, k, Rp, ia, u, seed, C);
 }
 
-cudaError_t launch_sis_level_fp64(const SweepTables<double>& t, int k, int64_t p0, int64_t p1, int Rp,
-                                  const IndArgs& ia, const double* u, uint64_t seed, uint8_t* C, cudaStream_t s) {
-    return sis_level<double>(t, k, p0, p1, Rp, ia, u, seed, C, s);
+cudaError_t launch_sis_flow_fp64(const SweepTables<double>& t, int k, int64_t N, int Rp, const IndArgs& ia,
+                                 const double* u, uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s) {
+    const size_t bytes = (size_t)N * Rp;
+    if (ia.ncat <= 2) return ind_flow(sis_flow_kernel<double, 2>, f, N, Rp, C, bytes, s, t, k, Rp, ia, u, seed, C);
+    if (ia.ncat <= 4) return ind_flow(sis_flow_kernel<double, 4>, f, N, Rp, C, bytes, s, t, k, Rp, ia, u, seed, C);
+    return ind_flow(sis_flow_kernel<double, 8>, f, N, Rp, C, bytes, s, t, k, Rp, ia, u, seed, C);
 }
 
 // ---------------------------------------------------------------------------
@@ -406,147 +522,168 @@ cudaError_t launch_cok_solve(const SolveArgs& a, const CokArgs& c, bool gaussian
     return gaussian ? cok_solve<true>(a, c, s) : cok_solve<false>(a, c, s);
 }
 
-// One level: one thread per (position, 4 realizations).
-__global__ void __launch_bounds__(256) cok_level_kernel(const CokArgs c, const int32_t* __restrict__ node, int k,
-                                                        int64_t p0, int64_t p1, int Rp, const double* __restrict__ u,
-                                                        uint64_t seed, uint8_t* __restrict__ C) {
-    const int cpn = Rp >> 2, L = c.ncat;
+template <int LM>
+__global__ void __launch_bounds__(256) cok_flow_kernel(const CokArgs c, const int32_t* __restrict__ node, int k, int Rp,
+                                                       const double* __restrict__ u, uint64_t seed, uint8_t* C,
+                                                       const __grid_constant__ FlowArgs f, int W) {
+    const int lane = threadIdx.x & 31, S = 32 / W, s = lane / W, L = c.ncat;
     IndArgs ia{};
     ia.ncat = L;
     for (int l = 0; l < IND_MAX_CAT; ++l) ia.prob[l] = c.prob[l];
-    const int64_t total = (p1 - p0) * cpn;
-    for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < total;
-         it += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pos = p0 + it / cpn;
-        const int ch = (int)(it % cpn);
+    bool ok = true;
+    for (FlowItems next(f); next.live(); next.step()) {
+        const int64_t pos = next.position();
+        const int r = (int)(next.it - pos * f.H) * W + lane % W;
+        const bool on = r < Rp;
         const int g = node[pos];
         const int m = c.m[pos];
-        double p[4][IND_MAX_CAT];
+        const double* w = c.w + pos * k * L * L;
+        for (int b = lane * 16; b < m * L * L; b += 512) asm volatile("prefetch.global.L1 [%0];" ::"l"(w + b));
+        float b0[LM];
+        double p[LM];
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int t = 0; t < IND_MAX_CAT; ++t) p[r][t] = t < L ? c.cst[pos * L + t] : 0.0;
-        for (int j = 0; j < m; ++j) {
-            const int64_t e = pos * k + j;
-            const uint32_t cats = *reinterpret_cast<const uint32_t*>(C + (int64_t)c.idx[e] * Rp + 4 * ch);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int b = (int)((cats >> (8 * r)) & 0xffu);
-                const double* wr = c.w + (e * L + b) * L;
-#pragma unroll
-                for (int t = 0; t < IND_MAX_CAT; ++t)
-                    if (t < L) p[r][t] += wr[t];
-            }
+        for (int t = 0; t < LM; ++t) {
+            b0[t] = t < L ? (float)c.cst[pos * L + t] : 0.f;
+            p[t] = 0.0;
         }
-        const float4 uf = u ? make_float4(0.f, 0.f, 0.f, 0.f) : uniforms4(seed, g, ch);
-        const float ufa[4] = {uf.x, uf.y, uf.z, uf.w};
-        uint32_t out = 0;
+        const double ur = on ? uniform_of(u, seed, g, Rp, r) : 0.0;
+        for (int j0 = 0; j0 < m; j0 += IND_AHEAD * S) {
+            uint32_t cat[IND_AHEAD];
+            ok = flow_categories(c.idx + pos * k, ok ? m : 0, j0 + s, S, on, C + r, Rp, f, cat) && ok;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const double ur = u ? u[(int64_t)g * Rp + 4 * ch + r] : (double)ufa[r];
-            out |= (uint32_t)draw_category(ia, p[r], ur) << (8 * r);
+            for (int h = 0; h < IND_AHEAD; ++h)
+                if (cat[h] < IND_MAX_CAT) {
+                    const double* wr = w + ((j0 + h * S + s) * L + cat[h]) * L;
+#pragma unroll
+                    for (int t = 0; t < LM; ++t)
+                        if (t < L) p[t] += wr[t];
+                }
         }
-        *reinterpret_cast<uint32_t*>(C + (int64_t)g * Rp + 4 * ch) = out;
+        __syncwarp();
+        for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+            for (int t = 0; t < LM; ++t)
+                if (t < L) p[t] += __shfl_xor_sync(FULL_MASK, p[t], o);
+        if (s == 0 && on) {
+            const int cat = draw_category32<LM>(
+                ia, b0, [&](int l) { return (float)p[l]; }, [&](int l) { return c.cst[pos * L + l] + p[l]; }, ur);
+            st_category(C + (int64_t)g * Rp + r, ok ? cat : 0);
+        }
     }
 }
 
-cudaError_t launch_cok_level(const CokArgs& c, const int32_t* node, int k, int64_t p0, int64_t p1, int Rp,
-                             const double* u, uint64_t seed, uint8_t* C, cudaStream_t s) {
-    if (p1 <= p0) return cudaSuccess;
-    int64_t blocks = ((p1 - p0) * (Rp / 4) + 255) / 256;
-    if (blocks > (1 << 20)) blocks = 1 << 20;
-    cok_level_kernel<<<(int)blocks, 256, 0, s>>>(c, node, k, p0, p1, Rp, u, seed, C);
-    return cudaGetLastError();
+cudaError_t launch_cok_flow(const CokArgs& c, const int32_t* node, int k, int64_t N, int Rp, const double* u,
+                            uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s) {
+    const size_t bytes = (size_t)N * Rp;
+    if (c.ncat <= 2) return ind_flow(cok_flow_kernel<2>, f, N, Rp, C, bytes, s, c, node, k, Rp, u, seed, C);
+    if (c.ncat <= 4) return ind_flow(cok_flow_kernel<4>, f, N, Rp, C, bytes, s, c, node, k, Rp, u, seed, C);
+    return ind_flow(cok_flow_kernel<8>, f, N, Rp, C, bytes, s, c, node, k, Rp, u, seed, C);
 }
 
-// One level of the multivariate Gaussian sweep: one thread per (position,
-// 4 realizations).  mu^_t = cst_t + sum_j sum_b w[j][b][t] v_b(x_j) over the
-// system's grid neighbours, then v = mu^ + F z with z the given normals or
-// the seeded ones of pseudo-node a*N + g (variable a of node g).
-__global__ void __launch_bounds__(256) mv_level_kernel(const CokArgs c, const int32_t* __restrict__ node, int k,
-                                                       int64_t N, int64_t p0, int64_t p1, int Rp,
-                                                       const double* __restrict__ z, uint64_t seed,
-                                                       double* __restrict__ V) {
-    const int cpn = Rp >> 2, L = c.ncat;
-    const int64_t total = (p1 - p0) * cpn;
-    for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < total;
-         it += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pos = p0 + it / cpn;
-        const int ch = (int)(it % cpn);
+// The multivariate Gaussian sweep: mu^_t = cst_t + sum_j sum_b w[j][b][t]
+// v_b(x_j) over the system's grid neighbours, then v = mu^ + F z with z the
+// given normals or the seeded ones of pseudo-node a*N + g (variable a of node
+// g).  LM: the variables' bound (2, 4, 8), 8 / LM neighbours at a time.  136
+// levels of 160 x 160 nodes, two variables x 16: 8.9 ms by level launches,
+// 0.44 so.
+template <int LM>
+__global__ void __launch_bounds__(256) mv_flow_kernel(const CokArgs c, const int32_t* __restrict__ node, int k, int64_t N,
+                                                      int Rp, const double* __restrict__ z, uint64_t seed, double* V,
+                                                      const __grid_constant__ FlowArgs f, int W) {
+    constexpr int AHEAD = 8 / LM;
+    const int lane = threadIdx.x & 31, S = 32 / W, s = lane / W, L = c.ncat;
+    bool ok = true;
+    for (FlowItems next(f); next.live(); next.step()) {
+        const int64_t pos = next.position();
+        const int r = (int)(next.it - pos * f.H) * W + lane % W;
+        const bool on = r < Rp;
         const int64_t g = node[pos];
         const int m = c.m[pos];
-        double mu[4][IND_MAX_CAT];
+        // what nothing has to wait for: the noise F z and the constant
+        double mu[LM], out[LM];
 #pragma unroll
-        for (int t = 0; t < IND_MAX_CAT; ++t) {
-            const double v = t < L ? c.cst[pos * L + t] : 0.0;
+        for (int t = 0; t < LM; ++t) mu[t] = out[t] = 0.0;
+        if (s == 0 && on) {
+            const double* F = c.fac + pos * L * L;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) mu[r][t] = v;
-        }
-        for (int j = 0; j < m; ++j) {
-            const int64_t e = pos * k + j;
-            const int64_t nb = c.idx[e];
-            for (int b = 0; b < L; ++b) {
-                const double* vb = V + ((int64_t)b * N + nb) * Rp + 4 * ch;
-                const double v0 = vb[0], v1 = vb[1], v2 = vb[2], v3 = vb[3];
-                const double* wr = c.w + (e * L + b) * L;
-#pragma unroll
-                for (int t = 0; t < IND_MAX_CAT; ++t)
-                    if (t < L) {
-                        const double wt = wr[t];
-                        mu[0][t] += wt * v0;
-                        mu[1][t] += wt * v1;
-                        mu[2][t] += wt * v2;
-                        mu[3][t] += wt * v3;
+            for (int b = 0; b < LM; ++b)
+                if (b < L) {
+                    double zb;
+                    if (z) {
+                        zb = z[((int64_t)b * N + g) * Rp + r];
+                    } else {
+                        const float4 n4 = normals4(seed, (int64_t)b * N + g, r >> 2);
+                        zb = (double)((r & 2) ? ((r & 1) ? n4.w : n4.z) : ((r & 1) ? n4.y : n4.x));
                     }
-            }
-        }
-        double zz[4][IND_MAX_CAT];
 #pragma unroll
-        for (int a = 0; a < IND_MAX_CAT; ++a) {
-            if (a < L) {
-                if (z) {
-                    const double* za = z + ((int64_t)a * N + g) * Rp + 4 * ch;
-                    zz[0][a] = za[0];
-                    zz[1][a] = za[1];
-                    zz[2][a] = za[2];
-                    zz[3][a] = za[3];
-                } else {
-                    const float4 f = normals4(seed, (int64_t)a * N + g, ch);
-                    zz[0][a] = f.x;
-                    zz[1][a] = f.y;
-                    zz[2][a] = f.z;
-                    zz[3][a] = f.w;
+                    for (int t = b; t < LM; ++t)
+                        if (t < L) out[t] += F[t * L + b] * zb;
                 }
-            } else {
-                zz[0][a] = zz[1][a] = zz[2][a] = zz[3][a] = 0.0;
-            }
+#pragma unroll
+            for (int t = 0; t < LM; ++t)
+                if (t < L) mu[t] = c.cst[pos * L + t];
         }
-        const double* F = c.fac + pos * L * L;
+        // the weights are on their way to L1 while the values are waited for
+        const double* w = c.w + pos * k * L * L;
+        for (int b = lane * 16; b < m * L * L; b += 512)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(w + b));
+        for (int j0 = 0; j0 < m; j0 += AHEAD * S) {
+            const double* p[AHEAD];
+            double v[AHEAD][LM];
 #pragma unroll
-        for (int t = 0; t < IND_MAX_CAT; ++t) {
-            if (t < L) {
+            for (int h = 0; h < AHEAD; ++h) {
+                const int j = j0 + h * S + s;
+                p[h] = ok && on && j < m ? V + (int64_t)c.idx[pos * k + j] * Rp + r : nullptr;
 #pragma unroll
-                for (int u = 0; u < IND_MAX_CAT; ++u)
-                    if (u <= t) {
-                        const double f = F[t * L + u];
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) mu[r][t] += f * zz[r][u];
-                    }
-                double* vt = V + ((int64_t)t * N + g) * Rp + 4 * ch;
-#pragma unroll
-                for (int r = 0; r < 4; ++r) vt[r] = mu[r][t];
+                for (int b = 0; b < LM; ++b)
+                    if (p[h] && b < L) v[h][b] = ld_value(p[h] + b * N * Rp);
             }
+            FlowBound bound;
+            while (ok) {
+                bool miss = false;
+#pragma unroll
+                for (int h = 0; h < AHEAD; ++h)
+#pragma unroll
+                    for (int b = 0; b < LM; ++b) miss |= p[h] && b < L && missing(v[h][b]);
+                if (!miss) break;
+                ok = bound.more(f.err, f.wait_ns);
+#pragma unroll
+                for (int h = 0; h < AHEAD; ++h)
+#pragma unroll
+                    for (int b = 0; b < LM; ++b)
+                        if (p[h] && b < L && missing(v[h][b])) v[h][b] = ld_value(p[h] + b * N * Rp);
+            }
+#pragma unroll
+            for (int h = 0; h < AHEAD; ++h)
+                if (p[h]) {
+#pragma unroll
+                    for (int b = 0; b < LM; ++b)
+                        if (b < L) {
+                            const double* wr = w + ((j0 + h * S + s) * L + b) * L;
+#pragma unroll
+                            for (int t = 0; t < LM; ++t)
+                                if (t < L) mu[t] += wr[t] * v[h][b];
+                        }
+                }
         }
+        __syncwarp();
+        for (int o = W; o < 32; o <<= 1)
+#pragma unroll
+            for (int t = 0; t < LM; ++t)
+                if (t < L) mu[t] += __shfl_xor_sync(FULL_MASK, mu[t], o);
+        if (s == 0 && on)
+#pragma unroll
+            for (int t = 0; t < LM; ++t)
+                if (t < L) st_value(V + ((int64_t)t * N + g) * Rp + r, ok ? mu[t] + out[t] : settle(unstored<double>()));
     }
 }
 
-cudaError_t launch_mv_level(const CokArgs& c, const int32_t* node, int k, int64_t N, int64_t p0, int64_t p1, int Rp,
-                            const double* z, uint64_t seed, double* V, cudaStream_t s) {
-    if (p1 <= p0) return cudaSuccess;
-    int64_t blocks = ((p1 - p0) * (Rp / 4) + 255) / 256;
-    if (blocks > (1 << 20)) blocks = 1 << 20;
-    mv_level_kernel<<<(int)blocks, 256, 0, s>>>(c, node, k, N, p0, p1, Rp, z, seed, V);
-    return cudaGetLastError();
+cudaError_t launch_mv_flow(const CokArgs& c, const int32_t* node, int k, int64_t N, int Rp, const double* z,
+                           uint64_t seed, double* V, const FlowArgs& f, cudaStream_t s) {
+    const size_t bytes = (size_t)N * c.ncat * Rp * sizeof(double);
+    if (c.ncat <= 2) return ind_flow(mv_flow_kernel<2>, f, N, Rp, V, bytes, s, c, node, k, N, Rp, z, seed, V);
+    if (c.ncat <= 4) return ind_flow(mv_flow_kernel<4>, f, N, Rp, V, bytes, s, c, node, k, N, Rp, z, seed, V);
+    return ind_flow(mv_flow_kernel<8>, f, N, Rp, V, bytes, s, c, node, k, N, Rp, z, seed, V);
 }
 
 // node-major category bytes [N][Rp] -> realization-major int32 [R][N]

@@ -257,10 +257,11 @@ struct IndArgs {
     const double* wsum;          // [P] sum of a system's weights (0 for the prior)
     const double* dsum;          // [P][ncat] weights of data of each category
 };
-cudaError_t launch_sis_level_fp32(const SweepTables<float>& t, int k, int64_t p0, int64_t p1, int Rp,
-                                  const IndArgs& ia, const double* u, uint64_t seed, uint8_t* C, cudaStream_t s);
-cudaError_t launch_sis_level_fp64(const SweepTables<double>& t, int k, int64_t p0, int64_t p1, int Rp,
-                                  const IndArgs& ia, const double* u, uint64_t seed, uint8_t* C, cudaStream_t s);
+// dataflow launches over all positions; f: error flag, tickets and wait_ns
+cudaError_t launch_sis_flow_fp32(const SweepTables<float>& t, int k, int64_t N, int Rp, const IndArgs& ia,
+                                 const double* u, uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s);
+cudaError_t launch_sis_flow_fp64(const SweepTables<double>& t, int k, int64_t N, int Rp, const IndArgs& ia,
+                                 const double* u, uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s);
 cudaError_t launch_cats_to_out(const uint8_t* C, int64_t N, int R, int Rp, int32_t* out, cudaStream_t s);
 
 // Full simple cokriging of the indicators (indicator.cu) for a linear model
@@ -288,13 +289,13 @@ struct CokArgs {
 // systems of every position (a: geometry, neighbours, order, status; the
 // status of each node is overwritten with its cokriging status)
 cudaError_t launch_cok_solve(const SolveArgs& a, const CokArgs& c, bool gaussian, cudaStream_t s);
-cudaError_t launch_cok_level(const CokArgs& c, const int32_t* node, int k, int64_t p0, int64_t p1, int Rp,
-                             const double* u, uint64_t seed, uint8_t* C, cudaStream_t s);
-// One level of the multivariate Gaussian sweep.  V: values [L][N][Rp]
-// (variable-major rows of Rp realizations); z: the normals in the same
-// layout, or null for the seeded normals of pseudo-node a*N + g.
-cudaError_t launch_mv_level(const CokArgs& c, const int32_t* node, int k, int64_t N, int64_t p0, int64_t p1, int Rp,
-                            const double* z, uint64_t seed, double* V, cudaStream_t s);
+cudaError_t launch_cok_flow(const CokArgs& c, const int32_t* node, int k, int64_t N, int Rp, const double* u,
+                            uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s);
+// The multivariate Gaussian sweep.  V: values [L][N][Rp] (variable-major rows
+// of Rp realizations); z: the normals in the same layout, or null for the
+// seeded normals of pseudo-node a*N + g.
+cudaError_t launch_mv_flow(const CokArgs& c, const int32_t* node, int k, int64_t N, int Rp, const double* z,
+                           uint64_t seed, double* V, const FlowArgs& f, cudaStream_t s);
 
 // Host-side description of one problem (api.cu: host_domain): everything
 // sgs_plan_create derives on the host before uploading.

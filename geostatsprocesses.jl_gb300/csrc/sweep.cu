@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "flow.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -30,30 +31,11 @@ struct Vec4<float> {
     __device__ static void store(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 };
 
-struct D4 {
-    double x, y, z, w;
-};
 __device__ __forceinline__ D4 load_d4(const double* p) {
     const double2 a = reinterpret_cast<const double2*>(p)[0];
     const double2 b = reinterpret_cast<const double2*>(p)[1];
     return {a.x, a.y, b.x, b.y};
 }
-// All ones in a value's words stands for "not yet stored" in a dataflow launch
-// (below); no other NaN does, and a stored value never has it.
-__device__ __forceinline__ bool missing(float v) { return __float_as_uint(v) == 0xffffffffu; }
-__device__ __forceinline__ bool missing(double v) { return __double2hiint(v) == -1 && __double2loint(v) == -1; }
-template <typename T>
-__device__ __forceinline__ T unstored();
-template <>
-__device__ __forceinline__ float unstored<float>() { return __uint_as_float(0xffffffffu); }
-template <>
-__device__ __forceinline__ double unstored<double>() { return __hiloint2double(-1, -1); }
-template <typename V>
-__device__ __forceinline__ bool missing4(const V& v) {
-    return missing(v.x) || missing(v.y) || missing(v.z) || missing(v.w);
-}
-__device__ __forceinline__ float settle(float v) { return missing(v) ? __uint_as_float(0x7fffffffu) : v; }
-__device__ __forceinline__ double settle(double v) { return missing(v) ? __hiloint2double(0x7fffffff, -1) : v; }
 __device__ __forceinline__ void store_d4(double* p, D4 v) {
     reinterpret_cast<double2*>(p)[0] = make_double2(settle(v.x), settle(v.y));
     reinterpret_cast<double2*>(p)[1] = make_double2(settle(v.z), settle(v.w));
@@ -524,47 +506,6 @@ cudaError_t launch_sweep_all_fp64(const SweepTables<double>& t, int k, const int
 // Lane layout inside a warp: W lanes per slice of the neighbour list (a
 // power of two), S = 32 / W slices, each lane G chunks of the piece
 // (P4 = W * G); the S partial sums are combined across lanes at the end.
-__device__ __forceinline__ float4 ld_value4(const float* p) {
-    float4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
-__device__ __forceinline__ D4 ld_value4(const double* p) {
-    D4 v;
-    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
-    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "l"(p + 2) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_value4(float* p, float4 v) {
-    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(settle(v.x)), "f"(settle(v.y)),
-                 "f"(settle(v.z)), "f"(settle(v.w))
-                 : "memory");
-}
-__device__ __forceinline__ void st_value4(double* p, D4 v) {
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(settle(v.x)), "d"(settle(v.y)) : "memory");
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + 2), "d"(settle(v.z)), "d"(settle(v.w))
-                 : "memory");
-}
-
-// A wait's bound: wait_ns of wall-clock time or, should the timer stall, a
-// count of polls (each a load from L2, far above 16 ns, so the count is
-// reached no earlier).  False once it has run out or another wait has.
-struct FlowBound {
-    uint64_t t0 = 0, polls = 0;
-    __device__ __forceinline__ bool more(int32_t* err, uint64_t wait_ns) {
-        if (++polls > 16) __nanosleep(32);
-        if (polls & 63) return true;
-        const uint64_t now = global_ns();
-        if (t0 == 0) t0 = now;
-        if (!*(volatile int32_t*)err && now - t0 <= wait_ns && polls <= wait_ns / 16 + 1024) return true;
-        atomicExch(err, 1);
-        return false;
-    }
-};
-
 // The sums of one chunk (4 realizations): FP32 values with (hi, lo) weights
 // and compensated sums, FP64 values with plain FMA sums.
 template <typename T>
@@ -655,39 +596,18 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
     using Weight = typename Sum::Weight;
     using Value = typename Sum::Value;
     const int lane = threadIdx.x & 31;
-    const int64_t items = f.item1;
     const int S = 32 / W, s = lane / W, cl = lane % W, cpn = Rp >> 2;
     const int64_t Rs = f.row_stride ? f.row_stride : Rp;
     const int pairs = CSR && sizeof(T) == 8 ? f.pairs : 0;
     if (CSR && f.seed_dev) seed = *f.seed_dev;
-    // a ticket of the warp's class, or the end once an error is raised (the
-    // two reads overlap)
-    const int cls = threadIdx.x >> 5;
-    auto take = [&]() {
-        unsigned long long base = 0;
-        if (lane == 0) {
-            base = f.item0 + (atomicAdd(f.ticket + cls * FLOW_TICKET_STRIDE, 1ull) * FLOW_CLASSES + cls) * f.chunk;
-            if (*(volatile int32_t*)f.err) base = (unsigned long long)items;
-        }
-        return base;
-    };
-    unsigned long long ticket = take();
-    int64_t it = 0, end = 0;  // the next item, and the end of its ticket
-    auto step = [&]() {
-        if (++it < end) return;
-        it = (int64_t)__shfl_sync(FULL_MASK, ticket, 0);
-        end = min(it + f.chunk, items);
-        if (it < items) ticket = take();
-    };
-    // it / H by a reciprocal: exact while it * H < 2^64
-    auto position = [&](int64_t i) { return f.H == 1 ? i : (int64_t)__umul64hi((uint64_t)i, f.rec); };
+    FlowItems next(f);
     // the next item's tables
     int64_t nrow = 0;
     int ng = 0, nm = 0, nidx = 0;
     Weight nw{};
     auto tables = [&]() {
-        if (it >= items) return;
-        const int64_t pos = position(it);
+        if (!next.live()) return;
+        const int64_t pos = next.position();
         ng = t.node[pos];
         nm = t.m[pos];
         nrow = CSR ? t.off[pos] : pos * (int64_t)k;
@@ -696,16 +616,15 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
             nw = Sum::entry(t.w, nrow + lane, pairs);
         }
     };
-    step();
     tables();
-    while (it < items) {
-        const int64_t pos = position(it);
-        const int c0 = (int)(it - pos * f.H) * (W * G);
+    while (next.live()) {
+        const int64_t pos = next.position();
+        const int c0 = (int)(next.it - pos * f.H) * (W * G);
         const int64_t row = nrow;
         const int g = ng, m = nm;
         int idx = nidx;
         Weight w = nw;
-        step();
+        next.step();
         tables();
         if (CSR && f.node_class && f.node_class[g] != f.cls) continue;  // the other launch's node
         // the draws and the node's own terms: nothing of them waits
