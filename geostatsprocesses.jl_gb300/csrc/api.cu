@@ -111,6 +111,7 @@ struct sgs_plan {
     double mv_mean[IND_MAX_CAT] = {};
     double* d_mv_dval = nullptr;  // [D][L]
     double* d_mv_fac = nullptr;   // [N][L][L]
+    double* d_cok_lut = nullptr;  // covariances by structure and lag
     // FP32 refinement whose weights amplify the rounding of FP32 values: the
     // sweep keeps FP64 values, from FP64 copies of the (hi, lo) tables
     unsigned int* d_wl1 = nullptr;
@@ -985,6 +986,7 @@ static CokArgs cok_args(const sgs_plan* P) {
     c.w = P->d_cok_w;
     c.cst = P->d_cok_cst;
     c.fac = P->d_mv_fac;
+    c.lut = P->d_cok_lut;
     return c;
 }
 
@@ -1198,6 +1200,14 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
         s.N = P->N;
         s.data_xyz = P->d_dxyz;
         s.status = P->d_status;
+        s.lut = P->lut;
+        if (P->d_lut64 && !P->d_cok_lut) {
+            const size_t lags = (size_t)P->lut.w[0] * P->lut.w[1] * P->lut.w[2];
+            if (lags * P->vario.ns <= (size_t)1 << 26) {
+                if ((rc = dalloc(P, &P->d_cok_lut, lags * P->vario.ns))) return rc;
+                LAUNCH(P, 1, launch_cok_lut(P->grid, P->vario, P->lut, P->d_cok_lut, st));
+            }
+        }
         LAUNCH(P, 1, launch_cok_solve(s, cok_args(P), P->mv, st));
     }
     CK(P, cudaEventRecord(P->ev[4], st));

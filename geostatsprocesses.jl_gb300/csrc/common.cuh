@@ -446,45 +446,71 @@ __device__ __forceinline__ int warp_levels(bool active, int g, const int32_t* __
     }
 }
 
-// Right-looking Cholesky of the lower triangle of A (leading dimension ld)
-// by one warp.  Fails (returns false) when a pivot is not > tau.
-template <typename T>
-__device__ bool warp_cholesky(T* A, int ld, int n, T tau, int lane) {
-    for (int j = 0; j < n; ++j) {
-        const T d = A[j * ld + j];
+// 1 / d of a pivot (positive, normal): an FP32 reciprocal r of its mantissa,
+// off by e = 1 - d r of some 2^-22, and one step of third order, r (1 + e +
+// e^2).  The exponents are handled as integers, off the FP64 pipe.
+__device__ __forceinline__ double reciprocal(double d) {
+    const unsigned hi = __double2hiint(d), lo = __double2loint(d);
+    float rf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(__uint_as_float(0x3f800000u | (hi & 0xfffffu) << 3 | lo >> 29)));
+    const unsigned u = __float_as_uint(rf);
+    const double r = __hiloint2double((int)((u >> 3) + (896u << 20) + (1023u << 20) - (hi & 0x7ff00000u)), (int)(u << 29));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// Rows of a symmetric FP64 system in shared memory: ld of them apart, 8 more
+// than a multiple of 16 doubles, so that 2 x 8 entries use all banks.
+__host__ __device__ constexpr int ldl_stride(int rows) { return (rows + 7) / 16 * 16 + 8; }
+
+// L D L' of the leading m rows of K (lower triangle) by one warp, carried on
+// through rows m .. M - 1: right-hand sides c, which end up as D^-1 L^-1 c,
+// with the lower triangle of any symmetric block C beyond column m, which
+// becomes the Schur complement C - c' K^-1 c.  False at the first pivot not
+// above tau.  Steps take 4 rows x 8 columns at a time, one FP64 instruction
+// each: about (M - j)^2 / 64 for step j instead of M - j with a row per lane,
+// and a reciprocal instead of a square root and three divisions a column.
+// av, fv: M entries of scratch.
+__device__ __forceinline__ bool warp_ldl(double* K, int ld, int m, int M, double tau, double* av, double* fv, int lane) {
+    const int r = lane >> 3, c = lane & 7;
+    for (int j = 0; j < m; ++j) {
+        const double d = K[j * ld + j];
         if (!(d > tau)) return false;
-        const T ljj = sqrt(d);
-        const T inv = T(1) / ljj;
+        const double inv = reciprocal(d);
+        for (int i = j + 1 + lane; i < M; i += 32) {
+            const double a = K[i * ld + j], f = a * inv;
+            av[i] = a;
+            fv[i] = -f;
+            K[i * ld + j] = f;
+        }
         __syncwarp();
-        for (int i = j + 1 + lane; i < n; i += 32) A[i * ld + j] *= inv;
-        if (lane == 0) A[j * ld + j] = ljj;
-        __syncwarp();
-        for (int i = j + 1 + lane; i < n; i += 32) {
-            const T lij = A[i * ld + j];
-            for (int l = j + 1; l <= i; ++l) A[i * ld + l] -= lij * A[l * ld + j];
+        for (int i0 = j + 1; i0 < M; i0 += 4) {
+            const int i = i0 + r, top = min(i, M - 1);
+            const double f = fv[top];
+            double* row = K + top * ld;
+#pragma unroll 4
+            for (int l = j + 1 + c; l - c <= min(i0 + 3, M - 1); l += 8)
+                if (i < M && l <= i) row[l] = fma(f, av[l], row[l]);
         }
         __syncwarp();
     }
     return true;
 }
 
-// Solve L L^T x = b in place (x overwrites b), L from warp_cholesky.
-template <typename T>
-__device__ void warp_chol_solve(const T* A, int ld, int n, T* b, int lane) {
-    for (int j = 0; j < n; ++j) {
-        const T yj = b[j] / A[j * ld + j];
-        __syncwarp();
-        if (lane == 0) b[j] = yj;
-        for (int i = j + 1 + lane; i < n; i += 32) b[i] -= A[i * ld + j] * yj;
-        __syncwarp();
+// Row `rhs` of a system warp_ldl has been through, D^-1 L^-1 c, becomes the
+// solution K^-1 c (m <= 64).
+__device__ __forceinline__ void warp_ldl_solve(double* K, int ld, int m, int rhs, int lane) {
+    double* z = K + rhs * ld;
+    double z0 = lane < m ? z[lane] : 0.0, z1 = lane + 32 < m ? z[lane + 32] : 0.0;
+    for (int j = m - 1; j > 0; --j) {
+        const double zj = __shfl_sync(FULL_MASK, j < 32 ? z0 : z1, j & 31);
+        const double* row = K + j * ld;
+        if (lane < j) z0 = fma(-row[lane], zj, z0);
+        if (j > 32 && lane + 32 < j) z1 = fma(-row[lane + 32], zj, z1);
     }
-    for (int j = n - 1; j >= 0; --j) {
-        const T wj = b[j] / A[j * ld + j];
-        __syncwarp();
-        if (lane == 0) b[j] = wj;
-        for (int i = lane; i < j; i += 32) b[i] -= A[j * ld + i] * wj;
-        __syncwarp();
-    }
+    if (lane < m) z[lane] = z0;
+    if (lane + 32 < m) z[lane + 32] = z1;
+    __syncwarp();
 }
 
 // ---- batches of domains: global numbering and per-domain descriptors ----

@@ -293,14 +293,14 @@ cudaError_t launch_sis_flow_fp64(const SweepTables<double>& t, int k, int64_t N,
 // the prior): v = mu^ + F z.  F's rule: a pivot not above tau contributes
 // nothing (its column of F is zero), so a conditional covariance that is zero
 // up to rounding (a node on a datum) draws no noise.
-constexpr int COK_WARPS = 2;
+constexpr int COK_WARPS = 4;
 
-__host__ __device__ constexpr size_t cok_smem_per_warp(bool gauss) {
-    return (size_t)COK_MAX * (COK_MAX + 1) * sizeof(double)                // LHS
-           + (size_t)COK_MAX * IND_MAX_CAT * sizeof(double)                // right-hand sides -> weights
-           + (size_t)COK_MAX * sizeof(double)                              // one column being solved
-           + (gauss ? (size_t)COK_MAX * IND_MAX_CAT * sizeof(double) : 0)  // right-hand sides kept
-           + (size_t)KMAX * 4 * sizeof(int);                               // neighbour cells / data ids
+// K, L right-hand sides and C(0) below it; two vectors; neighbour cells / data
+// ids; for up to n neighbours
+__host__ __device__ constexpr int cok_rows(int n, int L) { return n * L + L; }
+__host__ __device__ constexpr size_t cok_smem_per_warp(int n, int L) {
+    const int M = cok_rows(n, L);
+    return (size_t)(M * ldl_stride(M) + 2 * ((M + 1) / 2 * 2)) * sizeof(double) + (size_t)n * 4 * sizeof(int);
 }
 
 // lower Cholesky factor of the L x L symmetric matrix S (lower triangle,
@@ -312,12 +312,12 @@ __device__ __forceinline__ void mv_factor(const double* S, int L, double tau, do
         double d = S[j * L + j];
         for (int l = 0; l < j; ++l) d -= F[j * L + l] * F[j * L + l];
         if (!(d > tau)) continue;
-        const double fjj = sqrt(d);
+        const double fjj = sqrt_fp64(d), inv = reciprocal(fjj);
         F[j * L + j] = fjj;
         for (int i = j + 1; i < L; ++i) {
             double t = S[i * L + j];
             for (int l = 0; l < j; ++l) t -= F[i * L + l] * F[j * L + l];
-            F[i * L + j] = t / fjj;
+            F[i * L + j] = t * inv;
         }
     }
 }
@@ -343,28 +343,75 @@ __device__ __forceinline__ void cok_lag(const SolveArgs& a, const int* ca, const
     }
 }
 
+// C_s(h) of every structure: from the lag table, or evaluated
+__device__ __forceinline__ void cok_cov(const SolveArgs& a, const CokArgs& c, const int* ca, const int* cb, double* cs) {
+    const int S = a.vario.ns;
+    if (c.lut && ca[3] < 0 && cb[3] < 0) {
+        const CovLut& t = a.lut;
+        const int l0 = cb[0] - ca[0], l1 = cb[1] - ca[1], l2 = cb[2] - ca[2];
+        if (abs(l0) <= t.e[0] && abs(l1) <= t.e[1] && abs(l2) <= t.e[2]) {
+            const double* e = c.lut + ((l0 + t.e[0]) + t.w[0] * ((l1 + t.e[1]) + t.w[1] * (l2 + t.e[2])));
+            const int64_t total = (int64_t)t.w[0] * t.w[1] * t.w[2];
+            for (int s = 0; s < S; ++s) cs[s] = e[s * total];
+            return;
+        }
+    }
+    double h[3];
+    cok_lag(a, ca, cb, h);
+    for (int s = 0; s < S; ++s) cs[s] = structure_cov(a.vario.st[s], a.grid.dim, h[0], h[1], h[2]);
+}
+
+__global__ void cok_lut_kernel(const GridDev G, const VarioDev v, const CovLut t, int64_t total, double* out) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int L0 = (int)(i % t.w[0]) - t.e[0];
+        const int64_t r = i / t.w[0];
+        const int L1 = (int)(r % t.w[1]) - t.e[1];
+        const int L2 = (int)(r / t.w[1]) - t.e[2];
+        for (int s = 0; s < v.ns; ++s)
+            out[s * total + i] = structure_cov(v.st[s], G.dim, dmul((double)L0, G.spacing[0]), dmul((double)L1, G.spacing[1]),
+                                               G.dim == 3 ? dmul((double)L2, G.spacing[2]) : 0.0);
+    }
+}
+
+cudaError_t launch_cok_lut(const GridDev& g, const VarioDev& v, const CovLut& lut, double* out, cudaStream_t s) {
+    const int64_t total = (int64_t)lut.w[0] * lut.w[1] * lut.w[2];
+    cok_lut_kernel<<<(int)std::min<int64_t>((total + 127) / 128, 65535), 128, 0, s>>>(g, v, lut, total, out);
+    return cudaGetLastError();
+}
+
+// One warp per system: its n L equations, L right-hand sides and C(0) in
+// shared memory, eliminated together (warp_ldl), which leaves C(0) - c'
+// Lambda.  FP64 instructions bound it.  25.6k systems of 16 neighbours x 2
+// variables took 5.9 ms with covariances evaluated pair by pair, a Cholesky
+// factorization, two substitutions with divisions per variable and shared
+// memory for 64 equations whatever their number; 1.5 so.
 template <bool GAUSS>
-__global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const SolveArgs a, const CokArgs c) {
+__global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const __grid_constant__ SolveArgs a, const CokArgs c) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned char* base = smem + (size_t)wib * cok_smem_per_warp(GAUSS);
-    double* A = reinterpret_cast<double*>(base);
-    double* rhs = A + COK_MAX * (COK_MAX + 1);
-    double* col = rhs + COK_MAX * IND_MAX_CAT;
-    double* rhs0 = col + COK_MAX;  // GAUSS: the right-hand sides, kept
-    int* cell = reinterpret_cast<int*>(GAUSS ? rhs0 + COK_MAX * IND_MAX_CAT : rhs0);  // [n][4]: c0, c1, c2,
-                                                                                       // data id (-1: grid)
     const GridDev& G = a.grid;
-    const int L = c.ncat, k = a.k, S = a.vario.ns;
+    const int L = c.ncat, k = a.k, S = a.vario.ns, Mk = cok_rows(k, L), ld = ldl_stride(Mk);
+    double* A = reinterpret_cast<double*>(smem + (size_t)wib * cok_smem_per_warp(k, L));
+    double* av = A + Mk * ld;
+    double* fv = av + (Mk + 1) / 2 * 2;
+    int* cell = reinterpret_cast<int*>(fv + (Mk + 1) / 2 * 2);  // [n][4]: c0, c1, c2, data id (-1: grid)
     const int nwarps = gridDim.x * COK_WARPS;
     for (int64_t pos = (int64_t)blockIdx.x * COK_WARPS + wib; pos < a.P; pos += nwarps) {
         const int g = a.order[pos];
         const int n = a.cnt[g];
-        const int m = n * L, ld = m + 1;
+        const int m = n * L;
         int self[4];
         cell_of(G, g, self[0], self[1], self[2]);
         self[3] = -1;
         bool kriged = n >= a.nmin;
+        double* rhs = A + m * ld;  // row t: right-hand side t, then the weights Lambda[(i, a), t]
+        // C(0) beside the right-hand sides
+        for (int e = lane; e < L * L; e += 32) {
+            const int t = e / L, u = e - t * L;
+            double v = 0.0;
+            for (int s = 0; s < S; ++s) v += c.coef[(s * L + t) * L + u] * a.vario.st[s].sill;
+            rhs[t * ld + m + u] = v;
+        }
         if (kriged) {
             for (int q = lane; q < n; q += 32) {
                 const int id = a.nbr[(int64_t)g * k + q];
@@ -380,13 +427,12 @@ __global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const SolveAr
             __syncwarp();
             // lower triangle of the LHS, one neighbour pair (i >= j) per lane
             for (int item = lane; item < n * (n + 1) / 2; item += 32) {
-                int i = (int)((sqrt(8.0 * item + 1.0) - 1.0) * 0.5);
+                int i = (int)((sqrtf(8.0f * (float)item + 1.0f) - 1.0f) * 0.5f);
                 while (i * (i + 1) / 2 > item) --i;
                 while ((i + 1) * (i + 2) / 2 <= item) ++i;
                 const int j = item - i * (i + 1) / 2;
-                double h[3], cs[SGS_MAX_STRUCTURES];
-                cok_lag(a, cell + 4 * j, cell + 4 * i, h);
-                for (int s = 0; s < S; ++s) cs[s] = structure_cov(a.vario.st[s], G.dim, h[0], h[1], h[2]);
+                double cs[SGS_MAX_STRUCTURES];
+                cok_cov(a, c, cell + 4 * j, cell + 4 * i, cs);
                 for (int ai = 0; ai < L; ++ai)
                     for (int b = 0; b < L; ++b) {
                         const int r = i * L + ai, q = j * L + b;
@@ -397,45 +443,37 @@ __global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const SolveAr
                     }
             }
             for (int i = lane; i < n; i += 32) {
-                double h[3], cs[SGS_MAX_STRUCTURES];
-                cok_lag(a, self, cell + 4 * i, h);
-                for (int s = 0; s < S; ++s) cs[s] = structure_cov(a.vario.st[s], G.dim, h[0], h[1], h[2]);
+                double cs[SGS_MAX_STRUCTURES];
+                cok_cov(a, c, self, cell + 4 * i, cs);
                 for (int ai = 0; ai < L; ++ai)
                     for (int t = 0; t < L; ++t) {
                         double v = 0.0;
                         for (int s = 0; s < S; ++s) v += c.coef[(s * L + ai) * L + t] * cs[s];
-                        rhs[(i * L + ai) * IND_MAX_CAT + t] = v;
-                        if constexpr (GAUSS) rhs0[(i * L + ai) * IND_MAX_CAT + t] = v;
+                        rhs[t * ld + i * L + ai] = v;
                     }
             }
             __syncwarp();
-            kriged = warp_cholesky<double>(A, ld, m, c.tau, lane);
+            kriged = warp_ldl(A, ld, m, m + L, c.tau, av, fv, lane);
         }
-        if (kriged) {
-            for (int t = 0; t < L; ++t) {
-                for (int r = lane; r < m; r += 32) col[r] = rhs[r * IND_MAX_CAT + t];
-                __syncwarp();
-                warp_chol_solve<double>(A, ld, m, col, lane);
-                for (int r = lane; r < m; r += 32) rhs[r * IND_MAX_CAT + t] = col[r];  // Lambda[(i, a), t]
-                __syncwarp();
-            }
-        }
+        if (kriged)
+            for (int t = 0; t < L; ++t) warp_ldl_solve(A, ld, m, m + t, lane);
+        __syncwarp();
         if constexpr (GAUSS) {
-            // conditional covariance C(0) - c' Lambda (the prior's C(0) for a
-            // node without a system), lower triangle into col, then its factor
-            for (int e = lane; e < L * L; e += 32) {
-                const int t = e / L, u = e - t * L;
-                if (u > t) continue;
-                double v = 0.0;
-                for (int s = 0; s < S; ++s) v += c.coef[(s * L + t) * L + u] * a.vario.st[s].sill;
-                if (kriged)
-                    for (int r = 0; r < m; ++r) v -= rhs0[r * IND_MAX_CAT + t] * rhs[r * IND_MAX_CAT + u];
-                col[t * L + u] = v;
-            }
-            __syncwarp();
+            // the factor of the conditional covariance (the prior's C(0) for
+            // a node without a system)
             if (lane == 0) {
-                double F[IND_MAX_CAT * IND_MAX_CAT];
-                mv_factor(col, L, c.tau, F);
+                double C0[IND_MAX_CAT * IND_MAX_CAT], F[IND_MAX_CAT * IND_MAX_CAT];
+                for (int t = 0; t < L; ++t)
+                    for (int u = 0; u <= t; ++u) {
+                        double v = 0.0;
+                        if (kriged) {
+                            v = rhs[t * ld + m + u];
+                        } else {  // a factorization may have stopped halfway
+                            for (int s = 0; s < S; ++s) v += c.coef[(s * L + t) * L + u] * a.vario.st[s].sill;
+                        }
+                        C0[t * L + u] = v;
+                    }
+                mv_factor(C0, L, c.tau, F);
                 for (int i = 0; i < L * L; ++i) c.fac[pos * L * L + i] = F[i];
             }
             __syncwarp();
@@ -456,7 +494,7 @@ __global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const SolveAr
                         for (int t = 0; t < L; ++t) {
                             double v = 0.0;
                             for (int ai = 0; ai < L; ++ai) {
-                                const double lam = rhs[(i * L + ai) * IND_MAX_CAT + t];
+                                const double lam = rhs[t * ld + i * L + ai];
                                 v -= lam * c.prob[ai];
                                 if (d >= 0) v += lam * c.data_val[(int64_t)d * L + ai];
                             }
@@ -467,7 +505,7 @@ __global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const SolveAr
                         for (int t = 0; t < L; ++t) {
                             double v = 0.0;
                             for (int ai = 0; ai < L; ++ai) {
-                                const double lam = rhs[(i * L + ai) * IND_MAX_CAT + t];
+                                const double lam = rhs[t * ld + i * L + ai];
                                 v -= lam * c.prob[ai];
                                 if (ai == dcat) v += lam;
                             }
@@ -480,7 +518,7 @@ __global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const SolveAr
                         c.idx[e] = a.nbr[(int64_t)g * k + i];
                         for (int b = 0; b < L; ++b)
                             for (int t = 0; t < L; ++t)
-                                c.w[(e * L + b) * L + t] = rhs[(i * L + b) * IND_MAX_CAT + t];
+                                c.w[(e * L + b) * L + t] = rhs[t * ld + i * L + b];
                     }
                 }
                 mg += __popc(bal);
@@ -505,7 +543,7 @@ static cudaError_t cok_solve(const SolveArgs& a, const CokArgs& c, cudaStream_t 
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = cok_smem_per_warp(GAUSS) * COK_WARPS;
+    const size_t smem = cok_smem_per_warp(a.k, c.ncat) * COK_WARPS;
     cudaError_t e =
         cudaFuncSetAttribute(cok_solve_kernel<GAUSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

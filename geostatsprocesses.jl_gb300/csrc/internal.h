@@ -283,11 +283,14 @@ struct CokArgs {
     int32_t* idx;                // [P][k] their node ids
     double* w;                   // [P][k][L][L] weight of (grid neighbour j, its category b) for category t
     double* cst;                 // [P][L] prior term and the data's contribution
+    const double* lut;           // nullptr, or C_s by lag, [S][lags of SolveArgs::lut]
     double* fac;                 // [P][L][L] Gaussian: lower Cholesky factor of the conditional
                                  // covariance (of the prior's for prior nodes), row-major
 };
 // systems of every position (a: geometry, neighbours, order, status; the
 // status of each node is overwritten with its cokriging status)
+// C_s of every structure s over the lags of `lut` (out: [S][lags])
+cudaError_t launch_cok_lut(const GridDev& g, const VarioDev& v, const CovLut& lut, double* out, cudaStream_t s);
 cudaError_t launch_cok_solve(const SolveArgs& a, const CokArgs& c, bool gaussian, cudaStream_t s);
 cudaError_t launch_cok_flow(const CokArgs& c, const int32_t* node, int k, int64_t N, int Rp, const double* u,
                             uint64_t seed, uint8_t* C, const FlowArgs& f, cudaStream_t s);

@@ -12,9 +12,9 @@
 // bounded); lags involving data points are evaluated directly in FP64.
 //
 // Precision modes:
-//   FP64          one warp per system: FP64 LHS, right-looking Cholesky in
-//                 shared memory, FP64 weights (the plain path; also re-solves
-//                 queued systems)
+//   FP64          FP64 LHS, L D L' and weights: several systems of up to 16
+//                 neighbours per warp in registers, or one warp per system in
+//                 shared memory (the plain path; also re-solves queued systems)
 //   FP32+refine   half a warp per system: register-resident L D L' of the
 //                 FP32 LHS with L^-1 carried in place, refinement against the
 //                 LHS in fixed point with exact residuals, double-FP32
@@ -91,11 +91,9 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-template <typename T>
 __host__ __device__ constexpr size_t warp_smem_bytes(int k) {
-    // A (k x (k+1) of T), c and w (FP64), rhs (T), neighbour info
-    return ((size_t)k * (k + 1) * sizeof(T) + 15) / 16 * 16 + 2 * (size_t)k * sizeof(double) +
-           ((size_t)k * sizeof(T) + 15) / 16 * 16 + (size_t)k * sizeof(NbInfo);
+    // K and the right-hand side's row, two vectors of scratch, neighbour info
+    return (size_t)((k + 1) * ldl_stride(k + 1) + 2 * ((k + 2) / 2 * 2)) * sizeof(double) + (size_t)k * sizeof(NbInfo);
 }
 
 // Indicator sums of one system (SolveArgs::ind_*): w holds the weights of the
@@ -186,23 +184,23 @@ __device__ void write_row(const SolveArgs& a, const SweepTables<O>& tab, int64_t
 // One system (node g, sweep-table row pos) of the problem `a`, in this warp's
 // shared-memory slot `base` laid out for up to kl neighbours (kl >= a.k, or
 // >= the node's neighbour count).
-template <typename T, typename O>
+template <typename O>
 __device__ __forceinline__ void solve_system(const SolveArgs& a, const SweepTables<O>& tab, int64_t pos, int g,
                                              unsigned char* base, int kl, int lane) {
     const int k = a.k;
-    const int ld = kl + 1;
-    T* A = reinterpret_cast<T*>(base);
-    double* c = reinterpret_cast<double*>(base + ((size_t)kl * ld * sizeof(T) + 15) / 16 * 16);
-    double* w = c + kl;
-    T* rhs = reinterpret_cast<T*>(w + kl);
-    NbInfo* info = reinterpret_cast<NbInfo*>(reinterpret_cast<unsigned char*>(rhs) + ((size_t)kl * sizeof(T) + 15) / 16 * 16);
+    const int ld = ldl_stride(kl + 1);
+    double* A = reinterpret_cast<double*>(base);
+    double* av = A + (kl + 1) * ld;
+    double* fv = av + (kl + 2) / 2 * 2;
+    NbInfo* info = reinterpret_cast<NbInfo*>(fv + (kl + 2) / 2 * 2);
     const GridDev& G = a.grid;
     const double sill = a.vario.sill;
     const double prior_sd = sqrt(sill);
     {
         const int n = a.cnt[g];
+        double* c = A + n * ld;  // the right-hand side, then the weights
         if (n < a.nmin) {
-            write_row<O>(a, tab, pos, g, n, info, w, prior_sd, SGS_NODE_PRIOR_NMIN_, lane);
+            write_row<O>(a, tab, pos, g, n, info, c, prior_sd, SGS_NODE_PRIOR_NMIN_, lane);
             return;
         }
         NbInfo self;
@@ -222,62 +220,53 @@ __device__ __forceinline__ void solve_system(const SolveArgs& a, const SweepTabl
         }
         __syncwarp();
         for (int q = lane; q < n; q += 32) c[q] = kcov(a, info[q], self);
+        if (lane == 0) c[n] = sill;
         for (int r = 0; r < n; ++r) {
             const NbInfo ir = info[r];
             if (ir.did >= 0) continue;
             for (int q = lane; q <= r; q += 32) {
                 const NbInfo iq = info[q];
-                if (iq.did < 0) A[r * ld + q] = (T)kcov(a, iq, ir);
+                if (iq.did < 0) A[r * ld + q] = kcov(a, iq, ir);
             }
         }
         {
-            int* dl = reinterpret_cast<int*>(rhs);
+            int* dl = reinterpret_cast<int*>(av);
             const int nd = collect_data(info, n, dl, lane);
             for (int item = lane; item < nd * n; item += 32) {
                 const int da = dl[item / n], q = item % n;
                 const NbInfo iq = info[q];
                 if (iq.did >= 0 && q > da) continue;
-                A[(da >= q ? da : q) * ld + (da >= q ? q : da)] = (T)kcov(a, iq, info[da]);
+                A[(da >= q ? da : q) * ld + (da >= q ? q : da)] = kcov(a, iq, info[da]);
             }
         }
         __syncwarp();
 
-        const bool ok = warp_cholesky<T>(A, ld, n, (T)a.tau, lane);
-        if (ok) {
-            for (int q = lane; q < n; q += 32) rhs[q] = (T)c[q];
-            __syncwarp();
-            warp_chol_solve<T>(A, ld, n, rhs, lane);
-            for (int q = lane; q < n; q += 32) w[q] = (double)rhs[q];
-            __syncwarp();
-        }
-        if (!ok) {
-            write_row<O>(a, tab, pos, g, n, info, w, prior_sd, SGS_NODE_PRIOR_SINGULAR_, lane);
+        if (!warp_ldl(A, ld, n, n + 1, a.tau, av, fv, lane)) {
+            write_row<O>(a, tab, pos, g, n, info, c, prior_sd, SGS_NODE_PRIOR_SINGULAR_, lane);
             return;
         }
-        double wc = 0.0;
-        for (int q = lane; q < n; q += 32) wc += w[q] * c[q];
-        wc = warp_sum(wc);
-        const double var = sill - wc;
-        write_row<O>(a, tab, pos, g, n, info, w, sqrt(var > 0.0 ? var : 0.0), SGS_NODE_KRIGED_, lane);
+        const double var = c[n];  // sill - c' K^-1 c
+        warp_ldl_solve(A, ld, n, n, lane);
+        write_row<O>(a, tab, pos, g, n, info, c, sqrt(var > 0.0 ? var : 0.0), SGS_NODE_KRIGED_, lane);
         __syncwarp();
     }
 }
 
-// The plain FP64 path (T = double): FP64 LHS, Cholesky and weights.  O is the
+// The plain FP64 path: FP64 LHS, L D L' and weights.  O is the
 // table type: double for the FP64 path, float (hi, lo pairs) when it re-solves
 // the systems the FP32 path queued.  With a.list set, solves only the queued
 // positions.
-template <typename T, typename O>
+template <typename O>
 __global__ void __launch_bounds__(SOLVE_WARPS * 32) solve_kernel(const SolveArgs a, const SweepTables<O> tab) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    unsigned char* base = smem + (size_t)wib * warp_smem_bytes<T>(a.k);
+    unsigned char* base = smem + (size_t)wib * warp_smem_bytes(a.k);
     const int64_t count = a.list ? (int64_t)*a.nfallback : a.P;
     const int64_t nwarps = (int64_t)gridDim.x * SOLVE_WARPS;
     for (int64_t it = (int64_t)blockIdx.x * SOLVE_WARPS + wib; it < count; it += nwarps) {
         const int64_t pos = a.list ? (int64_t)a.list[it] : it;
-        solve_system<T, O>(a, tab, pos, a.order[pos], base, a.k, lane);
+        solve_system<O>(a, tab, pos, a.order[pos], base, a.k, lane);
     }
 }
 
@@ -285,7 +274,7 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32) solve_kernel(const SolveArgs
 // global node list `order`, each solved with its domain's descriptor (domain
 // d owns global node ids [noff[d], noff[d+1])); shared memory laid out for kl
 // neighbours.
-template <typename T, typename O>
+template <typename O>
 __global__ void __launch_bounds__(SOLVE_WARPS * 32)
 solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict__ noff, int ndom,
                    const int32_t* __restrict__ order, const int32_t* __restrict__ list,
@@ -294,7 +283,7 @@ solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict
     __shared__ SolveArgs s_dom[SOLVE_WARPS];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    unsigned char* base = smem + (size_t)wib * warp_smem_bytes<T>(kl);
+    unsigned char* base = smem + (size_t)wib * warp_smem_bytes(kl);
     const int64_t n = desc[0];
     const int32_t* lst = list + desc[1];
     const int64_t nwarps = (int64_t)gridDim.x * SOLVE_WARPS;
@@ -310,7 +299,7 @@ solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict
             warp_copy_struct(&s_dom[wib], &doms[d], lane);
             __syncwarp();
         }
-        solve_system<T, O>(s_dom[wib], tab, pos, (int)(gg - lo), base, kl, lane);
+        solve_system<O>(s_dom[wib], tab, pos, (int)(gg - lo), base, kl, lane);
     }
 }
 
@@ -325,19 +314,6 @@ solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict
 // chunks of 4 entries up to the longest system of the warp.  One warp per
 // system with a Cholesky factorization in shared memory and a division per
 // row in each substitution took 250k systems of 10 data 8.9 ms, this 2.6.
-// 1 / d of a pivot (positive, normal): an FP32 reciprocal r of its mantissa,
-// off by e = 1 - d r of some 2^-22, and one step of third order, r (1 + e +
-// e^2).  The exponents are handled as integers, off the FP64 pipe.
-__device__ __forceinline__ double reciprocal(double d) {
-    const unsigned hi = __double2hiint(d), lo = __double2loint(d);
-    float rf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(__uint_as_float(0x3f800000u | (hi & 0xfffffu) << 3 | lo >> 29)));
-    const unsigned u = __float_as_uint(rf);
-    const double r = __hiloint2double((int)((u >> 3) + (896u << 20) + (1023u << 20) - (hi & 0x7ff00000u)), (int)(u << 29));
-    const double e = fma(-d, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 template <int GS>
 struct Sys64 {
     static constexpr int SYS = 32 / GS;
@@ -544,29 +520,30 @@ static cudaError_t launch_solve64(const SolveArgs& a, const SweepTables<O>& t, c
     return cudaGetLastError();
 }
 
-template <typename T, typename O>
+template <typename O>
 static cudaError_t launch_solve(const SolveArgs& a, const SweepTables<O>& t, cudaStream_t s) {
-    // several systems share a warp (a lone one of 32 gains nothing: 27.8k took
-    // 1.56 ms in that form, 1.30 in this) and no category sums are wanted
+    // several systems share a warp, and no category sums are wanted (a lone
+    // system of 32 gains nothing from that form; 90k of 18 neighbours take
+    // 1.38 ms in the other, 4.1 with a Cholesky factorization)
     if (a.k <= 16 && !a.ind_wsum) return a.k <= 8 ? launch_solve64<8, O>(a, t, s) : launch_solve64<16, O>(a, t, s);
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = warp_smem_bytes<T>(a.k) * SOLVE_WARPS;
-    cudaError_t e = cudaFuncSetAttribute(solve_kernel<T, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = warp_smem_bytes(a.k) * SOLVE_WARPS;
+    cudaError_t e = cudaFuncSetAttribute(solve_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_kernel<T, O>, SOLVE_WARPS * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_kernel<O>, SOLVE_WARPS * 32, smem);
     if (per_sm < 1) per_sm = 1;
     int64_t want = a.list ? (int64_t)nsm * per_sm : (a.P + SOLVE_WARPS - 1) / SOLVE_WARPS;
     int blocks = (int)(want < (int64_t)nsm * per_sm ? want : (int64_t)nsm * per_sm);
     if (blocks < 1) blocks = 1;
-    solve_kernel<T, O><<<blocks, SOLVE_WARPS * 32, smem, s>>>(a, t);
+    solve_kernel<O><<<blocks, SOLVE_WARPS * 32, smem, s>>>(a, t);
     return cudaGetLastError();
 }
 
 cudaError_t launch_solve_fp64(const SolveArgs& a, const SweepTables<double>& t, cudaStream_t s) {
-    return launch_solve<double, double>(a, t, s);
+    return launch_solve<double>(a, t, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1601,7 +1578,7 @@ cudaError_t launch_solve_fp32(const SolveArgs& a, const SweepTables<float>& t, c
 }
 
 cudaError_t launch_solve_fp64_into_fp32(const SolveArgs& a, const SweepTables<float>& t, cudaStream_t s) {
-    return launch_solve<double, float>(a, t, s);
+    return launch_solve<float>(a, t, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1641,14 +1618,14 @@ static cudaError_t launch_solve64_batch(int kl, const SolveArgs* doms, const int
                                         const int32_t* order, const int32_t* list, const int32_t* desc,
                                         const SweepTables<O>& t, int nsm, cudaStream_t s) {
     if (kl < 1 || kl > KMAX) return cudaErrorInvalidValue;
-    const size_t smem = warp_smem_bytes<double>(kl) * SOLVE_WARPS;
-    cudaError_t e = cudaFuncSetAttribute(solve_batch_kernel<double, O>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const size_t smem = warp_smem_bytes(kl) * SOLVE_WARPS;
+    cudaError_t e = cudaFuncSetAttribute(solve_batch_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_batch_kernel<double, O>, SOLVE_WARPS * 32, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_batch_kernel<O>, SOLVE_WARPS * 32, smem);
     if (per_sm < 1) per_sm = 1;
-    solve_batch_kernel<double, O><<<nsm * per_sm, SOLVE_WARPS * 32, smem, s>>>(doms, noff, ndom, order, list, desc, kl, t);
+    solve_batch_kernel<O><<<nsm * per_sm, SOLVE_WARPS * 32, smem, s>>>(doms, noff, ndom, order, list, desc, kl, t);
     return cudaGetLastError();
 }
 
