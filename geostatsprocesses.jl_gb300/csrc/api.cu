@@ -609,6 +609,7 @@ int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err, boo
         d.type = u.type;
         d.sill = u.sill;
         d.nugget = u.nugget;
+        d.psill62 = std::ldexp(u.sill - u.nugget, -62);
         for (int j = 0; j < 3; ++j) d.inv_range[j] = j < dim ? 1.0 / u.ranges[j] : 1.0;
         for (int j = 0; j < 9; ++j) d.R[j] = u.rotation[j];
         for (int i = 0; i < 3; ++i)
@@ -901,6 +902,7 @@ static int run_solve(sgs_plan* P, double* w_full, double* sigma_full) {
     s.nmin = P->nmin;
     s.mu = P->mean;
     s.tau = kSingularTau * P->vario.sill;
+    s.ratio63 = (unsigned long long)std::ldexp((P->vario.st[0].sill - P->vario.st[0].nugget) / P->vario.sill, 63);
     s.inv_sill = 1.0 / P->vario.sill;
     s.sd_sill[0] = (float)std::sqrt(P->vario.sill);
     s.sd_sill[1] = (float)(std::sqrt(P->vario.sill) - (double)s.sd_sill[0]);

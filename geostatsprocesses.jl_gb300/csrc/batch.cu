@@ -752,6 +752,7 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
         s.nmin = h.nmin;
         s.mu = h.mean;
         s.tau = kSingularTau * h.vario.sill;
+        s.ratio63 = (unsigned long long)std::ldexp((h.vario.st[0].sill - h.vario.st[0].nugget) / h.vario.sill, 63);
         s.inv_sill = 1.0 / h.vario.sill;
         s.sd_sill[0] = (float)std::sqrt(h.vario.sill);
         s.sd_sill[1] = (float)(std::sqrt(h.vario.sill) - (double)s.sd_sill[0]);

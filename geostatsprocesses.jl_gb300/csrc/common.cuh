@@ -97,49 +97,103 @@ __device__ __forceinline__ void cell_of(const GridDev& g, int node, int& i0, int
 }
 
 // FP64 on this GPU issues one warp instruction in 64 cycles per scheduler, so
-// the covariance below counts its FP64 instructions: about 40 for an
-// exponential structure in 3D instead of about 150 with the library's exp and
-// sqrt, whose many special cases its arguments never need.
+// the covariance below keeps to three of them past the squared lag: square
+// roots are put together from FP32 corrections of exact FP64 remainders, and
+// the exponential is evaluated in 64-bit integers (some 85 instructions of a
+// cycle or two).  Errors below 2^-56 of the sill; the library's exp and sqrt
+// took about 100 FP64 instructions, FP64 forms of these two 30.
 //
-// 2^(j/64), j = 0 .. 63, rounded to double.
-static __device__ const double kExp2J64[64] = {
-    0x1.0000000000000p+0, 0x1.02c9a3e778061p+0, 0x1.059b0d3158574p+0, 0x1.0874518759bc8p+0,
-    0x1.0b5586cf9890fp+0, 0x1.0e3ec32d3d1a2p+0, 0x1.11301d0125b51p+0, 0x1.1429aaea92de0p+0,
-    0x1.172b83c7d517bp+0, 0x1.1a35beb6fcb75p+0, 0x1.1d4873168b9aap+0, 0x1.2063b88628cd6p+0,
-    0x1.2387a6e756238p+0, 0x1.26b4565e27cddp+0, 0x1.29e9df51fdee1p+0, 0x1.2d285a6e4030bp+0,
-    0x1.306fe0a31b715p+0, 0x1.33c08b26416ffp+0, 0x1.371a7373aa9cbp+0, 0x1.3a7db34e59ff7p+0,
-    0x1.3dea64c123422p+0, 0x1.4160a21f72e2ap+0, 0x1.44e086061892dp+0, 0x1.486a2b5c13cd0p+0,
-    0x1.4bfdad5362a27p+0, 0x1.4f9b2769d2ca7p+0, 0x1.5342b569d4f82p+0, 0x1.56f4736b527dap+0,
-    0x1.5ab07dd485429p+0, 0x1.5e76f15ad2148p+0, 0x1.6247eb03a5585p+0, 0x1.6623882552225p+0,
-    0x1.6a09e667f3bcdp+0, 0x1.6dfb23c651a2fp+0, 0x1.71f75e8ec5f74p+0, 0x1.75feb564267c9p+0,
-    0x1.7a11473eb0187p+0, 0x1.7e2f336cf4e62p+0, 0x1.82589994cce13p+0, 0x1.868d99b4492edp+0,
-    0x1.8ace5422aa0dbp+0, 0x1.8f1ae99157736p+0, 0x1.93737b0cdc5e5p+0, 0x1.97d829fde4e50p+0,
-    0x1.9c49182a3f090p+0, 0x1.a0c667b5de565p+0, 0x1.a5503b23e255dp+0, 0x1.a9e6b5579fdbfp+0,
-    0x1.ae89f995ad3adp+0, 0x1.b33a2b84f15fbp+0, 0x1.b7f76f2fb5e47p+0, 0x1.bcc1e904bc1d2p+0,
-    0x1.c199bdd85529cp+0, 0x1.c67f12e57d14bp+0, 0x1.cb720dcef9069p+0, 0x1.d072d4a07897cp+0,
-    0x1.d5818dcfba487p+0, 0x1.da9e603db3285p+0, 0x1.dfc97337b9b5fp+0, 0x1.e502ee78b3ff6p+0,
-    0x1.ea4afa2a490dap+0, 0x1.efa1bee615a27p+0, 0x1.f50765b6e4540p+0, 0x1.fa7c1819e90d8p+0,
+// 2^(-j/64) in units of 2^-63, j = 0 .. 63.
+static __device__ const unsigned long long kExp2J64[64] = {
+    0x8000000000000000ull, 0x7e9f06067a4360baull, 0x7d41d96db915019dull, 0x7be86fb985689ddcull,
+    0x7a92be8a92436616ull, 0x7940bb9e2cffd89dull, 0x77f25ccdee6d7ae6ull, 0x76a7980f6cca15c2ull,
+    0x75606373ee921c97ull, 0x741cb5281e25ee34ull, 0x72dc8373be41a454ull, 0x719fc4b95f452d29ull,
+    0x70666f76154a7089ull, 0x6f307a412f074892ull, 0x6dfddbcbed791babull, 0x6cce8ae13c57ebdbull,
+    0x6ba27e656b4eb57aull, 0x6a79ad55e7f6fd10ull, 0x69540ec8f895722dull, 0x683199ed779592caull,
+    0x6712460a8fc24072ull, 0x65f60a7f79393e2eull, 0x64dcdec3371793d1ull, 0x63c6ba6455dcd8aeull,
+    0x62b39508aa836d6full, 0x61a3666d124bb204ull, 0x6096266533384a2bull, 0x5f8bccdb3d398841ull,
+    0x5e8451cfac061b5full, 0x5d7fad59099f22feull, 0x5c7dd7a3b17dcf75ull, 0x5b7ec8f19468bbc9ull,
+    0x5a827999fcef3242ull, 0x5988e20954889245ull, 0x5891fac0e95612c8ull, 0x579dbc56b48521baull,
+    0x56ac1f752150a563ull, 0x55bd1cdad49f699cull, 0x54d0ad5a753e077cull, 0x53e6c9da74b29ab5ull,
+    0x52ff6b54d8a89c75ull, 0x521a8ad704f3404full, 0x513821818624b40cull, 0x50582887dcb8a7e1ull,
+    0x4f7a993048d088d7ull, 0x4e9f6cd3967fdba8ull, 0x4dc69cdceaa72a9cull, 0x4cf022c9905bfd32ull,
+    0x4c1bf828c6dc54b8ull, 0x4b4a169b900c2d00ull, 0x4a7a77d47f7b84b1ull, 0x49ad159789f37496ull,
+    0x48e1e9b9d588e19bull, 0x4818ee218a3358eeull, 0x47521cc5a2e6a9e0ull, 0x468d6fadbf2dd4f3ull,
+    0x45cae0f1f545eb73ull, 0x450a6abaa4b77ecdull, 0x444c0740496d4294ull, 0x438fb0cb4f468808ull,
+    0x42d561b3e6243d8aull, 0x421d1461d66f2023ull, 0x4166c34c5615d0ecull, 0x40b268f9de0183baull,
 };
 
-// exp(x) for x <= 0, table-driven (Tang 1989): x = (64 m + j) ln2 / 64 + r with
-// |r| <= ln2 / 128, exp(x) = 2^m 2^(j/64) exp(r), exp(r) by its Taylor
-// polynomial of degree 5 (truncation below 4e-17); 0 below -700.
-__device__ __forceinline__ double exp_nonpos(double x) {
-    if ((uint32_t)__double2hiint(x) > 0xC085E000u) return 0.0;  // x < -700
-    const double shift = 6755399441055744.0;  // 1.5 x 2^52: the sum's low word is the rounded integer
-    const double t = fma(x, 0x1.71547652b82fep+6, shift);
-    const int n = __double2loint(t);
-    const double nd = t - shift;
-    double r = fma(nd, -0x1.62e42fef00000p-7, x);  // ln2 / 64 in two parts, the first exact times nd
-    r = fma(nd, -0x1.473de6af278edp-40, r);
-    double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-    p = fma(p, r, 1.0 / 6.0);
-    p = fma(p, r, 0.5);
-    p = fma(p, r, 1.0);
-    p = p * r;
-    const double T = __ldg(&kExp2J64[n & 63]);
-    const double e = fma(T, p, T);
-    return __hiloint2double(__double2hiint(e) + ((n >> 6) << 20), __double2loint(e));
+// exp(-3 x) in units of 2^-62 of x < 16 in units of 2^-59, table-driven (Tang
+// 1989): 3 x / ln 2 = n + j / 64 + g with g < 1 / 64, exp(-3 x) = 2^-n 2^(-j/64)
+// exp(-z), z = g ln 2, exp(-z) by its Taylor polynomial of degree 7 as 1 - z
+// + z^2 q(z), with as many bits in each term as its size leaves to matter.
+__device__ __forceinline__ unsigned long long exp3_fixed(unsigned long long x) {
+    const unsigned long long C = 0x8a7fac5f0511f48dull;  // 3 / ln 2, 2^-61
+    const unsigned long long hi = __umul64hi(x, C);
+    if (hi >> 62) return 0;  // below 2^-64
+    const unsigned long long y = hi << 2 | (x * C) >> 62;  // 2^-58
+    const int n = (int)(y >> 58), j = (int)(y >> 52) & 63;
+    const unsigned long long z = __umul64hi(y << 12, 0xb17217f7d1cf79acull);  // g ln 2, 2^-70
+    const unsigned long long w = __umul64hi(z, z);                           // z^2, 2^-76
+    const uint32_t z32 = (uint32_t)(z >> 38), w32 = (uint32_t)(w >> 44);     // 2^-32
+    // z^2 / 24 (1 - z / 5 + z^2 / 30 - z^3 / 210), 2^-44
+    const uint32_t d = __umulhi(z32, 858993459u) - __umulhi(w32, 143165577u) + __umulhi(__umulhi(z32, w32), 20452225u);
+    uint32_t r = (uint32_t)(w >> 32);
+    r = __umulhi(r - __umulhi(r, d), 178956971u);
+    // q = 1/2 - z / 6 + .., 2^-64
+    const unsigned long long q = (1ull << 63) - __umul64hi(z >> 6, 0x2aaaaaaaaaaaaaabull) + ((unsigned long long)r << 20);
+    const unsigned long long p = (1ull << 63) - (z >> 7) + (__umul64hi(w, q) >> 13);
+    return __umul64hi(p, __ldg(&kExp2J64[j])) >> n;
+}
+
+// a positive double below 16 in units of 2^-59 (rounded down)
+__device__ __forceinline__ unsigned long long fixed59(double v) {
+    const unsigned hi = __double2hiint(v);
+    const unsigned long long m = (unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(v);
+    const int s = (int)(hi >> 20) - 1016;
+    return s >= 0 ? m << s : (s > -64 ? m >> -s : 0);
+}
+
+// the float nearest below a double's magnitude, its sign kept, and a float as
+// a double; by their bits (conversions use the FP64 pipe).  Magnitudes below
+// FP32's count as zero.
+__device__ __forceinline__ float to_float_bits(double v) {
+    const unsigned hi = __double2hiint(v), lo = __double2loint(v);
+    const unsigned u = ((hi << 3) | (lo >> 29)) - (896u << 23);
+    return (hi & 0x7ff00000u) > (896u << 20) ? __uint_as_float((u & 0x7fffffffu) | (hi & 0x80000000u)) : 0.0f;
+}
+__device__ __forceinline__ double to_double_bits(float v) {
+    const unsigned u = __float_as_uint(v);
+    return __hiloint2double((int)((((u & 0x7fffffffu) >> 3) + (896u << 20)) | (u & 0x80000000u)), (int)(u << 29));
+}
+
+// sqrt(s) in units of 2^-59 for s below 225: an FP32 root, corrected by e r / 2
+// (r the reciprocal root, e = s - h^2 exact) to some 46 bits, and once more
+__device__ __forceinline__ unsigned long long sqrt_fixed(double s) {
+    if ((unsigned)__double2hiint(s) < (1023u - 120u) << 20) return 0;
+    const float sf = to_float_bits(s);
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(sf));
+    double h = to_double_bits(__fmul_rn(sf, r));
+    const float half = 0.5f * r;
+    h += to_double_bits(__fmul_rn(to_float_bits(fma(-h, h, s)), half));
+    const float c = __fmul_rn(to_float_bits(fma(-h, h, s)), half);
+    return fixed59(h) + (long long)__float2int_rn(__fmul_rn(c, 576460752303423488.0f));
+}
+
+// covariance at a squared normalized lag s, as a part of its value short of
+// the nugget, in units of 2^-62
+__device__ __forceinline__ unsigned long long shape_fixed(int type, double s) {
+    if (!(s < 220.0)) return 0;
+    if (type == 3) return s < 16.0 ? exp3_fixed(fixed59(s)) : 0;
+    if (type == 1) {
+        if (!(s < 1.0)) return 0;
+        const unsigned long long h = sqrt_fixed(s), h64 = h >> 59 ? ~0ull : h << 5;  // below 1, 2^-64
+        const unsigned long long h3 = __umul64hi(__umul64hi(h64, h64), h64);
+        const long long v = (long long)((1ull << 62) - (h64 >> 2) - (h64 >> 3) + (h3 >> 3));  // 1 - 3/2 h + h^3 / 2
+        return v > 0 ? v : 0;
+    }
+    return exp3_fixed(sqrt_fixed(s));
 }
 
 // sqrt(s): FP32 reciprocal root and two Goldschmidt steps in FP64 (within an
@@ -158,41 +212,30 @@ __device__ __forceinline__ double sqrt_fp64(double s) {
     return fma(e, h, g);
 }
 
-// normalized variogram (0 at the origin, 1 at the sill) of a squared
-// normalized lag s
-__device__ __forceinline__ double structure_shape(int type, double s) {
-    if (type == 3) return 1.0 - exp_nonpos(-3.0 * s);
-    const double hn = sqrt_fp64(s);
-    if (type == 1) return hn < 1.0 ? 1.5 * hn - 0.5 * hn * hn * hn : 1.0;
-    return 1.0 - exp_nonpos(-3.0 * hn);
-}
-
-// gamma(h) of one structure at a nonzero lag (GeoStatsFunctions conventions:
+// covariance of one structure at a nonzero lag (GeoStatsFunctions conventions:
 // practical ranges, nugget for nonzero lags only)
-__device__ __forceinline__ double structure_gamma(const VarioStructDev& v, int dim, double h0, double h1, double h2) {
+__device__ __forceinline__ double structure_cov_nonzero(const VarioStructDev& v, int dim, double h0, double h1, double h2) {
     double s = 0.0;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         if (j < dim) {
-            double u = v.R[0 + 3 * j] * h0 + v.R[1 + 3 * j] * h1;
-            if (dim == 3) u += v.R[2 + 3 * j] * h2;
-            double q = u * v.inv_range[j];
-            s += q * q;
+            double u = fma(v.W[j], h0, v.W[3 + j] * h1);
+            if (dim == 3) u = fma(v.W[6 + j], h2, u);
+            s = fma(u, u, s);
         }
     }
-    return v.nugget + (v.sill - v.nugget) * structure_shape(v.type, s);
+    return v.psill62 * (double)(long long)shape_fixed(v.type, s);
 }
 
 __device__ __forceinline__ bool is_zero(double h) { return (__double_as_longlong(h) << 1) == 0; }
 
-// covariance C(h) = sill - gamma(h) in FP64, gamma summed over the model's
-// structures
+// covariance C(h) = sill - gamma(h), summed over the model's structures
 __device__ __forceinline__ double cov_fp64(const VarioDev& v, int dim, double h0, double h1, double h2) {
     if (is_zero(h0) && is_zero(h1) && (dim == 2 || is_zero(h2))) return v.sill;
-    double g = 0.0;
+    double c = 0.0;
 #pragma unroll 1
-    for (int i = 0; i < v.ns; ++i) g += structure_gamma(v.st[i], dim, h0, h1, h2);
-    return v.sill - g;
+    for (int i = 0; i < v.ns; ++i) c += structure_cov_nonzero(v.st[i], dim, h0, h1, h2);
+    return c;
 }
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw 2011) on counter (c0..c3), key (k0,k1)

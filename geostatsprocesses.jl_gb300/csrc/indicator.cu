@@ -324,7 +324,7 @@ __device__ __forceinline__ void mv_factor(const double* S, int L, double tau, do
 
 __device__ __forceinline__ double structure_cov(const VarioStructDev& v, int dim, double h0, double h1, double h2) {
     if (h0 == 0.0 && h1 == 0.0 && (dim == 2 || h2 == 0.0)) return v.sill;
-    return v.sill - structure_gamma(v, dim, h0, h1, h2);
+    return structure_cov_nonzero(v, dim, h0, h1, h2);
 }
 
 // lag between two points of the augmented set (grid cells or data), as the

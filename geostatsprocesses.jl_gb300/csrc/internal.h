@@ -56,6 +56,7 @@ struct VarioStructDev {
     // lag -> normalized lag, diag(1 / ranges) R': component j of lag h is
     // sum_i W[3 i + j] h_i, and of a lag of d cells sum_i E[3 i + j] d_i
     double W[9], E[9];
+    double psill62;  // (sill - nugget) 2^-62
 };
 
 // The process's variogram: ns structures summed (GeoStatsFunctions'
@@ -215,6 +216,7 @@ struct SolveArgs {
     int nmin;
     double mu;
     double tau;                  // singular pivot threshold (absolute)
+    unsigned long long ratio63;  // (sill - nugget) / sill of the first structure, 2^-63
     double inv_sill;             // 1 / sill (the FP32 path works on the correlation matrix)
     float sd_sill[2];            // sqrt(sill) as an FP32 (hi, lo) pair
     int s_near;                  // high word of the squared normalized lag up to which a lag

@@ -695,16 +695,26 @@ __device__ __noinline__ void datum_lag(const SolveArgs& a, int d, int c0, int c1
 // hit = false where the lag is too short to tell it from zero this way
 __device__ __noinline__ KF datum_cov(const SolveArgs& a, const double* u, int d0, int d1, int d2, bool& hit) {
     const VarioStructDev& v = a.vario.st[0];
-    const double x0 = (double)d0, x1 = (double)d1, x2 = (double)d2;
+    const double x0 = (double)d0, x1 = (double)d1;
     double s = 0.0;
+    if (a.grid.dim == 3) {
+        const double x2 = (double)d2;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const double t = fma(-v.E[j], x0, fma(-v.E[3 + j], x1, fma(-v.E[6 + j], x2, u[j])));
-        s = fma(t, t, s);
+        for (int j = 0; j < 3; ++j) {
+            const double t = fma(-v.E[j], x0, fma(-v.E[3 + j], x1, fma(-v.E[6 + j], x2, u[j])));
+            s = fma(t, t, s);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const double t = fma(-v.E[j], x0, fma(-v.E[3 + j], x1, u[j]));
+            s = fma(t, t, s);
+        }
     }
     hit = __double2hiint(s) > a.s_near;
-    const double f = structure_shape(v.type, s);
-    return kf_from_double((v.sill - fma(v.sill - v.nugget, f, v.nugget)) * a.inv_sill);
+    const unsigned long long x = __umul64hi(shape_fixed(v.type, s), a.ratio63);  // 2^-61
+    const int hi = (int)((x + (1ull << 32)) >> 33);
+    return {hi, __fmul_rn(__ll2float_rn((long long)(x - ((unsigned long long)hi << 33))), 4.3368086899420177e-19f)};
 }
 
 // the same, from the lag table where it holds the pair
