@@ -296,6 +296,18 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// a - b: the product with -1 is exact, so one rounding as in a subtraction
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, 0xbf800000bf800000ull, a); }
 
 // ---- double-FP32 ("float-float") arithmetic: a value is an unevaluated sum
 // hi + lo of two floats, |lo| <= ulp(hi)/2, about 48 significant bits.  Error-

@@ -19,8 +19,10 @@ template <>
 __device__ __forceinline__ float unstored<float>() { return __uint_as_float(0xffffffffu); }
 template <>
 __device__ __forceinline__ double unstored<double>() { return __hiloint2double(-1, -1); }
-template <typename V>
-__device__ __forceinline__ bool missing4(const V& v) {
+__device__ __forceinline__ bool missing4(const float4& v) {  // the largest word is all ones
+    return max(max(__float_as_uint(v.x), __float_as_uint(v.y)), max(__float_as_uint(v.z), __float_as_uint(v.w))) == ~0u;
+}
+__device__ __forceinline__ bool missing4(const D4& v) {
     return missing(v.x) || missing(v.y) || missing(v.z) || missing(v.w);
 }
 __device__ __forceinline__ float settle(float v) { return missing(v) ? __uint_as_float(0x7fffffffu) : v; }

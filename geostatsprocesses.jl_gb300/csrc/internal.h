@@ -180,8 +180,8 @@ constexpr int FLOW_WORDS = FLOW_TICKET_STRIDE + 2 * FLOW_TICKETS;  // error flag
 
 // More warps than a level has items only poll: the kernels compiled for
 // higher residency run from levels of 16 items per SM (the other form's
-// warps) on.  A mean of 4,096 items in a level: 4.29 ms with it, 4.60
-// without; of 905: 1.56 and 0.98.
+// warps) on.  A mean of 4,096 items in a level: 3.24 ms with it, 3.97
+// without; of 905: 1.10 and 0.81.
 inline int flow_tight(int64_t items, int levels, int nsm) { return items >= (int64_t)levels * 16 * nsm; }
 
 // Dataflow sweep state: warps take items (position in level order x piece of

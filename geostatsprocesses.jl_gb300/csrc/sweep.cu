@@ -491,17 +491,16 @@ cudaError_t launch_sweep_all_fp64(const SweepTables<double>& t, int k, const int
 // either has the value or loads again; nothing is ordered by it but the value
 // itself, so there are no fences and no flag reads.  With a flag per (node,
 // piece), a release fence and acquire polls, one dependent step took 2.6 us
-// (a chain of 2,125 levels: 5.6 ms) instead of 0.94.  Waits are bounded
+// (a chain of 2,125 levels: 5.6 ms) instead of 0.9.  Waits are bounded
 // (wait_ns of wall-clock time, or a count of polls reached no earlier); a
 // warp that gives up sets err and stores NaN, and no warp takes new tickets
 // once err is set.
 //
 // What bounds it: the neighbours' rows, gathered from anywhere in the values
 // (no reuse once they exceed L2), or on narrow levels the step above.  4M
-// nodes x 48 neighbours x 256 FP32 values: 40.8 ms, 65 with flags (37.6 by
-// per-level launches, whose half-empty warps of the narrow levels cost the
-// same on other shapes: 16.8M nodes x 64 values 33.7 ms, per level 36.3,
-// with flags 59; 1.2M x 100: 4.3, 5.9 and 6.8).
+// nodes x 48 neighbours x 256 FP32 values: 32.4 ms, 65 with flags, 37.6 by
+// per-level launches; 16.8M nodes x 64 values 27.2, 59 and 36.3; 1.2M x 100
+// 3.2, 6.8 and 5.9.
 //
 // Lane layout inside a warp: W lanes per slice of the neighbour list (a
 // power of two), S = 32 / W slices, each lane G chunks of the piece
@@ -514,11 +513,11 @@ template <>
 struct FlowSum<float> {
     using Weight = float2;
     using Value = float4;
-    Dot2 a[4];
-    __device__ __forceinline__ void init() {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) a[q].init(0.f, 0.f);
-    }
+    // Dot2 of two realizations at a time, the same operations on register
+    // pairs (f32x2): half the instructions to issue
+    // (4M nodes x 48 neighbours x 256 values 40.8 -> 35.5 ms)
+    F2 s[2], c[2];
+    __device__ __forceinline__ void init() { s[0] = s[1] = c[0] = c[1] = 0; }
     __device__ static Weight entry(const float* p, int64_t i, int) { return reinterpret_cast<const float2*>(p)[i]; }
     __device__ static Weight shfl(Weight w, int l) {
         return make_float2(__shfl_sync(FULL_MASK, w.x, l), __shfl_sync(FULL_MASK, w.y, l));
@@ -526,22 +525,39 @@ struct FlowSum<float> {
     __device__ static Value draws(const float* z, uint64_t seed, int g, int64_t row, int ch) {
         return z ? *reinterpret_cast<const float4*>(z + row + 4 * ch) : normals4(seed, g, ch);
     }
+    // s becomes s + p, the rounding error is returned
+    __device__ static F2 two_sum(F2& s, F2 p) {
+        const F2 t = f2_add(s, p), bp = f2_sub(t, s);
+        const F2 e = f2_add(f2_sub(s, f2_sub(t, bp)), f2_sub(p, bp));
+        s = t;
+        return e;
+    }
     __device__ __forceinline__ void add(Weight w, const Value& v) {
-        a[0].add(w.x, w.y, v.x);
-        a[1].add(w.x, w.y, v.y);
-        a[2].add(w.x, w.y, v.z);
-        a[3].add(w.x, w.y, v.w);
+        const F2 wh = f2_pack(w.x, w.x), wl = f2_pack(w.y, w.y);
+        const F2 x[2] = {f2_pack(v.x, v.y), f2_pack(v.z, v.w)};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const F2 p = f2_mul(wh, x[q]);
+            const F2 pe = f2_fma(wh, x[q], f2_mul(p, 0xbf800000bf800000ull));
+            const F2 e = two_sum(s[q], p);
+            c[q] = f2_add(c[q], f2_add(e, f2_fma(wl, x[q], pe)));
+        }
+    }
+    __device__ __forceinline__ void merge(int q, F2 s2, F2 c2) {
+        const F2 e = two_sum(s[q], s2);
+        c[q] = f2_add(c[q], f2_add(c2, e));
     }
     __device__ __forceinline__ void across(int o) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            dot2_merge(a[q], __shfl_xor_sync(FULL_MASK, a[q].s, o), __shfl_xor_sync(FULL_MASK, a[q].c, o));
+        for (int q = 0; q < 2; ++q)
+            merge(q, __shfl_xor_sync(FULL_MASK, s[q], o), __shfl_xor_sync(FULL_MASK, c[q], o));
     }
     __device__ __forceinline__ Value finish(Weight b0, Weight sg, const Value& z) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dot2_merge(a[q], b0.x, b0.y);
+        for (int q = 0; q < 2; ++q) merge(q, f2_pack(b0.x, b0.x), f2_pack(b0.y, b0.y));
         add(sg, z);
-        return make_float4(a[0].value(), a[1].value(), a[2].value(), a[3].value());
+        const F2 r0 = f2_add(s[0], c[0]), r1 = f2_add(s[1], c[1]);
+        return make_float4(f2_lo(r0), f2_hi(r0), f2_lo(r1), f2_hi(r1));
     }
 };
 template <>
@@ -599,6 +615,7 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
     const int S = 32 / W, s = lane / W, cl = lane % W, cpn = Rp >> 2;
     const int64_t Rs = f.row_stride ? f.row_stride : Rp;
     const int pairs = CSR && sizeof(T) == 8 ? f.pairs : 0;
+    const uint32_t stride16 = (uint32_t)(Rs * sizeof(T) / 16);  // a row, in 16 bytes: 32 x 32 bit products
     if (CSR && f.seed_dev) seed = *f.seed_dev;
     FlowItems next(f);
     // the next item's tables
@@ -640,6 +657,7 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
             }
         }
         bool stuck = false;
+        const uint4* Vl = reinterpret_cast<const uint4*>(V + 4 * (c0 + cl));
         Sum a[G];
 #pragma unroll
         for (int gi = 0; gi < G; ++gi) a[gi].init();
@@ -653,14 +671,17 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
                 Value v[AHEAD][G];
                 auto wanted = [&](int h, int gi) { return j0 + h * S + s < mm && c0 + cl + gi * W < cpn; };
                 auto chunk = [&](int h) {
-                    return V + (int64_t)__shfl_sync(FULL_MASK, idx, (j0 + h * S + s) & 31) * Rs + 4 * (c0 + cl);
+                    const uint32_t i = __shfl_sync(FULL_MASK, idx, (j0 + h * S + s) & 31);
+                    return reinterpret_cast<const T*>(Vl + (uint64_t)i * stride16);
                 };
 #pragma unroll
                 for (int h = 0; h < AHEAD; ++h) {
                     const T* p = chunk(h);
 #pragma unroll
-                    for (int gi = 0; gi < G; ++gi)
+                    for (int gi = 0; gi < G; ++gi) {
+                        v[h][gi] = Value{};
                         if (wanted(h, gi)) v[h][gi] = ld_value4(p + 4 * gi * W);
+                    }
                 }
                 // whatever is not stored yet is loaded again
                 FlowBound bound;
@@ -669,7 +690,7 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
 #pragma unroll
                     for (int h = 0; h < AHEAD; ++h)
 #pragma unroll
-                        for (int gi = 0; gi < G; ++gi) miss |= wanted(h, gi) && missing4(v[h][gi]);
+                        for (int gi = 0; gi < G; ++gi) miss |= missing4(v[h][gi]);
                     if (!__any_sync(FULL_MASK, miss) || stuck) break;
                     stuck = !bound.more(f.err, f.wait_ns);
                     stuck = __any_sync(FULL_MASK, stuck);
