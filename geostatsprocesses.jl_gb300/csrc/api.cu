@@ -82,7 +82,7 @@ struct sgs_plan {
     bool prepared = false;
     bool sweep_timed = false;     // ev[5]/ev[6] bracket the last sweep
     unsigned long long* d_sum_m = nullptr;
-    unsigned long long* d_stats = nullptr;  // [3] search candidates (grid, data), prior nodes
+    unsigned long long* d_stats = nullptr;  // [4] search candidates (grid, data), prior nodes, search ticket
     float* d_nn = nullptr;        // warm-start network parameters
     float* d_winit = nullptr;     // warm-start predictions [N][k]
     unsigned long long* d_flow = nullptr;  // dataflow sweep: error flag, tickets
@@ -1018,7 +1018,7 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
         if ((rc = dalloc(P, &P->d_status, N))) return rc;
         if ((rc = dalloc(P, &P->d_scratch, kScratchWords))) return rc;
         if ((rc = dalloc(P, &P->d_sum_m, 1))) return rc;
-        if ((rc = dalloc(P, &P->d_stats, 3))) return rc;
+        if ((rc = dalloc(P, &P->d_stats, 4))) return rc;
         if ((rc = dalloc(P, &P->d_wl1, 1))) return rc;
     }
     cudaStream_t st = P->stream;
@@ -1051,6 +1051,7 @@ extern "C" int sgs_plan_prepare(sgs_plan* P) {
     sa.ngrid = P->d_ngrid;
     sa.data_only = P->data_only;
     sa.scanned = P->d_stats;
+    sa.ticket = P->d_stats + 3;
     CK(P, cudaMemsetAsync(P->d_stats, 0, 3 * sizeof(unsigned long long), st));
     CK(P, cudaEventRecord(P->ev[0], st));
     LAUNCH(P, 1, launch_search(sa, st));

@@ -366,7 +366,7 @@ struct sgs_batch {
     int32_t *d_fallback = nullptr, *d_fbdesc = nullptr;
     int32_t* d_scratch = nullptr;  // [0] maxlevel [1] level-wait error
     int32_t* d_ticket = nullptr;             // levels tickets, one counter per domain
-    unsigned long long* d_sums = nullptr;    // [0] sum of grid neighbours (tables) [1] sum_m [2] priors
+    unsigned long long* d_sums = nullptr;    // [0] sum of grid neighbours (tables) [1] sum_m [2] priors [4] search ticket
     unsigned long long* d_flow = nullptr;    // sweep: error flag, tickets
     uint64_t* d_seed = nullptr;
     uint64_t* h_seed = nullptr;    // pinned
@@ -712,7 +712,7 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
     if ((rc = balloc(B, &B->d_fbdesc, 2))) return rc;
     if ((rc = balloc(B, &B->d_scratch, 4))) return rc;
     if ((rc = balloc(B, &B->d_ticket, nd))) return rc;
-    if ((rc = balloc(B, &B->d_sums, 4))) return rc;
+    if ((rc = balloc(B, &B->d_sums, 5))) return rc;
     if ((rc = balloc(B, &B->d_flow, FLOW_WORDS))) return rc;
     if ((rc = balloc(B, &B->d_seed, 1))) return rc;
     if ((rc = balloc(B, &B->d_wl1, nd))) return rc;
@@ -815,7 +815,7 @@ static int enqueue_prepare(sgs_batch* B, int64_t& launched, bool with_search) {
     const int nd = B->ndom;
     if (with_search) {
         BCK(B, cudaEventRecordWithFlags(B->ev[0], st, cudaEventRecordExternal));
-        BLAUNCH(B, launch_search_batch(B->d_search, B->d_noff, nd, N, B->nsm, st));
+        BLAUNCH(B, launch_search_batch(B->d_search, B->d_noff, nd, N, B->d_sums + 4, B->nsm, st));
         BCK(B, cudaEventRecordWithFlags(B->ev[1], st, cudaEventRecordExternal));
     }
     // levels and level order
@@ -880,7 +880,7 @@ extern "C" int sgs_batch_prepare(sgs_batch* B) {
         // size the packed sweep tables: one search, then the grid-neighbour
         // sum; this prepare then runs the rest of the sequence only
         BCK(B, cudaEventRecord(B->ev[0], st));
-        BLAUNCH(B, launch_search_batch(B->d_search, B->d_noff, B->ndom, B->Ntot, B->nsm, st));
+        BLAUNCH(B, launch_search_batch(B->d_search, B->d_noff, B->ndom, B->Ntot, B->d_sums + 4, B->nsm, st));
         BCK(B, cudaEventRecord(B->ev[1], st));
         searched = true;
         BCK(B, cudaMemsetAsync(B->d_sums, 0, sizeof(unsigned long long), st));

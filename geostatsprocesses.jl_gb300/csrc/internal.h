@@ -117,6 +117,7 @@ struct SearchArgs {
     // inside the grid, each one path rank read; data: bucket entries
     // screened), summed once per warp
     unsigned long long* scanned;
+    unsigned long long* ticket;  // hands out the nodes (single-problem search)
 };
 
 // The ring whose box of buckets holds 1.5 k of D evenly spread data.
@@ -379,8 +380,8 @@ cudaError_t launch_solve_fp64_into_fp32(const SolveArgs& a, const SweepTables<fl
 // list[desc[1] .. desc[1] + desc[0]), desc on the device)
 // *out += the number of nonzero entries of v[0, n) (device counter)
 cudaError_t launch_count_nonzero(int64_t n, const int8_t* v, unsigned long long* out, int nsm, cudaStream_t s);
-cudaError_t launch_search_batch(const SearchArgs* doms, const int64_t* noff, int ndom, int64_t total, int nsm,
-                                cudaStream_t s);
+cudaError_t launch_search_batch(const SearchArgs* doms, const int64_t* noff, int ndom, int64_t total,
+                                unsigned long long* ticket, int nsm, cudaStream_t s);
 cudaError_t launch_solve_fp32_batch(int nmax, const SolveArgs* doms, const int64_t* noff, int ndom,
                                     const int32_t* order, const int32_t* list, const int32_t* desc,
                                     const SweepTables<float>& t, int nsm, cudaStream_t s);

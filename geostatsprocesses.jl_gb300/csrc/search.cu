@@ -23,6 +23,7 @@
 namespace sgs {
 
 constexpr int SEARCH_WARPS = 8;
+constexpr int SEARCH_BLOCKS = 4;  // resident per SM: 64 registers (48 or 40 spill: 20.4, 25.2, 37 ms for 16.8M nodes)
 constexpr int SCAN_STEPS = 4;  // template steps of 32 entries loaded per pass
 constexpr int DCAP = 256;  // data candidate buffer per warp
 // Early path ranks: a node of rank t has exactly t simulated grid nodes, the
@@ -432,15 +433,48 @@ __device__ __forceinline__ void search_node(const SearchArgs& a, int g, int lane
     const int wib = threadIdx.x >> 5;                                     \
     const SearchSmem sm{s_gd2[wib], s_gidx[wib], s_dd2[wib], s_didx[wib], s_squ[wib], s_rows[wib], s_rows[wib] + 32}
 
-__global__ void __launch_bounds__(SEARCH_WARPS * 32) search_kernel(const SearchArgs a) {
+// Runs of `chunk` consecutive nodes, taken by warps as they become free (the
+// next run while the last is worked on): what a node costs varies with its
+// path rank by a factor of a hundred, and with the nodes dealt out beforehand
+// a fifth of the SMs' time was spent waiting for the last of them (4M nodes
+// 11.5 -> 8.6 ms, 16.8M 27.4 -> 20.4).  A warp's
+// nodes are neighbours, which share the rank and data cache lines they scan;
+// a node's result depends only on its path rank.  Below 8 nodes per warp the
+// counter would cost more than it evens out (10k nodes: 78 against 57 us), and
+// warps take every nwarps-th node (chunk 0).
+struct SearchRuns {
+    unsigned long long* ticket;
+    const int64_t total;
+    const int chunk, lane;
+    unsigned long long next;
+    __device__ __forceinline__ SearchRuns(unsigned long long* t, int64_t n, int c, int l)
+        : ticket(t), total(n), chunk(c), lane(l), next(blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) {
+        if (chunk) draw();
+    }
+    __device__ __forceinline__ void draw() {
+        if (lane == 0) next = atomicAdd(ticket, (unsigned long long)chunk);
+    }
+    __device__ __forceinline__ bool take(int64_t& g0, int64_t& g1) {
+        g0 = (int64_t)__shfl_sync(FULL_MASK, next, 0);
+        if (g0 >= total) return false;
+        if (chunk) {
+            g1 = min(g0 + chunk, total);
+            draw();
+        } else {
+            g1 = g0 + 1;
+            next += gridDim.x * SEARCH_WARPS;
+        }
+        return true;
+    }
+};
+
+__global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) search_kernel(const __grid_constant__ SearchArgs a,
+                                                                                  int chunk) {
     SEARCH_SMEM_DECL;
-    const int64_t nwarps = (int64_t)gridDim.x * SEARCH_WARPS;
-    // Nodes go in id order, so the warps of a block take neighbouring cells
-    // and share the rank and data cache lines they scan; the result of a
-    // node depends only on its path rank, not on when it is processed.
     unsigned long long ex_grid = 0, ex_data = 0;
-    for (int64_t gg = (int64_t)blockIdx.x * SEARCH_WARPS + wib; gg < a.grid.N; gg += nwarps)
-        search_node<true>(a, (int)gg, lane, sm, ex_grid, ex_data);
+    SearchRuns runs(a.ticket, a.grid.N, chunk, lane);
+    for (int64_t g0, g1; runs.take(g0, g1);)
+        for (int64_t g = g0; g < g1; ++g) search_node<true>(a, (int)g, lane, sm, ex_grid, ex_data);
     if (a.scanned && lane == 0) {
         atomicAdd(&a.scanned[0], ex_grid);
         atomicAdd(&a.scanned[1], ex_data);
@@ -451,44 +485,55 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32) search_kernel(const SearchA
 // belong to domain d, described by doms[d] (its own grid, metric, template,
 // data, path ranks and neighbour rows).  A warp copies its current domain's
 // descriptor to shared memory when it moves into another domain.
-__global__ void __launch_bounds__(SEARCH_WARPS * 32)
-search_batch_kernel(const SearchArgs* __restrict__ doms, const int64_t* __restrict__ noff, int ndom) {
+__global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS)
+search_batch_kernel(const SearchArgs* __restrict__ doms, const int64_t* __restrict__ noff, int ndom,
+                    unsigned long long* ticket, int chunk) {
     SEARCH_SMEM_DECL;
     __shared__ SearchArgs s_dom[SEARCH_WARPS];
     const int64_t total = noff[ndom];
-    const int64_t nwarps = (int64_t)gridDim.x * SEARCH_WARPS;
     int64_t lo = 0, hi = 0;
     unsigned long long ex_grid = 0, ex_data = 0;  // not counted for batches
-    for (int64_t gg = (int64_t)blockIdx.x * SEARCH_WARPS + wib; gg < total; gg += nwarps) {
-        if (gg < lo || gg >= hi) {
-            const int d = find_domain(noff, ndom, gg);
-            lo = noff[d];
-            hi = noff[d + 1];
-            __syncwarp();
-            warp_copy_struct(&s_dom[wib], &doms[d], lane);
-            __syncwarp();
+    SearchRuns runs(ticket, total, chunk, lane);
+    for (int64_t g0, g1; runs.take(g0, g1);)
+        for (int64_t gg = g0; gg < g1; ++gg) {
+            if (gg < lo || gg >= hi) {
+                const int d = find_domain(noff, ndom, gg);
+                lo = noff[d];
+                hi = noff[d + 1];
+                __syncwarp();
+                warp_copy_struct(&s_dom[wib], &doms[d], lane);
+                __syncwarp();
+            }
+            search_node<false>(s_dom[wib], (int)(gg - lo), lane, sm, ex_grid, ex_data);
         }
-        search_node<false>(s_dom[wib], (int)(gg - lo), lane, sm, ex_grid, ex_data);
-    }
 }
 
-cudaError_t launch_search_batch(const SearchArgs* doms, const int64_t* noff, int ndom, int64_t total, int nsm,
-                                cudaStream_t s) {
-    int64_t want = (total + SEARCH_WARPS - 1) / SEARCH_WARPS;
-    int blocks = (int)(want < (int64_t)nsm * 8 ? want : (int64_t)nsm * 8);
-    if (blocks < 1) blocks = 1;
-    search_batch_kernel<<<blocks, SEARCH_WARPS * 32, 0, s>>>(doms, noff, ndom);
+// resident blocks, and runs short enough that each warp takes some 16 of them
+static void search_launch(int64_t n, int nsm, int& blocks, int& chunk) {
+    const int64_t want = std::max<int64_t>(1, (n + SEARCH_WARPS - 1) / SEARCH_WARPS), resident = (int64_t)nsm * SEARCH_BLOCKS;
+    const int64_t warps = std::min(want, resident) * SEARCH_WARPS;
+    chunk = n < 8 * warps ? 0 : (int)std::max<int64_t>(1, std::min<int64_t>(16, n / (warps * 16)));
+    blocks = (int)std::min(want, chunk ? resident : 2 * resident);
+}
+
+cudaError_t launch_search_batch(const SearchArgs* doms, const int64_t* noff, int ndom, int64_t total,
+                                unsigned long long* ticket, int nsm, cudaStream_t s) {
+    int blocks, chunk;
+    search_launch(total, nsm, blocks, chunk);
+    cudaError_t e = chunk ? cudaMemsetAsync(ticket, 0, sizeof(unsigned long long), s) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+    search_batch_kernel<<<blocks, SEARCH_WARPS * 32, 0, s>>>(doms, noff, ndom, ticket, chunk);
     return cudaGetLastError();
 }
 
 cudaError_t launch_search(const SearchArgs& a, cudaStream_t s) {
-    int dev = 0, nsm = 0;
+    int dev = 0, nsm = 0, blocks, chunk;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    int64_t want = (a.grid.N + SEARCH_WARPS - 1) / SEARCH_WARPS;
-    int blocks = (int)(want < (int64_t)nsm * 8 ? want : (int64_t)nsm * 8);
-    if (blocks < 1) blocks = 1;
-    search_kernel<<<blocks, SEARCH_WARPS * 32, 0, s>>>(a);
+    search_launch(a.grid.N, nsm, blocks, chunk);
+    cudaError_t e = chunk ? cudaMemsetAsync(a.ticket, 0, sizeof(unsigned long long), s) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+    search_kernel<<<blocks, SEARCH_WARPS * 32, 0, s>>>(a, chunk);
     return cudaGetLastError();
 }
 
