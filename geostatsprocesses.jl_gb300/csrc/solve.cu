@@ -303,8 +303,8 @@ solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict
     }
 }
 
-// The plain FP64 path for at most 16 neighbours: GS lanes per system (8 or 16,
-// one per neighbour), 32 / GS systems per warp.  A warp FP64 instruction
+// The plain FP64 path for at most 16 neighbours: GS lanes per system (8, 10 or
+// 16, one per neighbour), 32 / GS systems per warp.  A warp FP64 instruction
 // holds its scheduler for 64 cycles whatever its lanes do, so what counts is
 // the number of instructions and the systems that share them.  Pairs with a
 // datum, the only ones evaluated, are queued and taken 32 at a time; lane i
@@ -313,7 +313,8 @@ solve_batch_kernel(const SolveArgs* __restrict__ doms, const int64_t* __restrict
 // taken of) by one reciprocal a column and rows broadcast by shuffles, in
 // chunks of 4 entries up to the longest system of the warp.  One warp per
 // system with a Cholesky factorization in shared memory and a division per
-// row in each substitution took 250k systems of 10 data 8.9 ms, this 2.6.
+// row in each substitution took 250k systems of 10 data 8.9 ms, this 1.4 (1.9 with
+// 16 lanes each: 10 neighbours are kriging's default).
 template <int GS>
 struct Sys64 {
     static constexpr int SYS = 32 / GS;
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
     constexpr int LD = S::LD;
     extern __shared__ __align__(16) unsigned char smem[];
     S& sh = reinterpret_cast<S*>(smem)[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31, grp = lane / GS, q = lane % GS;
+    const int lane = threadIdx.x & 31, grp = lane / GS, q = lane % GS, l0g = grp * GS;
     const int k = a.k;
     const GridDev& G = a.grid;
     const double sill = a.vario.sill;
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
     float l1max = 0.0f;
     for (int64_t it = (int64_t)blockIdx.x * SOLVE_WARPS + (threadIdx.x >> 5); it < rounds; it += nwarps) {
         const int64_t item = it * S::SYS + grp;
-        const bool have = item < count;
+        const bool have = grp < S::SYS && item < count;  // lanes past the last group are idle
         const int64_t pos = have ? (a.list ? (int64_t)a.list[item] : item) : 0;
         const int g = have ? a.order[pos] : 0;
         const int cnt = have ? a.cnt[g] : 0;
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
             else in.did = id - (int)G.N;
             sh.info[grp][q] = in;
         }
-        if (q == 0) {
+        if (q == 0 && grp < S::SYS) {
             NbInfo self{0, 0, 0, -1};
             cell_of(G, g, self.c0, self.c1, self.c2);
             sh.info[grp][n] = self;
@@ -424,18 +425,18 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
 #pragma unroll
         for (int j = 0; j < GS; ++j) {
             if (j < nmax) {
-                const double d = __shfl_sync(FULL_MASK, A[j], j, GS);
+                const double d = __shfl_sync(FULL_MASK, A[j], l0g + j);
                 ok = ok && (j >= n || d > a.tau);
                 const double inv = reciprocal(d);
                 if (q == j) dinv = inv;
                 const double f = q > j ? -A[j] * inv : 0.0;
-                y = fma(f, __shfl_sync(FULL_MASK, y, j, GS), y);
+                y = fma(f, __shfl_sync(FULL_MASK, y, l0g + j), y);
 #pragma unroll
                 for (int l0 = 0; l0 < GS; l0 += 4)
                     if (l0 + 3 > j && l0 < nmax) {
 #pragma unroll
-                        for (int l = l0; l < l0 + 4; ++l)
-                            if (l > j) A[l] = fma(f, __shfl_sync(FULL_MASK, A[l], j, GS), A[l]);
+                        for (int l = l0; l < l0 + 4 && l < GS; ++l)
+                            if (l > j) A[l] = fma(f, __shfl_sync(FULL_MASK, A[l], l0g + j), A[l]);
                     }
             }
         }
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
             if (j < nmax) {
                 const double t = y * dinv;
                 if (q == j) w = t;
-                const double wj = __shfl_sync(FULL_MASK, t, j, GS);
+                const double wj = __shfl_sync(FULL_MASK, t, l0g + j);
                 if (q < j) y = fma(-A[j], wj, y);
             }
         }
@@ -457,15 +458,20 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
         double wc = w * c;
         double b0 = kriged && q < n && in.did >= 0 ? w * (a.data_val[in.did] - a.mu) : 0.0;
         float l1 = isgrid ? (float)fabs(w) : 0.0f;
+        // sums over the group, in its first lane
 #pragma unroll
-        for (int o = GS / 2; o > 0; o >>= 1) {
-            wc += __shfl_xor_sync(FULL_MASK, wc, o);
-            b0 += __shfl_xor_sync(FULL_MASK, b0, o);
-            l1 += __shfl_xor_sync(FULL_MASK, l1, o);
+        for (int o = GS > 8 ? 8 : 4; o > 0; o >>= 1) {
+            const double tw = __shfl_down_sync(FULL_MASK, wc, o), tb = __shfl_down_sync(FULL_MASK, b0, o);
+            const float tl = __shfl_down_sync(FULL_MASK, l1, o);
+            if (q + o < GS) {
+                wc += tw;
+                b0 += tb;
+                l1 += tl;
+            }
         }
         const double var = kriged ? sill - wc : sill;
         const double sigma = sqrt(var > 0.0 ? var : 0.0);
-        const unsigned gb = (__ballot_sync(FULL_MASK, isgrid) >> (grp * GS)) & (0xffffffffu >> (32 - GS));
+        const unsigned gb = (__ballot_sync(FULL_MASK, isgrid) >> l0g) & (0xffffffffu >> (32 - GS));
         const int m = __popc(gb);
         if (have) {
             const int64_t row = table_row(tab, pos, k);
@@ -525,7 +531,9 @@ static cudaError_t launch_solve(const SolveArgs& a, const SweepTables<O>& t, cud
     // several systems share a warp, and no category sums are wanted (a lone
     // system of 32 gains nothing from that form; 90k of 18 neighbours take
     // 1.38 ms in the other, 4.1 with a Cholesky factorization)
-    if (a.k <= 16 && !a.ind_wsum) return a.k <= 8 ? launch_solve64<8, O>(a, t, s) : launch_solve64<16, O>(a, t, s);
+    if (a.k <= 16 && !a.ind_wsum)
+        return a.k <= 8 ? launch_solve64<8, O>(a, t, s)
+                        : (a.k <= 10 ? launch_solve64<10, O>(a, t, s) : launch_solve64<16, O>(a, t, s));
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

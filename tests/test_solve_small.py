@@ -37,7 +37,7 @@ def compare(oracle_mod, p, keep, sill, tol):
 
 
 # condition numbers below 1e4, two eliminations in FP64: 1e-11 and less
-@pytest.mark.parametrize("k", [1, 2, 7, 8, 9, 12, 15, 16, 17])
+@pytest.mark.parametrize("k", [1, 2, 7, 8, 9, 10, 11, 12, 15, 16, 17])
 @pytest.mark.parametrize("ndata", [0, 40])
 def test_small_fp64_systems(geosgs_lib, oracle_mod, k, ndata):
     xy = np.random.default_rng(k).uniform(0.0, 1.0, (ndata, 2)) * (31, 27) if ndata else None
