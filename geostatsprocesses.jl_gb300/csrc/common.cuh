@@ -434,6 +434,10 @@ __device__ __forceinline__ int warp_levels(bool active, int g, const int32_t* __
         }
     }
     bool pending = active;
+    constexpr int SLOTS = 8;
+    int ask[SLOTS], open = 0;  // neighbours asked for (-1: a free slot)
+#pragma unroll
+    for (int h = 0; h < SLOTS; ++h) ask[h] = -1;
     const volatile int32_t* verr = err;
     const uint64_t max_polls = wait_ns / 32 + 1024;
     uint64_t t0 = 0, idle = 0;
@@ -451,7 +455,7 @@ __device__ __forceinline__ int warp_levels(bool active, int g, const int32_t* __
                     moved = true;
                 }
             }
-            if (pending && !(near | mask)) {
+            if (pending && !(near | mask) && !open) {
                 lev[g] = lv;
                 s_lev[lane] = lv;
                 pending = false;
@@ -461,24 +465,30 @@ __device__ __forceinline__ int warp_levels(bool active, int g, const int32_t* __
             any = __any_sync(FULL_MASK, moved);
         }
         if (!__any_sync(FULL_MASK, pending)) return lv;
-        // one turn over global memory
+        // one turn over global memory: up to SLOTS neighbours are asked for at
+        // a time, their ids kept in registers until they answer (found again in
+        // the mask and row every turn, and 4 or 16 at a time, 5 to 30 % slower)
         bool moved = false;
-        if (pending && mask) {
-            unsigned long long left = mask;
-            int c[8], q[8], l[8];
+        if (pending && (mask || open)) {
+            if (mask && open < SLOTS) {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                q[h] = left ? 63 - __clzll((long long)left) : -1;
-                left = left ? left & ~(1ull << q[h]) : 0;
-                c[h] = q[h] >= 0 ? row[q[h]] : 0;
+                for (int h = 0; h < SLOTS; ++h)
+                    if (ask[h] < 0 && mask) {
+                        const int q = 63 - __clzll((long long)mask);
+                        mask &= ~(1ull << q);
+                        ask[h] = row[q];
+                        ++open;
+                    }
             }
+            int l[SLOTS];
 #pragma unroll
-            for (int h = 0; h < 8; ++h) l[h] = q[h] >= 0 ? lev[c[h]] : -1;
+            for (int h = 0; h < SLOTS; ++h) l[h] = ask[h] >= 0 ? lev[ask[h]] : -1;
 #pragma unroll
-            for (int h = 0; h < 8; ++h)
+            for (int h = 0; h < SLOTS; ++h)
                 if (l[h] >= 0) {
                     lv = max(lv, l[h] + 1);
-                    mask &= ~(1ull << q[h]);
+                    ask[h] = -1;
+                    --open;
                     moved = true;
                 }
         }

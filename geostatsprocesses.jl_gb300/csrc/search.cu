@@ -547,8 +547,8 @@ cudaError_t launch_search(const SearchArgs& a, cudaStream_t s) {
 // and on linear paths a trip through L2 per node; here there is one atomic per
 // 32 nodes and neighbours within a ticket are handed over on chip.  The
 // deepest level is kept per warp and published once.  Levels and their order,
-// one GB300: 4 M nodes 5.3 -> 1.6 ms, 16.8 M 19.9 -> 4.0 ms, 250 k 0.64 ->
-// 0.39 ms, a linear path over 300 x 300 (2,125 levels) 2.96 -> 1.5 ms.
+// one GB300: 4 M nodes 5.3 -> 1.5 ms, 16.8 M 19.9 -> 4.0 ms, 250 k 0.64 ->
+// 0.35 ms, a linear path over 300 x 300 (2,125 levels) 2.96 -> 1.44 ms.
 __global__ void __launch_bounds__(256) levels_kernel(const LevelArgs a) {
     __shared__ int32_t s_lev[8][32];
     const int lane = threadIdx.x & 31;
