@@ -63,7 +63,7 @@ extern "C" {
 
 /* ---- sgs_problem.flags --------------------------------------------------- */
 /* The default sweep is one persistent dataflow launch: warps take nodes in
-   level order and wait (bounded) on per-node flags of their neighbours, with
+   level order and wait (bounded) until their neighbours' values are there, with
    no barrier between levels.  These flags select the alternatives: */
 #define SGS_FLAG_ONE_LAUNCH_SWEEP 1  /* one cooperative launch with a grid barrier
                                         between dependency levels */
