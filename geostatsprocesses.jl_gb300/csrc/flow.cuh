@@ -60,6 +60,9 @@ __device__ __forceinline__ double ld_value(const double* p) {
 __device__ __forceinline__ void st_value(double* p, double v) {
     asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(settle(v)) : "memory");
 }
+__device__ __forceinline__ void st_value(float* p, float v) {
+    asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(settle(v)) : "memory");
+}
 // a category, 0xff where none is stored yet
 __device__ __forceinline__ uint32_t ld_category(const uint8_t* p) {
     uint32_t v;

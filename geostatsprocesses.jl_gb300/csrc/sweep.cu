@@ -491,7 +491,7 @@ cudaError_t launch_sweep_all_fp64(const SweepTables<double>& t, int k, const int
 // either has the value or loads again; nothing is ordered by it but the value
 // itself, so there are no fences and no flag reads.  With a flag per (node,
 // piece), a release fence and acquire polls, one dependent step took 2.6 us
-// (a chain of 2,125 levels: 5.6 ms) instead of 0.9.  Waits are bounded
+// (a chain of 2,125 levels: 5.6 ms) instead of 0.74.  Waits are bounded
 // (wait_ns of wall-clock time, or a count of polls reached no earlier); a
 // warp that gives up sets err and stores NaN, and no warp takes new tickets
 // once err is set.
@@ -644,11 +644,13 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
         next.step();
         tables();
         if (CSR && f.node_class && f.node_class[g] != f.cls) continue;  // the other launch's node
-        // FP64 sums over four slices and more are reduced with one realization
-        // left per lane (spread below): the first four slices finish one each
-        const bool spread = sizeof(T) == 8 && G == 1 && W <= 8;
+        // rows of up to 8 realizations (W <= 2, the kernels with AHEAD = 2): the
+        // sums over 16 or 32 slices are reduced with one realization left per
+        // lane, and the first four slices finish one each
+        constexpr bool spread = G == 1 && AHEAD == 2;
         // the draws and the node's own terms: nothing of them waits
         Value zz[G];
+        if (spread) zz[0] = Value{};
         Weight b0{}, sg{};
         if (s < (spread ? 4 : 1)) {
             b0 = Sum::entry(t.b0, pos, pairs);
@@ -714,26 +716,41 @@ __global__ void __launch_bounds__(256, MINB) sweep_flow_kernel(const SweepTables
                 }
             }
         }
-        if constexpr (sizeof(T) == 8 && G == 1) {
-            if (spread) {
-                // the additions of the tree below, each done once: 6 FP64
-                // instructions for 32 slices instead of 20, and 2 to finish
-                // instead of 8 (122 levels of 82 nodes, 4 realizations: 0.27 ->
-                // 0.15 ms)
-                const bool up = s & 1, up2 = s & 2;
+        if constexpr (spread) {
+            // the additions of the tree below, each done once: 6 FP64
+            // instructions for 32 slices instead of 20, and 2 to finish
+            // instead of 8 (122 levels of 82 nodes, 4 realizations: 0.27 ->
+            // 0.15 ms; FP32, 2,125 levels: 1.92 -> 1.56, 5.45M rows of 8
+            // 4.9 -> 4.4)
+            const bool up = s & 1, up2 = s & 2;
+            const int ch = c0 + cl;
+            const T zc = up ? (up2 ? zz[0].w : zz[0].z) : (up2 ? zz[0].y : zz[0].x);
+            T r;
+            if constexpr (sizeof(T) == 8) {
                 const D4 v = a[0].a;
                 const double k0 = (up ? v.z : v.x) + __shfl_xor_sync(FULL_MASK, up ? v.x : v.z, W);
                 const double k1 = (up ? v.w : v.y) + __shfl_xor_sync(FULL_MASK, up ? v.y : v.w, W);
                 double k = (up2 ? k1 : k0) + __shfl_xor_sync(FULL_MASK, up2 ? k0 : k1, 2 * W);
                 for (int o = 4 * W; o < 32; o <<= 1) k += __shfl_xor_sync(FULL_MASK, k, o);
-                const int ch = c0 + cl;
-                if (s < 4 && ch < cpn) {
-                    const double zc = up ? (up2 ? zz[0].w : zz[0].z) : (up2 ? zz[0].y : zz[0].x);
-                    const double r = fma(sg, zc, k + b0);
-                    st_value(V + (int64_t)g * Rs + 4 * ch + 2 * (s & 1) + (s >> 1), stuck ? settle(unstored<T>()) : r);
-                }
-                continue;
+                r = fma(sg, zc, k + b0);
+            } else {
+                F2 ks = up ? a[0].s[1] : a[0].s[0], kc = up ? a[0].c[1] : a[0].c[0];
+                const F2 os = __shfl_xor_sync(FULL_MASK, up ? a[0].s[0] : a[0].s[1], W);
+                const F2 oc = __shfl_xor_sync(FULL_MASK, up ? a[0].c[0] : a[0].c[1], W);
+                const F2 e = Sum::two_sum(ks, os);
+                kc = f2_add(kc, f2_add(oc, e));
+                Dot2 d{up2 ? f2_hi(ks) : f2_lo(ks), up2 ? f2_hi(kc) : f2_lo(kc)};
+                dot2_merge(d, __shfl_xor_sync(FULL_MASK, up2 ? f2_lo(ks) : f2_hi(ks), 2 * W),
+                           __shfl_xor_sync(FULL_MASK, up2 ? f2_lo(kc) : f2_hi(kc), 2 * W));
+                for (int o = 4 * W; o < 32; o <<= 1)
+                    dot2_merge(d, __shfl_xor_sync(FULL_MASK, d.s, o), __shfl_xor_sync(FULL_MASK, d.c, o));
+                dot2_merge(d, b0.x, b0.y);
+                d.add(sg.x, sg.y, zc);
+                r = d.value();
             }
+            if (s < 4 && ch < cpn)
+                st_value(V + (int64_t)g * Rs + 4 * ch + 2 * (s & 1) + (s >> 1), stuck ? settle(unstored<T>()) : r);
+            continue;
         }
         for (int o = W; o < 32; o <<= 1)
 #pragma unroll
