@@ -1262,8 +1262,12 @@ static int check_flow_error(sgs_plan* P) {
 static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, void* V, cudaStream_t st) {
     (void)R;
     const sgs_sweep_config& c = P->sweep;
-    P->last_sweep_mode = c.mode;
-    if (c.mode == SGS_SWEEP_COOPERATIVE) {
+    // A dataflow launch clears the rows it writes first, which would take the
+    // draws with them where both share a buffer; the other forms read a row's
+    // draws before they store its values.
+    const int mode = c.mode == SGS_SWEEP_FLOW && z && z == V ? SGS_SWEEP_LEVELS : c.mode;
+    P->last_sweep_mode = mode;
+    if (mode == SGS_SWEEP_COOPERATIVE) {
         // all levels in one cooperative launch (per-level launches if the
         // device or the launch configuration does not allow it)
         cudaError_t e;
@@ -1277,7 +1281,7 @@ static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, v
         }
         cudaGetLastError();
         P->last_sweep_mode = SGS_SWEEP_LEVELS;
-    } else if (c.mode == SGS_SWEEP_FLOW) {
+    } else if (mode == SGS_SWEEP_FLOW) {
         // leading levels by per-level launches, the rest in one dataflow launch
         int W = c.lanes_w, G = c.lanes_g;
         const int H = flow_layout(Rp, W, G);

@@ -195,8 +195,10 @@ int sgs_plan_simulate(sgs_plan* plan, int32_t nreals, const double* z,
  * [N][nreals rounded up to a multiple of 4], float when sgs_info.values_fp64
  * is 0 — SGS_PREC_FP32_REFINE with moderate weights — and double when it is
  * 1, or NULL for seeded draws) and vals_dev (node-major, same shape and type,
- * centred values v - mean) are device pointers; stream is a cudaStream_t
- * (NULL = the plan's stream).  Same reference counterpart as
+ * centred values v - mean) are device pointers; vals_dev may be z_dev itself
+ * (the values replace the draws, one launch per level where the sweep would be
+ * a dataflow launch), but must not overlap it otherwise.  stream is a
+ * cudaStream_t (NULL = the plan's stream).  Same reference counterpart as
  * sgs_plan_simulate. */
 int sgs_plan_simulate_device(sgs_plan* plan, int32_t nreals, const void* z_dev,
                              uint64_t seed, void* vals_dev, void* stream);
