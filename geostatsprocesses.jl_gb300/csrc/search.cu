@@ -291,6 +291,8 @@ __device__ __forceinline__ void search_node(const SearchArgs& a, int g, int lane
                     });
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) far = fmaxf(far, __shfl_xor_sync(FULL_MASK, far, o));
+                // lengths whose squares leave FP32's range bound nothing
+                ring = ring && far > 1e-30f;
                 // above the true distance: each lag is off by at most dh
                 const float d = sqrtf(far) * 1.0001f + sqrtf((float)G.dim) * a.metric.dh_f * 1.0001f;
                 far = d * d;

@@ -51,3 +51,21 @@ def test_clustered_data_match_oracle(geosgs_lib, oracle_mod, dims, ndata):
     # neighbour moves the values by 1e-6 and more
     np.testing.assert_allclose(mean, want_mean, rtol=0, atol=1e-10)
     np.testing.assert_allclose(var, want_var, rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize("scale", [1e-25, 1e-23, 1e-19, 1e-15, 1e15, 1e19, 1e25])
+@pytest.mark.parametrize("radius", [None, 30.0])
+def test_lengths_whose_squares_leave_fp32(geosgs_lib, scale, radius):
+    rng = np.random.default_rng(3)
+    z = rng.standard_normal(300)
+    u = rng.uniform(size=(300, 2)) * 64.0
+
+    def mean(s):
+        process = geosgs.GaussianProcess(geosgs.ExponentialVariogram(range=20.0 * s, sill=1.0, nugget=0.1), 0.0)
+        grid = geosgs.CartesianGrid((64, 64), spacing=(s, s))
+        ball = None if radius is None else geosgs.MetricBall(radius * s)
+        return geosgs.posterior(process, grid, geosgs.georef({"Z": z}, u * s), maxneighbors=10, neighborhood=ball)[0]
+
+    # the same neighbours: lags rounded at another scale, systems of condition
+    # below 1e3; other neighbours move the values by 1e-3 and more
+    np.testing.assert_allclose(mean(scale), mean(1.0), rtol=0, atol=1e-10)
