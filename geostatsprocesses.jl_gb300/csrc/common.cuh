@@ -196,22 +196,6 @@ __device__ __forceinline__ unsigned long long shape_fixed(int type, double s) {
     return exp3_fixed(sqrt_fixed(s));
 }
 
-// sqrt(s): FP32 reciprocal root and two Goldschmidt steps in FP64 (within an
-// ulp); values far outside FP32's range go to the library
-__device__ __forceinline__ double sqrt_fp64(double s) {
-    const uint32_t hi = (uint32_t)__double2hiint(s);
-    if (hi - 0x39B00000u > 0x46300000u - 0x39B00000u) return sqrt(s);  // outside 2^-100 .. 2^100
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((float)s));
-    const double yd = (double)y;
-    double g = s * yd, h = 0.5 * yd;
-    double e = fma(-g, h, 0.5);
-    g = fma(g, e, g);
-    h = fma(h, e, h);
-    e = fma(-g, g, s);
-    return fma(e, h, g);
-}
-
 // covariance of one structure at a nonzero lag (GeoStatsFunctions conventions:
 // practical ranges, nugget for nonzero lags only)
 __device__ __forceinline__ double structure_cov_nonzero(const VarioStructDev& v, int dim, double h0, double h1, double h2) {
@@ -512,8 +496,9 @@ __device__ __forceinline__ int warp_levels(bool active, int g, const int32_t* __
 }
 
 // 1 / d of a pivot (positive, normal): an FP32 reciprocal r of its mantissa,
-// off by e = 1 - d r of some 2^-22, and one step of third order, r (1 + e +
-// e^2).  The exponents are handled as integers, off the FP64 pipe.
+// off by e = 1 - d r of some 2^-22, and one step of the third-order iteration
+// for reciprocals, r (1 + e + e^2) (Householder 1970), off by e^3 and a
+// rounding.  The exponents are handled as integers, off the FP64 pipe.
 __device__ __forceinline__ double reciprocal(double d) {
     const unsigned hi = __double2hiint(d), lo = __double2loint(d);
     float rf;

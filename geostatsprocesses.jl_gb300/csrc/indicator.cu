@@ -312,12 +312,12 @@ __device__ __forceinline__ void mv_factor(const double* S, int L, double tau, do
         double d = S[j * L + j];
         for (int l = 0; l < j; ++l) d -= F[j * L + l] * F[j * L + l];
         if (!(d > tau)) continue;
-        const double fjj = sqrt_fp64(d), inv = reciprocal(fjj);
+        const double fjj = sqrt(d);
         F[j * L + j] = fjj;
         for (int i = j + 1; i < L; ++i) {
             double t = S[i * L + j];
             for (int l = 0; l < j; ++l) t -= F[i * L + l] * F[j * L + l];
-            F[i * L + j] = t * inv;
+            F[i * L + j] = t / fjj;
         }
     }
 }

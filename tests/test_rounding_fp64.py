@@ -1,5 +1,6 @@
 """FP64 results at their own rounding: the deviations of small systems against
-extended precision."""
+extended precision, and the factor of a multivariate prior against correctly
+rounded roots and quotients."""
 import numpy as np
 import pytest
 
@@ -52,3 +53,21 @@ def test_deviations_of_small_systems(geosgs_lib, k):
 
     # no further off than a plain FP64 Cholesky of the same systems
     assert rms(sigma[g]) <= rms(deviation(cov, *lags))
+
+
+def test_factor_of_a_multivariate_prior(geosgs_lib):
+    rng = np.random.default_rng(0)
+    L = 8
+    for _ in range(40):
+        B = rng.standard_normal((L, L))
+        A = B @ B.T + 0.1 * np.eye(L)
+        A = 0.5 * (A + A.T)
+        method = geosgs.GPUSEQSIM(path=geosgs.LinearPath(), maxneighbors=1, precision="fp64")
+        process = geosgs.GaussianProcess(geosgs.SphericalVariogram(range=2.0, sill=1.0, nugget=0.0), 0.0)
+        p, keep = geosgs.build_problem(process, geosgs.CartesianGrid((2, 1)), None, method)
+        plan = geosgs.Plan(p, keep).set_multivariate(np.zeros(L), A[None]).prepare()
+        z = np.zeros((1, L, 2))
+        z[0, 0] = 1.0
+        got = plan.simulate_multivariate(1, z=z)[0, :, 0]  # the first node: the factor's first column
+        plan.close()
+        assert np.array_equal(got, np.r_[np.sqrt(A[0, 0]), A[1:, 0] / np.sqrt(A[0, 0])])
