@@ -100,6 +100,7 @@ struct sgs_plan {
     bool cok = false;
     double* d_cok_coef = nullptr;
     double cok_tau = 0.0;
+    double cok_unit = 1.0;  // the matrices are kept divided by its square (variance_unit)
     int32_t *d_cok_m = nullptr, *d_cok_idx = nullptr;
     double *d_cok_w = nullptr, *d_cok_cst = nullptr;
     int cok_L = 0;                // L the cokriging tables were allocated for
@@ -620,6 +621,17 @@ int sgs::host_domain(const sgs_problem* pr, HostDomain& H, std::string& err, boo
         H.vario.sill += u.sill;
         H.vario.nugget += u.nugget;
     }
+    const double unit = H.vario.unit = variance_unit(H.vario.sill);
+    if (unit != 1.0) {
+        for (int i = 0; i < H.vario.ns; ++i) {
+            VarioStructDev& d = H.vario.st[i];
+            d.psill62 = std::ldexp((d.sill - d.nugget) / unit / unit, -62);
+            d.sill = d.sill / unit / unit;
+            d.nugget = d.nugget / unit / unit;
+        }
+        H.vario.sill = H.vario.sill / unit / unit;
+        H.vario.nugget = H.vario.nugget / unit / unit;
+    }
     H.vario.type = H.vario.st[0].type;
     for (int j = 0; j < 3; ++j) H.vario.inv_range[j] = H.vario.st[0].inv_range[j];
     for (int j = 0; j < 9; ++j) H.vario.R[j] = H.vario.st[0].R[j];
@@ -904,8 +916,9 @@ static int run_solve(sgs_plan* P, double* w_full, double* sigma_full) {
     s.tau = kSingularTau * P->vario.sill;
     s.ratio63 = (unsigned long long)std::ldexp((P->vario.st[0].sill - P->vario.st[0].nugget) / P->vario.sill, 63);
     s.inv_sill = 1.0 / P->vario.sill;
-    s.sd_sill[0] = (float)std::sqrt(P->vario.sill);
-    s.sd_sill[1] = (float)(std::sqrt(P->vario.sill) - (double)s.sd_sill[0]);
+    const double sd = std::sqrt(P->vario.sill) * P->vario.unit;
+    s.sd_sill[0] = (float)sd;
+    s.sd_sill[1] = (float)(sd - (double)s.sd_sill[0]);
     s.s_near = P->s_near;
     s.refine_steps = P->refine_steps;
     s.P = P->N;
@@ -983,6 +996,7 @@ static CokArgs cok_args(const sgs_plan* P) {
     c.data_cat = P->d_ind_cat;
     c.data_val = P->d_mv_dval;
     c.tau = P->cok_tau;
+    c.unit = P->cok_unit * P->vario.unit;
     c.m = P->d_cok_m;
     c.idx = P->d_cok_idx;
     c.w = P->d_cok_w;
@@ -1762,7 +1776,7 @@ extern "C" int sgs_krige(const sgs_problem* problem, double* mean, double* var) 
     if (P->D == 0) {  // no data: the prior (priormean, src/expectation/field/gaussian.jl:5-19)
         for (int64_t g = 0; g < N; ++g) {
             mean[g] = P->mean;
-            if (var) var[g] = P->vario.sill;
+            if (var) var[g] = P->vario.sill * P->vario.unit * P->vario.unit;
         }
         sgs_plan_destroy(P);
         return SGS_OK;
@@ -1823,6 +1837,33 @@ extern "C" int sgs_plan_set_indicator(sgs_plan* P, int32_t ncat, const double* p
     return SGS_OK;
 }
 
+// The largest variance of a variable: coef is S x L x L, of the plan's S structures.
+static double largest_variance(const sgs_plan* P, const double* coef, int L) {
+    const double u = P->vario.unit;
+    double vmax = 0.0;
+    for (int a = 0; a < L; ++a) {
+        double v = 0.0;
+        for (int s = 0; s < P->vario.ns; ++s) v += coef[((size_t)s * L + a) * L + a] * (P->vario.st[s].sill * u * u);
+        vmax = std::max(vmax, v);
+    }
+    return vmax;
+}
+
+// Uploads the coregionalization matrices and sets the singular rule's scale.
+static int upload_coef(sgs_plan* P, const double* coef, int L, double vmax) {
+    const double u = P->vario.unit, c = variance_unit(vmax / u / u);
+    dfree(P, P->d_cok_coef);
+    P->d_cok_coef = nullptr;
+    std::vector<double> cf(coef, coef + (size_t)P->vario.ns * L * L);
+    for (double& x : cf) x = x / c / c;
+    int rc;
+    if ((rc = upload(P, &P->d_cok_coef, cf.data(), cf.size()))) return rc;
+    CK(P, cudaStreamSynchronize(P->stream));
+    P->cok_unit = c;
+    P->cok_tau = kSingularTau * (vmax / u / u / c / c);
+    return SGS_OK;
+}
+
 extern "C" int sgs_plan_set_indicator_cokriging(sgs_plan* P, int32_t ncat, const double* prob, const int32_t* data_cat,
                                                 const double* coef) {
     if (!P) return set_err(nullptr, SGS_ERR_ARG, "null plan");
@@ -1837,19 +1878,9 @@ extern "C" int sgs_plan_set_indicator_cokriging(sgs_plan* P, int32_t ncat, const
     if (rc) return rc;
     if (old_ncat != ncat) free_cok_tables(P);  // table sizes change: reallocate at the next prepare
     // the singular rule's scale: the largest indicator variance
-    double vmax = 0.0;
-    for (int a = 0; a < ncat; ++a) {
-        double v = 0.0;
-        for (int s = 0; s < S; ++s) v += coef[((size_t)s * ncat + a) * ncat + a] * P->vario.st[s].sill;
-        vmax = std::max(vmax, v);
-    }
+    const double vmax = largest_variance(P, coef, ncat);
     if (!(vmax > 0.0)) return set_err(P, SGS_ERR_ARG, "the model's indicator variances must be positive");
-    dfree(P, P->d_cok_coef);
-    P->d_cok_coef = nullptr;
-    std::vector<double> cf(coef, coef + (size_t)S * ncat * ncat);
-    if ((rc = upload(P, &P->d_cok_coef, cf.data(), cf.size()))) return rc;
-    CK(P, cudaStreamSynchronize(P->stream));
-    P->cok_tau = kSingularTau * vmax;
+    if ((rc = upload_coef(P, coef, ncat, vmax))) return rc;
     P->cok = true;
     return SGS_OK;
 }
@@ -1943,19 +1974,11 @@ extern "C" int sgs_plan_set_multivariate(sgs_plan* P, int32_t nvars, const doubl
     for (int64_t i = 0; i < P->D * L; ++i)
         if (!std::isfinite(data_values[i])) return set_err(P, SGS_ERR_ARG, "data values must be finite");
     // the singular rule's scale: the largest variance of a variable
-    double vmax = 0.0;
-    for (int a = 0; a < L; ++a) {
-        double v = 0.0;
-        for (int s = 0; s < S; ++s) v += coef[((size_t)s * L + a) * L + a] * P->vario.st[s].sill;
-        vmax = std::max(vmax, v);
-    }
+    const double vmax = largest_variance(P, coef, L);
     if (!(vmax > 0.0)) return set_err(P, SGS_ERR_ARG, "the model's variances must be positive");
     CK(P, cudaSetDevice(P->device));
     int rc;
-    dfree(P, P->d_cok_coef);
-    P->d_cok_coef = nullptr;
-    std::vector<double> cf(coef, coef + (size_t)S * L * L);
-    if ((rc = upload(P, &P->d_cok_coef, cf.data(), cf.size()))) return rc;
+    if ((rc = upload_coef(P, coef, L, vmax))) return rc;
     dfree(P, P->d_mv_dval);
     P->d_mv_dval = nullptr;
     if (P->D > 0) {
@@ -1971,7 +1994,6 @@ extern "C" int sgs_plan_set_multivariate(sgs_plan* P, int32_t nvars, const doubl
     P->cok = false;
     for (int a = 0; a < IND_MAX_CAT; ++a) P->mv_mean[a] = a < L ? mean[a] : 0.0;
     P->mv_nvars = L;
-    P->cok_tau = kSingularTau * vmax;
     P->mv = true;
     P->prepared = false;
     return SGS_OK;

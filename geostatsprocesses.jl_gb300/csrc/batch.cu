@@ -754,8 +754,9 @@ static int batch_init(sgs_batch* B, const sgs_problem* pr, int nd) {
         s.tau = kSingularTau * h.vario.sill;
         s.ratio63 = (unsigned long long)std::ldexp((h.vario.st[0].sill - h.vario.st[0].nugget) / h.vario.sill, 63);
         s.inv_sill = 1.0 / h.vario.sill;
-        s.sd_sill[0] = (float)std::sqrt(h.vario.sill);
-        s.sd_sill[1] = (float)(std::sqrt(h.vario.sill) - (double)s.sd_sill[0]);
+        const double sd = std::sqrt(h.vario.sill) * h.vario.unit;
+        s.sd_sill[0] = (float)sd;
+        s.sd_sill[1] = (float)(sd - (double)s.sd_sill[0]);
         s.s_near = h.s_near;
         s.refine_steps = pr[d].refine_steps;
         s.P = h.N;

@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(COK_WARPS * 32) cok_solve_kernel(const __grid_
                         C0[t * L + u] = v;
                     }
                 mv_factor(C0, L, c.tau, F);
-                for (int i = 0; i < L * L; ++i) c.fac[pos * L * L + i] = F[i];
+                for (int i = 0; i < L * L; ++i) c.fac[pos * L * L + i] = F[i] * c.unit;
             }
             __syncwarp();
         }

@@ -62,10 +62,13 @@ struct VarioStructDev {
 // The process's variogram: ns structures summed (GeoStatsFunctions'
 // NestedVariogram; ns = 1 for a single variogram).  type, inv_range and R
 // repeat the first structure (the learned warm start's frame); sill and
-// nugget are the model's, the structures' summed.
+// nugget are the model's, the structures' summed.  Sills whose systems would
+// meet FP64's smallest or largest numbers are kept divided by unit^2, a power
+// of four: weights do not depend on it, and deviations are `unit` times theirs.
 struct VarioDev {
     int type;
     double sill, nugget;
+    double unit;
     double inv_range[3];
     double R[9];
     int ns;
@@ -282,6 +285,7 @@ struct CokArgs {
     const int32_t* data_cat;     // [D] data categories (indicator)
     const double* data_val;      // [D][L] data values (Gaussian)
     double tau;                  // singular pivot threshold (absolute)
+    double unit;                 // factor of the deviations (VarioDev::unit, and the same of coef)
     int32_t* m;                  // [P] grid neighbours of the position's system
     int32_t* idx;                // [P][k] their node ids
     double* w;                   // [P][k][L][L] weight of (grid neighbour j, its category b) for category t
@@ -302,6 +306,15 @@ cudaError_t launch_cok_flow(const CokArgs& c, const int32_t* node, int k, int64_
 // seeded normals of pseudo-node a*N + g.
 cudaError_t launch_mv_flow(const CokArgs& c, const int32_t* node, int k, int64_t N, int Rp, const double* z,
                            uint64_t seed, double* V, const FlowArgs& f, cudaStream_t s);
+
+// The power of two u for which variances of size v are kept as v / u^2: 1
+// within 2^-900 .. 2^900, where pivots down to 1e-10 v, their reciprocals and
+// products keep all their bits.
+inline double variance_unit(double v) {
+    int e = 0;
+    std::frexp(v, &e);
+    return e > 900 || e < -900 ? std::ldexp(1.0, e / 2) : 1.0;
+}
 
 // Host-side description of one problem (api.cu: host_domain): everything
 // sgs_plan_create derives on the host before uploading.

@@ -195,7 +195,7 @@ __device__ __forceinline__ void solve_system(const SolveArgs& a, const SweepTabl
     NbInfo* info = reinterpret_cast<NbInfo*>(fv + (kl + 2) / 2 * 2);
     const GridDev& G = a.grid;
     const double sill = a.vario.sill;
-    const double prior_sd = sqrt(sill);
+    const double prior_sd = sqrt(sill) * a.vario.unit;
     {
         const int n = a.cnt[g];
         double* c = A + n * ld;  // the right-hand side, then the weights
@@ -247,7 +247,7 @@ __device__ __forceinline__ void solve_system(const SolveArgs& a, const SweepTabl
         }
         const double var = c[n];  // sill - c' K^-1 c
         warp_ldl_solve(A, ld, n, n, lane);
-        write_row<O>(a, tab, pos, g, n, info, c, sqrt(var > 0.0 ? var : 0.0), SGS_NODE_KRIGED_, lane);
+        write_row<O>(a, tab, pos, g, n, info, c, sqrt(var > 0.0 ? var : 0.0) * a.vario.unit, SGS_NODE_KRIGED_, lane);
         __syncwarp();
     }
 }
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(SOLVE_WARPS * 32, 4) solve64_kernel(const __gr
             }
         }
         const double var = kriged ? sill - wc : sill;
-        const double sigma = sqrt(var > 0.0 ? var : 0.0);
+        const double sigma = sqrt(var > 0.0 ? var : 0.0) * a.vario.unit;
         const unsigned gb = (__ballot_sync(FULL_MASK, isgrid) >> l0g) & (0xffffffffu >> (32 - GS));
         const int m = __popc(gb);
         if (have) {
