@@ -180,13 +180,13 @@ constexpr int ENS_DONE = INT_MIN;
 constexpr int ENS_FIXED_MAX = 512;  // values of a row in the integer form
 
 // Mean and variance in integers.  With |x| < 2^e over a row, X = x 2^(51 - e)
-// is an integer (values below 2^-27 of the largest are rounded to it), sums of
-// at most 512 of them are exact, and so are the three partial sums of the
-// squares of X - M, M an integer near the mean, taken as 26-bit halves:
-// sum (X - M)^2 = hh 2^52 + 2 hl 2^26 + ll.  The variance is the sum less
-// (sum (X - M))^2 / R.  FP64 is left to the last dozen operations, for 32
-// nodes at a time.  Rows with infinities, NaN or magnitudes beyond 2^60 or
-// below 2^-60 are summed in FP64.
+// is an integer where no value but 0 is below 2^(e - 28) (whose last bit is
+// 2^(e - 51)); sums of at most 512 of them are exact, and so are the three
+// partial sums of the squares of X - M, M an integer near the mean, taken as
+// 26-bit halves: sum (X - M)^2 = hh 2^52 + 2 hl 2^26 + ll.  The variance is
+// the sum less (sum (X - M))^2 / R.  FP64 is left to the last dozen
+// operations, for 32 nodes at a time.  Rows with smaller values, infinities, NaN or magnitudes
+// beyond 2^60 or below 2^-60 are summed in FP64.
 template <int LPN, int V>
 __global__ void __launch_bounds__(ENS_WARPS * 32) ens_stats_fixed_kernel(const EnsArgs a, int rounds, double* mean,
                                                                          double* var) {
@@ -204,13 +204,21 @@ __global__ void __launch_bounds__(ENS_WARPS * 32) ens_stats_fixed_kernel(const E
             const float* row = vals + g * a.stride;
             float x[V];
             ens_load<LPN, V>(row, a.R, q, g < a.N, 0.0f, x);
-            unsigned mx = 0;
+            unsigned mx = 0, mn = ~0u;  // of the magnitudes; the smallest less 1, zeros left out
 #pragma unroll
-            for (int i = 0; i < V; ++i) mx = max(mx, __float_as_uint(x[i]) & 0x7fffffffu);
+            for (int i = 0; i < V; ++i) {
+                const unsigned v = __float_as_uint(x[i]) & 0x7fffffffu;
+                mx = max(mx, v);
+                mn = min(mn, v - 1);
+            }
 #pragma unroll
-            for (int o = LPN / 2; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+            for (int o = LPN / 2; o > 0; o >>= 1) {
+                mx = max(mx, __shfl_xor_sync(FULL_MASK, mx, o));
+                mn = min(mn, __shfl_xor_sync(FULL_MASK, mn, o));
+            }
             const int e = mx ? (int)(mx >> 23) - 126 : 0;
-            const bool fixed = e >= -60 && e <= 60;
+            // 27 binades below the largest one's at most
+            const bool fixed = e >= -60 && e <= 60 && ((mn + 1) >> 23) + 27 >= mx >> 23;
             const float sc = __uint_as_float((unsigned)(127 + 25 - (fixed ? e : 0)) << 23);
             long long X[V], s = 0;
 #pragma unroll
