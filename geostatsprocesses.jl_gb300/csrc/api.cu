@@ -86,8 +86,7 @@ struct sgs_plan {
     float* d_nn = nullptr;        // warm-start network parameters
     float* d_winit = nullptr;     // warm-start predictions [N][k]
     unsigned long long* d_flow = nullptr;  // dataflow sweep: error flag, tickets
-    sgs_sweep_config sweep{SGS_SWEEP_FLOW, 1, 0, 1, 0, 0, 0, 0, 0, 0.f};
-    bool sweep_auto = true;  // not set or tuned by the user: the launch chooses `tight`
+    sgs_sweep_config sweep{SGS_SWEEP_FLOW, 1, 0, 1, 0, 0, 0, -1, 0, 0.f};
     int last_sweep_mode = SGS_SWEEP_FLOW;  // mode of the last sweep launched
     int data_only = 0;            // neighbours from the data alone (sgs_krige)
     // indicator simulation (sgs_plan_set_indicator)
@@ -1313,7 +1312,7 @@ static int run_sweep(sgs_plan* P, int R, int Rp, const void* z, uint64_t seed, v
             if (l0 > 0) f.ticket += FLOW_TICKETS;
             f.chunk = std::max(1, c.chunk);
             f.blocks_per_sm = c.blocks_per_sm;
-            f.tight = P->sweep_auto ? flow_tight((p1 - p0) * H, l1 - l0, P->nsm) : c.tight;
+            f.tight = c.tight < 0 ? flow_tight((p1 - p0) * H, l1 - l0, P->nsm) : c.tight;
             cudaError_t e = launch_flow_clear(values_fp64(P) ? sweep64(P).node : P->t32.node, p0, p1, P->N,
                                               (size_t)Rp * (values_fp64(P) ? sizeof(double) : sizeof(float)), V, st);
             if (e != cudaSuccess) return cuda_err(P, e, "sweep clear");
@@ -1593,12 +1592,11 @@ extern "C" int sgs_plan_set_sweep(sgs_plan* P, const sgs_sweep_config* c) {
     if (c->mode == SGS_SWEEP_FLOW &&
         (c->chunk < 0 || c->chunk > 64 || c->blocks_per_sm < 0 || c->blocks_per_sm > 32 || c->lanes_g < 0 ||
          c->lanes_g > 2 || c->lanes_w < 0 || c->lanes_w > 32 || (c->lanes_w & (c->lanes_w - 1)) ||
-         c->level_lo < 0 || c->level_hi < 0 || c->tight < 0 || c->tight > 1 || c->split_nodes < 0))
+         c->level_lo < 0 || c->level_hi < 0 || c->tight < -1 || c->tight > 1 || c->split_nodes < 0))
         return set_err(P, SGS_ERR_ARG, "invalid dataflow sweep parameters");
     if (c->mode == SGS_SWEEP_LEVELS && (c->lanes_g < 0 || c->lanes_g > 4 || c->lanes_g == 3 || c->split_nodes < 0))
         return set_err(P, SGS_ERR_ARG, "invalid per-level sweep parameters (lanes_g 0, 1, 2 or 4, split_nodes >= 0)");
     P->sweep = *c;
-    P->sweep_auto = false;
     if (P->sweep.chunk < 1) P->sweep.chunk = 1;
     return SGS_OK;
 }
@@ -1606,7 +1604,6 @@ extern "C" int sgs_plan_set_sweep(sgs_plan* P, const sgs_sweep_config* c) {
 // time one sweep configuration (after a warm-up run); < 0 on failure
 static int time_sweep(sgs_plan* P, const sgs_sweep_config& c, int R, int Rp, void* V, float* ms) {
     P->sweep = c;
-    P->sweep_auto = false;
     cudaStream_t st = P->stream;
     int rc;
     if ((rc = run_sweep(P, R, Rp, nullptr, 7, V, st))) return rc;
@@ -1633,7 +1630,6 @@ extern "C" int sgs_plan_tune_sweep(sgs_plan* P, int32_t R, sgs_sweep_config* cho
     int rc;
     if ((rc = dalloc(P, (unsigned char**)&V, (size_t)P->N * Rp * es))) return rc;
     const sgs_sweep_config saved = P->sweep;
-    const bool saved_auto = P->sweep_auto;
     std::vector<sgs_sweep_config> done;
     int best = -1;
     auto run = [&](sgs_sweep_config c) -> int {
@@ -1728,7 +1724,6 @@ extern "C" int sgs_plan_tune_sweep(sgs_plan* P, int32_t R, sgs_sweep_config* cho
     dfree(P, V);
     if (rc || best < 0) {
         P->sweep = saved;
-        P->sweep_auto = saved_auto;
         return rc ? rc : set_err(P, SGS_ERR_CUDA, "no sweep configuration could be timed");
     }
     P->sweep = done[best];

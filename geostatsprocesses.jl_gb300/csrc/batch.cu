@@ -384,8 +384,7 @@ struct sgs_batch {
     int sweep_Rp = 0;
     void* sweep_V = nullptr;
     cudaStream_t sweep_stream = nullptr;
-    sgs_sweep_config sweep{SGS_SWEEP_FLOW, 1, 0, 1, 0, 0, 0, 0, 0, 0.f};
-    bool sweep_auto = true;  // not set or tuned by the user: the launch chooses `tight`
+    sgs_sweep_config sweep{SGS_SWEEP_FLOW, 1, 0, 1, 0, 0, 0, -1, 0, 0.f};
     bool sweep_graph_valid = false;
     bool sweep_pending = false;    // a device-resident sweep not yet checked
     unsigned int* d_wl1 = nullptr; // per domain: largest sum of |grid weights| (FP32 bits)
@@ -1028,7 +1027,7 @@ static int enqueue_sweep(sgs_batch* B, int Rp, const void* z, void* V, cudaStrea
     f.err = reinterpret_cast<int32_t*>(B->d_flow);
     f.chunk = std::max(1, c.chunk);
     f.blocks_per_sm = c.blocks_per_sm;
-    f.tight = B->sweep_auto ? flow_tight(f.item1, B->info.nlevels, B->nsm) : c.tight;
+    f.tight = c.tight < 0 ? flow_tight(f.item1, B->info.nlevels, B->nsm) : c.tight;
     f.wait_ns = 10000000000ull;  // 10 s: far beyond any dependency chain
     f.seed_dev = B->d_seed;
     f.pairs = B->promote ? 1 : 0;
@@ -1294,11 +1293,10 @@ extern "C" int sgs_batch_set_sweep(sgs_batch* B, const sgs_sweep_config* c) {
     if (!c) return berr(B, SGS_ERR_ARG, "null sweep configuration");
     if (c->mode != SGS_SWEEP_FLOW) return berr(B, SGS_ERR_ARG, "batches sweep in the dataflow form only");
     if (c->chunk < 0 || c->chunk > 64 || c->blocks_per_sm < 0 || c->blocks_per_sm > 32 || c->lanes_g < 0 ||
-        c->lanes_g > 2 || c->lanes_w < 0 || c->lanes_w > 32 || (c->lanes_w & (c->lanes_w - 1)) || c->tight < 0 ||
+        c->lanes_g > 2 || c->lanes_w < 0 || c->lanes_w > 32 || (c->lanes_w & (c->lanes_w - 1)) || c->tight < -1 ||
         c->tight > 1)
         return berr(B, SGS_ERR_ARG, "invalid dataflow sweep parameters");
     B->sweep = *c;
-    B->sweep_auto = false;
     B->sweep.level_lo = B->sweep.level_hi = B->sweep.split_nodes = 0;
     if (B->sweep.chunk < 1) B->sweep.chunk = 1;
     B->sweep_graph_valid = false;
@@ -1317,13 +1315,11 @@ extern "C" int sgs_batch_tune_sweep(sgs_batch* B, int32_t R, sgs_sweep_config* c
     unsigned char* V = nullptr;
     if ((rc = balloc(B, &V, (size_t)B->Ntot * Rp * es))) return rc;
     const sgs_sweep_config saved = B->sweep;
-    const bool saved_auto = B->sweep_auto;
     std::vector<sgs_sweep_config> done;
     int best = -1;
     cudaStream_t st = B->stream;
     auto time_one = [&](sgs_sweep_config c) -> int {
         B->sweep = c;
-        B->sweep_auto = false;
         int r;
         int64_t launched = 0;
         *B->h_seed = 7;
@@ -1353,7 +1349,6 @@ extern "C" int sgs_batch_tune_sweep(sgs_batch* B, int32_t R, sgs_sweep_config* c
     bfree(B, V);
     if (rc || best < 0) {
         B->sweep = saved;
-        B->sweep_auto = saved_auto;
         B->sweep_graph_valid = false;
         return rc ? rc : berr(B, SGS_ERR_CUDA, "no sweep configuration could be timed");
     }

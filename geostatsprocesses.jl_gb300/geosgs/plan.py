@@ -47,7 +47,7 @@ class Plan:
         self.prepared = False
         self._sweep = _abi.SgsSweepConfig(2 if problem.flags & _abi.SGS_FLAG_LEVEL_SWEEP else
                                           1 if problem.flags & _abi.SGS_FLAG_ONE_LAUNCH_SWEEP else 0,
-                                          1, 0, 1, 0, 0, 0, 0, 0, 0.0).as_dict()
+                                          1, 0, 1, 0, 0, 0, -1, 0, 0.0).as_dict()
 
     def close(self):
         if getattr(self, "h", None):
@@ -193,7 +193,8 @@ class Plan:
         return self
 
     def sweep_config(self) -> dict:
-        """The sweep configuration set last (set_sweep / tune_sweep)."""
+        """The sweep configuration set last (set_sweep / tune_sweep), or the
+        default; set_sweep(**config) restores it."""
         return dict(self._sweep)
 
     def tune_sweep(self, nreals: int):

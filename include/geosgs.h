@@ -301,7 +301,9 @@ typedef struct sgs_sweep_config {
     int32_t level_hi;         /* swept by per-level launches, the levels before and
                                  after them by one dataflow launch each             */
     int32_t tight;            /* flow: 1 = the kernel variant compiled for higher
-                                 residency (register cap)                           */
+                                 residency (register cap), 0 = the other, -1 = by
+                                 the items of a level (plans and batches that were
+                                 given no configuration)                          */
     int32_t split_nodes;      /* levels (FP32, rows of a multiple of 8 realizations):
                                  levels of fewer nodes than this take one block per
                                  node, its 8 warps splitting the neighbour list
