@@ -1,5 +1,5 @@
-"""Means of float rows whose values differ by more than 27 binades: the small
-ones count with all their bits."""
+"""Statistics of float rows: means where values differ by more than 27 binades
+(the small ones count with all their bits), and counts beside NaN."""
 import math
 
 import numpy as np
@@ -35,3 +35,14 @@ def test_means_with_small_values(geosgs_lib, r, binades):
     # the same sums of squares, each value's difference from the mean rounded
     # (to 2^-53 of numbers up to 1, twice where the mean is, too)
     assert np.all(np.abs(var - exact) <= (steps + 8) * 2.0**-53 * np.abs(exact) + 4 * r * 2.0**-53 * 2.0**-53)
+
+
+def test_counts_of_rows_with_nan(geosgs_lib):
+    x = np.random.default_rng(0).standard_normal((40, 24)).astype(np.float32)
+    x[::5, 3] = np.nan
+    v = torch.from_numpy(x).cuda()
+    for complement in (False, True):
+        got = ensemble.cdf(v, 24, [0.5, -1.0], 24, complement=complement).cpu().numpy()
+        with np.errstate(invalid="ignore"):
+            hit = x[:, :, None] > np.float32([0.5, -1.0]) if complement else x[:, :, None] <= np.float32([0.5, -1.0])
+        assert np.array_equal(got, hit.sum(axis=1) / 24)
