@@ -100,7 +100,9 @@ __device__ __forceinline__ void cell_of(const GridDev& g, int node, int& i0, int
 // the covariance below keeps to three of them past the squared lag: square
 // roots are put together from FP32 corrections of exact FP64 remainders, and
 // the exponential is evaluated in 64-bit integers (some 85 instructions of a
-// cycle or two).  Errors below 2^-56 of the sill; the library's exp and sqrt
+// cycle or two).  Errors below 2^-56 of the sill, which is also what small
+// covariances are accurate to (sill - gamma, their other form, loses its bits to
+// the same cancellation from 2^-52 of the sill on); the library's exp and sqrt
 // took about 100 FP64 instructions, FP64 forms of these two 30.
 //
 // 2^(-j/64) in units of 2^-63, j = 0 .. 63.
@@ -358,12 +360,6 @@ __device__ __forceinline__ DF df_sqrt(DF v) {
 
 __device__ __forceinline__ DF shfl_xor_df(DF v, int o) {
     return {__shfl_xor_sync(FULL_MASK, v.hi, o), __shfl_xor_sync(FULL_MASK, v.lo, o)};
-}
-
-__device__ __forceinline__ DF warp_sum_df(DF v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = df_add(v, shfl_xor_df(v, o));
-    return v;
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() {

@@ -18,7 +18,7 @@
 // instruction holds its scheduler for 64 cycles): exact sums in integers,
 // sorting networks in registers, thresholds moved to the floats between which
 // they fall.  1M nodes x 100 float values, one GB300: mean and variance 4.57
-// -> 0.22 ms, 3 quantiles 4.36 -> 0.30, 3 thresholds 1.79 -> 0.11 (0.06 each
+// -> 0.23 ms, 3 quantiles 4.36 -> 0.30, 3 thresholds 1.79 -> 0.11 (0.06 each
 // to read).  Nothing is allocated: the threshold and probability lists (at
 // most 32 per launch) travel in the kernel parameters, and the host wrapper
 // launches once per 32 of them.

@@ -66,12 +66,13 @@ __device__ __forceinline__ int draw_category(const IndArgs& ia, const double* p,
 
 // The sweeps below are dataflow launches (sweep.cu): an item is a node and up
 // to 32 of its realizations, W lanes one realization each and 32 / W slices of
-// the neighbour list.  A lane loads its realization's value of 8
-// neighbours and adds them once they are stored.  One launch per level, with
-// the categories of 4 realizations and up to 28 FP64 divisions to a thread,
-// took 48 us for a level (174 levels of 256 x 256 nodes x 32: 8.3 ms); this
-// takes 2.4 (0.42 ms).  8, 16 or 24 neighbours at a time are slower, and so is
-// a branch on the category instead of adding zero to the others (0.70 ms).
+// the neighbour list.  A lane loads its realization's category of 4 neighbours
+// (the multivariate sweep: its LM variables of 8 / LM neighbours) and adds
+// them once they are stored; with 8, 16 or 24 it is slower.  One launch per
+// level, with the categories of 4 realizations and up to 28 FP64 divisions to
+// a thread, took 48 us for a level (174 levels of 256 x 256 nodes x 32: 8.3
+// ms); this takes 2.4 (0.42 ms; 0.70 with a branch on the category instead of
+// adding zero to the others).
 constexpr int IND_AHEAD = 4;
 
 // The category drawn at u for probabilities proportional to base + sum,

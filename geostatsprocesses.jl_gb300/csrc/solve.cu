@@ -589,8 +589,8 @@ cudaError_t launch_solve_fp64(const SolveArgs& a, const SweepTables<double>& t, 
 // 250k systems of 32 went through FP64 in 1.3 ms), a weight of 32 or more (the integer sums' range) or whose refinement does
 // not contract is queued for the FP64 kernel.
 //
-// Bound: latency and issue slots of 8 to 24 warps per SM (shared memory holds
-// the systems; counters of the 32-neighbour form: issue slots 49 % used, L1's
+// Bound: latency and issue slots of 6 (above 48 neighbours) to 24 warps per SM
+// (shared memory and registers hold the systems; counters of the 32-neighbour form: issue slots 49 % used, L1's
 // data pipe 73 % before the table gathers were put in lag order), and the
 // FP64 pipe where many pairs involve data.  Measured against one warp per
 // system with a full Gauss-Jordan inverse (CUDA events, one GB300): 2 M
