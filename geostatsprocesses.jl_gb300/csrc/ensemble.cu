@@ -560,8 +560,10 @@ extern "C" int sgs_ensemble_quantile(const void* vals, int32_t precision, int64_
         for (int i = 0; i < a.nlist; ++i) a.list[i] = p[i0 + i];
         if (a.fp64) {
             const size_t smem = (size_t)ENS_WARPS * P * sizeof(double);
-            if ((rc = ens_done(cudaFuncSetAttribute(ens_quantile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    (int)smem), "sgs_ensemble_quantile")))
+            // the limit for the longest rows: it is one for all threads of the process
+            constexpr int most = ENS_WARPS * ENS_RMAX * (int)sizeof(double);
+            if ((rc = ens_done(cudaFuncSetAttribute(ens_quantile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                               "sgs_ensemble_quantile")))
                 return rc;
             ens_quantile_kernel<<<ens_grid(nnodes), ENS_WARPS * 32, smem, st>>>(a, out);
         } else {

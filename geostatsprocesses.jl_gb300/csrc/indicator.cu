@@ -304,6 +304,16 @@ __host__ __device__ constexpr size_t cok_smem_per_warp(int n, int L) {
     return (size_t)(M * ldl_stride(M) + 2 * ((M + 1) / 2 * 2)) * sizeof(double) + (size_t)n * 4 * sizeof(int);
 }
 
+// the largest of any call (a kernel's limit is one for all threads of the process)
+constexpr int cok_smem_max() {
+    size_t m = 0;
+    for (int L = 1; L <= IND_MAX_CAT; ++L) {
+        const size_t s = cok_smem_per_warp(COK_MAX / L, L);
+        m = s > m ? s : m;
+    }
+    return (int)(m * COK_WARPS);
+}
+
 // lower Cholesky factor of the L x L symmetric matrix S (lower triangle,
 // row-major) into F (full L x L, zero above the diagonal); pivots not above
 // tau give zero columns
@@ -546,7 +556,7 @@ static cudaError_t cok_solve(const SolveArgs& a, const CokArgs& c, cudaStream_t 
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const size_t smem = cok_smem_per_warp(a.k, c.ncat) * COK_WARPS;
     cudaError_t e =
-        cudaFuncSetAttribute(cok_solve_kernel<GAUSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(cok_solve_kernel<GAUSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, cok_smem_max());
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cok_solve_kernel<GAUSS>, COK_WARPS * 32, smem);

@@ -96,6 +96,10 @@ __host__ __device__ constexpr size_t warp_smem_bytes(int k) {
     return (size_t)((k + 1) * ldl_stride(k + 1) + 2 * ((k + 2) / 2 * 2)) * sizeof(double) + (size_t)k * sizeof(NbInfo);
 }
 
+// A kernel's shared-memory limit is one for all threads of the process: it is set
+// to the largest that any call needs, not to a call's own.
+constexpr int kSolveSmemMax = (int)(warp_smem_bytes(KMAX) * SOLVE_WARPS);
+
 // Indicator sums of one system (SolveArgs::ind_*): w holds the weights of the
 // system's n neighbours (FP64 values `wq(q)`), kriged = false for a prior
 // node (all sums zero).
@@ -541,7 +545,7 @@ static cudaError_t launch_solve(const SolveArgs& a, const SweepTables<O>& t, cud
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const size_t smem = warp_smem_bytes(a.k) * SOLVE_WARPS;
-    cudaError_t e = cudaFuncSetAttribute(solve_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(solve_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmemMax);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_kernel<O>, SOLVE_WARPS * 32, smem);
@@ -1641,7 +1645,7 @@ static cudaError_t launch_solve64_batch(int kl, const SolveArgs* doms, const int
     if (kl < 1 || kl > KMAX) return cudaErrorInvalidValue;
     const size_t smem = warp_smem_bytes(kl) * SOLVE_WARPS;
     cudaError_t e = cudaFuncSetAttribute(solve_batch_kernel<O>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         kSolveSmemMax);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_batch_kernel<O>, SOLVE_WARPS * 32, smem);
