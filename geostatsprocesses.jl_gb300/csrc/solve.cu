@@ -650,8 +650,11 @@ struct Sys32 {
         unsigned long long mask[SYS];  // the systems' neighbours that are data
         int n[SYS], g[SYS], dom[SYS];
         unsigned short row[CHUNK];     // system << 6 | neighbour
+        unsigned short first[2][CHUNK];  // their pairs' numbers: with the grid and the node, with earlier data
         unsigned char place[SYS][NMAX];  // row of the matrix a neighbour stands in
+        unsigned char order[SYS][NMAX];  // the grid neighbours, then the data
         unsigned char same[SYS];  // 1: a datum and another neighbour are one point
+        unsigned short total[2];
     };
     static constexpr int block_bytes = SYS * bytes + (int)sizeof(Shared);
 };
@@ -999,6 +1002,13 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
             __syncwarp();
         }
         // ---- pairs with a datum: FP64, over the whole block ----
+#pragma unroll
+        for (int s = 0; s < NMAX / 16; ++s) {
+            const int q = l16 + 16 * s;
+            const unsigned long long lower = (1ull << q) - 1;
+            const int nd = __popcll(dmask & lower);
+            if (q < n) sh.order[sys][(dmask >> q) & 1 ? n - __popcll(dmask) + nd : q - nd] = (unsigned char)q;
+        }
         if (l16 == 0) {
             sh.mask[sys] = dmask;
             sh.same[sys] = 0;
@@ -1014,53 +1024,79 @@ __device__ __forceinline__ void solve32_pair(const SolveArgs& a, const SolveArgs
             for (int e = 0; e < S::SYS; ++e) total += __popcll(sh.mask[e]);
             const int nr = min(total - r0, S::CHUNK);
             left = total - r0 - nr;
-            if ((int)threadIdx.x < nr) {
-                int t = r0 + threadIdx.x, es = 0;
-                while (t >= __popcll(sh.mask[es])) t -= __popcll(sh.mask[es++]);
-                unsigned long long mk = sh.mask[es];
-                for (; t > 0; --t) mk &= mk - 1;
-                const int da = __ffsll((long long)mk) - 1;
-                sh.row[threadIdx.x] = (unsigned short)(es << 6 | da);
-                const SolveArgs& ah = problem(es);
-                if (ah.vario.ns == 1) {
-                    int c0, c1, c2;
-                    cell_of(ah.grid, sh.g[es], c0, c1, c2);
-                    datum_lag(ah, ah.nbr[(int64_t)sh.g[es] * ah.k + da] - (int)ah.grid.N, c0, c1, c2, sh.u[threadIdx.x]);
+            int counts[2] = {0, 0};  // pairs of each kind in the chunk
+            if (threadIdx.x < 32) {
+                if (lane < nr) {
+                    int t = r0 + lane, es = 0;
+                    while (t >= __popcll(sh.mask[es])) t -= __popcll(sh.mask[es++]);
+                    const int ng = sh.n[es] - __popcll(sh.mask[es]), da = sh.order[es][ng + t];
+                    sh.row[lane] = (unsigned short)(es << 6 | da);
+                    counts[0] = ng + 1;
+                    counts[1] = t;
+                    const SolveArgs& ah = problem(es);
+                    if (ah.vario.ns == 1) {
+                        int c0, c1, c2;
+                        cell_of(ah.grid, sh.g[es], c0, c1, c2);
+                        datum_lag(ah, ah.nbr[(int64_t)sh.g[es] * ah.k + da] - (int)ah.grid.N, c0, c1, c2, sh.u[lane]);
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int kind = 0; kind < 2; ++kind) {
+                    int end = counts[kind];
+#pragma unroll
+                    for (int o = 1; o < S::CHUNK; o <<= 1) {
+                        const int y = __shfl_up_sync(FULL_MASK, end, o);
+                        if (lane >= o) end += y;
+                    }
+                    if (lane < S::CHUNK) sh.first[kind][lane] = (unsigned short)(end - counts[kind]);
+                    if (lane == S::CHUNK - 1) sh.total[kind] = (unsigned short)end;
                 }
             }
             __syncthreads();
+            // A pair to a thread, none of them idle: first the rows' pairs with
+            // grid neighbours and the node, then those with earlier data, so that a
+            // warp takes one kind.  With a slot for every pair of a row and the
+            // system's largest size, two thirds of them empty, 40k systems of
+            // 40 data (spherical) took 6.5 ms, more than one warp per system
+            // had (4.9); this takes 3.0, and systems of 20 0.76 (1.93, 1.35).
 #pragma unroll 1
-            for (int item = threadIdx.x; item < nr * NMAX; item += 32 * S::WARPS) {
-                const int ei = item / NMAX, q = item - ei * NMAX;
-                const int e = sh.row[ei], es = e >> 6, da = e & 63;
-                if (q >= sh.n[es]) continue;
-                const SolveArgs& ah = problem(es);
-                unsigned char* bh = smem + es * S::bytes;
-                const int gh = sh.g[es];
-                const int32_t* rowh = ah.nbr + (int64_t)gh * ah.k;
-                const int id = rowh[q];
-                if (id >= ah.grid.N && q > da) continue;  // data-data pair once
-                // q == da stands for the pair with the node (its own diagonal is 1)
-                const NbInfo nq = nb_of(ah, q == da ? gh : id);
-                KF x;
-                bool hit = false;
-                if (ah.vario.ns == 1 && nq.did < 0) {
-                    int c0, c1, c2;
-                    cell_of(ah.grid, gh, c0, c1, c2);
-                    x = datum_cov(ah, sh.u[ei], nq.c0 - c0, nq.c1 - c1, nq.c2 - c2, hit);
-                }
-                if (!hit) x = kcov64n(ah, nq, nb_of(ah, rowh[da]));
-                const int pd = sh.place[es][da];
-                if (q == da) {
-                    reinterpret_cast<KF*>(bh + S::K)[pd] = x;
-                    *reinterpret_cast<KF*>(bh + S::at(pd, pd)) = {(int)KFIX, 0.0f};
-                } else {
-                    // Correlation 1: the variance of their difference, 2 (1 - K), bounds the
-                    // later one's pivot, which is then far below the singular rule's 1e-10.
-                    if (x.hi == (int)KFIX && fabsf(x.lo) <= 1e-12f) sh.same[es] = 1;
-                    const int pq = sh.place[es][q], i = max(pq, pd), j = min(pq, pd);
-                    *reinterpret_cast<KF*>(bh + S::at(i, j)) = x;
-                    if ((i >> 2) == (j >> 2)) *reinterpret_cast<KF*>(bh + S::at(j, i)) = x;
+            for (int kind = 0; kind < 2; ++kind) {
+                const int pairs = sh.total[kind];
+#pragma unroll 1
+                for (int item = threadIdx.x; item < pairs; item += 32 * S::WARPS) {
+                    int ei = 0;
+#pragma unroll
+                    for (int step = 8; step > 0; step >>= 1)
+                        if (ei + step < nr && sh.first[kind][ei + step] <= item) ei += step;
+                    const int e = sh.row[ei], es = e >> 6, da = e & 63, j = item - sh.first[kind][ei];
+                    const SolveArgs& ah = problem(es);
+                    unsigned char* bh = smem + es * S::bytes;
+                    const int gh = sh.g[es], ng = sh.n[es] - __popcll(sh.mask[es]);
+                    const int32_t* rowh = ah.nbr + (int64_t)gh * ah.k;
+                    const bool own = kind == 0 && j == ng;  // the pair with the node (its own diagonal is 1)
+                    const int q = own ? da : sh.order[es][kind ? ng + j : j];
+                    const NbInfo nq = nb_of(ah, own ? gh : rowh[q]);
+                    KF x;
+                    bool hit = false;
+                    if (kind == 0 && ah.vario.ns == 1) {
+                        int c0, c1, c2;
+                        cell_of(ah.grid, gh, c0, c1, c2);
+                        x = datum_cov(ah, sh.u[ei], nq.c0 - c0, nq.c1 - c1, nq.c2 - c2, hit);
+                    }
+                    if (!hit) x = kcov64n(ah, nq, nb_of(ah, rowh[da]));
+                    const int pd = sh.place[es][da];
+                    if (own) {
+                        reinterpret_cast<KF*>(bh + S::K)[pd] = x;
+                        *reinterpret_cast<KF*>(bh + S::at(pd, pd)) = {(int)KFIX, 0.0f};
+                    } else {
+                        // Correlation 1: the variance of their difference, 2 (1 - K), bounds the
+                        // later one's pivot, which is then far below the singular rule's 1e-10.
+                        if (x.hi == (int)KFIX && fabsf(x.lo) <= 1e-12f) sh.same[es] = 1;
+                        const int pq = sh.place[es][q], i = max(pq, pd), jj = min(pq, pd);
+                        *reinterpret_cast<KF*>(bh + S::at(i, jj)) = x;
+                        if ((i >> 2) == (jj >> 2)) *reinterpret_cast<KF*>(bh + S::at(jj, i)) = x;
+                    }
                 }
             }
             __syncthreads();
